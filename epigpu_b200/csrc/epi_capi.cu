@@ -25,7 +25,7 @@ cudaError_t launch_unpack(const int32_t *raw, int nsnp, int nid, int npack, int 
                           cudaStream_t stream);
 cudaError_t launch_qmiss(const uint32_t *missbits, int nsnp, int Wp, const uint32_t *wmask, const double *qd,
                         const double *qr, int Np, int ntraits, double *qm, double *rm, double *nm,
-                        cudaStream_t stream);
+                        float *qmf, cudaStream_t stream);
 cudaError_t launch_major(const uint4 *planes, int nsnp, int Wp, uint8_t *maj, cudaStream_t stream);
 cudaError_t launch_marg(const uint4 *planes, int nsnp, int Wp, const float *y, const uint32_t *wmask, int Np,
                         int ntraits, double *pmC, int32_t *pmN, double *pmQ, cudaStream_t stream);
@@ -38,25 +38,29 @@ cudaError_t popc_encode_planes(int v, PopcMaps *maps, const uint4 *planes, int n
 // tensor form (scan_mma.cu)
 bool mma_available();
 int mma_tile_i();
-int mma_tile_j();
+int mma_tile_j(int screen);
+int mma_x_rows(int screen);
 int mma_min_nid();
 int mma_max_nid();
+int mma_screen_max_nid();
 int mma_shapes();
 void mma_shape(int v, const char **desc);
-cudaError_t mma_prepare(int v, int ntraits, int grid_request, int *grid);
-cudaError_t mma_enqueue(int v, const ScanArgs &a, const MmaMaps &maps, int grid, cudaStream_t stream);
+cudaError_t mma_prepare(int v, int screen, int ntraits, int grid_request, int *grid);
+cudaError_t mma_enqueue(int v, int screen, const ScanArgs &a, const MmaMaps &maps, int grid,
+                        cudaStream_t stream);
+cudaError_t exact_enqueue(const ScanArgs &a, int sm_count, cudaStream_t stream);
 cudaError_t mma_encode_genotypes(MmaMaps *maps, const uint8_t *hcodes, const uint8_t *h3, int nsnp, int Np);
 cudaError_t mma_encode_traits(MmaMaps *maps, const int8_t *ydig, int ntraits, int Np);
-cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits);
+cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits, int screen);
 bool mma_needs_x(int v);
-cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int8_t *x,
-                          cudaStream_t stream);
-// Start of a scan: counters (hits, tile queue, error flag and site) to zero, the per-trait
-// maxima of F and F2 to the order-encoded -inf.
+cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int screen,
+                          int8_t *x, cudaStream_t stream);
+// Start of a scan: counters to zero, the per-trait maxima of F and F2 and the screen's lower
+// bounds of them to the order-encoded -inf.
 __global__ void k_scan_init(unsigned long long *counters, unsigned int *maxf, int n)
 {
-    if (threadIdx.x < 4) counters[threadIdx.x] = 0ull;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) maxf[i] = 0x007fffffu;
+    if (threadIdx.x < NCOUNTERS) counters[threadIdx.x] = 0ull;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) maxf[i] = ENC_NEG_INF;
 }
 }  // namespace epi
 
@@ -94,7 +98,18 @@ struct epi_ctx {
     // SNP, individual and trait), built on first use after each genotype or trait load
     int8_t *d_x = nullptr;
     size_t x_cap = 0;
-    bool x_valid = false;
+    int x_valid = -1;  // -1: none, 0: of all digits, 1, 2: of the screen with that many digits
+    // screened scan: constants per trait and per (trait, SNP), the candidate list; per trait
+    // E / sigma of either screen and the number of valid individuals (screen_scan); the thresholds of a scan
+    // whose candidates did not fit the list (no scan at these or lower ones is screened again
+    // until other genotypes or traits are loaded)
+    float4 *d_tscr = nullptr;
+    float *d_qmf = nullptr;
+    epi::Cand *d_cand = nullptr;
+    size_t tscr_cap = 0, qmf_cap = 0, cand_cap = 0;
+    std::vector<double> scr_r[2], scr_nv;
+    bool scr_full = false;
+    float scr_full_t1 = 0.0f, scr_full_t2 = 0.0f;
     std::vector<double> qc;
     // plain form: marginals per (trait, SNP) and the sum of y^2 per trait
     double *d_pmC = nullptr, *d_pmQ = nullptr, *d_ysq = nullptr;
@@ -113,7 +128,7 @@ struct epi_ctx {
     // counters and maxima it reads back
     BlockDesc *h_blocks = nullptr;
     int h_blocks_cap = 0;
-    unsigned long long *h_state = nullptr;  // counters[4], then 2 x ntraits encoded maxima
+    unsigned long long *h_state = nullptr;  // the counters, then 2 x ntraits encoded maxima
     size_t h_state_cap = 0;
     // the device part of the last scan, captured as a CUDA graph, and what it was captured for
     cudaGraphExec_t gexec = nullptr;
@@ -213,7 +228,7 @@ epi_status epi_open(int32_t device, epi_ctx **out)
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->d_counters, 4 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->d_counters, epi::NCOUNTERS * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         epi_close(ctx);
         return EPI_E_CUDA;
@@ -230,7 +245,7 @@ epi_status epi_close(epi_ctx *ctx)
     void *bufs[] = {ctx->d_raw, ctx->d_planes, ctx->d_hcodes, ctx->d_h3, ctx->d_missbits, ctx->d_y, ctx->d_q,
                     ctx->d_wmask, ctx->d_qc, ctx->d_yscale, ctx->d_qd, ctx->d_qtot, ctx->d_qm, ctx->d_ydig,
                     ctx->d_hits, ctx->d_counters, ctx->d_maxf, ctx->d_blocks, ctx->d_maj, ctx->d_pmC,
-                    ctx->d_pmQ, ctx->d_ysq, ctx->d_pmN, ctx->d_x};
+                    ctx->d_pmQ, ctx->d_ysq, ctx->d_pmN, ctx->d_x, ctx->d_tscr, ctx->d_qmf, ctx->d_cand};
     for (void *p : bufs)
         if (p) cudaFree(p);
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
@@ -277,7 +292,8 @@ epi_status epi_load_packed(epi_ctx *ctx, const int32_t *gpack, int32_t nid, int3
     CK(epi::launch_major(ctx->d_planes, nsnp, Wp, ctx->d_maj, ctx->stream));
     ctx->qm_valid = false;
     ctx->pm_valid = false;
-    ctx->x_valid = false;
+    ctx->x_valid = -1;
+    ctx->scr_full = false;
     CK(epi::mma_encode_genotypes(&ctx->maps, ctx->d_hcodes, ctx->d_h3, nsnp, 32 * Wp));
     if (ctx->traits_nid != nid) ctx->ntraits = 0;  // traits no longer match
     ctx->nid = nid;
@@ -349,7 +365,14 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
     // Y = round(y * 2^sy) (|Y| <= 8355711); hqd holds ytilde^2 = (Y 2^-sy)^2 (exact in FP64:
     // |Y| < 2^23) and Y; hsc per trait 2^-sy, the sum of Y and the number of valid individuals;
     // hqtot the sum of ytilde^2.
-    constexpr int ND = 4;
+    // (rows: the highest digit first). The screen's 8-bit phenotype in front of them: D = round(s (ytilde - c)) with c the middle of
+    // the values and s the scale that spreads them over -127..127, d0 = -s c (the D of the mean),
+    // E the norm of what the rounding leaves (scan_mma.cu).
+    constexpr int ND = 5;
+    std::vector<float4> hts(2 * (size_t)ntraits);
+    ctx->scr_r[0].assign(ntraits, 0.0);
+    ctx->scr_r[1].assign(ntraits, 0.0);
+    ctx->scr_nv.assign(ntraits, 0.0);
     std::vector<int8_t> hd((size_t)ntraits * ND * Np, 0);
     std::vector<double> hqd(2 * (size_t)ntraits * Np, 0.0), hqtot(ntraits, 0.0), hsc(3 * (size_t)ntraits, 1.0);
     for (int t = 0; t < ntraits; ++t) {
@@ -372,17 +395,21 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
         hsc[t] = std::ldexp(1.0, -sy);
         int8_t *d0 = hd.data() + (size_t)t * ND * Np;
         long long ysum = 0;
+        double ymin = INFINITY, ymax = -INFINITY, e16 = 0.0;
         for (int k = 0; k < nid; ++k) {
             if (!ok(k)) continue;
             long long Y = std::llround(((double)yt[k] - mu) * p2 * scale);
             Y = std::min(8355711LL, std::max(-8355711LL, Y));
             const long long a0 = ((Y + 128) & 255) - 128, Y1 = (Y - a0) / 256;
             const long long a1 = ((Y1 + 128) & 255) - 128, a2 = (Y1 - a1) / 256;
-            d0[k] = 1;
-            d0[Np + k] = (int8_t)a0;
-            d0[2 * (size_t)Np + k] = (int8_t)a1;
-            d0[3 * (size_t)Np + k] = (int8_t)a2;
+            d0[Np + k] = 1;
+            d0[2 * (size_t)Np + k] = (int8_t)a2;
+            d0[3 * (size_t)Np + k] = (int8_t)a1;
+            d0[4 * (size_t)Np + k] = (int8_t)a0;
+            e16 += (double)(a0 * a0);
             const double yq = (double)Y * hsc[t];
+            ymin = std::min(ymin, yq);
+            ymax = std::max(ymax, yq);
             hqd[(size_t)t * Np + k] = yq * yq;
             hqd[((size_t)ntraits + t) * Np + k] = (double)Y;
             hqtot[t] += yq * yq;
@@ -390,6 +417,27 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
         }
         hsc[ntraits + t] = (double)ysum;
         hsc[2 * (size_t)ntraits + t] = (double)nv;
+        const double mid = nv ? 0.5 * (ymin + ymax) : 0.0, half = nv ? 0.5 * (ymax - ymin) : 0.0;
+        const double s = half > 0.0 ? 127.0 / half : 1.0;
+        const float dm = (float)(-s * mid);
+        const double *yv = hqd.data() + ((size_t)ntraits + t) * Np;
+        double e2 = 0.0;
+        for (int k = 0; k < nid; ++k) {
+            if (!ok(k)) continue;
+            const double x = s * hsc[t] * yv[k], D = std::min(127.0, std::max(-127.0, std::nearbyint(x + dm)));
+            d0[k] = (int8_t)D;
+            const double e = x - (D - dm);
+            e2 += e * e;
+        }
+        const double qs = s * s * hqtot[t];
+        hts[2 * t] = make_float4(dm, (float)(std::sqrt(e2) * (1.0 + 1e-6)), (float)qs, (float)(s * s));
+        // two digits: D = d1 + 256 d2 = (Y - d0) / 256
+        const double s16 = scale / 256.0, q16 = s16 * s16 * hqtot[t];
+        e16 /= 65536.0;
+        hts[2 * t + 1] = make_float4(0.0f, (float)(std::sqrt(e16) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
+        ctx->scr_nv[t] = (double)nv;
+        ctx->scr_r[0][t] = qs > 0.0 ? std::sqrt(e2 * (double)nv / qs) : INFINITY;
+        ctx->scr_r[1][t] = qs > 0.0 ? std::sqrt(e16 * (double)nv / q16) : INFINITY;
     }
     size_t need = (size_t)ntraits * Np * sizeof(float);
     size_t cap_y = ctx->traits_cap, cap_q = ctx->traits_cap;
@@ -412,6 +460,8 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
     CK(ensure(&ctx->d_yscale, &ctx->yscale_cap, hsc.size() * sizeof(double)));
     CK(cudaMemcpyAsync(ctx->d_ydig, hd.data(), hd.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(epi::mma_encode_traits(&ctx->maps, ctx->d_ydig, ntraits, Np));
+    CK(ensure(&ctx->d_tscr, &ctx->tscr_cap, hts.size() * sizeof(float4)));
+    CK(cudaMemcpyAsync(ctx->d_tscr, hts.data(), hts.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_qd, hqd.data(), hqd.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_qtot, hqtot.data(), ntraits * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_yscale, hsc.data(), hsc.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -420,7 +470,8 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
     ctx->traits_nid = nid;
     ctx->qm_valid = false;
     ctx->pm_valid = false;
-    ctx->x_valid = false;
+    ctx->x_valid = -1;
+    ctx->scr_full = false;
     return EPI_OK;
 }
 
@@ -446,17 +497,14 @@ void epi_permute_phenotype(float *phen, int32_t nid, uint32_t seed)
 
 }  // extern "C"
 
-// number of pairs (gx, gy) of a block with start1+gx > start2+gy
+// number of pairs (gx, gy) of a block with start1+gx > start2+gy: the sum over gx of
+// clamp(gx + d, 0, size2), d = start1 - start2
 static int64_t block_pairs(const epi_block &b)
 {
-    int64_t n = 0;
-    const int64_t d = (int64_t)b.start1 - b.start2;
-    for (int64_t gx = 0; gx < b.size1; ++gx) {
-        int64_t lim = gx + d;
-        if (lim > b.size2) lim = b.size2;
-        if (lim > 0) n += lim;
-    }
-    return n;
+    const int64_t d = (int64_t)b.start1 - b.start2, m1 = b.size1, m2 = b.size2;
+    const int64_t lo = std::min(m1, std::max<int64_t>(0, -d));      // gx + d <= 0 below lo
+    const int64_t hi = std::min(m1, std::max<int64_t>(lo, m2 - d));  // gx + d >= m2 from hi on
+    return (hi - lo) * d + (lo + hi - 1) * (hi - lo) / 2 + (m1 - hi) * m2;
 }
 
 namespace {
@@ -465,6 +513,26 @@ struct ScanRun {
     epi::ScanArgs args;
     int form;
     int variant;  // the form's kernel variant (tile shape or ring depths)
+    int screen;   // tensor form: the digits of the screened scan, 0: all digits
+    int segments;
+    // tensor form: units in all and of one trait, and where each row group begins (units of the
+    // trait before it, block, group)
+    struct Start {
+        int64_t units;
+        int block, group;
+    };
+    int64_t units, trait_units;
+    int xsi, xsj;
+    std::vector<Start> starts;
+    // the first row group at or past `u` units
+    epi::SegPos at(int64_t u, int ntraits) const
+    {
+        if (u >= units) return {ntraits, 0, 0};
+        const auto it = std::lower_bound(starts.begin(), starts.end(), u % trait_units,
+                                         [](const Start &x, int64_t y) { return x.units < y; });
+        const int t = (int)(u / trait_units);
+        return it == starts.end() ? epi::SegPos{t + 1, 0, 0} : epi::SegPos{t, it->block, it->group};
+    }
     int64_t ntiles;
     std::vector<BlockDesc> desc;
 };
@@ -496,10 +564,13 @@ int pick_form(const epi_ctx *ctx, const epi_scan_opts *o)
 // Builds the kernel arguments and tile schedule for `blocks` and uploads the schedule.
 // Bytes of the streamed-B variant's expanded rows, and whether they may be allocated: at most
 // 32 GiB and half the device's free memory (beyond, that variant is not a candidate).
-static size_t x_bytes(const epi_ctx *ctx) { return 12 * (size_t)ctx->nsnp * ctx->Np * ctx->ntraits; }
-static bool x_usable(const epi_ctx *ctx)
+static size_t x_bytes(const epi_ctx *ctx, int screen)
 {
-    const size_t need = x_bytes(ctx);
+    return (size_t)epi::mma_x_rows(screen) * ctx->nsnp * ctx->Np * ctx->ntraits;
+}
+static bool x_usable(const epi_ctx *ctx, int screen)
+{
+    const size_t need = x_bytes(ctx, screen);
     if (need <= ctx->x_cap) return true;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
@@ -512,13 +583,88 @@ static bool x_usable(const epi_ctx *ctx)
 // cap (SM clock ~1,350 MHz against ~1,935 MHz for the shared-memory producers) and ends 12%
 // slower, although the autotuner's short sample, run before the cap bites, ranks it 15% faster.
 // At N = 4,000 it is 10-14% faster at full clock. tile_config can still force it.
-static bool x_candidate(const epi_ctx *ctx) { return ctx->Np <= 6144 && x_usable(ctx); }
+// The screen needs half the rows per pair: there it is the fastest at every size, also at
+// N = 10,000 under the power cap (605 ms at 1,567 MHz against 640 ms for two producer groups).
+static bool x_candidate(const epi_ctx *ctx, int screen) { return (screen || ctx->Np <= 6144) && x_usable(ctx, screen); }
+
+// Upper tails of the chi-squared distribution with 8 and 4 degrees of freedom.
+static double chi8(double x) { const double h = 0.5 * x; return std::exp(-h) * (1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0))); }
+static double chi4(double x) { const double h = 0.5 * x; return std::exp(-h) * (1.0 + h); }
+
+// x with tail(x) = p (bisection; both tails fall from 1)
+static double chi_quantile(double (*tail)(double), double p)
+{
+    double lo = 0.0, hi = 1500.0;
+    for (int k = 0; k < 60; ++k) {
+        const double mid = 0.5 * (lo + hi);
+        (tail(mid) > p ? lo : hi) = mid;
+    }
+    return lo;
+}
+
+// The share of a scan's pair tests that the screen with `digits` phenotype digits (1 or 2,
+// scan_mma.cu) is expected to pass on, for unassociated genotypes. SSB and SSI are then about
+// sigma^2 times chi-squared with 8 and 4 degrees of freedom; a pair is passed on when its root is
+// within R = E / sigma of the threshold's, or of the largest lower bound so far, itself R below
+// the largest of `pairs` draws.
+static double screen_share(const epi_ctx *ctx, const epi_scan_opts *o, double pairs, int digits)
+{
+    const bool want_int = o->test == 'i';
+    const double top8 = std::sqrt(chi_quantile(chi8, std::min(0.5, 1.0 / pairs)));
+    const double top4 = std::sqrt(chi_quantile(chi4, std::min(0.5, 1.0 / pairs)));
+    double share = 0.0;
+    for (int t = 0; t < ctx->ntraits; ++t) {
+        const double r = ctx->scr_r[digits - 1][t], nv = ctx->scr_nv[t];
+        if (!std::isfinite(r)) return INFINITY;
+        const bool report = o->report_trait < 0 || o->report_trait == t;
+        auto part = [&](double thr, double df, double top, double (*tail)(double)) {
+            double root = std::max(0.0, top - r);
+            if (report) {
+                if (!(thr > 0.0)) return 1.0;
+                const double d2 = std::max(1.0, nv - 9.0);
+                root = std::min(root, std::sqrt(df * thr * nv / (d2 + df * thr)));
+            }
+            root = std::max(0.0, root - r);
+            return tail(root * root);
+        };
+        share += part(o->t1, 8.0, top8, chi8);
+        if (want_int) share += part(o->t2, 4.0, top4, chi4);
+    }
+    return share / ctx->ntraits;
+}
+
+// The digits of the screen for a scan of `pairs` pairs, or 0 for all digits without a screen. A
+// candidate costs about as much as 110 pairs of the one-digit screen (11 ns against 0.1 ns at
+// N = 10,000, both in proportion to N), a pair with two digits 1.5 and with all digits 2 of them:
+// so one digit up to a share of 1 in 250 (0.72 of the time with all digits there), two up to 1 in
+// 400, or where that is at most 1,024 candidates in all (fewer than the exact kernel's warps). For
+// a normal trait R is 0.0092 sqrt(N) with one digit: the rule turns to two at 10,000 to 14,000
+// individuals at p = 1e-6, and to all digits at thresholds that let one pair in 400 through.
+static int screen_digits(const epi_ctx *ctx, const epi_scan_opts *o, double pairs)
+{
+    if (ctx->scr_full && o->t1 <= ctx->scr_full_t1 && o->t2 <= ctx->scr_full_t2) return 0;
+    if (!(pairs >= 1.0) || ctx->Np > epi::mma_screen_max_nid()) return 0;
+    const double tests = pairs * ctx->ntraits;
+    const double one = screen_share(ctx, o, pairs, 1);
+    if (one <= 1.0 / 250.0 || one * tests <= 1024.0) return 1;
+    const double two = screen_share(ctx, o, pairs, 2);
+    return two <= 1.0 / 400.0 || two * tests <= 1024.0 ? 2 : 0;
+}
+
+// Capacity of the candidate list: one percent of the pair tests (where the screen stops paying),
+// 2^16 to 2^22 entries (100 MB); a longer list ends the screened scan.
+static int64_t cand_capacity(double tests)
+{
+    return (int64_t)std::min(4194304.0, std::max(65536.0, tests / 100.0));
+}
 
 epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const epi_scan_opts *o, ScanRun &r,
-                     int variant)
+                     int variant, int screen)
 {
     r.form = pick_form(ctx, o);
     r.variant = variant;
+    r.screen = screen;
+    r.segments = 1;
     if (r.form == EPI_FORM_TENSOR && !epi::mma_available())
         return set_err(ctx, EPI_E_UNSUPPORTED, "tensor form not available in this library");
     if (r.form == EPI_FORM_TENSOR && ctx->Np > epi::mma_max_nid())
@@ -527,18 +673,18 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         return set_err(ctx, EPI_E_UNSUPPORTED, "popcount form counts in 16 bits: at most 65535 individuals "
                        "(the reference's unsigned short counts, EpiOpenCL.c:68)");
     if (r.form == EPI_FORM_TENSOR && epi::mma_needs_x(variant)) {
-        if (!x_usable(ctx))
+        if (!x_usable(ctx, screen))
             return set_err(ctx, EPI_E_UNSUPPORTED, "tensor variant %d: its %zu bytes of expanded B rows do not fit",
-                           variant + 1, x_bytes(ctx));
-        if (!ctx->x_valid) {
-            CK(ensure(&ctx->d_x, &ctx->x_cap, x_bytes(ctx)));
-            CK(epi::launch_expand(ctx->d_hcodes, ctx->d_ydig, ctx->nsnp, ctx->Np, ctx->ntraits, ctx->d_x,
+                           variant + 1, x_bytes(ctx, screen));
+        if (ctx->x_valid != screen) {
+            CK(ensure(&ctx->d_x, &ctx->x_cap, x_bytes(ctx, screen)));
+            CK(epi::launch_expand(ctx->d_hcodes, ctx->d_ydig, ctx->nsnp, ctx->Np, ctx->ntraits, screen, ctx->d_x,
                                   ctx->stream));
-            CK(epi::mma_encode_x(&ctx->maps, ctx->d_x, ctx->nsnp, ctx->Np, ctx->ntraits));
-            ctx->x_valid = true;
+            CK(epi::mma_encode_x(&ctx->maps, ctx->d_x, ctx->nsnp, ctx->Np, ctx->ntraits, screen));
+            ctx->x_valid = screen;
         }
     }
-    int TI = epi::mma_tile_i(), TJ = epi::mma_tile_j();
+    int TI = epi::mma_tile_i(), TJ = epi::mma_tile_j(screen);
     if (r.form == EPI_FORM_POPC) {
         epi::popc_shape(variant, &TI, &TJ, nullptr);
         CK(epi::popc_encode_planes(variant, &ctx->pmaps, ctx->d_planes, ctx->nsnp, ctx->Wp));
@@ -571,7 +717,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         CK(cudaHostAlloc((void **)&ctx->h_blocks, (size_t)nblocks * sizeof(BlockDesc), cudaHostAllocDefault));
         ctx->h_blocks_cap = nblocks;
     }
-    const size_t state = 4 * sizeof(unsigned long long) + 2 * (size_t)ctx->ntraits * sizeof(unsigned int);
+    const size_t state = epi::NCOUNTERS * sizeof(unsigned long long) + 2 * (size_t)ctx->ntraits * sizeof(unsigned int);
     if (ctx->h_state_cap < state) {
         if (ctx->h_state) cudaFreeHost(ctx->h_state);
         ctx->h_state = nullptr;
@@ -579,18 +725,53 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         CK(cudaHostAlloc((void **)&ctx->h_state, state, cudaHostAllocDefault));
         ctx->h_state_cap = state;
     }
-    if (ctx->maxf_cap < 2 * ctx->ntraits) {
+    if (ctx->maxf_cap < 4 * ctx->ntraits) {  // maxima, then the screen's lower bounds of them
         if (ctx->d_maxf) cudaFree(ctx->d_maxf);
         ctx->d_maxf = nullptr;
-        CK(cudaMalloc((void **)&ctx->d_maxf, 2 * ctx->ntraits * sizeof(unsigned int)));
-        ctx->maxf_cap = 2 * ctx->ntraits;
+        CK(cudaMalloc((void **)&ctx->d_maxf, 4 * (size_t)ctx->ntraits * sizeof(unsigned int)));
+        ctx->maxf_cap = 4 * ctx->ntraits;
+    }
+    // the tensor form's order of units (scan_mma.cu: Walker): super-tiles of about 40 MB of A rows
+    // (3 bytes per SNP and individual) and expanded B rows for the streamed-B variant, equal
+    // sides in pair tiles; row by row over all j-tiles otherwise
+    r.xsi = 1;
+    r.xsj = 1 << 30;
+    r.starts.clear();
+    r.units = base * ctx->ntraits;
+    if (r.form == EPI_FORM_TENSOR) {
+        if (epi::mma_needs_x(variant)) {
+            const double per = (3.0 * TI + (double)epi::mma_x_rows(screen) * TJ) * ctx->Np;
+            r.xsi = r.xsj = std::max(1, (int)(40e6 / per));
+        }
+        r.units = 0;
+        for (const BlockDesc &d : r.desc)
+            for (int ti = 0; ti < d.tiles_i; ++ti) {
+                if (ti % r.xsi == 0) r.starts.push_back({r.units, (int)(&d - r.desc.data()), ti / r.xsi});
+                const int64_t x = (int64_t)d.start1 + std::min((ti + 1) * TI, d.size1) - 1 - d.start2;
+                r.units += x <= 0 ? 0 : std::min<int64_t>(d.tiles_j, (x + TJ - 1) / TJ);
+            }
+        r.trait_units = r.units;
+        r.units *= ctx->ntraits;
+        if (r.units == 0) r.ntiles = 0;  // no pair at all
+    }
+    if (screen) {
+        double tests = 0.0;
+        for (int b = 0; b < nblocks; ++b) tests += (double)block_pairs(blocks[b]) * ctx->ntraits;
+        // Segments: the list of each is worked off before the next begins, so the list stays
+        // short, the exact maxima of the first ones tighten the screen of the later ones and a
+        // list that runs over costs a part of the scan only. A segment boundary idles the GPU for
+        // about 30 us, so a segment lasts 5 ms or more (600 cycles a stage, two SMs a unit).
+        const double ms = (double)r.units / (ctx->sm_count / 2) * (ctx->Np / 128) * 600.0 / 1.9e6;
+        r.segments = (int)std::min((double)epi::MAX_SEGMENTS, std::max(1.0, ms / 5.0));
+        CK(ensure(&ctx->d_cand, &ctx->cand_cap, (size_t)cand_capacity(tests / r.segments) * sizeof(epi::Cand)));
     }
     if (r.form == EPI_FORM_TENSOR && !ctx->qm_valid) {
         const size_t tn = (size_t)ctx->ntraits * ctx->nsnp;
         CK(ensure(&ctx->d_qm, &ctx->qm_cap, 3 * tn * sizeof(double)));
+        CK(ensure(&ctx->d_qmf, &ctx->qmf_cap, tn * sizeof(float)));
         CK(epi::launch_qmiss(ctx->d_missbits, ctx->nsnp, ctx->Wp, ctx->d_wmask, ctx->d_qd,
                              ctx->d_qd + (size_t)ctx->ntraits * ctx->Np, ctx->Np, ctx->ntraits, ctx->d_qm,
-                             ctx->d_qm + tn, ctx->d_qm + 2 * tn, ctx->stream));
+                             ctx->d_qm + tn, ctx->d_qm + 2 * tn, ctx->d_qmf, ctx->stream));
         ctx->qm_valid = true;
     }
     if (r.form == EPI_FORM_POPC && !ctx->pm_valid) {
@@ -641,12 +822,15 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     a.t2 = o->t2;
     a.wait_ns = o->wait_limit_ms > 0 ? (unsigned long long)o->wait_limit_ms * 1000000ull : 2000000000ull;
     a.debug_stall = o->debug == EPI_DEBUG_STALL;
-    // streamed-B variant: super-tiles of about 40 MB of A rows (3 bytes per SNP and individual)
-    // and expanded B rows (12 per SNP, individual and trait), equal sides in pair tiles
-    {
-        const double per = (3.0 * epi::mma_tile_i() + 12.0 * epi::mma_tile_j() * ctx->ntraits) * ctx->Np;
-        a.xsi = a.xsj = std::max(1, (int)(40e6 / per));
-    }
+    a.xsi = r.xsi;
+    a.xsj = r.xsj;
+    a.seg1 = {ctx->ntraits, 0, 0};
+    a.tscr = ctx->d_tscr;
+    a.qmf = ctx->d_qmf;
+    a.cand = ctx->d_cand;
+    a.cand_cap = (int64_t)(ctx->cand_cap / sizeof(epi::Cand));
+    a.lowf = ctx->d_maxf + 2 * (size_t)ctx->ntraits;
+    a.lowf2 = ctx->d_maxf + 3 * (size_t)ctx->ntraits;
     a.counters = ctx->d_counters;
     a.maxf = ctx->d_maxf;
     a.maxf2 = ctx->d_maxf + ctx->ntraits;
@@ -663,19 +847,32 @@ cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, int nblocks, 
     // under stream capture the timing events are recorded as external records, which become
     // event nodes of the graph (so they time every replay); a direct launch records them plainly
     const unsigned int ev_flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-    epi::k_scan_init<<<1, 256, 0, s>>>(ctx->d_counters, ctx->d_maxf, 2 * ctx->ntraits);
+    epi::k_scan_init<<<1, 256, 0, s>>>(ctx->d_counters, ctx->d_maxf, 4 * ctx->ntraits);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && nblocks)
         e = cudaMemcpyAsync(ctx->d_blocks, ctx->h_blocks, nblocks * sizeof(BlockDesc), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev0, s, ev_flags);
-    if (e == cudaSuccess && r.ntiles > 0)
-        e = r.form == EPI_FORM_TENSOR ? epi::mma_enqueue(r.variant, r.args, ctx->maps, grid, s)
-                                      : epi::popc_enqueue(r.variant, r.args, ctx->pmaps, grid, s);
+    if (e == cudaSuccess && r.ntiles > 0) {
+        if (r.form != EPI_FORM_TENSOR) e = epi::popc_enqueue(r.variant, r.args, ctx->pmaps, grid, s);
+        else if (!r.screen) e = epi::mma_enqueue(r.variant, 0, r.args, ctx->maps, grid, s);
+        else {
+            epi::ScanArgs a = r.args;
+            for (int k = 0; k < r.segments && e == cudaSuccess; ++k) {
+                a.segment = k;
+                a.seg0 = r.at(r.units / r.segments * k, ctx->ntraits);
+                a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), ctx->ntraits);
+                if (memcmp(&a.seg0, &a.seg1, sizeof(a.seg0)) == 0) continue;
+                e = epi::mma_enqueue(r.variant, r.screen, a, ctx->maps, grid, s);
+                if (e == cudaSuccess) e = epi::exact_enqueue(a, ctx->sm_count, s);
+            }
+        }
+    }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev1, s, ev_flags);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ctx->h_state, ctx->d_counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+        e = cudaMemcpyAsync(ctx->h_state, ctx->d_counters, epi::NCOUNTERS * sizeof(unsigned long long),
+                            cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ctx->h_state + 4, ctx->d_maxf, 2 * (size_t)ctx->ntraits * sizeof(unsigned int),
+        e = cudaMemcpyAsync(ctx->h_state + epi::NCOUNTERS, ctx->d_maxf, 2 * (size_t)ctx->ntraits * sizeof(unsigned int),
                             cudaMemcpyDeviceToHost, s);
     return e;
 }
@@ -695,10 +892,10 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
 {
     int grid = 0;
     if (r.ntiles > 0) {
-        const int64_t units = r.ntiles * (int64_t)ctx->ntraits;
+        const int64_t units = r.units;
         if (r.form == EPI_FORM_TENSOR) {
             // one CTA pair per unit (tile x trait) up to every SM
-            CK(epi::mma_prepare(r.variant, ctx->ntraits, (int)std::min<int64_t>(2 * units, ctx->sm_count), &grid));
+            CK(epi::mma_prepare(r.variant, r.screen, ctx->ntraits, (int)std::min<int64_t>(2 * units, ctx->sm_count), &grid));
         } else {
             // one CTA per unit up to every SM
             CK(epi::popc_prepare(r.variant));
@@ -706,7 +903,8 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
         }
     }
     if (nblocks) memcpy(ctx->h_blocks, r.desc.data(), nblocks * sizeof(BlockDesc));
-    ctx->last_launches = r.ntiles > 0 ? 2 : 1;  // the state reset and the scan kernel
+    // the state reset and the scan kernel, or the screen and the exact kernel of every segment
+    ctx->last_launches = 1 + (r.ntiles > 0 ? (r.screen ? 2 * r.segments : 1) : 0);
     ctx->last_form = r.form;
     if (!use_graph) {
         CK(enqueue_scan(ctx, r, grid, nblocks, false));
@@ -716,6 +914,8 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
     key_add(key, r.args);
     key_add(key, r.form);
     key_add(key, r.variant);
+    key_add(key, r.screen);
+    key_add(key, r.segments);
     key_add(key, grid);
     key_add(key, ctx->ntraits);
     if (r.form == EPI_FORM_TENSOR) key_add(key, ctx->maps);
@@ -753,6 +953,7 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
 // launches (src/main.c:115-130, src/EpiOpenCL.c:1353-1362), set by hand.
 struct TuneEntry {
     int device, form, Np, ntraits, variant;
+    int screen;
     std::string how;
 };
 static std::mutex g_tune_mu;
@@ -769,7 +970,7 @@ std::string variant_desc(int form, int v)
     return std::string(form == EPI_FORM_TENSOR ? "tensor form, " : "plain form, ") + d;
 }
 
-epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int *v, std::string *how)
+epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int screen, int *v, std::string *how)
 {
     const int nv = form_variants(form);
     if (o->tile_config > 0) {
@@ -785,7 +986,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int *v, 
         // would fit: another context of the same shape may hold more SNPs)
         for (const TuneEntry &t : g_tune)
             if (t.device == ctx->device && t.form == form && t.Np == ctx->Np && t.ntraits == ctx->ntraits &&
-                !(form == EPI_FORM_TENSOR && epi::mma_needs_x(t.variant) && !x_candidate(ctx))) {
+                t.screen == screen && !(form == EPI_FORM_TENSOR && epi::mma_needs_x(t.variant) && !x_candidate(ctx, screen))) {
                 *v = t.variant;
                 *how = t.how;
                 return EPI_OK;
@@ -818,12 +1019,12 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int *v, 
     for (int c = 0; c < nv; ++c) {
         // the streamed-B variant is no candidate where its expanded rows would not fit or would
         // run into the power cap (x_candidate)
-        if (form == EPI_FORM_TENSOR && epi::mma_needs_x(c) && !x_candidate(ctx)) {
+        if (form == EPI_FORM_TENSOR && epi::mma_needs_x(c) && !x_candidate(ctx, screen)) {
             ms[c] = INFINITY;
             continue;
         }
         ScanRun r;
-        epi_status st = setup_run(ctx, &blk, 1, &o2, r, c);
+        epi_status st = setup_run(ctx, &blk, 1, &o2, r, c, screen);
         if (st != EPI_OK) return st;
         r.args.hits = ctx->d_hits;
         r.args.cap = ctx->hit_cap;
@@ -839,7 +1040,8 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int *v, 
     }
     const int best = (int)(std::min_element(ms.begin(), ms.end()) - ms.begin());
     char buf[256];
-    int len = snprintf(buf, sizeof(buf), "autotuned on a %d x %d-SNP block:", blk.size1, blk.size2);
+    int len = snprintf(buf, sizeof(buf), "autotuned on a %d x %d-SNP block%s:", blk.size1, blk.size2,
+                       screen == 1 ? ", 8-bit screen" : screen == 2 ? ", 16-bit screen" : "");
     for (int c = 0; c < nv && len < (int)sizeof(buf); ++c)
         len += std::isfinite(ms[c]) ? snprintf(buf + len, sizeof(buf) - len, "%s %.3f ms", c ? " /" : "", ms[c])
                                     : snprintf(buf + len, sizeof(buf) - len, "%s n/a", c ? " /" : "");
@@ -851,10 +1053,10 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int *v, 
         cudaFree(ctx->d_x);
         ctx->d_x = nullptr;
         ctx->x_cap = 0;
-        ctx->x_valid = false;
+        ctx->x_valid = -1;
     }
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_tune.push_back({ctx->device, form, ctx->Np, ctx->ntraits, best, *how});
+    g_tune.push_back({ctx->device, form, ctx->Np, ctx->ntraits, best, screen, *how});
     return EPI_OK;
 }
 
@@ -881,10 +1083,19 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     const int form = pick_form(ctx, opts);
     int variant = 0;
     std::string how;
-    s = pick_variant(ctx, opts, form, &variant, &how);
+    int64_t pairs = 0;
+    for (int b = 0; b < nblocks; ++b) {
+        const epi_block &e = blocks[b];
+        if (e.size1 < 0 || e.size2 < 0 || e.start1 < 0 || e.start2 < 0 || (int64_t)e.start1 + e.size1 > ctx->nsnp ||
+            (int64_t)e.start2 + e.size2 > ctx->nsnp)
+            return set_err(ctx, EPI_E_INVALID, "block %d out of range", b);
+        pairs += block_pairs(e);
+    }
+    int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs) : 0;
+    s = pick_variant(ctx, opts, form, screen, &variant, &how);
     if (s != EPI_OK) return s;
     ScanRun r;
-    s = setup_run(ctx, blocks, nblocks, opts, r, variant);
+    s = setup_run(ctx, blocks, nblocks, opts, r, variant, screen);
     if (s != EPI_OK) return s;
     if (ctx->hit_cap == 0) {
         const int64_t initial = 1 << 20;
@@ -903,6 +1114,18 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
         if (cnt[2] != 0)
             return set_err(ctx, EPI_E_TIMEOUT, "a bounded device wait of the scan kernel gave up (site %llu)",
                            cnt[3]);
+        if (screen && cnt[epi::CNT_OVERFLOW] != 0) {
+            // more candidates than the list holds: once more with all digits, directly
+            ctx->scr_full = true;
+            ctx->scr_full_t1 = opts->t1;
+            ctx->scr_full_t2 = opts->t2;
+            screen = 0;
+            s = pick_variant(ctx, opts, form, screen, &variant, &how);
+            if (s == EPI_OK) s = setup_run(ctx, blocks, nblocks, opts, r, variant, screen);
+            if (s != EPI_OK) return s;
+            attempt = -1;
+            continue;
+        }
         found = cnt[0];
         if ((int64_t)found <= ctx->hit_cap) break;
         // every hit is needed to put the first `cap` in output order: grow and rescan
@@ -916,11 +1139,9 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     ctx->last_ms = ms;
     ctx->last_config = variant_desc(form, variant) + " (" + how + ")";
-    int64_t pairs = 0;
-    for (int b = 0; b < nblocks; ++b) pairs += block_pairs(blocks[b]);
     ctx->last_pairs = pairs * ctx->ntraits;
 
-    const unsigned int *mx = reinterpret_cast<const unsigned int *>(ctx->h_state + 4);
+    const unsigned int *mx = reinterpret_cast<const unsigned int *>(ctx->h_state + epi::NCOUNTERS);
     std::vector<DevHit> dh((size_t)found);
     if (found) {
         CK(cudaMemcpyAsync(dh.data(), ctx->d_hits, (size_t)found * sizeof(DevHit), cudaMemcpyDeviceToHost,
@@ -991,10 +1212,10 @@ extern "C" epi_status epi_scan_dump(epi_ctx *ctx, const epi_block *block, const 
     const int form = pick_form(ctx, &o);
     int variant = 0;
     std::string how;
-    s = pick_variant(ctx, &o, form, &variant, &how);
+    s = pick_variant(ctx, &o, form, 0, &variant, &how);
     if (s != EPI_OK) return s;
     ScanRun r;
-    s = setup_run(ctx, block, 1, &o, r, variant);
+    s = setup_run(ctx, block, 1, &o, r, variant, 0);
     if (s != EPI_OK) return s;
     const size_t np = (size_t)block->size1 * block->size2;
     int32_t *dc = nullptr, *dd1 = nullptr, *dd2 = nullptr;

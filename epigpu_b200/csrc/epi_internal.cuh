@@ -14,8 +14,15 @@
 // and for the tensor-core form
 //   hcodes  uint8 [nsnp][Np]      one-hot genotype byte: 1 << g for g in 0..2, 0 if missing
 //   missbits uint32 [nsnp][Wp]    missing-genotype bits
-//   ydig    int8 [T][4][Np]       per individual: phenotype-valid flag and the three balanced
-//                                 base-256 digits (low first) of Y = round(y * 2^sy)
+//   ydig    int8 [T][5][Np]       per individual: the screen's 8-bit phenotype D (below), the
+//                                 phenotype-valid flag and the three balanced base-256 digits
+//                                 (the highest first) of Y = round(y * 2^sy)
+//   tscr    float4 [T][2]         the screen with one digit and with two: (d0, E, s^2 Qtot, s^2);
+//                                 one digit: D approximates s (ytilde - c) with |D| <= 127,
+//                                 d0 = -s c is the D of the mean; two: D is the two upper digits
+//                                 of Y and d0 = 0; E = ||s ytilde - (D - d0)||_2 over the valid
+//                                 individuals
+//   qmf     float [T][nsnp]       qm as floats
 //   qd      double [2][T][Np]     ytilde^2 (ytilde = Y 2^-sy, the quantised y), then Y itself;
 //                                 0 where invalid; per trait qtot = sum of ytilde^2, ytot = sum
 //                                 of Y, nvalid = count over the valid individuals
@@ -62,6 +69,22 @@ struct HitRow {
     float F, F2;
 };
 
+// A place in the tensor form's order of units: the begin of a row group.
+struct SegPos {
+    int32_t trait, block, group;
+};
+
+// A pair that the screen of the tensor form could not settle, with upper bounds of its F and
+// F2 (NaN: unknown): the list that k_exact goes through.
+struct Cand {
+    int32_t snp1, snp2, trait, block;
+    float fu, f2u;
+};
+
+// 64-bit counters of a scan: hits found, tile queue (plain form), error flag and site, then
+// whether the candidate list overflowed, and from CNT_CAND on the candidates of each segment
+constexpr int CNT_OVERFLOW = 4, CNT_CAND = 5, MAX_SEGMENTS = 8, NCOUNTERS = CNT_CAND + MAX_SEGMENTS + 3;
+
 struct ScanArgs {
     // genotypes
     const uint4 *planes;
@@ -95,13 +118,24 @@ struct ScanArgs {
     // tensor form: limit of every device-side wait (ns); test hook that makes one wait run out
     unsigned long long wait_ns;
     int32_t debug_stall;
-    // tensor form, streamed-B variant: the unit order walks super-tiles of xsi x xsj pair
-    // tiles, so that their A rows and expanded B rows stay in L2 together
+    // tensor form: for each trait the unit order walks groups of xsi i-tile rows in chunks of xsj
+    // j-tiles (the streamed-B variant: super-tiles whose A rows and expanded B rows stay in L2
+    // together); this launch's part of it begins at seg0 and ends before seg1
     int32_t xsi, xsj;
+    SegPos seg0, seg1;
+    // tensor form, screened scan: per trait and per (trait, SNP) constants of the screen, the
+    // segment's candidate list and the per-trait lower bounds of the largest F and F2 so far
+    // (order-encoded, as the maxima)
+    const float4 *tscr;
+    const float *qmf;
+    Cand *cand;
+    int64_t cand_cap;
+    int32_t segment;
+    unsigned int *lowf, *lowf2;
     // outputs
     DevHit *hits;
     int64_t cap;
-    unsigned long long *counters;  // [0] hits found, [1] tile queue, [2] error flag, [3] error site
+    unsigned long long *counters;  // NCOUNTERS: [0] hits found, [1] tile queue, [2] error flag, [3] error site, ...
     unsigned int *maxf, *maxf2;    // [T] order-preserving encoded floats
     // optional dump of one block (pair (gx, gy) at gx*size2 + gy)
     int32_t *dump_counts;
@@ -117,7 +151,10 @@ struct ScanArgs {
 
 // TMA descriptors of the tensor form (kernel parameter, __grid_constant__)
 struct MmaMaps {
-    CUtensorMap hi, hj, dg, hx;  // hx: the expanded B rows of the streamed-B variant
+    // dg: the trait's four digit rows (w, Y digits); ds, ds2: the rows of the screen with one digit
+    // (D, w) and with two (w, d2, d1), whose j-tile is narrower (hj2); hx: the expanded B rows of
+    // the streamed-B variant
+    CUtensorMap hi, hj, hj2, dg, ds, ds2, hx;
 };
 
 // TMA descriptors of the plain form: the genotype plane words, in boxes of the tile's i-SNPs
@@ -125,6 +162,8 @@ struct MmaMaps {
 struct PopcMaps {
     CUtensorMap planes_i, planes_j;
 };
+
+constexpr unsigned int ENC_NEG_INF = 0x007fffffu;  // f2ord(-inf)
 
 // float -> unsigned with the same order (for atomicMax over possibly negative F)
 __device__ __forceinline__ unsigned int f2ord(float f)

@@ -71,10 +71,12 @@ __global__ void k_unpack(const int32_t *__restrict__ raw, int nsnp, int nid, int
 }
 
 // Per trait t and SNP s, over the individuals missing at s (and phenotype-valid for t):
-// qm[t][s] = sum of qd[t][k], rm[t][s] = sum of qr[t][k] and nm[t][s] = their number
+// qm[t][s] = sum of qd[t][k], rm[t][s] = sum of qr[t][k] and nm[t][s] = their number; qmf[t][s]
+// = qm as a float
 __global__ void k_qmiss(const uint32_t *__restrict__ missbits, int nsnp, int Wp, const uint32_t *__restrict__ wmask,
                         const double *__restrict__ qd, const double *__restrict__ qr, int Np, int ntraits,
-                        double *__restrict__ qm, double *__restrict__ rm, double *__restrict__ nm)
+                        double *__restrict__ qm, double *__restrict__ rm, double *__restrict__ nm,
+                        float *__restrict__ qmf)
 {
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (long long)nsnp * ntraits) return;
@@ -95,27 +97,34 @@ __global__ void k_qmiss(const uint32_t *__restrict__ missbits, int nsnp, int Wp,
     qm[gid] = x;
     rm[gid] = r;
     nm[gid] = (double)cnt;
+    qmf[gid] = (float)x;
 }
 
-// The streamed-B variant's expanded B rows: for trait t, CTA half h, SNP s and local column
-// type q = 2b + r (genotype b, digit row 2h + r of the trait: w, d0 for h = 0, d1, d2 for h = 1)
-// row ((t 2 + h) nsnp + s) 6 + q holds [g_s(k) == b] * digit(k) for every individual k -- the
-// rows the tensor form's producers otherwise build in shared memory. One thread per 16
-// individuals of (t, h, s).
+// The streamed-B variant's expanded B rows: row (u nsnp + s) R + r of the u-th set of R = 3 G rows
+// per SNP holds [g_s(k) == b] * digit(k) for every individual k, r = G b + i and digit the i-th of
+// the set's G digit rows -- the rows the tensor form's producers otherwise build in shared
+// memory. Full digits: two sets of G = 2 rows per trait, (w, d2) for CTA 0's half and (d1, d0) for
+// CTA 1's; the screen: one set per trait, (w, D) or (w, d2, d1). ydig's rows per trait are D, w,
+// d2, d1, d0. One thread per 16 individuals of (set, s).
+template <int G, bool FULL>
 __global__ void k_expand(const uint8_t *__restrict__ hcodes, const int8_t *__restrict__ ydig, int nsnp, int Np,
-                         int ntraits, int8_t *__restrict__ x)
+                         int sets, int8_t *__restrict__ x)
 {
     const int nc = Np / 16;
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (long long)ntraits * 2 * nsnp * nc) return;
+    if (gid >= (long long)sets * nsnp * nc) return;
     const int c = (int)(gid % nc);
     const long long rest = gid / nc;
-    const int s = (int)(rest % nsnp);
-    const int h = (int)((rest / nsnp) % 2), t = (int)(rest / nsnp / 2);
+    const int s = (int)(rest % nsnp), u = (int)(rest / nsnp);
+    const int trait = FULL ? u / 2 : u;
     const uint4 hc = reinterpret_cast<const uint4 *>(hcodes + (size_t)s * Np)[c];
-    const uint4 d0 = reinterpret_cast<const uint4 *>(ydig + ((size_t)t * 4 + 2 * h) * Np)[c];
-    const uint4 d1 = reinterpret_cast<const uint4 *>(ydig + ((size_t)t * 4 + 2 * h + 1) * Np)[c];
-    uint4 *out = reinterpret_cast<uint4 *>(x + (((size_t)t * 2 + h) * nsnp + s) * 6 * (size_t)Np) + c;
+    uint4 d[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+        const int row = FULL ? 1 + 2 * (u & 1) + i : G == 2 ? 1 - i : 1 + i;
+        d[i] = reinterpret_cast<const uint4 *>(ydig + ((size_t)trait * 5 + row) * Np)[c];
+    }
+    uint4 *out = reinterpret_cast<uint4 *>(x + ((size_t)u * nsnp + s) * 3 * G * (size_t)Np) + c;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
         uint4 m;
@@ -123,8 +132,9 @@ __global__ void k_expand(const uint8_t *__restrict__ hcodes, const int8_t *__res
         m.y = ((hc.y >> b) & 0x01010101u) * 0xFFu;
         m.z = ((hc.z >> b) & 0x01010101u) * 0xFFu;
         m.w = ((hc.w >> b) & 0x01010101u) * 0xFFu;
-        out[(size_t)(2 * b) * nc] = make_uint4(m.x & d0.x, m.y & d0.y, m.z & d0.z, m.w & d0.w);
-        out[(size_t)(2 * b + 1) * nc] = make_uint4(m.x & d1.x, m.y & d1.y, m.z & d1.z, m.w & d1.w);
+#pragma unroll
+        for (int i = 0; i < G; ++i)
+            out[(size_t)(G * b + i) * nc] = make_uint4(m.x & d[i].x, m.y & d[i].y, m.z & d[i].z, m.w & d[i].w);
     }
 }
 
@@ -238,21 +248,25 @@ cudaError_t launch_unpack(const int32_t *raw, int nsnp, int nid, int npack, int 
 
 cudaError_t launch_qmiss(const uint32_t *missbits, int nsnp, int Wp, const uint32_t *wmask, const double *qd,
                         const double *qr, int Np, int ntraits, double *qm, double *rm, double *nm,
-                        cudaStream_t stream)
+                        float *qmf, cudaStream_t stream)
 {
     const long long total = (long long)nsnp * ntraits;
     const int nt = 256;
     k_qmiss<<<(unsigned)((total + nt - 1) / nt), nt, 0, stream>>>(missbits, nsnp, Wp, wmask, qd, qr, Np, ntraits, qm,
-                                                                     rm, nm);
+                                                              rm, nm, qmf);
     return cudaGetLastError();
 }
 
-cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int8_t *x,
-                          cudaStream_t stream)
+cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int screen,
+                          int8_t *x, cudaStream_t stream)
 {
-    const long long total = (long long)ntraits * 2 * nsnp * (Np / 16);
+    const int sets = screen ? ntraits : 2 * ntraits;
+    const long long total = (long long)sets * nsnp * (Np / 16);
     const int nt = 256;
-    k_expand<<<(unsigned)((total + nt - 1) / nt), nt, 0, stream>>>(hcodes, ydig, nsnp, Np, ntraits, x);
+    const unsigned nb = (unsigned)((total + nt - 1) / nt);
+    if (screen == 0) k_expand<2, true><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
+    else if (screen == 1) k_expand<2, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
+    else k_expand<3, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
     return cudaGetLastError();
 }
 

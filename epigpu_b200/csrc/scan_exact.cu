@@ -1,0 +1,118 @@
+// scan_exact.cu -- the exact statistics of the pairs that the tensor form's screen could not
+// settle (the candidate list of k_scan_mma's screened variants, scan_mma.cu).
+//
+// One warp per candidate: the 3x3 counts and the three digit sums of every cell over the
+// one-hot genotype bytes and the trait's digit rows, 16 individuals per lane and step, as byte
+// masks and dp4a (36 accumulators; int32, so the sums are the same integers that the full
+// MMA gives), then the same FP64 statistics (pair_stat_exact). The reference's per-pair loop is
+// src/EpiOpenCL.c:110-247 and :452-489.
+// About 57 instructions per 128 individuals and warp: 5,000 per candidate at 10,000
+// individuals. At 1e-4 of the pairs that is under 1% of the screen's time, which is why the
+// list is worked off pair by pair and not as tiles.
+#include "epi_internal.cuh"
+#include "pair_exact.cuh"
+
+namespace epi {
+
+constexpr int EXACT_NT = 256;
+
+__global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
+{
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * EXACT_NT + threadIdx.x) >> 5, nwarps = (long long)gridDim.x * (EXACT_NT / 32);
+    const long long found = (long long)a.counters[CNT_CAND + a.segment];
+    if (found > a.cand_cap || a.counters[CNT_OVERFLOW]) {
+        // the list does not hold them all: the host scans again without the screen
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.counters[CNT_OVERFLOW] = 1ull;
+        return;
+    }
+    const float t1c = screen_lo(a.t1), t2c = screen_lo(a.t2);
+    const int nc = a.Np / 16;
+    for (long long q = warp; q < found; q += nwarps) {
+        const Cand c = a.cand[q];
+        const int t = c.trait;
+        const bool report = a.report_trait < 0 || a.report_trait == t;
+        // against the lower bounds of the maxima as they stand now (the same for every lane)
+        unsigned int lF = 0u, lI = 0u;
+        if (lane == 0) {
+            lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
+            lI = reinterpret_cast<volatile unsigned int *>(a.lowf2)[t];
+        }
+        const float mF = screen_lo(ord2f(__shfl_sync(0xffffffffu, lF, 0)));
+        const float mI = screen_lo(ord2f(__shfl_sync(0xffffffffu, lI, 0)));
+        if (c.fu <= (report ? fminf(t1c, mF) : mF) && (!a.test_int || c.f2u <= (report ? fminf(t2c, mI) : mI))) continue;
+
+        const uint4 *hi = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp1 * a.Np);
+        const uint4 *hj = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp2 * a.Np);
+        const uint4 *dg = reinterpret_cast<const uint4 *>(a.ydig + ((size_t)t * 5 + 1) * a.Np);
+        int acc[9][4];
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[k][r] = 0;
+        for (int k = lane; k < nc; k += 32) {
+            const uint4 vi = hi[k], vj = hj[k];
+            const uint4 d[4] = {dg[k], dg[nc + k], dg[2 * nc + k], dg[3 * nc + k]};
+            const uint32_t wi[4] = {vi.x, vi.y, vi.z, vi.w}, wj[4] = {vj.x, vj.y, vj.z, vj.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                int dx[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) dx[r] = (int)(x == 0 ? d[r].x : x == 1 ? d[r].y : x == 2 ? d[r].z : d[r].w);
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    const uint32_t mi = (wi[x] >> g) & 0x01010101u;
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        const int m = (int)(mi & (wj[x] >> b));
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) acc[3 * g + b][r] = __dp4a(m, dx[r], acc[3 * g + b][r]);
+                    }
+                }
+            }
+        }
+        int n[9], N = 0;
+        double si[9], st = 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            n[k] = __reduce_add_sync(0xffffffffu, acc[k][0]);
+            const int x3 = __reduce_add_sync(0xffffffffu, acc[k][1]);
+            const int x2 = __reduce_add_sync(0xffffffffu, acc[k][2]);
+            const int x1 = __reduce_add_sync(0xffffffffu, acc[k][3]);
+            si[k] = fma(65536.0, (double)x3, fma(256.0, (double)x2, (double)x1));
+            st += si[k];
+            N += n[k];
+        }
+        // the sum of squares: see scan_mma.cu
+        const size_t mi = (size_t)t * a.nsnp + c.snp1, mj = (size_t)t * a.nsnp + c.snp2;
+        const double sc = a.yscale[t];
+        const int nmm = N + (int)(a.nm[mi] - a.nvalid[t] + a.nm[mj]);
+        double qmm = 0.0;
+        if (nmm == 1) {
+            const double ymm = (st - a.ytot[t] + a.sm[mi] + a.sm[mj]) * sc;
+            qmm = ymm * ymm;
+        } else if (nmm >= 2) {
+            qmm = missing_both_q(a, t, c.snp1, c.snp2);
+        }
+        const PairStat s = pair_stat_exact(n, si, sc, a.qtot[t] - a.qm[mi] - a.qm[mj] + qmm, a.test_int != 0);
+        emit_hit(a, lane == 0 && report && is_hit(a, s), c.snp1, c.snp2, s, t, c.block);
+        if (lane == 0) {
+            auto raise = [](unsigned int *max, unsigned int *low, double F) {
+                if (!(F == F)) return;
+                const unsigned int v = f2ord((float)F);
+                if (v > *reinterpret_cast<volatile unsigned int *>(max)) atomicMax(max, v);
+                if (v > *reinterpret_cast<volatile unsigned int *>(low)) atomicMax(low, v);
+            };
+            raise(&a.maxf[t], &a.lowf[t], s.F);
+            if (a.test_int) raise(&a.maxf2[t], &a.lowf2[t], s.F2);
+        }
+    }
+}
+
+cudaError_t exact_enqueue(const ScanArgs &a, int sm_count, cudaStream_t stream)
+{
+    k_exact<<<2 * sm_count, EXACT_NT, 0, stream>>>(a);
+    return cudaGetLastError();
+}
+
+}  // namespace epi

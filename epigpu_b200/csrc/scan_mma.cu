@@ -7,13 +7,13 @@
 //     D[128 x 252] = A[128 x K] * B[K x 252]
 //   A rows (row 32w + l, l < 30): i-SNP 10w + l/3, genotype a = l%3: [g_i(k) == a]
 //   B cols: type t = 4b + s (b = 0..2 the j genotype, s = 0..3), [g_j(k) == b] * D_s(k), with
-//     D_0 = w_k (phenotype valid) and D_1..3 the balanced base-256 digits of the fixed-point
-//     phenotype Y_k = round(y_k * 2^sy) (y centred, 0 when invalid); CTA 0 of the pair holds
+//     D_0 = w_k (phenotype valid) and D_1..3 the balanced base-256 digits, the highest first, of
+//     the fixed-point phenotype Y_k = round(y_k * 2^sy) (y centred, 0 when invalid); CTA 0 of the pair holds
 //     the types of D_0 and D_1, CTA 1 those of D_2 and D_3, so each builds its half from two
 //     digit rows: column of (t, j') in the pair MMA 128 (s / 2) + 6 j' + (2b + s % 2), the six
 //     columns of a j-SNP side by side in each half.
 // int8 operands, int32 accumulation: counts and digit sums are exact, so
-//     S_ab = (D1 + 256 D2 + 65536 D3) * 2^-sy exactly for the quantised phenotype.
+//     S_ab = (65536 D1 + 256 D2 + D3) * 2^-sy exactly for the quantised phenotype.
 // The sum of ytilde^2 (ytilde = Y 2^-sy) over the pair's valid individuals (both genotypes
 // known, phenotype valid) follows from per-SNP sums over each SNP's missing individuals:
 //     Q_ij = Qtot - QM_i - QM_j + QMM_ij,   QMM_ij = sum of ytilde^2 over the individuals
@@ -62,6 +62,7 @@
 #include <vector>
 
 #include "epi_internal.cuh"
+#include "pair_exact.cuh"
 #include "tc_ptx.cuh"
 
 namespace epi {
@@ -69,7 +70,7 @@ namespace mma {
 
 constexpr int TI = 40;         // i-SNPs per CTA (4 lane quarters x 10 triplets)
 constexpr int TIP = 2 * TI;    // i-SNPs per pair tile
-constexpr int TJ = 21;         // j-SNPs per tile
+constexpr int TJ = 21;         // j-SNPs per tile of the full digits (the screen: 2 x 21)
 constexpr int NTYPE = 12;      // B column types per j-SNP: b (3) x {w, d0, d1, d2}
 constexpr int NCOL = TJ * NTYPE;  // 252 columns in use
 constexpr int N = 256;         // MMA width (pair MMAs take multiples of 32)
@@ -78,6 +79,7 @@ constexpr int TYH = NTYPE / 2; // column types held by each CTA (6 x 21 = 126 of
 constexpr int M = 256;         // MMA height over the pair
 constexpr int KS = 128;        // individuals per pipeline stage
 constexpr int ND = 4;          // digit rows per trait: w, Y digits (3)
+constexpr int DROWS = 1 + ND;  // rows per trait in ydig: D, w, then the Y digits, the highest first
 constexpr int ROUNDS = (TJ + 2) / 3;  // j rounds of the epilogue (3 j-SNPs per round)
 constexpr uint32_t ACC_COL1 = N;
 __host__ __device__ constexpr uint32_t acc_col(uint32_t buf) { return buf ? ACC_COL1 : 0u; }
@@ -97,7 +99,6 @@ constexpr uint32_t XB_BYTES = 6 * TJ * KS;     // the streamed-B variant: one CT
 // raw stage: the j-tile's one-hot rows and the trait's digit rows, 1024-aligned sections
 constexpr int RAW_J = 0, RAW_D = (TJ * KS + 1023) / 1024 * 1024;
 constexpr int RAW_STAGE = 4 * 1024;
-constexpr uint32_t RAW_BYTES = (TJ + ND) * KS;
 // producer work items per stage: (j-SNP, 16-individual chunk); 128 producer threads take the
 // first 128 and the threads below XTRA one more (the j-SNPs 16..20, same chunk)
 constexpr int XTRA = TJ * 8 - 128;
@@ -134,10 +135,20 @@ static_assert(6 * 3 * (ROUNDS - 1) + RCOLS <= NH && bcol(11, TJ - 1) < N && bcol
 // bytes per SNP and individual: `hx`, rows ((t 2 + half) M + snp) 6 + q) and TMA-loaded with
 // the A rows, one 126-row box per CTA half per stage; no producers or raw loader run (warps 4-7
 // and 14 idle) and CTA 0's full barrier counts two arrivals (its loader, CTA 1's forward).
-template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false>
+//
+// SCR (the screened scan, 1 or 2 phenotype digits; 0: all digits): B holds the column types of w
+// and of the screen's digits only, 3 (1 + SCR) per j-SNP and TJH j-SNPs in each CTA's half: a
+// tile is 42 j-SNPs wide with one digit, 28 with two (screen_epilogue below).
+template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false, int SCR_ = 0>
 struct Rings {
-    static constexpr int STAGES = S, RSTAGES = RSx, EPW = EPW_, PW = PW_;
+    static constexpr int STAGES = S, RSTAGES = RSx, EPW = EPW_, PW = PW_, SCR = SCR_;
     static constexpr bool XF = XF_;
+    static constexpr int TY = SCR ? 3 * (1 + SCR) : TYH;  // column types of a j-SNP in a CTA's half
+    static constexpr int TJH = (TYH * TJ) / TY;           // j-SNPs in a half: 21 (all digits, one), 14 (two)
+    static constexpr int TJT = SCR ? 2 * TJH : TJ;        // j-SNPs per tile
+    static constexpr int RAW_ROWS = SCR == 0 ? ND : 1 + SCR;  // digit rows of a raw stage
+    static constexpr uint32_t RAW_BYTES = (TJH + RAW_ROWS) * KS;
+    static_assert(TY * TJH == TYH * TJ, "every variant fills 126 of a half's 128 rows");
     static_assert(!XF || (EPW == 2 && PW == 1), "the streamed-B variant runs the 15-warp layout");
     static constexpr int NWARPS = (EPW == 2 && PW == 1) ? 15 : 20;
     static constexpr int NTHREADS = NWARPS * 32;
@@ -165,45 +176,86 @@ __device__ __forceinline__ uint4 ld_sw128(const uint8_t *base, int r, int c)
     return *reinterpret_cast<const uint4 *>(base + r * 128 + ((c ^ (r & 7)) << 4));
 }
 
-struct Unit {
-    int block, trait, i0, j0;
+// The units (trait, pair tile) of one cluster, in order: every npairs-th one of the tiles that
+// hold a pair snp1 > snp2, of one trait after the other (with traits innermost the expanded B
+// rows of the streamed-B variant, which differ per trait, came from DRAM for every i-tile). Each
+// role walks its own copy. Tiles outside the
+// triangle are not in the sequence at all, so the clusters' shares differ by one unit at most
+// (a fixed stride over all tiles gave some clusters twice the work of others on a diagonal
+// block, and a 64-bit division per unit and role). A block's tiles run in groups of xsi i-tile
+// rows and within a group in chunks of xsj j-tiles, row by row inside a chunk: with xsi = 1 and
+// one chunk row by row over all j-tiles; the streamed-B variant keeps super-tiles, whose A rows
+// and expanded B rows then stay in L2 together.
+template <class C>
+struct Walker {
     BlockDesc bd;
-    bool skip;
-};
+    int block, trait, i0, j0;  // the unit: its block, trait, first i-SNP (of the pair) and first j-SNP
+    bool done;
 
-// Unit u -> (trait, block, pair tile). Units run trait-fastest over the block's tiles. XF (the
-// streamed-B variant): a block's tiles are walked in groups of xsi i-tiles, and within a group
-// in chunks of xsj j-tiles, i-tile by i-tile inside a chunk, so the clusters working at the same
-// time share a super-tile's A rows and expanded B rows in L2; otherwise i-tile by i-tile.
-template <bool XF = false>
-__device__ __forceinline__ Unit decode(const ScanArgs &a, long long u)
-{
-    Unit r;
-    const long long tile = u / a.ntraits;
-    r.trait = (int)(u % a.ntraits);
-    r.block = find_block(a.blocks, a.nblocks, tile);
-    r.bd = a.blocks[r.block];
-    const long long lt = tile - r.bd.tile_base;
-    int ti, tj;
-    if (XF) {
-        const long long grp_tiles = (long long)a.xsi * r.bd.tiles_j;
-        const int grp = (int)(lt / grp_tiles);
-        const int ni = min(a.xsi, r.bd.tiles_i - grp * a.xsi);
-        const long long q = lt - (long long)grp * grp_tiles;
-        const int jc = (int)(q / ((long long)ni * a.xsj));
-        const int q2 = (int)(q - (long long)jc * ni * a.xsj);
-        const int nj = min(a.xsj, r.bd.tiles_j - jc * a.xsj);
-        ti = grp * a.xsi + q2 / nj;
-        tj = jc * a.xsj + q2 % nj;
-    } else {
-        ti = (int)(lt / r.bd.tiles_j);
-        tj = (int)(lt % r.bd.tiles_j);
+    __device__ __forceinline__ Walker(const ScanArgs &args, int first, int step_)
+        : block(args.seg0.block), trait(args.seg0.trait), done(false), a(args), step(step_), grp(args.seg0.group - 1),
+          jc(0), q(0), rows(0), chunks(0), off(0), len(0)
+    {
+        bd = a.blocks[block];
+        move(first);
     }
-    r.i0 = ti * TIP;  // the pair tile's first i-SNP
-    r.j0 = tj * TJ;
-    r.skip = r.bd.start1 + min(r.i0 + TIP, r.bd.size1) - 1 <= r.bd.start2 + r.j0;
-    return r;
-}
+    __device__ __forceinline__ void next() { move(step); }
+
+private:
+    const ScanArgs &a;
+    int step;
+    int grp, jc, q, rows, chunks;  // the row group, the chunk of j-tiles, the row in the group
+    int off, len;                  // the tile in the row's part of the chunk, and that part's length
+
+    // how many tiles of row ti hold a pair: those that begin below the row's last i-SNP
+    __device__ __forceinline__ int valid_tiles(int ti) const
+    {
+        const int x = bd.start1 + min((ti + 1) * TIP, bd.size1) - 1 - bd.start2;
+        return x <= 0 ? 0 : min(bd.tiles_j, (x + C::TJT - 1) / C::TJT);
+    }
+    __device__ __forceinline__ bool at_end() const
+    {
+        if (trait != a.seg1.trait) return trait > a.seg1.trait;
+        return block > a.seg1.block || (block == a.seg1.block && grp >= a.seg1.group);
+    }
+    __device__ __forceinline__ bool next_row()
+    {
+        ++q;
+        while (q >= rows) {  // next chunk
+            q = 0;
+            if (++jc < chunks) break;
+            jc = 0;
+            ++grp;
+            while (!at_end() && grp * a.xsi >= bd.tiles_i) {  // next block, or trait
+                grp = 0;
+                if (++block == a.nblocks) {
+                    block = 0;
+                    ++trait;
+                }
+                if (!at_end()) bd = a.blocks[block];
+            }
+            if (at_end()) return false;
+            rows = min(a.xsi, bd.tiles_i - grp * a.xsi);
+            chunks = (valid_tiles(grp * a.xsi + rows - 1) + a.xsj - 1) / a.xsj;
+            if (chunks == 0) q = rows;  // a group above the diagonal
+        }
+        len = max(0, min(a.xsj, valid_tiles(grp * a.xsi + q) - jc * a.xsj));
+        return true;
+    }
+    __device__ __forceinline__ void move(int tiles)
+    {
+        off += tiles;
+        while (off >= len) {
+            off -= len;
+            if (!next_row()) {
+                done = true;
+                return;
+            }
+        }
+        i0 = (grp * a.xsi + q) * TIP;
+        j0 = (jc * a.xsj + off) * C::TJT;
+    }
+};
 
 template <class Smem>
 __device__ __forceinline__ void fail(const ScanArgs &a, Smem &sm, int where)
@@ -221,82 +273,6 @@ template <class T>
 __device__ __forceinline__ T pick3(T x0, T x1, T x2, int idx)
 {
     return idx == 0 ? x0 : (idx == 1 ? x1 : x2);
-}
-
-// 1/x for x > 0: single-precision seed (__frcp_rn) refined by one Newton step in FP64,
-// e = 1 - x r, r' = r + r e, which squares the seed's relative error (2^-24 -> ~2^-48).
-__device__ __forceinline__ double rcp_d(double x)
-{
-    double r = (double)__frcp_rn((float)x);
-    const double e = fma(-x, r, 1.0);
-    return fma(r, e, r);
-}
-
-// num / den in FP64: by rcp_d when den is a normal single-precision magnitude (relative error
-// ~2^-46), else by IEEE division (zero, tiny or huge denominators keep division's inf / NaN).
-__device__ __forceinline__ double div_fast(double num, double den)
-{
-    const double ad = fabs(den);
-    return (ad > 1e-30 && ad < 1e30) ? num * rcp_d(den) : num / den;
-}
-
-// The reference's 8 df / 4 df statistics (src/EpiOpenCL.c:231-247, :452-486) in FP64 from
-// the exact integer cell counts n and digit sums si (S = si * sc), and Q = sum of y^2 over
-// the pair's valid individuals. Same quantities as pair_stat, arranged to avoid division
-// chains: reciprocals by rcp_d.
-__device__ __forceinline__ PairStat pair_stat_exact(const int n[9], const double si[9], double sc, double Q,
-                                                    bool want_int)
-{
-    // si are integers below 2^53 in magnitude (digit sums), so every sum of them is exact
-    PairStat r;
-    int N = 0, nfac = 0;
-    double St_i = 0.0;
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        N += n[c];
-        St_i += si[c];
-        nfac += n[c] > 0;
-    }
-    const double St = St_i * sc;
-    const double m = St * rcp_d((double)N);
-    double mc[9], SSB = 0.0;
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        mc[c] = 0.0;
-        if (n[c] > 0) {
-            mc[c] = si[c] * sc * rcp_d((double)n[c]);
-            const double d = mc[c] - m;
-            SSB = fma((double)n[c] * d, d, SSB);
-        }
-    }
-    const double SSW = ssw_floored(Q - St * m, SSB, SSW_FLOOR_EXACT);
-    r.nfac = nfac;
-    r.d1 = nfac - 1;
-    r.d2 = N - nfac;
-    r.F = div_fast(SSB * (double)r.d2, SSW * (double)r.d1);
-    r.F2 = 0.0;
-    if (want_int) {
-        double row[3], col[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double rs = si[3 * i] + si[3 * i + 1] + si[3 * i + 2];
-            const double cs = si[i] + si[i + 3] + si[i + 6];
-            const int rn = n[3 * i] + n[3 * i + 1] + n[3 * i + 2];
-            const int cn = n[i] + n[i + 3] + n[i + 6];
-            row[i] = rn > 0 ? rs * sc * rcp_d((double)rn) : 0.0;
-            col[i] = cn > 0 ? cs * sc * rcp_d((double)cn) : 0.0;
-        }
-        double SSI = 0.0;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            if (n[c] > 0) {
-                const double t = mc[c] - row[c / 3] - col[c % 3] + m;
-                SSI = fma((double)n[c] * t, t, SSI);
-            }
-        }
-        r.F2 = div_fast(SSI * (double)r.d2, 4.0 * SSW);
-    }
-    return r;
 }
 
 // approximate reciprocal of the screen (one MUFU operation, relative error ~2^-23; 1/0 = +inf)
@@ -362,15 +338,322 @@ __device__ __forceinline__ void pair_stat_f32(const int n[9], const float sd[9],
     }
 }
 
-// x lowered by the screen's margin (relative 1e-3); -inf and NaN stay as they are
-__device__ __forceinline__ float screen_lo(float x) { return x - 1e-3f * fabsf(x); }
-
 template <int RING>
 __device__ __forceinline__ void advance(uint32_t &slot, uint32_t &phase)
 {
     if (++slot == RING) {
         slot = 0;
         phase ^= 1u;
+    }
+}
+
+// ---- the screen (SCR) ----
+//
+// For deciding which pairs can matter an 8-bit phenotype is enough (16 bits, the two upper
+// digits of Y, where N is so large that 8 let too many pairs through). With D (|D| <= 127, one
+// int8 digit) approximating s (ytilde - c) and E = ||s ytilde - (D - d0)||_2 over the valid
+// individuals, SSB is the squared norm of an orthogonal projection of ytilde (onto the cells'
+// indicators less the constant) and SSI that of a symmetric map of norm <= 1 (the cells' mean
+// less the row and column means plus the grand mean), so in units of D
+//     sqrt(SSB) <= sqrt(SSB_D) + E,     sqrt(SSI) <= sqrt(SSI_D) + E,
+// and likewise from below with - E. The sum of squares is exact up to the individuals missing
+// at both SNPs: Qtot - QM_i - QM_j <= Q <= Qtot - max(QM_i, QM_j). A pair whose upper bounds of
+// F and F2 stay below the thresholds and below the largest lower bounds met so far is neither
+// a hit nor a maximum; every other pair (about 1e-4 of them at the usual thresholds) goes to
+// the candidate list, which k_exact evaluates from the 24-bit digits. The bounds of FP32
+// rounding: P, R, C, M and X below are sums of squares of the centred trait's cell sums, each
+// at most P in magnitude and good to ~1e-6 of it, hence the slack SLK_B and SLK_I; the
+// thresholds are lowered by a relative 1e-3, which covers the rest.
+//
+// Six column types (nine) instead of twelve per j-SNP: a pair MMA serves 80 x 42 (28) pairs
+// instead of 80 x 21.
+constexpr float SLK_B = 4e-6f, SLK_I = 1.2e-5f;
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(rcp_fast(a.x), rcp_fast(a.y)); }
+__device__ __forceinline__ float sqrt_fast(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Integers below 2^22 in magnitude as floats (exact): an integer addition into the mantissa of
+// 1.5 x 2^23 and a float subtraction. The conversion instruction runs on the pipe of the
+// reciprocals, at a sixteenth of the rate: 36 of them a round made it the epilogue's bound
+// (85% busy at 500 individuals).
+__device__ __forceinline__ float2 int_float2(uint32_t x, uint32_t y)
+{
+    const float2 m = make_float2(-12582912.0f, -12582912.0f);
+    return add2(make_float2(__int_as_float((int)(x + 0x4B400000u)), __int_as_float((int)(y + 0x4B400000u))), m);
+}
+
+// The pair sums that the common path needs, per genotype row of the i-SNP and added up over
+// the triplet of lanes that holds the three rows: sum of S^2 / n, the count (plus 65,536 times
+// the number of occupied cells: both are exact together, below 2^24) and the sum.
+struct RowSums {
+    float2 P, NF, S;
+};
+
+// A lane's accumulator row of a round, the j-SNPs 3 r .. 3 r + 2 of each half (the last three
+// where fewer are left): v[h][TY c + (1 + SCR) b + s], the count (s = 0) and the digit sums of
+// genotype b of j-SNP c
+template <class C>
+__device__ __forceinline__ int round_j(int r) { return min(3 * r, C::TJH - 3); }
+
+template <class C>
+__device__ __forceinline__ void load_round(uint32_t acc, int r, uint32_t v[2][3 * C::TY])
+{
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t col = acc + h * NH + C::TY * round_j<C>(r);
+        tc::tmem_ld16(col, v[h]);
+        if constexpr (C::SCR == 2) tc::tmem_ld8(col + 16, v[h] + 16);
+        tc::tmem_ld2(col + 3 * C::TY - 2 - C::SCR / 2, v[h] + 3 * C::TY - 2 - C::SCR / 2);
+        if constexpr (C::SCR == 2) tc::tmem_ld1(col + 26, v[h][26]);
+    }
+    tc::tmem_wait_ld();
+}
+
+// The count and the sum (about the trait's mean) of a cell, of the pairs of both halves
+template <class C>
+__device__ __forceinline__ void cell2(const uint32_t v[2][3 * C::TY], int k, float2 md0, float2 &n, float2 &S)
+{
+    n = int_float2(v[0][k], v[1][k]);
+    S = int_float2(v[0][k + 1], v[1][k + 1]);
+    if constexpr (C::SCR == 2) S = fma2(S, make_float2(256.0f, 256.0f), int_float2(v[0][k + 2], v[1][k + 2]));
+    else S = fma2(md0, n, S);  // exactly 0 in an empty cell
+}
+
+// 2 X - R - C - M of the lane's pair in half h: SSI_D = P + this (all nine cells, gathered
+// from the triplet's rows; the rows' order does not matter)
+template <class C>
+__device__ __forceinline__ float interaction(const uint32_t v[3 * C::TY], float d0, int ga, int s1, int s2)
+{
+    const int o1 = (ga + 2) % 3, o2 = (ga + 1) % 3;  // the columns this lane offers the others
+    float n[9], S[9];
+#pragma unroll
+    for (int q = 0; q < C::TY; ++q) {
+        const uint32_t x0 = v[q], x1 = v[C::TY + q], x2 = v[2 * C::TY + q];
+        const uint32_t w[3] = {pick3(x0, x1, x2, ga), __shfl_sync(0xffffffffu, pick3(x0, x1, x2, o1), s1),
+                               __shfl_sync(0xffffffffu, pick3(x0, x1, x2, o2), s2)};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int cell = 3 * k + q / (1 + C::SCR), s = q % (1 + C::SCR);
+            const float f = (float)(int)w[k];
+            if (s == 0) n[cell] = f;
+            else if (C::SCR == 1) S[cell] = fmaf(-d0, n[cell], f);
+            else S[cell] = s == 1 ? 256.0f * f : S[cell] + f;
+        }
+    }
+    float cb[3], N = 0.f, St = 0.f, RC = 0.f, X = 0.f;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+        const float nb = n[b] + n[3 + b] + n[6 + b], Sb = S[b] + S[3 + b] + S[6 + b];
+        cb[b] = Sb * rcp_fast(nb + 1e-30f);
+        RC = fmaf(Sb, cb[b], RC);
+        N += nb;
+        St += Sb;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float na = n[3 * k] + n[3 * k + 1] + n[3 * k + 2], Sa = S[3 * k] + S[3 * k + 1] + S[3 * k + 2];
+        const float ra = Sa * rcp_fast(na + 1e-30f);
+        RC = fmaf(Sa, ra, RC);
+        X = fmaf(ra, fmaf(n[3 * k + 2], cb[2], fmaf(n[3 * k + 1], cb[1], n[3 * k] * cb[0])), X);
+    }
+    return fmaf(2.0f, X, -RC) - St * St * rcp_fast(N + 1e-30f);
+}
+
+// One warp of the epilogue: its j rounds of every unit. A round is three j-SNPs of each B half
+// (columns 18 r of either half), so a lane forms the pairs (i, j0 + 3 r + ga) and
+// (i, j0 + 21 + 3 r + ga), the two halves side by side in packed FP32 (f32x2) operations. SSI
+// is at most SSB (the map above has norm <= 1 on the cells' means), so one sum over the cells
+// settles both tests for all but a few pairs in a thousand: each lane forms the sums of its own
+// genotype row for the three j-SNPs and the triplet adds them up, three values a pair instead of
+// twelve; all nine cells meet in one lane only where a pair passes (the columns are read again).
+template <class C>
+__device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::Smem &sm, uint32_t tmem, uint32_t rank,
+                                                int pair, int npairs)
+{
+    constexpr int EPW = C::EPW;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int *abort = &sm.abort;
+    const int e = warp & 3, grp = warp < 4 ? 0 : (warp < 12 ? 1 : 2);
+    constexpr int RND = (C::TJH + 2) / 3;
+    const int r_begin = (grp * RND + EPW - 1) / EPW, r_end = ((grp + 1) * RND + EPW - 1) / EPW;
+    const int ii = 10 * e + lane / 3, ga = lane % 3, tbase = (lane / 3) * 3;
+    const int s1 = tbase + (ga + 1) % 3, s2 = tbase + (ga + 2) % 3;  // the triplet's other rows
+    const bool is1 = ga == 1, is2 = ga == 2;
+    const uint32_t tl = tmem + ((uint32_t)(32 * e) << 16);
+    const bool ti = a.test_int != 0;
+    const float t1c = screen_lo(a.t1), t2c = screen_lo(a.t2);
+    uint32_t accph = 0u;  // bit b: the parity of accumulator b's next phase
+    int buf = 0;
+    for (Walker<C> un(a, pair, npairs); !un.done; un.next()) {
+        const int t = un.trait;
+        const int di = un.i0 + TI * (int)rank + ii;
+        const int gi = un.bd.start1 + di;
+        const bool ivalid = lane < 30 && di < un.bd.size1;
+        const float4 ts = a.tscr[2 * t + C::SCR - 1];
+        const float d0 = ts.x, E = ts.y, qtot = ts.z, s2y = ts.w;
+        const float *qmf = a.qmf + (size_t)t * a.nsnp;
+        const float qmi = ivalid ? s2y * qmf[gi] : 0.0f;
+        const bool report = a.report_trait < 0 || a.report_trait == t;
+        unsigned int lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
+        unsigned int lI = ti ? reinterpret_cast<volatile unsigned int *>(a.lowf2)[t] : 0u;
+        auto threshold = [&](unsigned int low, float tc) {
+            const float l = screen_lo(ord2f(low));
+            return report ? fminf(tc, l) : l;
+        };
+        float tF = threshold(lF, t1c), tI = ti ? 4.0f * threshold(lI, t2c) : INFINITY;
+        // SSY >= Q - (sqrt(M) + E)^2 >= Q - 2 M - 2 E^2
+        const float qi = qtot - qmi - 2.0f * E * E;
+        if (!tc::mbar_wait(&sm.acc_full[buf], (accph >> buf) & 1u, abort, a.wait_ns)) {
+            fail(a, sm, 3);
+            break;
+        }
+        tc::tc_fence_after();
+        const uint32_t acc = tl + acc_col(buf);
+        // Nothing is known of the trait's maxima yet (its first units, which every cluster begins
+        // at once): the rounds run twice, first only to raise the lower bounds. Listing pairs in
+        // that pass would list a tenth of them.
+        bool seed = lF == ENC_NEG_INF || (ti && lI == ENC_NEG_INF);
+#pragma unroll 1
+        for (int r = r_begin; r < r_end; ++r) {
+            const int dj = un.j0 + round_j<C>(r) + ga, gj = un.bd.start2 + dj;
+            bool valid[2];
+            float qmj[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                valid[h] = ivalid && dj + C::TJH * h < un.bd.size2 && gi > gj + C::TJH * h;
+                // (the last round takes in the j-SNPs of the one before where three do not divide)
+                if (C::TJH % 3 != 0) valid[h] = valid[h] && round_j<C>(r) + ga >= 3 * r;
+                qmj[h] = valid[h] ? s2y * qmf[gj + C::TJH * h] : 0.0f;
+            }
+            uint32_t v[2][3 * C::TY];
+            load_round<C>(acc, r, v);
+            const float2 tiny = make_float2(1e-30f, 1e-30f), md0 = make_float2(-d0, -d0);
+            const float2 k64 = make_float2(65536.0f, 65536.0f);
+            RowSums w[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                float2 nf = make_float2(0.f, 0.f), n = nf;
+                w[c].P = w[c].S = nf;
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    float2 nb, Sb;
+                    cell2<C>(v, C::TY * c + (1 + C::SCR) * b, md0, nb, Sb);
+                    w[c].P = fma2(Sb, mul2(Sb, rcp2(add2(nb, tiny))), w[c].P);
+                    w[c].S = add2(w[c].S, Sb);
+                    n = add2(n, nb);
+                    nf = add2(nf, make_float2(__saturatef(nb.x), __saturatef(nb.y)));
+                }
+                w[c].NF = fma2(nf, k64, n);
+            }
+            // the pair (i, j-SNP c = ga) is this lane's: each lane adds what the triplet's other
+            // two offer it, the lane of row ga + 1 its column (ga + 1) + 2 = ga (mod 3)
+            auto gather = [&](float x0, float x1, float x2) {
+                const float own = is1 ? x1 : is2 ? x2 : x0;
+                const float for1 = is1 ? x0 : is2 ? x1 : x2, for2 = is1 ? x2 : is2 ? x0 : x1;
+                return own + __shfl_sync(0xffffffffu, for1, s1) + __shfl_sync(0xffffffffu, for2, s2);
+            };
+            bool cand[2];
+            float P[2], M[2], d1[2], d2[2], uB[2], W[2];
+            bool any = false;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                auto x = [&](const float2 &y) { return h ? y.y : y.x; };
+                P[h] = gather(x(w[0].P), x(w[1].P), x(w[2].P));
+                const float St = gather(x(w[0].S), x(w[1].S), x(w[2].S));
+                const float NF = gather(x(w[0].NF), x(w[1].NF), x(w[2].NF));
+                // NF = 65536 nfac + N with N < 32768: nfac by rounding to the nearest integer
+                const float nf = fmaf(NF, 1.0f / 65536.0f, 12582912.0f) - 12582912.0f;
+                const float N = fmaf(-65536.0f, nf, NF);
+                M[h] = St * St * rcp_fast(N + 1e-30f);
+                d1[h] = nf - 1.0f;
+                d2[h] = N - nf;
+                // upper bound of SSB, lower bounds of SSY and SSW
+                const float sB = sqrt_fast(fmaxf(fmaf(P[h], 1.0f + SLK_B, -M[h]), 0.0f)) + E;
+                const float Y = fmaf(-2.0f, M[h], qi - qmj[h]);
+                uB[h] = sB * sB;
+                W[h] = Y - uB[h];
+                const float lhs = uB[h] * d2[h];
+                // one occupied cell: F is 0/0, never a hit or a maximum (F2 is 0); no individual:
+                // neither is defined. W too small a part of Y to be told from rounding: unknown
+                cand[h] = valid[h] && ((d1[h] > 0.0f && !(lhs <= tF * d1[h] * W[h])) ||
+                                       (d1[h] >= 0.0f && (!(W[h] > 1e-3f * Y) || !(lhs <= tI * W[h]))));
+                cand[h] = cand[h] && (ti || d1[h] > 0.0f);
+                W[h] = W[h] > 1e-3f * Y ? W[h] : __int_as_float(0x7fc00000);
+                any = any || cand[h];
+            }
+            if (__any_sync(0xffffffffu, any)) {
+                // raise the lower bounds of the maxima by this round's pairs first, then list the
+                // pairs that still matter
+                if (ti) load_round<C>(acc, r, v);
+                float fu[2], f2u[2];
+                unsigned int bF = 0u, bI = 0u;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float I0 = ti ? interaction<C>(v[h], d0, ga, s1, s2) : 0.0f;
+                    const float sI = sqrt_fast(fmaxf(fmaf(P[h], 1.0f + SLK_I, I0), 0.0f)) + E;
+                    fu[h] = d1[h] > 0.0f ? uB[h] * d2[h] / (d1[h] * W[h]) : -INFINITY;
+                    f2u[h] = ti ? sI * sI * d2[h] / (4.0f * W[h]) : -INFINITY;
+                    const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(P[h], 1.0f - SLK_B, -M[h]), 0.0f)) - E, 0.0f);
+                    const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(P[h], 1.0f - SLK_I, I0), 0.0f)) - E, 0.0f);
+                    const float Wu = (qtot - fmaxf(qmi, qmj[h])) - lB * lB;  // SSW <= Q - SSB
+                    if (cand[h] && W[h] == W[h] && Wu > 0.0f) {
+                        if (d1[h] > 0.0f) bF = max(bF, f2ord(screen_lo(lB * lB * d2[h] / (d1[h] * Wu))));
+                        if (ti) bI = max(bI, f2ord(screen_lo(lo * lo * d2[h] / (4.0f * Wu))));
+                    }
+                }
+                bF = __reduce_max_sync(0xffffffffu, bF);
+                bI = __reduce_max_sync(0xffffffffu, bI);
+                if (bF > lF) {
+                    lF = bF;
+                    tF = threshold(lF, t1c);
+                    if (lane == 0) atomicMax(&a.lowf[t], lF);
+                }
+                if (ti && bI > lI) {
+                    lI = bI;
+                    tI = 4.0f * threshold(lI, t2c);
+                    if (lane == 0) atomicMax(&a.lowf2[t], lI);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const bool c = cand[h] && !seed && (!(fu[h] <= tF) || !(4.0f * f2u[h] <= tI));
+                    const unsigned int mask = __ballot_sync(0xffffffffu, c);
+                    if (!mask) continue;
+                    const int leader = __ffs(mask) - 1;
+                    unsigned long long base = 0ull;
+                    if (lane == leader)
+                        base = atomicAdd(&a.counters[CNT_CAND + a.segment], (unsigned long long)__popc(mask));
+                    base = __shfl_sync(0xffffffffu, base, leader) + __popc(mask & ((1u << lane) - 1u));
+                    if (c && (long long)base < a.cand_cap)
+                        a.cand[base] = Cand{gi, gj + C::TJH * h, t, un.block, fu[h], f2u[h]};
+                }
+            }
+            if (seed && r + 1 == r_end) {
+                seed = false;
+                r = r_begin - 1;
+                lF = max(lF, reinterpret_cast<volatile unsigned int *>(a.lowf)[t]);
+                tF = threshold(lF, t1c);
+                if (ti) {
+                    lI = max(lI, reinterpret_cast<volatile unsigned int *>(a.lowf2)[t]);
+                    tI = 4.0f * threshold(lI, t2c);
+                }
+            }
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (rank == 0) tc::mbar_arrive(&sm.acc_empty[buf]);
+            else tc::mbar_arrive_remote(&sm.acc_empty[buf], 0);
+        }
+        accph ^= 1u << buf;
+        buf ^= 1;
     }
 }
 
@@ -386,9 +669,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw + (((raw_s + 1023u) & ~1023u) - raw_s));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = tc::cluster_rank();  // 0: issues the MMAs
-    const long long pair = tc::cluster_id(), npairs = tc::cluster_count();
-    const long long units = a.ntiles * (long long)a.ntraits;
+    const int pair = (int)tc::cluster_id(), npairs = (int)tc::cluster_count();
     const int nks = a.Np / KS;
+    // an earlier segment's candidates did not fit: the host scans again without the screen (the
+    // flag is written between the segments' kernels only, so every thread reads the same)
+    if (C::SCR && a.counters[CNT_OVERFLOW]) return;
 
     if (warp == 12) {
         tc::tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);
@@ -450,12 +735,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
         // the ring positions of the others without touching them)
         const int pg = warp >= 16 ? 1 : 0;
         const int t = threadIdx.x - (pg ? 512 : 128), jj = t >> 3, c = t & 7;
-        const bool xtra = t < XTRA;
+        const bool xtra = C::TJH > 16 && t < XTRA, mine = jj < C::TJH;
+        constexpr int DG = C::SCR ? 1 + C::SCR : 2;  // digit rows of this CTA's half
         uint32_t stage = 0, phase = 0, rs = 0, rph = 0, seq = 0;
         bool ok = true;
-        for (long long u = pair; u < units && ok; u += npairs) {
-            const Unit un = decode<C::XF>(a, u);
-            if (un.skip) continue;
+        for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
             for (int ks = 0; ks < nks; ++ks) {
                 if ((int)(seq++ % (uint32_t)PW) != pg) {
                     advance<STAGES>(stage, phase);
@@ -469,13 +753,16 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 }
                 const uint8_t *raw = sm.raw[rs];
                 uint8_t *base = sm.b[stage];
-                // this CTA's two digit rows: 2 rank and 2 rank + 1
-                const uint4 d[2] = {ld_sw128(raw + RAW_D, 2 * (int)rank, c), ld_sw128(raw + RAW_D, 2 * (int)rank + 1, c)};
-                // local type q = 2b + s' (genotype b, this CTA's digit row s') of j-SNP jx at
-                // local row 6 jx + q
+                // the digit rows of this CTA's half: all digits -- 2 rank and 2 rank + 1 of w, d2,
+                // d1, d0; one digit -- w and D of the rows D, w; two -- w, d2, d1
+                uint4 d[DG];
+#pragma unroll
+                for (int r = 0; r < DG; ++r)
+                    d[r] = ld_sw128(raw + RAW_D, C::SCR == 0 ? 2 * (int)rank + r : C::SCR == 1 ? 1 - r : r, c);
+                // local type q = DG b + r (genotype b, digit row r) of j-SNP jx at local row TY jx + q
                 auto put = [&](int q, int jx, const uint4 &m) {
-                    const int n = 6 * jx + q;
-                    const uint4 &dv = d[q & 1];
+                    const int n = C::TY * jx + q;
+                    const uint4 &dv = d[q % DG];
                     uint4 o;
                     o.x = m.x & dv.x;
                     o.y = m.y & dv.y;
@@ -497,11 +784,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
 #pragma unroll
                     for (int b = 0; b < 3; ++b) {
                         const uint4 m = gmask(h, b);
-                        put(2 * b, jx, m);
-                        put(2 * b + 1, jx, m);
+#pragma unroll
+                        for (int r = 0; r < DG; ++r) put(DG * b + r, jx, m);
                     }
                 };
-                build(jj);
+                if (mine) build(jj);
                 if (xtra) build(16 + jj);
                 // the raw slot is released only after the stores above, which consume every
                 // value loaded from it (an arrive right after the loads can overtake them)
@@ -516,6 +803,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 advance<RSTAGES>(rs, rph);
             }
         }
+    } else if (C::SCR && epi_warp) {
+        screen_epilogue<C>(a, sm, tmem, rank, pair, npairs);
     } else if (epi_warp) {
         // ---------------- epilogue: the j rounds split over the warps of each lane quarter ----------------
         // warps 0-3 (group 0), 8-11 (group 1), 16-19 (group 2): rounds [rb(g), rb(g + 1))
@@ -526,13 +815,10 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
         const uint32_t tl = tmem + ((uint32_t)(32 * e) << 16);
         uint32_t accph[2] = {0u, 0u};
         int buf = 0;
-        for (long long u = pair; u < units; u += npairs) {
-            Unit un = decode<C::XF>(a, u);
-            if (un.skip) continue;
-            un.i0 += TI * (int)rank;  // this CTA's i-SNPs
+        for (Walker<C> un(a, pair, npairs); !un.done; un.next()) {
             const int t = un.trait;
             const double sc = a.yscale[t];
-            const int di = un.i0 + ii;
+            const int di = un.i0 + TI * (int)rank + ii;  // this CTA's i-SNPs
             const bool ivalid = rowok && di < un.bd.size1;
             const int gi = un.bd.start1 + (ivalid ? di : 0);
             const size_t mi = (size_t)t * a.nsnp + gi;
@@ -594,8 +880,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
 #pragma unroll
                     for (int b = 0; b < 3; ++b) {
                         cn[c][b] = (int)v[4 * b][c];
-                        cs[c][b] = fmaf(65536.0f, (float)(int)v[4 * b + 3][c],
-                                        fmaf(256.0f, (float)(int)v[4 * b + 2][c], (float)(int)v[4 * b + 1][c]));
+                        cs[c][b] = fmaf(65536.0f, (float)(int)v[4 * b + 1][c],
+                                        fmaf(256.0f, (float)(int)v[4 * b + 2][c], (float)(int)v[4 * b + 3][c]));
                     }
                 }
                 // the pair (SNP i, j-SNP jb + ga) is this lane's: its own row directly, the rows of
@@ -661,9 +947,9 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                         double st = 0.0;
 #pragma unroll
                         for (int b = 0; b < 3; ++b) {
-                            const uint32_t c1[3] = {sel3(v[4 * b + 1], ga), r1[4 * b + 1], r2[4 * b + 1]};
+                            const uint32_t c3[3] = {sel3(v[4 * b + 1], ga), r1[4 * b + 1], r2[4 * b + 1]};
                             const uint32_t c2[3] = {sel3(v[4 * b + 2], ga), r1[4 * b + 2], r2[4 * b + 2]};
-                            const uint32_t c3[3] = {sel3(v[4 * b + 3], ga), r1[4 * b + 3], r2[4 * b + 3]};
+                            const uint32_t c1[3] = {sel3(v[4 * b + 3], ga), r1[4 * b + 3], r2[4 * b + 3]};
 #pragma unroll
                             for (int r = 0; r < 3; ++r) {
                                 si[3 * r + b] = fma(65536.0, (double)(int)c3[r],
@@ -686,19 +972,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                         const int src = __ffs(need) - 1;
                         need &= need - 1;
                         const int si_ = __shfl_sync(0xffffffffu, gi, src), sj_ = __shfl_sync(0xffffffffu, gj, src);
-                        const uint32_t *mbi = a.missbits + (size_t)si_ * a.Wp, *mbj = a.missbits + (size_t)sj_ * a.Wp;
-                        const uint32_t *wm = a.wmask + (size_t)t * a.Wp;
-                        const double *qdt = a.qd + (size_t)t * a.Np;
-                        double part = 0.0;
-                        for (int w = lane; w < a.Wp; w += 32) {
-                            uint32_t bits = mbi[w] & mbj[w] & wm[w];
-                            while (bits) {
-                                part += qdt[32 * w + __ffs(bits) - 1];
-                                bits &= bits - 1;
-                            }
-                        }
-#pragma unroll
-                        for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+                        const double part = missing_both_q(a, t, si_, sj_);
                         if (lane == src) qmm = part;
                     }
                     if (exact) s = pair_stat_exact(n, si, sc, pki - qmj + qmm, a.test_int != 0);
@@ -741,11 +1015,10 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
         if (lane == 0) {
             uint32_t as = 0, aph = 0, issued_a = 0;
             bool ok = true;
-            for (long long u = pair; u < units && ok; u += npairs) {
-                const Unit un = decode<C::XF>(a, u);
-                if (un.skip) continue;
+            for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
                 const int arow = 3 * (un.bd.start1 + un.i0 + TI * (int)rank);
-                const int xrow = ((un.trait * 2 + (int)rank) * a.nsnp + un.bd.start2 + un.j0) * 6;
+                const int xrow = C::SCR ? (un.trait * a.nsnp + un.bd.start2 + un.j0 + C::TJH * (int)rank) * C::TY
+                                        : ((un.trait * 2 + (int)rank) * a.nsnp + un.bd.start2 + un.j0) * C::TY;
                 for (int ks = 0; ks < nks; ++ks) {
                     if (!tc::mbar_wait(&sm.empty[as], aph ^ 1u, abort, a.wait_ns)) {
                         fail(a, sm, 7);
@@ -780,9 +1053,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
         if (lane == 0) {
             uint32_t rs = 0, rph = 0, issued_r = 0;
             bool ok = true;
-            for (long long u = pair; u < units && ok; u += npairs) {
-                const Unit un = decode<C::XF>(a, u);
-                if (un.skip) continue;
+            for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
                 for (int ks = 0; ks < nks; ++ks) {
                     if (!tc::mbar_wait(&sm.raw_empty[rs], rph ^ 1u, abort, a.wait_ns)) {
                         fail(a, sm, 10);
@@ -790,9 +1061,15 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                         break;
                     }
                     uint8_t *raw = sm.raw[rs];
-                    tc::mbar_arrive_expect_tx(&sm.raw_full[rs], RAW_BYTES);
-                    tc::tma_load_2d(raw + RAW_J, &maps.hj, ks * KS, un.bd.start2 + un.j0, &sm.raw_full[rs]);
-                    tc::tma_load_2d(raw + RAW_D, &maps.dg, ks * KS, ND * un.trait, &sm.raw_full[rs]);
+                    tc::mbar_arrive_expect_tx(&sm.raw_full[rs], C::RAW_BYTES);
+                    tc::tma_load_2d(raw + RAW_J, C::SCR == 2 ? &maps.hj2 : &maps.hj, ks * KS,
+                                    un.bd.start2 + un.j0 + (C::SCR ? C::TJH * (int)rank : 0), &sm.raw_full[rs]);
+                    if constexpr (C::SCR == 0)
+                        tc::tma_load_2d(raw + RAW_D, &maps.dg, ks * KS, DROWS * un.trait + 1, &sm.raw_full[rs]);
+                    else if constexpr (C::SCR == 1)
+                        tc::tma_load_2d(raw + RAW_D, &maps.ds, ks * KS, DROWS * un.trait, &sm.raw_full[rs]);
+                    else
+                        tc::tma_load_2d(raw + RAW_D, &maps.ds2, ks * KS, DROWS * un.trait + 1, &sm.raw_full[rs]);
                     ++issued_r;
                     advance<RSTAGES>(rs, rph);
                 }
@@ -808,9 +1085,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
         // each of this CTA's A stages, once landed, counts as one arrival on CTA 0's full
         uint32_t as = 0, aph = 0;
         bool ok = true;
-        for (long long u = pair; u < units && ok; u += npairs) {
-            const Unit un = decode<C::XF>(a, u);
-            if (un.skip) continue;
+        for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
             for (int ks = 0; ks < nks; ++ks) {
                 if (!tc::mbar_wait(&sm.full[as], aph, abort, a.wait_ns)) {
                     fail(a, sm, 9);
@@ -832,9 +1107,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             fail(a, sm, 12);
             ok = false;
         }
-        for (long long u = pair; u < units && ok; u += npairs) {
-            const Unit un = decode<C::XF>(a, u);
-            if (un.skip) continue;
+        for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
             if (!tc::mbar_wait_cluster(&sm.acc_empty[buf], accph[buf] ^ 1u, abort, a.wait_ns)) {
                 fail(a, sm, 4);
                 break;
@@ -883,6 +1156,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
 
 }  // namespace mma
 
+using Screen2Digits = mma::Rings<6, 6, 2, 1, false, 2>;
+
 // Tensor maps of the tensor form's TMA loads: the genotype-indicator rows h3 [3 nsnp][Np]
 // with 30-row boxes (A), the one-hot genotype bytes [nsnp][Np] with 16-row boxes (j side) and
 // the trait digit rows [7T][Np] with 7-row boxes; all 128 bytes wide, 128-byte swizzled,
@@ -911,26 +1186,36 @@ cudaError_t mma_encode_genotypes(MmaMaps *maps, const uint8_t *hcodes, const uin
 {
     cudaError_t e = encode_2d(&maps->hi, h3, (uint64_t)Np, 3 * (uint64_t)nsnp, mma::A_BOX);
     if (e == cudaSuccess) e = encode_2d(&maps->hj, hcodes, (uint64_t)Np, (uint64_t)nsnp, mma::TJ);
+    if (e == cudaSuccess) e = encode_2d(&maps->hj2, hcodes, (uint64_t)Np, (uint64_t)nsnp, Screen2Digits::TJH);
     return e;
 }
 
 cudaError_t mma_encode_traits(MmaMaps *maps, const int8_t *ydig, int ntraits, int Np)
 {
-    return encode_2d(&maps->dg, ydig, (uint64_t)Np, (uint64_t)mma::ND * ntraits, mma::ND);
+    const uint64_t rows = (uint64_t)mma::DROWS * ntraits;
+    cudaError_t e = encode_2d(&maps->dg, ydig, (uint64_t)Np, rows, mma::ND);
+    if (e == cudaSuccess) e = encode_2d(&maps->ds, ydig, (uint64_t)Np, rows, 2);
+    if (e == cudaSuccess) e = encode_2d(&maps->ds2, ydig, (uint64_t)Np, rows, 3);
+    return e;
 }
 
 // The streamed-B variant's expanded rows [ntraits][2][nsnp][6][Np], in boxes of one CTA half
 // of a j tile (21 SNPs x 6 types = 126 rows)
-cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits)
+// expanded rows per SNP and trait
+int mma_x_rows(int screen) { return screen ? 3 * (1 + screen) : mma::NTYPE; }
+
+cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits, int screen)
 {
-    return encode_2d(&maps->hx, x, (uint64_t)Np, 12 * (uint64_t)nsnp * ntraits, 6 * mma::TJ);
+    return encode_2d(&maps->hx, x, (uint64_t)Np, (uint64_t)mma_x_rows(screen) * nsnp * ntraits, mma::TYH * mma::TJ);
 }
 
 bool mma_available() { return true; }
 int mma_tile_i() { return mma::TIP; }  // the host tiles blocks by CTA-pair tiles
-int mma_tile_j() { return mma::TJ; }
+int mma_tile_j(int screen) { return screen == 0 ? mma::TJ : screen == 1 ? 2 * mma::TJ : Screen2Digits::TJT; }
 int mma_min_nid() { return 256; }
 int mma_max_nid() { return 1 << 24; }  // digit sums stay within int32
+// the screen's sums (127 per individual) stay below 2^22, its counts below 2^15
+int mma_screen_max_nid() { return (1 << 15) - mma::KS; }
 int mma_stage_individuals() { return mma::KS; }
 
 // The variants the autotuner chooses among -- operand slots and raw stages (each ~200-216 KB
@@ -938,13 +1223,16 @@ int mma_stage_individuals() { return mma::KS; }
 //   0  6 slots / 6 raw, 2 epilogue warps   1  5 / 10, 2   2  6 / 4, 2   3  6 / 6, 3
 //   4  6 / 6, 2 epilogue warps, two producer groups on alternate stages
 //   5  6 slots, streamed B (expanded rows TMA-loaded from HBM; no producers, no raw ring)
-using Rings0 = mma::Rings<6, 6>;
-using Rings1 = mma::Rings<5, 10>;
-using Rings2 = mma::Rings<6, 4>;
-using Rings3 = mma::Rings<6, 6, 3>;
-using Rings4 = mma::Rings<6, 6, 2, 2>;
-using Rings5 = mma::Rings<6, 1, 2, 1, true>;
 constexpr int MMA_SHAPES = 6;
+// variant v with SCR digits in the screen (0: all digits)
+template <int V, int SCR>
+struct VariantOf;
+template <int SCR> struct VariantOf<0, SCR> { using type = mma::Rings<6, 6, 2, 1, false, SCR>; };
+template <int SCR> struct VariantOf<1, SCR> { using type = mma::Rings<5, 10, 2, 1, false, SCR>; };
+template <int SCR> struct VariantOf<2, SCR> { using type = mma::Rings<6, 4, 2, 1, false, SCR>; };
+template <int SCR> struct VariantOf<3, SCR> { using type = mma::Rings<6, 6, 3, 1, false, SCR>; };
+template <int SCR> struct VariantOf<4, SCR> { using type = mma::Rings<6, 6, 2, 2, false, SCR>; };
+template <int SCR> struct VariantOf<5, SCR> { using type = mma::Rings<6, 1, 2, 1, true, SCR>; };
 
 bool mma_needs_x(int v) { return v == 5; }
 
@@ -1031,34 +1319,47 @@ static cudaError_t enqueue(const ScanArgs &a, const MmaMaps &maps, int grid, cud
     return cudaGetLastError();
 }
 
-// The launch shape of a scan with variant v, resolved before any stream capture: the kernel's
-// shared-memory attribute and the number of co-resident clusters, then whole clusters of two --
-// at least one, never more than can be resident at once.
-cudaError_t mma_prepare(int v, int ntraits, int grid_request, int *grid)
+// f(VariantOf<v, screen>())
+template <int SCR, class F>
+static cudaError_t with_rings(int v, F f)
 {
     switch (v) {
-    case 0: return prepare<Rings0>(v, ntraits, grid_request, grid);
-    case 1: return prepare<Rings1>(v, ntraits, grid_request, grid);
-    case 2: return prepare<Rings2>(v, ntraits, grid_request, grid);
-    case 3: return prepare<Rings3>(v, ntraits, grid_request, grid);
-    case 4: return prepare<Rings4>(v, ntraits, grid_request, grid);
-    case 5: return prepare<Rings5>(v, ntraits, grid_request, grid);
+    case 0: return f(VariantOf<0, SCR>());
+    case 1: return f(VariantOf<1, SCR>());
+    case 2: return f(VariantOf<2, SCR>());
+    case 3: return f(VariantOf<3, SCR>());
+    case 4: return f(VariantOf<4, SCR>());
+    case 5: return f(VariantOf<5, SCR>());
     }
     return cudaErrorInvalidValue;
 }
 
-// The launch itself (a stream operation only, so it can be captured into a CUDA graph).
-cudaError_t mma_enqueue(int v, const ScanArgs &a, const MmaMaps &maps, int grid, cudaStream_t stream)
+template <class F>
+static cudaError_t with_variant(int v, int screen, F f)
 {
-    switch (v) {
-    case 0: return enqueue<Rings0>(a, maps, grid, stream);
-    case 1: return enqueue<Rings1>(a, maps, grid, stream);
-    case 2: return enqueue<Rings2>(a, maps, grid, stream);
-    case 3: return enqueue<Rings3>(a, maps, grid, stream);
-    case 4: return enqueue<Rings4>(a, maps, grid, stream);
-    case 5: return enqueue<Rings5>(a, maps, grid, stream);
+    switch (screen) {
+    case 0: return with_rings<0>(v, f);
+    case 1: return with_rings<1>(v, f);
+    case 2: return with_rings<2>(v, f);
     }
     return cudaErrorInvalidValue;
+}
+
+// The launch shape of a scan with variant v, resolved before any stream capture: the kernel's
+// shared-memory attribute and the number of co-resident clusters, then whole clusters of two --
+// at least one, never more than can be resident at once.
+cudaError_t mma_prepare(int v, int screen, int ntraits, int grid_request, int *grid)
+{
+    return with_variant(v, screen, [&](auto c) {
+        return prepare<typename decltype(c)::type>(v + MMA_SHAPES * screen, ntraits, grid_request, grid);
+    });
+}
+
+// The launch itself (a stream operation only, so it can be captured into a CUDA graph).
+cudaError_t mma_enqueue(int v, int screen, const ScanArgs &a, const MmaMaps &maps, int grid, cudaStream_t stream)
+{
+    return with_variant(v, screen,
+                        [&](auto c) { return enqueue<typename decltype(c)::type>(a, maps, grid, stream); });
 }
 
 }  // namespace epi

@@ -1,0 +1,115 @@
+"""The screened scan of the tensor form (8-bit phenotype bounds, then the exact statistics of
+the pairs that pass) against the same library's per-pair dump, which goes through the full
+digits: the same hits, F and F2 and the same largest F and F2, bit for bit, at the edges of its
+tiles (80 x 42 SNPs), of the packed layouts (128 individuals a stage) and of its range (thresholds
+and individuals where it turns to the full digits), over several blocks, traits and masks; and
+where the candidate list overflows, since the traits make nearly every pair a hit."""
+import numpy as np
+import pytest
+
+from epigpu_b200 import capi, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _expected(ctx, blocks, t, test, t1, t2):
+    """Hits (as a set of rows) and maxima of trait t from the dump of every block."""
+    rows, mf, mf2 = set(), -np.inf, -np.inf
+    for b, (s1, m1, s2, m2) in enumerate(blocks):
+        d = ctx.scan_dump((s1, m1, s2, m2), capi.default_opts(test=test, t1=t1, t2=t2, form=capi.FORM_TENSOR), trait=t)
+        tri = (np.arange(m1)[:, None] + s1) > (np.arange(m2)[None, :] + s2)
+        F, F2 = d["F"], d["F2"]
+        with np.errstate(invalid="ignore"):
+            hit = (F > np.float32(t1)) & tri if test == "f" else \
+                ((F > np.float32(t1)) | (F2 > np.float32(t2))) & (d["df1"] > 5) & tri
+        for i, j in zip(*np.nonzero(hit)):
+            rows.add((t, b, i + s1, j + s2, d["df1"][i, j], d["df2"][i, j], F[i, j], F2[i, j] if test == "i" else 0.0))
+        ok = tri & ~np.isnan(F)
+        if ok.any():
+            mf = max(mf, F[ok].max())
+        ok = tri & ~np.isnan(F2)
+        if test == "i" and ok.any():
+            mf2 = max(mf2, F2[ok].max())
+    return rows, mf, (mf2 if test == "i" else 0.0)
+
+
+def _check(ctx, blocks, ntraits, test, t1, t2, tile=0, screened=None):
+    opts = capi.default_opts(test=test, t1=t1, t2=t2, form=capi.FORM_TENSOR, report_trait=-1, tile_config=tile)
+    hits, total, ex = ctx.scan(blocks, opts, ntraits=ntraits, want_blocks=True, want_traits=True)
+    if screened is not None:  # the state reset, the screen and the exact kernel, or the reset and one kernel
+        assert (ctx.last_timing()[2] >= 3) == screened
+    got = set(zip(ex["trait"], ex["block"], hits["snp1"], hits["snp2"], hits["df1"], hits["df2"], hits["F"], hits["F2"]))
+    want = set()
+    for t in range(ntraits):
+        rows, mf, mf2 = _expected(ctx, blocks, t, test, t1, t2)
+        want |= rows
+        assert ex["max_f"][t] == np.float32(mf) and ex["max_f2"][t] == np.float32(mf2), t
+    assert total == len(hits) == len(got) and got == want
+    return total
+
+
+def _load(ctx, nid, sizes, ntraits, seed, miss=0.01, masks=True):
+    nsnp = sum(sizes)
+    codes = synth.genotype_codes(nid, nsnp, seed=seed, miss=miss)
+    if nsnp > 20:
+        codes[3], codes[7], codes[11] = 0, 3, 2   # monomorphic, all missing, monomorphic
+    rng = np.random.default_rng(seed + 1)
+    pairs = [tuple(rng.choice(nsnp, 2, replace=False)) for _ in range(2)]
+    cols = []
+    for t in range(ntraits):
+        y = synth.planted_phenotype(codes, pairs, seed=seed + 10 + t, var_frac=min(0.3, 60.0 / nid), miss=0.0)
+        cols.append(y if t % 2 == 0 else np.exp(y).astype(np.float32))  # every second one skewed
+    valid = rng.random((nid, ntraits)) >= (0.03 if masks else 0.0)
+    ctx.load_packed(synth.pack(codes), nid)
+    ctx.set_traits(np.stack(cols, 1), valid)
+    starts = np.concatenate([[0], np.cumsum(sizes)[:-1]])
+    return [(int(starts[i]), sizes[i], int(starts[j]), sizes[j]) for i in range(len(sizes)) for j in range(i + 1)]
+
+
+@pytest.mark.parametrize("nid", [256, 257, 511, 1153])
+@pytest.mark.parametrize("sizes", [[2], [42], [43, 80], [81, 85, 1], [167, 121]], ids=str)
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_tile_edges(gpu_ctx, nid, sizes, test):
+    blocks = _load(gpu_ctx, nid, sizes, 2, seed=nid + len(sizes))
+    t1, t2 = synth.f_threshold(8, nid - 9, 1e-6), synth.f_threshold(4, nid - 9, 1e-6)
+    _check(gpu_ctx, blocks, 2, test, t1, t2, screened=True)
+
+
+@pytest.mark.parametrize("tile", [1, 2, 3, 4, 5, 6])
+def test_variants_and_maxima(gpu_ctx, tile):
+    """Every kernel variant with one digit and with two (15,000 individuals); thresholds out of reach, so that the maxima alone drive the screen."""
+    for nid, p in ((1500, 1e-5), (15000, 1e-5)):
+        blocks = _load(gpu_ctx, nid, [190, 93], 3, seed=5)
+        assert _check(gpu_ctx, blocks, 3, "i", synth.f_threshold(8, nid - 9, p), synth.f_threshold(4, nid - 9, p), tile) > 0
+        assert _check(gpu_ctx, blocks, 3, "i", 1e6, 1e6, tile) == 0
+
+
+@pytest.mark.parametrize("nid,screened", [(6017, True), (12200, None), (32641, False)])
+def test_many_individuals(gpu_ctx, nid, screened):
+    blocks = _load(gpu_ctx, nid, [300, 41], 1, seed=nid, miss=0.02)
+    p = 1e-6 if nid < 10000 else 1e-9  # (12,200: two digits)
+    _check(gpu_ctx, blocks, 1, "i", synth.f_threshold(8, nid - 9, p), synth.f_threshold(4, nid - 9, p), screened=screened)
+
+
+def test_thresholds_that_let_many_through_are_not_screened(gpu_ctx):
+    blocks = _load(gpu_ctx, 900, [500], 1, seed=77)
+    for p, screened in ((1e-2, False), (1e-6, True)):
+        _check(gpu_ctx, blocks, 1, "i", synth.f_threshold(8, 891, p), synth.f_threshold(4, 891, p), screened=screened)
+
+
+def test_candidate_list_overflow():
+    """SNPs in strong linkage disequilibrium with a causal one: nearly every pair passes, more than
+    the list holds, and the scan is made again with the full digits; the next is not screened."""
+    nid, nsnp = 600, 600
+    codes = synth.genotype_codes(nid, nsnp, seed=91, miss=0.0)
+    rng = np.random.default_rng(92)
+    codes = np.where(rng.random((nsnp, nid)) < 0.7, codes[:1], codes).astype(np.uint8)
+    y = (codes[0] + 0.5 * rng.standard_normal(nid)).astype(np.float32)
+    t1 = synth.f_threshold(8, nid - 9, 1e-6)
+    blocks = [(0, nsnp, 0, nsnp)]
+    with capi.Context(0) as ctx:  # a new one: its list has the smallest capacity
+        ctx.load_packed(synth.pack(codes), nid)
+        ctx.set_traits(y)
+        total = _check(ctx, blocks, 1, "f", t1, 0.0, screened=False)
+        assert total > 1 << 16
+        assert _check(ctx, blocks, 1, "f", t1, 0.0, screened=False) == total
