@@ -26,6 +26,8 @@ cudaError_t launch_unpack(const int32_t *raw, int nsnp, int nid, int npack, int 
 cudaError_t launch_qmiss(const uint32_t *missbits, int nsnp, int Wp, const uint32_t *wmask, const double *qd,
                         const double *qr, int Np, int ntraits, double *qm, double *rm, double *nm,
                         float *qmf, cudaStream_t stream);
+cudaError_t launch_traits(const float *yraw, const uint8_t *valid, int mode, int nid, int Np, int ntraits,
+                          const TraitArrays &o, TraitInfo *info, cudaStream_t stream);
 cudaError_t launch_major(const uint4 *planes, int nsnp, int Wp, uint8_t *maj, cudaStream_t stream);
 cudaError_t launch_marg(const uint4 *planes, int nsnp, int Wp, const float *y, const uint32_t *wmask, int Np,
                         int ntraits, double *pmC, int32_t *pmN, double *pmQ, cudaStream_t stream);
@@ -70,7 +72,6 @@ using epi::DevHit;
 struct epi_ctx {
     int device = -1;
     int sm_count = 0;
-    char name[256] = {0};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // genotypes
@@ -86,37 +87,43 @@ struct epi_ctx {
     epi::PopcMaps pmaps;
     // traits
     int ntraits = 0, traits_nid = 0;
-    float *d_y = nullptr, *d_q = nullptr;
+    float *d_y = nullptr, *d_yraw = nullptr;  // centred, and as given
+    uint8_t *d_yvalid = nullptr;
     uint32_t *d_wmask = nullptr;
-    double *d_qc = nullptr, *d_yscale = nullptr, *d_qd = nullptr, *d_qtot = nullptr, *d_qm = nullptr;
+    double *d_yscale = nullptr, *d_qd = nullptr, *d_qtot = nullptr, *d_qm = nullptr;
     int8_t *d_ydig = nullptr;
-    size_t traits_cap = 0, ydig_cap = 0, qd_cap = 0, qm_cap = 0, wmask_cap = 0, qc_cap = 0, qtot_cap = 0,
+    size_t y_cap = 0, yraw_cap = 0, yvalid_cap = 0, ydig_cap = 0, qd_cap = 0, qm_cap = 0, wmask_cap = 0, qtot_cap = 0,
            yscale_cap = 0;
     bool qm_valid = false;
     epi::MmaMaps maps;
     // tensor form, streamed-B variant: the expanded B rows of every SNP and trait (12 bytes per
     // SNP, individual and trait), built on first use after each genotype or trait load
-    int8_t *d_x = nullptr;
+    int8_t *d_x = nullptr;  // (own_x below)
     size_t x_cap = 0;
     int x_valid = -1;  // -1: none, 0: of all digits, 1, 2: of the screen with that many digits
     // screened scan: constants per trait and per (trait, SNP), the candidate list; per trait
-    // E / sigma of either screen and the number of valid individuals (screen_scan); the thresholds of a scan
+    // E / sigma of either screen and the number of valid individuals (pinned, written by k_traits;
+    // screen_digits); the thresholds of a scan
     // whose candidates did not fit the list (no scan at these or lower ones is screened again
     // until other genotypes or traits are loaded)
     float4 *d_tscr = nullptr;
-    float *d_qmf = nullptr;
     epi::Cand *d_cand = nullptr;
-    size_t tscr_cap = 0, qmf_cap = 0, cand_cap = 0;
-    std::vector<double> scr_r[2], scr_nv;
+    size_t tscr_cap = 0, cand_cap = 0;
+    epi::TraitInfo *h_info = nullptr;
+    int h_info_cap = 0;
     bool scr_full = false;
     float scr_full_t1 = 0.0f, scr_full_t2 = 0.0f;
-    std::vector<double> qc;
     // plain form: marginals per (trait, SNP) and the sum of y^2 per trait
     double *d_pmC = nullptr, *d_pmQ = nullptr, *d_ysq = nullptr;
     int32_t *d_pmN = nullptr;
     size_t pmC_cap = 0, pmQ_cap = 0, pmN_cap = 0, ysq_cap = 0;
     bool pm_valid = false;
-    // scan scratch
+    // scan scratch. The first scan of a context takes one allocation (d_slab) for its hits, its
+    // candidates and, up to 256 MB, its expanded B rows: a cudaMalloc of a megabyte or more costs
+    // about 0.35 ms, as much as a small scan's whole pass. What outgrows its part of it gets
+    // memory of its own (own_*).
+    void *d_slab = nullptr;
+    bool own_hits = false, own_cand = false, own_x = false;
     DevHit *d_hits = nullptr;
     int64_t hit_cap = 0;
     unsigned long long *d_counters = nullptr;
@@ -124,10 +131,11 @@ struct epi_ctx {
     int maxf_cap = 0;
     BlockDesc *d_blocks = nullptr;
     int blocks_cap = 0;
-    // pinned host staging of the device part of a scan: the block schedule it uploads, the
+    // pinned host staging of the device part of a scan (parts of h_arena where they fit): the block schedule it uploads, the
     // counters and maxima it reads back
     BlockDesc *h_blocks = nullptr;
     int h_blocks_cap = 0;
+    unsigned char *h_arena = nullptr;
     unsigned long long *h_state = nullptr;  // the counters, then 2 x ntraits encoded maxima
     size_t h_state_cap = 0;
     // the device part of the last scan, captured as a CUDA graph, and what it was captured for
@@ -164,6 +172,43 @@ static epi_status set_err(epi_ctx *ctx, epi_status s, const char *fmt, ...)
                            "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);      \
         }                                                                                             \
     } while (0)
+
+// ensure() for memory that may be a part of the context's slab: that is not freed by itself.
+template <class T>
+static cudaError_t ensure_own(T **p, size_t *cap_bytes, size_t bytes, bool *own)
+{
+    if (*p && *cap_bytes >= bytes) return cudaSuccess;
+    if (*p && *own) cudaFree(*p);
+    *p = nullptr;
+    *cap_bytes = 0;
+    cudaError_t e = cudaMalloc((void **)p, bytes ? bytes : 16);
+    if (e == cudaSuccess) {
+        *cap_bytes = bytes;
+        *own = true;
+    }
+    return e;
+}
+
+// Pinned host memory of `count` elements: the arena's part for it, or an allocation of its own
+// where that is too small.
+constexpr size_t ARENA_STATE = 0, ARENA_INFO = 16384, ARENA_BLOCKS = 32768, ARENA_BYTES = 65536;
+template <class T, class N>
+static cudaError_t ensure_pinned(epi_ctx *ctx, T **p, N *cap, size_t count, size_t at, size_t end)
+{
+    if (*p && (size_t)*cap >= count) return cudaSuccess;
+    T *const part = reinterpret_cast<T *>(ctx->h_arena + at);
+    if (*p && *p != part) cudaFreeHost(*p);
+    *p = nullptr;
+    *cap = 0;
+    if (count <= (end - at) / sizeof(T)) {
+        *p = part;
+        *cap = (N)((end - at) / sizeof(T));
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaHostAlloc((void **)p, count * sizeof(T), cudaHostAllocDefault);
+    if (e == cudaSuccess) *cap = (N)count;
+    return e;
+}
 
 template <class T>
 static cudaError_t ensure(T **p, size_t *cap_bytes, size_t bytes)
@@ -217,14 +262,17 @@ epi_status epi_open(int32_t device, epi_ctx **out)
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) return EPI_E_NODEVICE;
     if (device < 0 || device >= n) return EPI_E_NODEVICE;
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return EPI_E_NODEVICE;
-    if (prop.major != 10) return EPI_E_NODEVICE;  // the library carries sm_100a code only
+    // (single attributes: the whole property structure, with the name, takes 3 ms to fill)
+    int major = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return EPI_E_NODEVICE;
+    if (major != 10) return EPI_E_NODEVICE;  // the library carries sm_100a code only
     epi_ctx *ctx = new epi_ctx();
     ctx->device = device;
-    ctx->sm_count = prop.multiProcessorCount;
-    snprintf(ctx->name, sizeof(ctx->name), "%s", prop.name);
+    ctx->sm_count = sms;
     cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&ctx->h_arena, ARENA_BYTES, cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
@@ -242,15 +290,20 @@ epi_status epi_close(epi_ctx *ctx)
     if (!ctx) return EPI_OK;
     if (ctx->device >= 0) cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    void *bufs[] = {ctx->d_raw, ctx->d_planes, ctx->d_hcodes, ctx->d_h3, ctx->d_missbits, ctx->d_y, ctx->d_q,
-                    ctx->d_wmask, ctx->d_qc, ctx->d_yscale, ctx->d_qd, ctx->d_qtot, ctx->d_qm, ctx->d_ydig,
-                    ctx->d_hits, ctx->d_counters, ctx->d_maxf, ctx->d_blocks, ctx->d_maj, ctx->d_pmC,
-                    ctx->d_pmQ, ctx->d_ysq, ctx->d_pmN, ctx->d_x, ctx->d_tscr, ctx->d_qmf, ctx->d_cand};
+    void *bufs[] = {ctx->d_raw, ctx->d_planes, ctx->d_hcodes, ctx->d_h3, ctx->d_missbits, ctx->d_y, ctx->d_yraw, ctx->d_yvalid,
+                    ctx->d_wmask, ctx->d_yscale, ctx->d_qd, ctx->d_qtot, ctx->d_qm, ctx->d_ydig,
+                    ctx->d_slab, ctx->own_hits ? ctx->d_hits : nullptr, ctx->d_counters, ctx->d_maxf, ctx->d_blocks, ctx->d_maj, ctx->d_pmC,
+                    ctx->d_pmQ, ctx->d_ysq, ctx->d_pmN, ctx->own_x ? ctx->d_x : nullptr, ctx->d_tscr,
+                    ctx->own_cand ? ctx->d_cand : nullptr};
     for (void *p : bufs)
         if (p) cudaFree(p);
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-    if (ctx->h_blocks) cudaFreeHost(ctx->h_blocks);
-    if (ctx->h_state) cudaFreeHost(ctx->h_state);
+    const auto inside = [&](const void *p) {
+        return p >= ctx->h_arena && p < ctx->h_arena + ARENA_BYTES;
+    };
+    for (void *p : {(void *)ctx->h_blocks, (void *)ctx->h_state, (void *)ctx->h_info})
+        if (p && !inside(p)) cudaFreeHost(p);
+    if (ctx->h_arena) cudaFreeHost(ctx->h_arena);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -261,7 +314,11 @@ epi_status epi_close(epi_ctx *ctx)
 epi_status epi_device_info(const epi_ctx *ctx, char *name, int32_t name_len, int32_t *sm_count)
 {
     if (!ctx) return EPI_E_INVALID;
-    if (name && name_len > 0) snprintf(name, (size_t)name_len, "%s", ctx->name);
+    if (name && name_len > 0) {
+        cudaDeviceProp prop;
+        if (cudaGetDeviceProperties(&prop, ctx->device) != cudaSuccess) return EPI_E_CUDA;
+        snprintf(name, (size_t)name_len, "%s", prop.name);
+    }
     if (sm_count) *sm_count = ctx->sm_count;
     return EPI_OK;
 }
@@ -306,7 +363,9 @@ epi_status epi_load_packed(epi_ctx *ctx, const int32_t *gpack, int32_t nid, int3
     return EPI_OK;
 }
 
-epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntraits, const uint8_t *valid)
+// The phenotype columns as given are uploaded and k_traits (prep.cu) makes all that the scans
+// need of them on the device.
+static epi_status set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntraits, const uint8_t *valid, int mode)
 {
     if (!ctx) return EPI_E_INVALID;
     if (!y || nid < 1 || ntraits < 1) return set_err(ctx, EPI_E_INVALID, "epi_set_traits: bad arguments");
@@ -315,156 +374,28 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
         return set_err(ctx, EPI_E_INVALID, "epi_set_traits: %d individuals, genotypes have %d", nid, ctx->nid);
     CK(cudaSetDevice(ctx->device));
     const int Np = ctx->Np, Wp = ctx->Wp;
-    std::vector<float> hy((size_t)ntraits * Np, 0.0f), hq((size_t)ntraits * Np, 0.0f);
-    std::vector<uint32_t> hw((size_t)ntraits * Wp, 0u);
-    ctx->qc.assign(ntraits, 0.0);
-    // Each centred trait is scaled by a power of two that brings its largest magnitude into
-    // [0.5, 1). F and F2 do not depend on the trait's scale, and a power-of-two factor is
-    // exact in binary floating point, so in the normal range every result is bit-identical
-    // to the unscaled computation; a trait in units of 1e20 or 1e-20 no longer overflows or
-    // underflows the single-precision sums of squares.
-    std::vector<double> p2s(ntraits, 1.0), ysq(ntraits, 0.0);
-    for (int t = 0; t < ntraits; ++t) {
-        const float *yt = y + (size_t)t * nid;
-        const uint8_t *vt = valid ? valid + (size_t)t * nid : nullptr;
-        double sum = 0.0;
-        long long nv = 0;
-        for (int k = 0; k < nid; ++k) {
-            const bool ok = vt ? vt[k] != 0 : yt[k] != -9.0f;
-            if (ok) {
-                sum += (double)yt[k];
-                ++nv;
-                hw[(size_t)t * Wp + k / 32] |= 1u << (k % 32);
-            }
-        }
-        const double mu = nv ? sum / (double)nv : 0.0;
-        double maxabs = 0.0;
-        for (int k = 0; k < nid; ++k)
-            if (hw[(size_t)t * Wp + k / 32] >> (k % 32) & 1u) maxabs = std::max(maxabs, std::fabs((double)yt[k] - mu));
-        const double p2 = (maxabs > 0.0 && std::isfinite(maxabs)) ? std::ldexp(1.0, -(std::ilogb(maxabs) + 1)) : 1.0;
-        p2s[t] = p2;
-        double s2 = 0.0;
-        for (int k = 0; k < nid; ++k) {
-            if (hw[(size_t)t * Wp + k / 32] >> (k % 32) & 1u) {
-                const float yc = (float)(((double)yt[k] - mu) * p2);
-                hy[(size_t)t * Np + k] = yc;
-                s2 += (double)yc * (double)yc;
-            }
-        }
-        const double c = nv ? s2 / (double)nv : 0.0;
-        ctx->qc[t] = c;
-        ysq[t] = s2;
-        for (int k = 0; k < nid; ++k) {
-            if (hw[(size_t)t * Wp + k / 32] >> (k % 32) & 1u) {
-                const double yc = hy[(size_t)t * Np + k];
-                hq[(size_t)t * Np + k] = (float)(yc * yc - c);
-            }
-        }
-    }
-    // tensor form: per valid individual the flag and three balanced base-256 digits of
-    // Y = round(y * 2^sy) (|Y| <= 8355711); hqd holds ytilde^2 = (Y 2^-sy)^2 (exact in FP64:
-    // |Y| < 2^23) and Y; hsc per trait 2^-sy, the sum of Y and the number of valid individuals;
-    // hqtot the sum of ytilde^2.
-    // (rows: the highest digit first). The screen's 8-bit phenotype in front of them: D = round(s (ytilde - c)) with c the middle of
-    // the values and s the scale that spreads them over -127..127, d0 = -s c (the D of the mean),
-    // E the norm of what the rounding leaves (scan_mma.cu).
-    constexpr int ND = 5;
-    std::vector<float4> hts(2 * (size_t)ntraits);
-    ctx->scr_r[0].assign(ntraits, 0.0);
-    ctx->scr_r[1].assign(ntraits, 0.0);
-    ctx->scr_nv.assign(ntraits, 0.0);
-    std::vector<int8_t> hd((size_t)ntraits * ND * Np, 0);
-    std::vector<double> hqd(2 * (size_t)ntraits * Np, 0.0), hqtot(ntraits, 0.0), hsc(3 * (size_t)ntraits, 1.0);
-    for (int t = 0; t < ntraits; ++t) {
-        const float *yt = y + (size_t)t * nid;
-        auto ok = [&](int k) { return (hw[(size_t)t * Wp + k / 32] >> (k % 32) & 1u) != 0; };
-        double sum = 0.0;
-        long long nv = 0;
-        for (int k = 0; k < nid; ++k)
-            if (ok(k)) {
-                sum += (double)yt[k];
-                ++nv;
-            }
-        const double mu = nv ? sum / (double)nv : 0.0;
-        const double p2 = p2s[t];
-        double maxabs = 0.0;
-        for (int k = 0; k < nid; ++k)
-            if (ok(k)) maxabs = std::max(maxabs, std::fabs(((double)yt[k] - mu) * p2));
-        const int sy = (maxabs > 0.0 && std::isfinite(maxabs)) ? (int)std::floor(std::log2(8355000.0 / maxabs)) : 0;
-        const double scale = std::ldexp(1.0, sy);
-        hsc[t] = std::ldexp(1.0, -sy);
-        int8_t *d0 = hd.data() + (size_t)t * ND * Np;
-        long long ysum = 0;
-        double ymin = INFINITY, ymax = -INFINITY, e16 = 0.0;
-        for (int k = 0; k < nid; ++k) {
-            if (!ok(k)) continue;
-            long long Y = std::llround(((double)yt[k] - mu) * p2 * scale);
-            Y = std::min(8355711LL, std::max(-8355711LL, Y));
-            const long long a0 = ((Y + 128) & 255) - 128, Y1 = (Y - a0) / 256;
-            const long long a1 = ((Y1 + 128) & 255) - 128, a2 = (Y1 - a1) / 256;
-            d0[Np + k] = 1;
-            d0[2 * (size_t)Np + k] = (int8_t)a2;
-            d0[3 * (size_t)Np + k] = (int8_t)a1;
-            d0[4 * (size_t)Np + k] = (int8_t)a0;
-            e16 += (double)(a0 * a0);
-            const double yq = (double)Y * hsc[t];
-            ymin = std::min(ymin, yq);
-            ymax = std::max(ymax, yq);
-            hqd[(size_t)t * Np + k] = yq * yq;
-            hqd[((size_t)ntraits + t) * Np + k] = (double)Y;
-            hqtot[t] += yq * yq;
-            ysum += Y;
-        }
-        hsc[ntraits + t] = (double)ysum;
-        hsc[2 * (size_t)ntraits + t] = (double)nv;
-        const double mid = nv ? 0.5 * (ymin + ymax) : 0.0, half = nv ? 0.5 * (ymax - ymin) : 0.0;
-        const double s = half > 0.0 ? 127.0 / half : 1.0;
-        const float dm = (float)(-s * mid);
-        const double *yv = hqd.data() + ((size_t)ntraits + t) * Np;
-        double e2 = 0.0;
-        for (int k = 0; k < nid; ++k) {
-            if (!ok(k)) continue;
-            const double x = s * hsc[t] * yv[k], D = std::min(127.0, std::max(-127.0, std::nearbyint(x + dm)));
-            d0[k] = (int8_t)D;
-            const double e = x - (D - dm);
-            e2 += e * e;
-        }
-        const double qs = s * s * hqtot[t];
-        hts[2 * t] = make_float4(dm, (float)(std::sqrt(e2) * (1.0 + 1e-6)), (float)qs, (float)(s * s));
-        // two digits: D = d1 + 256 d2 = (Y - d0) / 256
-        const double s16 = scale / 256.0, q16 = s16 * s16 * hqtot[t];
-        e16 /= 65536.0;
-        hts[2 * t + 1] = make_float4(0.0f, (float)(std::sqrt(e16) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
-        ctx->scr_nv[t] = (double)nv;
-        ctx->scr_r[0][t] = qs > 0.0 ? std::sqrt(e2 * (double)nv / qs) : INFINITY;
-        ctx->scr_r[1][t] = qs > 0.0 ? std::sqrt(e16 * (double)nv / q16) : INFINITY;
-    }
-    size_t need = (size_t)ntraits * Np * sizeof(float);
-    size_t cap_y = ctx->traits_cap, cap_q = ctx->traits_cap;
-    CK(ensure(&ctx->d_y, &cap_y, need));
-    CK(ensure(&ctx->d_q, &cap_q, need));
-    ctx->traits_cap = std::min(cap_y, cap_q);
+    const size_t T = (size_t)ntraits, cells = T * nid;
+    ctx->ntraits = 0;  // until the new ones are there
     // buffers are kept across calls while they are large enough: a cudaFree would
     // synchronise the device on every trait upload
-    CK(ensure(&ctx->d_wmask, &ctx->wmask_cap, (size_t)ntraits * Wp * sizeof(uint32_t)));
-    CK(ensure(&ctx->d_qc, &ctx->qc_cap, (size_t)ntraits * sizeof(double)));
-    CK(cudaMemcpyAsync(ctx->d_y, hy.data(), need, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_q, hq.data(), need, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_wmask, hw.data(), hw.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_qc, ctx->qc.data(), ntraits * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(ensure(&ctx->d_ysq, &ctx->ysq_cap, (size_t)ntraits * sizeof(double)));
-    CK(cudaMemcpyAsync(ctx->d_ysq, ysq.data(), ntraits * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(ensure(&ctx->d_ydig, &ctx->ydig_cap, hd.size()));
-    CK(ensure(&ctx->d_qd, &ctx->qd_cap, hqd.size() * sizeof(double)));
-    CK(ensure(&ctx->d_qtot, &ctx->qtot_cap, (size_t)ntraits * sizeof(double)));
-    CK(ensure(&ctx->d_yscale, &ctx->yscale_cap, hsc.size() * sizeof(double)));
-    CK(cudaMemcpyAsync(ctx->d_ydig, hd.data(), hd.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(ensure(&ctx->d_yraw, &ctx->yraw_cap, cells * sizeof(float)));
+    if (mode == epi::VALID_BYTES) CK(ensure(&ctx->d_yvalid, &ctx->yvalid_cap, cells));
+    CK(ensure(&ctx->d_y, &ctx->y_cap, T * Np * sizeof(float)));
+    CK(ensure(&ctx->d_wmask, &ctx->wmask_cap, T * Wp * sizeof(uint32_t)));
+    CK(ensure(&ctx->d_ysq, &ctx->ysq_cap, T * sizeof(double)));
+    CK(ensure(&ctx->d_ydig, &ctx->ydig_cap, 5 * T * Np));
+    CK(ensure(&ctx->d_qd, &ctx->qd_cap, 2 * T * Np * sizeof(double)));
+    CK(ensure(&ctx->d_qtot, &ctx->qtot_cap, T * sizeof(double)));
+    CK(ensure(&ctx->d_yscale, &ctx->yscale_cap, 3 * T * sizeof(double)));
+    CK(ensure(&ctx->d_tscr, &ctx->tscr_cap, 2 * T * sizeof(float4)));
+    CK(ensure_pinned(ctx, &ctx->h_info, &ctx->h_info_cap, T, ARENA_INFO, ARENA_BLOCKS));
     CK(epi::mma_encode_traits(&ctx->maps, ctx->d_ydig, ntraits, Np));
-    CK(ensure(&ctx->d_tscr, &ctx->tscr_cap, hts.size() * sizeof(float4)));
-    CK(cudaMemcpyAsync(ctx->d_tscr, hts.data(), hts.size() * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_qd, hqd.data(), hqd.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_qtot, hqtot.data(), ntraits * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_yscale, hsc.data(), hsc.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_yraw, y, cells * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+    if (mode == epi::VALID_BYTES)
+        CK(cudaMemcpyAsync(ctx->d_yvalid, valid, cells, cudaMemcpyHostToDevice, ctx->stream));
+    const epi::TraitArrays out = {ctx->d_y,  ctx->d_wmask, ctx->d_ydig,   ctx->d_qd,
+                                  ctx->d_ysq, ctx->d_qtot, ctx->d_yscale, ctx->d_tscr};
+    CK(epi::launch_traits(ctx->d_yraw, ctx->d_yvalid, mode, nid, Np, ntraits, out, ctx->h_info, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->ntraits = ntraits;
     ctx->traits_nid = nid;
@@ -475,12 +406,14 @@ epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntr
     return EPI_OK;
 }
 
+epi_status epi_set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t ntraits, const uint8_t *valid)
+{
+    return set_traits(ctx, y, nid, ntraits, valid, valid ? epi::VALID_BYTES : epi::VALID_NOT9);
+}
+
 epi_status epi_set_phenotype(epi_ctx *ctx, const float *phen, int32_t nid, int32_t safe)
 {
-    if (!ctx) return EPI_E_INVALID;
-    if (!safe) return epi_set_traits(ctx, phen, nid, 1, nullptr);
-    std::vector<uint8_t> v((size_t)(nid > 0 ? nid : 0), 1);
-    return epi_set_traits(ctx, phen, nid, 1, v.data());
+    return set_traits(ctx, phen, nid, 1, nullptr, safe ? epi::VALID_ALL : epi::VALID_NOT9);
 }
 
 void epi_permute_phenotype(float *phen, int32_t nid, uint32_t seed)
@@ -614,7 +547,7 @@ static double screen_share(const epi_ctx *ctx, const epi_scan_opts *o, double pa
     const double top4 = std::sqrt(chi_quantile(chi4, std::min(0.5, 1.0 / pairs)));
     double share = 0.0;
     for (int t = 0; t < ctx->ntraits; ++t) {
-        const double r = ctx->scr_r[digits - 1][t], nv = ctx->scr_nv[t];
+        const double r = digits == 1 ? ctx->h_info[t].r1 : ctx->h_info[t].r2, nv = ctx->h_info[t].nv;
         if (!std::isfinite(r)) return INFINITY;
         const bool report = o->report_trait < 0 || o->report_trait == t;
         auto part = [&](double thr, double df, double top, double (*tail)(double)) {
@@ -672,18 +605,10 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     if (r.form == EPI_FORM_POPC && ctx->nid > 65535)
         return set_err(ctx, EPI_E_UNSUPPORTED, "popcount form counts in 16 bits: at most 65535 individuals "
                        "(the reference's unsigned short counts, EpiOpenCL.c:68)");
-    if (r.form == EPI_FORM_TENSOR && epi::mma_needs_x(variant)) {
-        if (!x_usable(ctx, screen))
-            return set_err(ctx, EPI_E_UNSUPPORTED, "tensor variant %d: its %zu bytes of expanded B rows do not fit",
-                           variant + 1, x_bytes(ctx, screen));
-        if (ctx->x_valid != screen) {
-            CK(ensure(&ctx->d_x, &ctx->x_cap, x_bytes(ctx, screen)));
-            CK(epi::launch_expand(ctx->d_hcodes, ctx->d_ydig, ctx->nsnp, ctx->Np, ctx->ntraits, screen, ctx->d_x,
-                                  ctx->stream));
-            CK(epi::mma_encode_x(&ctx->maps, ctx->d_x, ctx->nsnp, ctx->Np, ctx->ntraits, screen));
-            ctx->x_valid = screen;
-        }
-    }
+    const bool needs_x = r.form == EPI_FORM_TENSOR && epi::mma_needs_x(variant);
+    if (needs_x && !x_usable(ctx, screen))
+        return set_err(ctx, EPI_E_UNSUPPORTED, "tensor variant %d: its %zu bytes of expanded B rows do not fit",
+                       variant + 1, x_bytes(ctx, screen));
     int TI = epi::mma_tile_i(), TJ = epi::mma_tile_j(screen);
     if (r.form == EPI_FORM_POPC) {
         epi::popc_shape(variant, &TI, &TJ, nullptr);
@@ -710,21 +635,9 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     size_t bcap = (size_t)ctx->blocks_cap * sizeof(BlockDesc);
     CK(ensure(&ctx->d_blocks, &bcap, (size_t)std::max(nblocks, 1) * sizeof(BlockDesc)));
     ctx->blocks_cap = (int)(bcap / sizeof(BlockDesc));
-    if (ctx->h_blocks_cap < nblocks) {
-        if (ctx->h_blocks) cudaFreeHost(ctx->h_blocks);
-        ctx->h_blocks = nullptr;
-        ctx->h_blocks_cap = 0;
-        CK(cudaHostAlloc((void **)&ctx->h_blocks, (size_t)nblocks * sizeof(BlockDesc), cudaHostAllocDefault));
-        ctx->h_blocks_cap = nblocks;
-    }
-    const size_t state = epi::NCOUNTERS * sizeof(unsigned long long) + 2 * (size_t)ctx->ntraits * sizeof(unsigned int);
-    if (ctx->h_state_cap < state) {
-        if (ctx->h_state) cudaFreeHost(ctx->h_state);
-        ctx->h_state = nullptr;
-        ctx->h_state_cap = 0;
-        CK(cudaHostAlloc((void **)&ctx->h_state, state, cudaHostAllocDefault));
-        ctx->h_state_cap = state;
-    }
+    CK(ensure_pinned(ctx, &ctx->h_blocks, &ctx->h_blocks_cap, (size_t)nblocks, ARENA_BLOCKS, ARENA_BYTES));
+    CK(ensure_pinned(ctx, &ctx->h_state, &ctx->h_state_cap, epi::NCOUNTERS + (size_t)ctx->ntraits, ARENA_STATE,
+                     ARENA_INFO));
     if (ctx->maxf_cap < 4 * ctx->ntraits) {  // maxima, then the screen's lower bounds of them
         if (ctx->d_maxf) cudaFree(ctx->d_maxf);
         ctx->d_maxf = nullptr;
@@ -754,6 +667,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         r.units *= ctx->ntraits;
         if (r.units == 0) r.ntiles = 0;  // no pair at all
     }
+    size_t cand = 0;  // bytes of the candidate list
     if (screen) {
         double tests = 0.0;
         for (int b = 0; b < nblocks; ++b) tests += (double)block_pairs(blocks[b]) * ctx->ntraits;
@@ -763,15 +677,39 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         // about 30 us, so a segment lasts 5 ms or more (600 cycles a stage, two SMs a unit).
         const double ms = (double)r.units / (ctx->sm_count / 2) * (ctx->Np / 128) * 600.0 / 1.9e6;
         r.segments = (int)std::min((double)epi::MAX_SEGMENTS, std::max(1.0, ms / 5.0));
-        CK(ensure(&ctx->d_cand, &ctx->cand_cap, (size_t)cand_capacity(tests / r.segments) * sizeof(epi::Cand)));
+        cand = (size_t)cand_capacity(tests / r.segments) * sizeof(epi::Cand);
+    }
+    if (!ctx->d_slab) {
+        // the first scan's memory in one piece: hits (2^20), candidates, expanded B rows
+        const size_t hits = sizeof(DevHit) << 20, cand_part = (cand + 255) & ~(size_t)255;
+        const size_t x = needs_x && x_bytes(ctx, screen) <= (256u << 20) ? x_bytes(ctx, screen) : 0;
+        CK(cudaMalloc(&ctx->d_slab, hits + cand_part + x));
+        unsigned char *const p = (unsigned char *)ctx->d_slab;
+        ctx->d_hits = (DevHit *)p;
+        ctx->hit_cap = 1 << 20;
+        if (cand) {
+            ctx->d_cand = (epi::Cand *)(p + hits);
+            ctx->cand_cap = cand;
+        }
+        if (x) {
+            ctx->d_x = (int8_t *)(p + hits + cand_part);
+            ctx->x_cap = x;
+        }
+    }
+    if (cand) CK(ensure_own(&ctx->d_cand, &ctx->cand_cap, cand, &ctx->own_cand));
+    if (needs_x && ctx->x_valid != screen) {
+        CK(ensure_own(&ctx->d_x, &ctx->x_cap, x_bytes(ctx, screen), &ctx->own_x));
+        CK(epi::launch_expand(ctx->d_hcodes, ctx->d_ydig, ctx->nsnp, ctx->Np, ctx->ntraits, screen, ctx->d_x,
+                              ctx->stream));
+        CK(epi::mma_encode_x(&ctx->maps, ctx->d_x, ctx->nsnp, ctx->Np, ctx->ntraits, screen));
+        ctx->x_valid = screen;
     }
     if (r.form == EPI_FORM_TENSOR && !ctx->qm_valid) {
         const size_t tn = (size_t)ctx->ntraits * ctx->nsnp;
-        CK(ensure(&ctx->d_qm, &ctx->qm_cap, 3 * tn * sizeof(double)));
-        CK(ensure(&ctx->d_qmf, &ctx->qmf_cap, tn * sizeof(float)));
+        CK(ensure(&ctx->d_qm, &ctx->qm_cap, tn * (3 * sizeof(double) + sizeof(float))));
         CK(epi::launch_qmiss(ctx->d_missbits, ctx->nsnp, ctx->Wp, ctx->d_wmask, ctx->d_qd,
                              ctx->d_qd + (size_t)ctx->ntraits * ctx->Np, ctx->Np, ctx->ntraits, ctx->d_qm,
-                             ctx->d_qm + tn, ctx->d_qm + 2 * tn, ctx->d_qmf, ctx->stream));
+                             ctx->d_qm + tn, ctx->d_qm + 2 * tn, (float *)(ctx->d_qm + 3 * tn), ctx->stream));
         ctx->qm_valid = true;
     }
     if (r.form == EPI_FORM_POPC && !ctx->pm_valid) {
@@ -807,9 +745,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     a.pmQ = ctx->d_pmQ;
     a.ysq = ctx->d_ysq;
     a.y = ctx->d_y;
-    a.q = ctx->d_q;
     a.wmask = ctx->d_wmask;
-    a.qc = ctx->d_qc;
     a.Np = ctx->Np;
     a.ntraits = ctx->ntraits;
     a.blocks = ctx->d_blocks;
@@ -826,7 +762,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     a.xsj = r.xsj;
     a.seg1 = {ctx->ntraits, 0, 0};
     a.tscr = ctx->d_tscr;
-    a.qmf = ctx->d_qmf;
+    a.qmf = (const float *)(ctx->d_qm + 3 * (size_t)ctx->ntraits * ctx->nsnp);
     a.cand = ctx->d_cand;
     a.cand_cap = (int64_t)(ctx->cand_cap / sizeof(epi::Cand));
     a.lowf = ctx->d_maxf + 2 * (size_t)ctx->ntraits;
@@ -916,6 +852,8 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
     key_add(key, r.variant);
     key_add(key, r.screen);
     key_add(key, r.segments);
+    key_add(key, ctx->h_state);
+    key_add(key, ctx->h_blocks);
     key_add(key, grid);
     key_add(key, ctx->ntraits);
     if (r.form == EPI_FORM_TENSOR) key_add(key, ctx->maps);
@@ -1008,11 +946,6 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     epi_block blk;
     if (ctx->nsnp >= 2 * s) blk = {s, s, 0, s};
     else blk = {0, ctx->nsnp, 0, ctx->nsnp};
-    if (ctx->hit_cap == 0) {
-        const int64_t initial = 1 << 20;
-        CK(cudaMalloc((void **)&ctx->d_hits, initial * sizeof(DevHit)));
-        ctx->hit_cap = initial;
-    }
     epi_scan_opts o2 = *o;
     o2.report_trait = 0;
     std::vector<float> ms(nv, 0.0f);
@@ -1048,10 +981,11 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     *v = best;
     *how = buf;
     // the streamed-B candidate's expanded rows (up to 32 GiB) are released when it lost
-    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best) && ctx->d_x) {
+    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best) && ctx->d_x && ctx->own_x) {
         CK(cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->d_x);
         ctx->d_x = nullptr;
+        ctx->own_x = false;
         ctx->x_cap = 0;
         ctx->x_valid = -1;
     }
@@ -1097,11 +1031,6 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     ScanRun r;
     s = setup_run(ctx, blocks, nblocks, opts, r, variant, screen);
     if (s != EPI_OK) return s;
-    if (ctx->hit_cap == 0) {
-        const int64_t initial = 1 << 20;
-        CK(cudaMalloc((void **)&ctx->d_hits, initial * sizeof(DevHit)));
-        ctx->hit_cap = initial;
-    }
     unsigned long long found = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
         r.args.hits = ctx->d_hits;
@@ -1129,10 +1058,9 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
         found = cnt[0];
         if ((int64_t)found <= ctx->hit_cap) break;
         // every hit is needed to put the first `cap` in output order: grow and rescan
-        cudaFree(ctx->d_hits);
-        ctx->d_hits = nullptr;
+        size_t hits_bytes = (size_t)ctx->hit_cap * sizeof(DevHit);
         ctx->hit_cap = 0;
-        CK(cudaMalloc((void **)&ctx->d_hits, (size_t)found * sizeof(DevHit)));
+        CK(ensure_own(&ctx->d_hits, &hits_bytes, (size_t)found * sizeof(DevHit), &ctx->own_hits));
         ctx->hit_cap = (int64_t)found;
     }
     float ms = 0.0f;

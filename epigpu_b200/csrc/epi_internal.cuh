@@ -6,7 +6,6 @@
 //   codes   uint32 [nsnp][Wc]     2-bit codes, 16 individuals per word, LSB first,
 //                                 padding individuals coded 3 (missing)
 //   y       float [T][Np]         trait column centred by its valid mean, 0 where invalid
-//   q       float [T][Np]         y^2 - qc[t] (qc = mean of y^2 over valid), 0 where invalid
 //   wmask   uint32 [T][Wp]        phenotype-valid bits
 //   maj     uint8 [nsnp]          most frequent genotype of each SNP (plain form)
 //   pmC, pmN, pmQ                 plain form: per (trait, SNP) the sums of y and the counts by
@@ -69,6 +68,25 @@ struct HitRow {
     float F, F2;
 };
 
+// Which phenotype values count: those that are not -9, those whose `valid` byte is set, or all.
+enum { VALID_NOT9 = 0, VALID_BYTES = 1, VALID_ALL = 2 };
+
+// What k_traits (prep.cu) makes of the phenotype columns; layouts above and in ScanArgs. yscale
+// holds 2^-sy, the sums of Y and the numbers of valid individuals, [T] each.
+struct TraitArrays {
+    float *y;
+    uint32_t *wmask;
+    int8_t *ydig;
+    double *qd, *ysq, *qtot, *yscale;
+    float4 *tscr;
+};
+
+// Per trait, for the choice of the screen: the number of valid individuals and E / sigma of the
+// screen with one digit and with two (+inf where the trait has no variance).
+struct TraitInfo {
+    double nv, r1, r2;
+};
+
 // A place in the tensor form's order of units: the begin of a row group.
 struct SegPos {
     int32_t trait, block, group;
@@ -93,9 +111,8 @@ struct ScanArgs {
     const uint32_t *missbits;
     int32_t Wp, Wc, nid, nsnp;
     // traits
-    const float *y, *q;
+    const float *y;
     const uint32_t *wmask;
-    const double *qc;          // [T]
     const double *yscale;      // [T] (tensor form: 2^-sy)
     const double *qd, *qtot, *qm, *sm, *nm;  // tensor form (layout above)
     const double *ytot, *nvalid;             // [T] (tensor form)
@@ -142,7 +159,9 @@ struct ScanArgs {
     float *dump_F, *dump_F2;
     int32_t *dump_df1, *dump_df2;
     // allocation-free entry point only: genotypes read straight from the reference's
-    // packed words, hits written as 24-byte result rows
+    // packed words, hits written as 24-byte result rows; q = y^2 - qc (qc = mean of y^2)
+    const float *q;
+    const double *qc;
     const int32_t *gpack;
     int32_t npack, remain;
     HitRow *rows;

@@ -9,6 +9,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "epi_internal.cuh"
+
 namespace epi {
 
 __device__ __forceinline__ uint32_t ref_code(const int32_t *row, int k, int nid, int npack, int remain)
@@ -70,21 +72,183 @@ __global__ void k_unpack(const int32_t *__restrict__ raw, int nsnp, int nid, int
     }
 }
 
+// Sum over the block of up to four values at once; every thread gets the sums. `sv` holds
+// 32 x N doubles.
+template <int N>
+__device__ __forceinline__ void block_sum(double (&v)[N], double *sv)
+{
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+    __syncthreads();
+    if (l == 0)
+        for (int i = 0; i < N; ++i) sv[N * w + i] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        double x = l < (int)(blockDim.x >> 5) ? sv[N * l + i] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        v[i] = x;
+    }
+}
+
+// The largest of each of two values over the block (NaN is never the larger one).
+__device__ __forceinline__ void block_max2(double &a, double &b, double *sv)
+{
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    auto warp_max = [](double x) {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double y = __shfl_xor_sync(0xffffffffu, x, o);
+            x = y > x ? y : x;
+        }
+        return x;
+    };
+    a = warp_max(a);
+    b = warp_max(b);
+    __syncthreads();
+    if (l == 0) {
+        sv[2 * w] = a;
+        sv[2 * w + 1] = b;
+    }
+    __syncthreads();
+    const int nw = blockDim.x >> 5;
+    a = warp_max(sv[2 * (l < nw ? l : 0)]);
+    b = warp_max(sv[2 * (l < nw ? l : 0) + 1]);
+}
+
+// Everything that the scans need of a phenotype column, one block per trait, in FP64:
+//   * centred by its valid mean and scaled by the power of two that brings its largest magnitude
+//     into [0.5, 1). F and F2 do not depend on the trait's scale, and a power-of-two factor is
+//     exact in binary floating point, so in the normal range every result is bit-identical to
+//     the unscaled computation; a trait in units of 1e20 or 1e-20 no longer overflows or
+//     underflows the single-precision sums of squares;
+//   * tensor form: Y = round(y 2^sy) (|Y| <= 8355711), three balanced base-256 digits of it
+//     and the valid flag; ytilde^2 = (Y 2^-sy)^2 (exact in FP64: |Y| < 2^23) and Y; their sums;
+//   * the screen's 8-bit phenotype D = round(s (ytilde - c)), c the middle of the values and s
+//     the scale that spreads them over -127..127, d0 = -s c (the D of the mean), and the norm
+//     E of what the rounding leaves; the same for the two upper digits of Y (scan_mma.cu).
+// Four passes over the column; at 10,000 individuals about 15 us, where the same loops on one
+// host core and the upload of their eight arrays took 200 to 300 us.
+__global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw, const uint8_t *__restrict__ valid,
+                                                 int mode, int nid, int Np, int ntraits, TraitArrays o,
+                                                 TraitInfo *__restrict__ info)
+{
+    __shared__ double sv[32 * 4];
+    const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const float *y = yraw + (size_t)t * nid;
+    const uint8_t *vb = mode == VALID_BYTES ? valid + (size_t)t * nid : nullptr;
+    auto ok = [&](int k) { return k < nid && (mode == VALID_ALL || (vb ? vb[k] != 0 : y[k] != -9.0f)); };
+
+    double s0[2] = {0.0, 0.0};
+    for (int k = tid; k < Np; k += nt) {  // (Np and the block are multiples of a warp)
+        const bool v = ok(k);
+        const unsigned int bits = __ballot_sync(0xffffffffu, v);
+        if ((tid & 31) == 0) o.wmask[((size_t)t * Np + k) >> 5] = bits;
+        if (v) {
+            s0[0] += (double)y[k];
+            s0[1] += 1.0;
+        }
+    }
+    block_sum(s0, sv);
+    const double nv = s0[1], mu = nv > 0.0 ? s0[0] / nv : 0.0;
+
+    double maxabs = 0.0, unused = 0.0;
+    for (int k = tid; k < nid; k += nt)
+        if (ok(k)) {
+            const double d = fabs((double)y[k] - mu);
+            maxabs = d > maxabs ? d : maxabs;
+        }
+    block_max2(maxabs, unused, sv);
+    const bool scaled = maxabs > 0.0 && isfinite(maxabs);
+    const double p2 = scaled ? ldexp(1.0, -(ilogb(maxabs) + 1)) : 1.0;
+    // the largest power of two with maxabs p2 2^sy <= 8355000, maxabs p2 in [0.5, 1)
+    const double scale = scaled ? (maxabs * p2 * 8388608.0 <= 8355000.0 ? 8388608.0 : 4194304.0) : 1.0;
+    const double unit = 1.0 / scale;  // 2^-sy
+
+    int8_t *dg = o.ydig + (size_t)t * 5 * Np;  // rows D, w, d2, d1, d0
+    double *qd = o.qd + (size_t)t * Np, *Yd = o.qd + ((size_t)ntraits + t) * Np;
+    double s1[4] = {0.0, 0.0, 0.0, 0.0};  // sums of y^2 (as floats), ytilde^2, Y, d0^2
+    double ymax = -INFINITY, nymin = -INFINITY;
+    for (int k = tid; k < Np; k += nt) {
+        float yc = 0.0f;
+        long long Y = 0;
+        const bool v = ok(k);
+        if (v) {
+            const double x = ((double)y[k] - mu) * p2, z = x * scale;
+            yc = (float)x;
+            Y = isfinite(z) ? llround(z) : -8355711LL;
+            Y = min(8355711LL, max(-8355711LL, Y));
+        }
+        const long long a0 = ((Y + 128) & 255) - 128, Y1 = (Y - a0) / 256;
+        const long long a1 = ((Y1 + 128) & 255) - 128, a2 = (Y1 - a1) / 256;
+        const double yq = (double)Y * unit;
+        o.y[(size_t)t * Np + k] = yc;
+        dg[(size_t)Np + k] = (int8_t)v;
+        dg[2 * (size_t)Np + k] = (int8_t)a2;
+        dg[3 * (size_t)Np + k] = (int8_t)a1;
+        dg[4 * (size_t)Np + k] = (int8_t)a0;
+        qd[k] = yq * yq;
+        Yd[k] = (double)Y;
+        if (v) {
+            s1[0] += (double)yc * (double)yc;
+            s1[1] += yq * yq;
+            s1[2] += (double)Y;
+            s1[3] += (double)(a0 * a0);
+            ymax = yq > ymax ? yq : ymax;
+            nymin = -yq > nymin ? -yq : nymin;
+        }
+    }
+    block_sum(s1, sv);
+    block_max2(ymax, nymin, sv);
+
+    const double mid = nv > 0.0 ? 0.5 * (ymax - nymin) : 0.0, half = nv > 0.0 ? 0.5 * (ymax + nymin) : 0.0;
+    const double s = half > 0.0 ? 127.0 / half : 1.0;
+    const float dm = (float)(-s * mid);
+    double e[1] = {0.0};
+    for (int k = tid; k < Np; k += nt) {  // (each thread reads what it wrote)
+        double D = 0.0;
+        if (dg[(size_t)Np + k]) {
+            const double x = s * (Yd[k] * unit);
+            D = fmin(127.0, fmax(-127.0, rint(x + (double)dm)));
+            const double r = x - (D - (double)dm);
+            e[0] += r * r;
+        }
+        dg[k] = (int8_t)D;
+    }
+    block_sum(e, sv);
+    if (tid != 0) return;
+    const double s16 = scale / 256.0, e16 = s1[3] / 65536.0;  // two digits: D = d1 + 256 d2 = (Y - d0) / 256
+    const double q8 = s * s * s1[1], q16 = s16 * s16 * s1[1];
+    o.ysq[t] = s1[0];
+    o.qtot[t] = s1[1];
+    o.yscale[t] = unit;
+    o.yscale[ntraits + t] = s1[2];
+    o.yscale[2 * (size_t)ntraits + t] = nv;
+    o.tscr[2 * t] = make_float4(dm, (float)(sqrt(e[0]) * (1.0 + 1e-6)), (float)q8, (float)(s * s));
+    o.tscr[2 * t + 1] = make_float4(0.0f, (float)(sqrt(e16) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
+    info[t].nv = nv;
+    info[t].r1 = q8 > 0.0 ? sqrt(e[0] * nv / q8) : INFINITY;
+    info[t].r2 = q16 > 0.0 ? sqrt(e16 * nv / q16) : INFINITY;
+}
+
 // Per trait t and SNP s, over the individuals missing at s (and phenotype-valid for t):
 // qm[t][s] = sum of qd[t][k], rm[t][s] = sum of qr[t][k] and nm[t][s] = their number; qmf[t][s]
-// = qm as a float
+// = qm as a float. One warp per (t, s), lanes over the words (one thread per SNP walked its words
+// one after the other: 200 us for 20,000 SNPs at 10,000 individuals, and as long for few SNPs).
 __global__ void k_qmiss(const uint32_t *__restrict__ missbits, int nsnp, int Wp, const uint32_t *__restrict__ wmask,
                         const double *__restrict__ qd, const double *__restrict__ qr, int Np, int ntraits,
                         double *__restrict__ qm, double *__restrict__ rm, double *__restrict__ nm,
                         float *__restrict__ qmf)
 {
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (gid >= (long long)nsnp * ntraits) return;
     const int t = (int)(gid / nsnp), s = (int)(gid % nsnp);
     double x = 0.0, r = 0.0;
     int cnt = 0;
     const uint32_t *mb = missbits + (size_t)s * Wp;
-    for (int w = 0; w < Wp; ++w) {
+    for (int w = lane; w < Wp; w += 32) {
         uint32_t bits = mb[w] & wmask[(size_t)t * Wp + w];
         cnt += __popc(bits);
         while (bits) {
@@ -94,10 +258,18 @@ __global__ void k_qmiss(const uint32_t *__restrict__ missbits, int nsnp, int Wp,
             bits &= bits - 1;
         }
     }
-    qm[gid] = x;
-    rm[gid] = r;
-    nm[gid] = (double)cnt;
-    qmf[gid] = (float)x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        r += __shfl_xor_sync(0xffffffffu, r, o);
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        qm[gid] = x;
+        rm[gid] = r;
+        nm[gid] = (double)cnt;
+        qmf[gid] = (float)x;
+    }
 }
 
 // The streamed-B variant's expanded B rows: row (u nsnp + s) R + r of the u-th set of R = 3 G rows
@@ -217,6 +389,13 @@ __global__ void k_marg(const uint4 *__restrict__ planes, int nsnp, int Wp, const
     }
 }
 
+cudaError_t launch_traits(const float *yraw, const uint8_t *valid, int mode, int nid, int Np, int ntraits,
+                          const TraitArrays &o, TraitInfo *info, cudaStream_t stream)
+{
+    k_traits<<<ntraits, Np < 1024 ? Np : 1024, 0, stream>>>(yraw, valid, mode, nid, Np, ntraits, o, info);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_major(const uint4 *planes, int nsnp, int Wp, uint8_t *maj, cudaStream_t stream)
 {
     const long long threads = 32LL * nsnp;
@@ -250,7 +429,7 @@ cudaError_t launch_qmiss(const uint32_t *missbits, int nsnp, int Wp, const uint3
                         const double *qr, int Np, int ntraits, double *qm, double *rm, double *nm,
                         float *qmf, cudaStream_t stream)
 {
-    const long long total = (long long)nsnp * ntraits;
+    const long long total = 32LL * nsnp * ntraits;
     const int nt = 256;
     k_qmiss<<<(unsigned)((total + nt - 1) / nt), nt, 0, stream>>>(missbits, nsnp, Wp, wmask, qd, qr, Np, ntraits, qm,
                                                               rm, nm, qmf);
