@@ -46,7 +46,7 @@ int mma_min_nid();
 int mma_max_nid();
 int mma_screen_max_nid();
 int mma_shapes();
-void mma_shape(int v, const char **desc);
+void mma_shape(int v, int screen, const char **desc);
 cudaError_t mma_prepare(int v, int screen, int ntraits, int grid_request, int *grid);
 cudaError_t mma_enqueue(int v, int screen, const ScanArgs &a, const MmaMaps &maps, int grid,
                         cudaStream_t stream);
@@ -54,7 +54,7 @@ cudaError_t exact_enqueue(const ScanArgs &a, int sm_count, cudaStream_t stream);
 cudaError_t mma_encode_genotypes(MmaMaps *maps, const uint8_t *hcodes, const uint8_t *h3, int nsnp, int Np);
 cudaError_t mma_encode_traits(MmaMaps *maps, const int8_t *ydig, int ntraits, int Np);
 cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits, int screen);
-bool mma_needs_x(int v);
+bool mma_needs_x(int v, int screen);
 cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int screen,
                           int8_t *x, cudaStream_t stream);
 // Start of a scan: counters to zero, the per-trait maxima of F and F2 and the screen's lower
@@ -457,13 +457,15 @@ struct ScanRun {
     int64_t units, trait_units;
     int xsi, xsj;
     std::vector<Start> starts;
-    // the first row group at or past `u` units
-    epi::SegPos at(int64_t u, int ntraits) const
+    // the first row group at or past `u` units, and the units before it
+    epi::SegPos at(int64_t u, int ntraits, int64_t *before) const
     {
+        *before = units;
         if (u >= units) return {ntraits, 0, 0};
         const auto it = std::lower_bound(starts.begin(), starts.end(), u % trait_units,
                                          [](const Start &x, int64_t y) { return x.units < y; });
         const int t = (int)(u / trait_units);
+        *before = t * trait_units + (it == starts.end() ? trait_units : it->units);
         return it == starts.end() ? epi::SegPos{t + 1, 0, 0} : epi::SegPos{t, it->block, it->group};
     }
     int64_t ntiles;
@@ -605,7 +607,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     if (r.form == EPI_FORM_POPC && ctx->nid > 65535)
         return set_err(ctx, EPI_E_UNSUPPORTED, "popcount form counts in 16 bits: at most 65535 individuals "
                        "(the reference's unsigned short counts, EpiOpenCL.c:68)");
-    const bool needs_x = r.form == EPI_FORM_TENSOR && epi::mma_needs_x(variant);
+    const bool needs_x = r.form == EPI_FORM_TENSOR && epi::mma_needs_x(variant, screen);
     if (needs_x && !x_usable(ctx, screen))
         return set_err(ctx, EPI_E_UNSUPPORTED, "tensor variant %d: its %zu bytes of expanded B rows do not fit",
                        variant + 1, x_bytes(ctx, screen));
@@ -652,7 +654,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     r.starts.clear();
     r.units = base * ctx->ntraits;
     if (r.form == EPI_FORM_TENSOR) {
-        if (epi::mma_needs_x(variant)) {
+        if (epi::mma_needs_x(variant, screen)) {
             const double per = (3.0 * TI + (double)epi::mma_x_rows(screen) * TJ) * ctx->Np;
             r.xsi = r.xsj = std::max(1, (int)(40e6 / per));
         }
@@ -761,6 +763,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     a.xsi = r.xsi;
     a.xsj = r.xsj;
     a.seg1 = {ctx->ntraits, 0, 0};
+    a.seg_units = r.units;
     a.tscr = ctx->d_tscr;
     a.qmf = (const float *)(ctx->d_qm + 3 * (size_t)ctx->ntraits * ctx->nsnp);
     a.cand = ctx->d_cand;
@@ -795,9 +798,11 @@ cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, int nblocks, 
             epi::ScanArgs a = r.args;
             for (int k = 0; k < r.segments && e == cudaSuccess; ++k) {
                 a.segment = k;
-                a.seg0 = r.at(r.units / r.segments * k, ctx->ntraits);
-                a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), ctx->ntraits);
-                if (memcmp(&a.seg0, &a.seg1, sizeof(a.seg0)) == 0) continue;
+                int64_t u0 = 0, u1 = 0;
+                a.seg0 = r.at(r.units / r.segments * k, ctx->ntraits, &u0);
+                a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), ctx->ntraits, &u1);
+                a.seg_units = u1 - u0;
+                if (a.seg_units == 0) continue;
                 e = epi::mma_enqueue(r.variant, r.screen, a, ctx->maps, grid, s);
                 if (e == cudaSuccess) e = epi::exact_enqueue(a, ctx->sm_count, s);
             }
@@ -899,11 +904,11 @@ static std::vector<TuneEntry> g_tune;
 
 int form_variants(int form) { return form == EPI_FORM_TENSOR ? epi::mma_shapes() : epi::popc_shapes(); }
 
-std::string variant_desc(int form, int v)
+std::string variant_desc(int form, int v, int screen)
 {
     const char *d = nullptr;
     int ti = 0, tj = 0;
-    if (form == EPI_FORM_TENSOR) epi::mma_shape(v, &d);
+    if (form == EPI_FORM_TENSOR) epi::mma_shape(v, screen, &d);
     else epi::popc_shape(v, &ti, &tj, &d);
     return std::string(form == EPI_FORM_TENSOR ? "tensor form, " : "plain form, ") + d;
 }
@@ -924,7 +929,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
         // would fit: another context of the same shape may hold more SNPs)
         for (const TuneEntry &t : g_tune)
             if (t.device == ctx->device && t.form == form && t.Np == ctx->Np && t.ntraits == ctx->ntraits &&
-                t.screen == screen && !(form == EPI_FORM_TENSOR && epi::mma_needs_x(t.variant) && !x_candidate(ctx, screen))) {
+                t.screen == screen && !(form == EPI_FORM_TENSOR && epi::mma_needs_x(t.variant, screen) && !x_candidate(ctx, screen))) {
                 *v = t.variant;
                 *how = t.how;
                 return EPI_OK;
@@ -952,7 +957,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     for (int c = 0; c < nv; ++c) {
         // the streamed-B variant is no candidate where its expanded rows would not fit or would
         // run into the power cap (x_candidate)
-        if (form == EPI_FORM_TENSOR && epi::mma_needs_x(c) && !x_candidate(ctx, screen)) {
+        if (form == EPI_FORM_TENSOR && epi::mma_needs_x(c, screen) && !x_candidate(ctx, screen)) {
             ms[c] = INFINITY;
             continue;
         }
@@ -981,7 +986,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     *v = best;
     *how = buf;
     // the streamed-B candidate's expanded rows (up to 32 GiB) are released when it lost
-    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best) && ctx->d_x && ctx->own_x) {
+    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best, screen) && ctx->d_x && ctx->own_x) {
         CK(cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->d_x);
         ctx->d_x = nullptr;
@@ -1066,7 +1071,7 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     ctx->last_ms = ms;
-    ctx->last_config = variant_desc(form, variant) + " (" + how + ")";
+    ctx->last_config = variant_desc(form, variant, screen) + " (" + how + ")";
     ctx->last_pairs = pairs * ctx->ntraits;
 
     const unsigned int *mx = reinterpret_cast<const unsigned int *>(ctx->h_state + epi::NCOUNTERS);

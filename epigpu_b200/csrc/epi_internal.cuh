@@ -140,6 +140,7 @@ struct ScanArgs {
     // together); this launch's part of it begins at seg0 and ends before seg1
     int32_t xsi, xsj;
     SegPos seg0, seg1;
+    int64_t seg_units;  // units in it
     // tensor form, screened scan: per trait and per (trait, SNP) constants of the screen, the
     // segment's candidate list and the per-trait lower bounds of the largest F and F2 so far
     // (order-encoded, as the maxima)

@@ -120,7 +120,8 @@ static_assert(6 * 3 * (ROUNDS - 1) + RCOLS <= NH && bcol(11, TJ - 1) < N && bcol
 // wait and one commit: the issuer is the pipeline's critical path (a barrier wait costs about a
 // hundred cycles even when the barrier is ready).
 //
-// EPW epilogue warps per TMEM lane quarter: 2 (epilogue warps 0-3 and 8-11) or 3 (also 16-19).
+// EPW epilogue warps per TMEM lane quarter: 2 (epilogue warps 0-3 and 8-11) or 3 (also 16-19);
+// 4 in the screen's streamed-B variant, which has no producers (0-3, 4-7, 8-11 and 16-19).
 // PW producer groups of 4 warps: 1 (warps 4-7) or 2 (also 16-19, the groups taking alternate
 // stages, so each has two stage times for its loads, stores, proxy fence and arrivals: the
 // producers' per-stage latency, not their throughput, bounds the pipeline). One group and two
@@ -134,7 +135,8 @@ static_assert(6 * 3 * (ROUNDS - 1) + RCOLS <= NH && bcol(11, TJ - 1) < N && bcol
 // not built in shared memory but precomputed once per genotype and trait load into HBM (12
 // bytes per SNP and individual: `hx`, rows ((t 2 + half) M + snp) 6 + q) and TMA-loaded with
 // the A rows, one 126-row box per CTA half per stage; no producers or raw loader run (warps 4-7
-// and 14 idle) and CTA 0's full barrier counts two arrivals (its loader, CTA 1's forward).
+// and 14 idle); both CTAs' loads complete on CTA 0's full barrier, which counts one arrival (its
+// loader) and the bytes of both.
 //
 // SCR (the screened scan, 1 or 2 phenotype digits; 0: all digits): B holds the column types of w
 // and of the screen's digits only, 3 (1 + SCR) per j-SNP and TJH j-SNPs in each CTA's half: a
@@ -149,16 +151,18 @@ struct Rings {
     static constexpr int RAW_ROWS = SCR == 0 ? ND : 1 + SCR;  // digit rows of a raw stage
     static constexpr uint32_t RAW_BYTES = (TJH + RAW_ROWS) * KS;
     static_assert(TY * TJH == TYH * TJ, "every variant fills 126 of a half's 128 rows");
-    static_assert(!XF || (EPW == 2 && PW == 1), "the streamed-B variant runs the 15-warp layout");
+    static_assert(!XF || (EPW == 2 && PW == 1) || (EPW == 4 && PW == 1 && SCR), "streamed-B layouts");
     static constexpr int NWARPS = (EPW == 2 && PW == 1) ? 15 : 20;
     static constexpr int NTHREADS = NWARPS * 32;
     static constexpr int PROD_REGS = PW == 2 ? 88 : 56;
-    static_assert((EPW == 2 || EPW == 3) && (PW == 1 || PW == 2) && !(EPW == 3 && PW == 2), "warp roles");
-    static_assert(NWARPS == 15 || EPW * 128 * 128 + PW * 128 * PROD_REGS + 128 * 40 <= NTHREADS * 96, "register split");
+    // register budgets by warpgroup (setmaxnreg); with four epilogue warpgroups all keep the launch's 96
+    static constexpr bool REBALANCE = NWARPS == 20 && EPW < 4;
+    static_assert((EPW == 2 || EPW == 3 || XF) && (PW == 1 || PW == 2) && !(EPW == 3 && PW == 2), "warp roles");
+    static_assert(!REBALANCE || EPW * 128 * 128 + PW * 128 * PROD_REGS + 128 * 40 <= NTHREADS * 96, "register split");
     struct Smem {
         uint8_t a[STAGES][A_STAGE];
         uint8_t b[STAGES][B_STAGE];
-        uint8_t raw[RSTAGES][RAW_STAGE];
+        uint8_t raw[RSTAGES][XF ? 16 : RAW_STAGE];  // (unused with streamed B)
         // full: CTA 0 -- its A stage landed (its TMA), CTA 1's forward of its own, and both B
         // halves built (4 local + 4 remote producer warps): 10 arrivals; CTA 1 -- its A stage
         // landed (1). empty: the MMAs reading the slot are done (both CTAs, one commit)
@@ -481,9 +485,10 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
     constexpr int EPW = C::EPW;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *abort = &sm.abort;
-    const int e = warp & 3, grp = warp < 4 ? 0 : (warp < 12 ? 1 : 2);
     constexpr int RND = (C::TJH + 2) / 3;
-    const int r_begin = (grp * RND + EPW - 1) / EPW, r_end = ((grp + 1) * RND + EPW - 1) / EPW;
+    const int e = warp & 3;  // TMEM lane quarter, and the warp's number among those of its quarter
+    const int part = EPW == 4 ? (warp < 12 ? warp >> 2 : 3) : warp < 4 ? 0 : (warp < 12 ? 1 : 2);
+    const int r_begin = (part * RND + EPW - 1) / EPW, r_end = ((part + 1) * RND + EPW - 1) / EPW;
     const int ii = 10 * e + lane / 3, ga = lane % 3, tbase = (lane / 3) * 3;
     const int s1 = tbase + (ga + 1) % 3, s2 = tbase + (ga + 2) % 3;  // the triplet's other rows
     const bool is1 = ga == 1, is2 = ga == 2;
@@ -688,7 +693,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     tc::fence_proxy_async_smem();
     // maxima of F and F2 per trait: per CTA in shared memory (flushed to global memory once,
     // at the end) up to SMAX_TRAITS traits, else the global maxima directly
-    const bool smax_local = a.ntraits <= SMAX_TRAITS;
+    // (the screen keeps none)
+    const bool smax_local = !C::SCR && a.ntraits <= SMAX_TRAITS;
     unsigned int *smax = reinterpret_cast<unsigned int *>(reinterpret_cast<uint8_t *>(&sm) + sizeof(Smem));
     if (smax_local)
         for (int w = threadIdx.x; w < 2 * a.ntraits; w += blockDim.x) smax[w] = 0u;
@@ -696,7 +702,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     unsigned int *const mxf2 = smax_local ? smax + a.ntraits : a.maxf2;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            tc::mbar_init(&sm.full[s], rank == 0 ? (C::XF ? 2 : 10) : 1);
+            tc::mbar_init(&sm.full[s], rank == 0 ? (C::XF ? 1 : 10) : 1);
             tc::mbar_init(&sm.empty[s], 1);
         }
         for (int r = 0; r < RSTAGES; ++r) {
@@ -719,11 +725,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     const uint32_t tmem = sm.tmem_base;
     volatile int *abort = &sm.abort;
 
-    // epilogue warps: 0-3, 8-11 (and 16-19 with three per lane quarter); producer warps: 4-7
+    // epilogue warps: 0-3, 8-11 (and 16-19 with three per lane quarter, 4-7 too with four); producer warps: 4-7
     // (and 16-19 with two producer groups)
-    const bool epi_warp = warp < 4 || (warp >= 8 && warp < 12) || (EPW == 3 && warp >= 16);
+    const bool epi_warp = warp < 4 || (warp >= 8 && warp < 12) || (EPW >= 3 && warp >= 16) || (EPW == 4 && warp < 8);
     const bool prod_warp = !C::XF && ((warp >= 4 && warp < 8) || (PW == 2 && warp >= 16));
-    if constexpr (C::NWARPS == 20) {
+    if constexpr (C::REBALANCE) {
         if (epi_warp) tc::setmaxnreg_inc<128>();
         else if (prod_warp) tc::setmaxnreg_dec<C::PROD_REGS>();
         else tc::setmaxnreg_dec<40>();
@@ -1025,12 +1031,22 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                         ok = false;
                         break;
                     }
-                    tc::mbar_arrive_expect_tx(&sm.full[as], C::XF ? A_BYTES + XB_BYTES : A_BYTES);
+                    if constexpr (C::XF) {
+                        // both CTAs' loads complete on CTA 0's barrier, which expects the bytes of
+                        // both (no forward through CTA 1); this CTA's half of the B stage: 126
+                        // expanded rows
+                        if (rank == 0) tc::mbar_arrive_expect_tx(&sm.full[as], 2 * (A_BYTES + XB_BYTES));
+                        const uint32_t bar = tc::mapa(&sm.full[as], 0);
 #pragma unroll
-                    for (int w = 0; w < 4; ++w)
-                        tc::tma_load_2d(sm.a[as] + 32 * w * KS, &maps.hi, ks * KS, arow + A_BOX * w, &sm.full[as]);
-                    // the streamed-B variant: this CTA's half of the B stage, 126 expanded rows
-                    if constexpr (C::XF) tc::tma_load_2d(sm.b[as], &maps.hx, ks * KS, xrow, &sm.full[as]);
+                        for (int w = 0; w < 4; ++w)
+                            tc::tma_load_2d_pair(sm.a[as] + 32 * w * KS, &maps.hi, ks * KS, arow + A_BOX * w, bar);
+                        tc::tma_load_2d_pair(sm.b[as], &maps.hx, ks * KS, xrow, bar);
+                    } else {
+                        tc::mbar_arrive_expect_tx(&sm.full[as], A_BYTES);
+#pragma unroll
+                        for (int w = 0; w < 4; ++w)
+                            tc::tma_load_2d(sm.a[as] + 32 * w * KS, &maps.hi, ks * KS, arow + A_BOX * w, &sm.full[as]);
+                    }
                     ++issued_a;
                     advance<STAGES>(as, aph);
                 }
@@ -1039,9 +1055,10 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             // the last loads issued into every slot. A stages of CTA 1 complete on its local
             // barrier; CTA 0's also need CTA 1's forward, so CTA 0 waits for its own bytes only
             // through the phases it can observe (all its issued phases complete on the normal
-            // path; after an abort the bounded wait ends).
+            // path; after an abort the bounded wait ends). With streamed B CTA 0 waits for both
+            // CTAs' loads, and CTA 1 for CTA 0 in the cluster barrier below.
             int no_abort = 0;
-            for (uint32_t back = 1; back <= STAGES && back <= issued_a; ++back) {
+            for (uint32_t back = 1; back <= STAGES && back <= issued_a && !(C::XF && rank == 1); ++back) {
                 const uint32_t slot = (as + STAGES - back) % STAGES, par = back > as ? (aph ^ 1u) : aph;
                 if (!tc::mbar_wait(&sm.full[slot], par, &no_abort, a.wait_ns)) fail(a, sm, 8);
             }
@@ -1080,12 +1097,12 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 if (!tc::mbar_wait(&sm.raw_full[slot], par, &no_abort, a.wait_ns)) fail(a, sm, 11);
             }
         }
-    } else if (warp == 12 && lane == 0 && rank == 1) {
+    } else if (warp == 12 && lane == 0 && rank == 1 && !C::XF) {
         // ---------------- A forwarder (CTA 1, warp 12) ----------------
         // each of this CTA's A stages, once landed, counts as one arrival on CTA 0's full
         uint32_t as = 0, aph = 0;
         bool ok = true;
-        for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
+        for (long long u = pair; u < a.seg_units && ok; u += npairs) {
             for (int ks = 0; ks < nks; ++ks) {
                 if (!tc::mbar_wait(&sm.full[as], aph, abort, a.wait_ns)) {
                     fail(a, sm, 9);
@@ -1096,8 +1113,10 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 advance<STAGES>(as, aph);
             }
         }
-    } else if (warp == 12 && lane == 0) {
+    } else if (warp == 12 && lane == 0 && rank == 0) {
         // ---------------- MMA issuer (CTA 0, warp 12) ----------------
+        // (it needs the number of this cluster's units only: walking them would cost it about 900
+        // cycles between two units, and it is the critical path)
         uint32_t as = 0, aph = 0, accph[2] = {0u, 0u};
         int buf = 0;
         bool ok = true;
@@ -1107,7 +1126,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             fail(a, sm, 12);
             ok = false;
         }
-        for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
+        for (long long u = pair; u < a.seg_units && ok; u += npairs) {
             if (!tc::mbar_wait_cluster(&sm.acc_empty[buf], accph[buf] ^ 1u, abort, a.wait_ns)) {
                 fail(a, sm, 4);
                 break;
@@ -1218,27 +1237,33 @@ int mma_max_nid() { return 1 << 24; }  // digit sums stay within int32
 int mma_screen_max_nid() { return (1 << 15) - mma::KS; }
 int mma_stage_individuals() { return mma::KS; }
 
-// The variants the autotuner chooses among -- operand slots and raw stages (each ~200-216 KB
+// The variants the autotuner chooses among -- operand slots and raw stages (each ~200-230 KB
 // of shared memory) and epilogue warps per TMEM lane quarter:
 //   0  6 slots / 6 raw, 2 epilogue warps   1  5 / 10, 2   2  6 / 4, 2   3  6 / 6, 3
 //   4  6 / 6, 2 epilogue warps, two producer groups on alternate stages
 //   5  6 slots, streamed B (expanded rows TMA-loaded from HBM; no producers, no raw ring)
+// The screen needs half the expanded rows per pair, so streamed B is its fastest variant at every
+// size and comes twice, with 7 slots: 5 with 2 epilogue warps per lane quarter, 2 with 4 (the
+// faster one below about 1,500 individuals, where the epilogue bounds a unit: N = 500 x 4,000
+// SNPs 130 us against 146; N = 4,000 x 20,000 SNPs 8.70 ms against 8.55).
 constexpr int MMA_SHAPES = 6;
+
 // variant v with SCR digits in the screen (0: all digits)
 template <int V, int SCR>
 struct VariantOf;
 template <int SCR> struct VariantOf<0, SCR> { using type = mma::Rings<6, 6, 2, 1, false, SCR>; };
 template <int SCR> struct VariantOf<1, SCR> { using type = mma::Rings<5, 10, 2, 1, false, SCR>; };
-template <int SCR> struct VariantOf<2, SCR> { using type = mma::Rings<6, 4, 2, 1, false, SCR>; };
+template <int SCR> struct VariantOf<2, SCR> { using type = mma::Rings<7, 1, 4, 1, true, SCR>; };
+template <> struct VariantOf<2, 0> { using type = mma::Rings<6, 4, 2, 1, false, 0>; };
 template <int SCR> struct VariantOf<3, SCR> { using type = mma::Rings<6, 6, 3, 1, false, SCR>; };
 template <int SCR> struct VariantOf<4, SCR> { using type = mma::Rings<6, 6, 2, 2, false, SCR>; };
-template <int SCR> struct VariantOf<5, SCR> { using type = mma::Rings<6, 1, 2, 1, true, SCR>; };
+template <int SCR> struct VariantOf<5, SCR> { using type = mma::Rings<SCR ? 7 : 6, 1, 2, 1, true, SCR>; };
 
-bool mma_needs_x(int v) { return v == 5; }
+bool mma_needs_x(int v, int screen) { return v == 5 || (v == 2 && screen); }
 
 int mma_shapes() { return MMA_SHAPES; }
 
-void mma_shape(int v, const char **desc)
+void mma_shape(int v, int screen, const char **desc)
 {
     static const char *names[MMA_SHAPES] = {"6 operand slots / 6 raw stages, 8 epilogue warps",
                                             "5 operand slots / 10 raw stages, 8 epilogue warps",
@@ -1246,7 +1271,9 @@ void mma_shape(int v, const char **desc)
                                             "6 operand slots / 6 raw stages, 12 epilogue warps (setmaxnreg)",
                                             "6 operand slots / 6 raw stages, 8 epilogue warps, 2 producer groups (setmaxnreg)",
                                             "6 operand slots, B streamed from HBM, 8 epilogue warps"};
-    if (desc) *desc = names[v];
+    if (desc) *desc = screen && v == 2   ? "7 operand slots, B streamed from HBM, 16 epilogue warps"
+                      : screen && v == 5 ? "7 operand slots, B streamed from HBM, 8 epilogue warps"
+                                         : names[v];
 }
 
 // Launch shape per (device, variant, dynamic shared memory size): the attribute set and the
@@ -1273,7 +1300,7 @@ static cudaLaunchConfig_t mma_config(int ntraits, int grid, cudaStream_t stream,
     cfg.blockDim = dim3(C::NTHREADS, 1, 1);
     // more than half of the SM's shared memory: one CTA per SM, which owns all 512 TMEM
     // columns; the tail holds the per-CTA maxima
-    cfg.dynamicSmemBytes = sizeof(typename C::Smem) + 1024 + smax_bytes(ntraits);
+    cfg.dynamicSmemBytes = sizeof(typename C::Smem) + 1024 + (C::SCR ? 0 : smax_bytes(ntraits));
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -1297,7 +1324,7 @@ static cudaError_t prepare(int v, int ntraits, int grid_request, int *grid)
         if (clusters == 0) {
             // the attribute admits the largest size any trait count asks for
             e = cudaFuncSetAttribute(mma::k_scan_mma<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(sizeof(typename C::Smem) + 1024 + smax_bytes(SMAX_TRAITS)));
+                                     (int)(sizeof(typename C::Smem) + 1024 + (C::SCR ? 0 : smax_bytes(SMAX_TRAITS))));
             if (e != cudaSuccess) return e;
             e = cudaOccupancyMaxActiveClusters(&clusters, mma::k_scan_mma<C>, &cfg);
             if (e != cudaSuccess) return e;
