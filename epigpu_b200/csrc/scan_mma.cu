@@ -1231,7 +1231,11 @@ cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int n
 bool mma_available() { return true; }
 int mma_tile_i() { return mma::TIP; }  // the host tiles blocks by CTA-pair tiles
 int mma_tile_j(int screen) { return screen == 0 ? mma::TJ : screen == 1 ? 2 * mma::TJ : Screen2Digits::TJT; }
-int mma_min_nid() { return 256; }
+// The automatic choice takes this form from here on. Kernel time against the plain form, 8 df and
+// 4 df, B200: N = 64 x 2,000 SNPs 64 us and 320, N = 150 x 240 22 and 88, N = 231 x 2,003 69 and
+// 443, N = 126 x 30,000 6.3 ms and 61. With few individuals many pairs fit nearly perfectly and
+// the screen settles none of them: at N = 20 both take 0.3 ms.
+int mma_min_nid() { return 64; }
 int mma_max_nid() { return 1 << 24; }  // digit sums stay within int32
 // the screen's sums (127 per individual) stay below 2^22, its counts below 2^15
 int mma_screen_max_nid() { return (1 << 15) - mma::KS; }

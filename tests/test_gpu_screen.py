@@ -66,7 +66,7 @@ def _load(ctx, nid, sizes, ntraits, seed, miss=0.01, masks=True):
     return [(int(starts[i]), sizes[i], int(starts[j]), sizes[j]) for i in range(len(sizes)) for j in range(i + 1)]
 
 
-@pytest.mark.parametrize("nid", [256, 257, 511, 1153])
+@pytest.mark.parametrize("nid", [64, 200, 256, 257, 511, 1153])
 @pytest.mark.parametrize("sizes", [[2], [42], [43, 80], [81, 85, 1], [167, 121]], ids=str)
 @pytest.mark.parametrize("test", ["f", "i"])
 def test_tile_edges(gpu_ctx, nid, sizes, test):
@@ -113,3 +113,23 @@ def test_candidate_list_overflow():
         total = _check(ctx, blocks, 1, "f", t1, 0.0, screened=False)
         assert total > 1 << 16
         assert _check(ctx, blocks, 1, "f", t1, 0.0, screened=False) == total
+
+
+@pytest.mark.parametrize("nid", [63, 64, 131, 255])
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_automatic_form_of_few_individuals(gpu_ctx, nid, test):
+    """The automatic choice takes the tensor form from 64 individuals on: the hits of the plain
+    form on the same call, with F and F2 within the parity bar (1e-5 SSY / SSW)."""
+    blocks = _load(gpu_ctx, nid, [150, 77], 1, seed=nid)
+    t1, t2 = synth.f_threshold(8, nid - 9, 1e-4), synth.f_threshold(4, nid - 9, 1e-4)
+    opts = dict(test=test, t1=t1, t2=t2)
+    auto, n, ex = gpu_ctx.scan(blocks, capi.default_opts(**opts), want_blocks=True)
+    assert gpu_ctx.last_timing()[3] == (capi.FORM_TENSOR if nid >= 64 else capi.FORM_POPC)
+    plain, m, px = gpu_ctx.scan(blocks, capi.default_opts(form=capi.FORM_POPC, **opts), want_blocks=True)
+    assert n == m and np.array_equal(ex["block"], px["block"])
+    for f in ("snp1", "snp2", "df1", "df2"):
+        assert np.array_equal(auto[f], plain[f])
+    kappa = 1.0 + px["max_f"].max() * 8 / (nid - 9)  # the largest SSY / SSW about
+    assert np.all(np.abs(auto["F"] - plain["F"]) <= 2e-5 * kappa * np.maximum(plain["F"], 1.0))
+    assert np.all(np.abs(auto["F2"] - plain["F2"]) <= 2e-5 * kappa * np.maximum(plain["F2"], 1.0))
+    assert np.allclose(ex["max_f"], px["max_f"], rtol=2e-5 * kappa)
