@@ -766,6 +766,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     a.seg_units = r.units;
     a.tscr = ctx->d_tscr;
     a.qmf = (const float *)(ctx->d_qm + 3 * (size_t)ctx->ntraits * ctx->nsnp);
+    a.qmf_j = a.qmf;
     a.cand = ctx->d_cand;
     a.cand_cap = (int64_t)(ctx->cand_cap / sizeof(epi::Cand));
     a.lowf = ctx->d_maxf + 2 * (size_t)ctx->ntraits;

@@ -71,8 +71,8 @@ struct HitRow {
 // Which phenotype values count: those that are not -9, those whose `valid` byte is set, or all.
 enum { VALID_NOT9 = 0, VALID_BYTES = 1, VALID_ALL = 2 };
 
-// What k_traits (prep.cu) makes of the phenotype columns; layouts above and in ScanArgs. yscale
-// holds 2^-sy, the sums of Y and the numbers of valid individuals, [T] each.
+// What k_traits (prep.cu) makes of the phenotype columns; layouts above and in ScanArgs; y and qd
+// may be left out (null). yscale holds 2^-sy, the sums of Y and the numbers of valid individuals, [T] each.
 struct TraitArrays {
     float *y;
     uint32_t *wmask;
@@ -98,6 +98,9 @@ struct Cand {
     int32_t snp1, snp2, trait, block;
     float fu, f2u;
 };
+
+// epi_scan_block_noalloc goes through its block in parts of at most this many SNPs a side
+constexpr int RAW_SNPS = 2048;
 
 // 64-bit counters of a scan: hits found, tile queue (plain form), error flag and site, then
 // whether the candidate list overflowed, and from CNT_CAND on the candidates of each segment
@@ -145,7 +148,7 @@ struct ScanArgs {
     // segment's candidate list and the per-trait lower bounds of the largest F and F2 so far
     // (order-encoded, as the maxima)
     const float4 *tscr;
-    const float *qmf;
+    const float *qmf, *qmf_j;  // indexed by SNP; qmf_j: of the j side (the same array but in epi_scan_block_noalloc)
     Cand *cand;
     int64_t cand_cap;
     int32_t segment;
@@ -168,6 +171,52 @@ struct ScanArgs {
     HitRow *rows;
 };
 
+// ---- the reference's packed words (src/readplink.c:1066-1102), read as they are ----
+
+// Word `idx` of a SNP's row as it stands; words past the last one and rows that are not there
+// (row == nullptr) read as all codes 3 (missing).
+__device__ __forceinline__ uint32_t packed_raw(const uint32_t *row, int idx, int npack1)
+{
+    return row != nullptr && idx < npack1 ? __ldg(row + idx) : 0xFFFFFFFFu;
+}
+
+// The same with its first individual in bits 31:30, as in the full words, and every position
+// without an individual coded 3: the tail word (idx == npack) holds its codes right-aligned.
+__device__ __forceinline__ uint32_t packed_aligned(uint32_t w, int idx, int npack, int remain)
+{
+    return idx == npack && remain ? (w << (32 - 2 * remain)) | (0xFFFFFFFFu >> (2 * remain)) : w;
+}
+
+__device__ __forceinline__ uint32_t packed_word(const uint32_t *row, int idx, int npack, int remain)
+{
+    return packed_aligned(packed_raw(row, idx, npack + (remain > 0)), idx, npack, remain);
+}
+
+// Byte-permute selectors of an aligned word's 16 individuals, four per selector, first individual
+// lowest: the code with its two bits swapped (0, 2, 1, 3 for 0, 1, 2, 3), so that
+// __byte_perm(table, 0, sel[q]) looks four individuals up in a table of four bytes. (PACKED_TABLE
+// puts the bytes for genotypes 0, 1, 2 and for missing in their places.)
+#define PACKED_TABLE(g0, g1, g2, miss) ((g0) | (g2) << 8 | (g1) << 16 | (miss) << 24)
+__device__ __forceinline__ void packed_selectors(uint32_t w, uint32_t sel[4])
+{
+    const uint32_t x = __brev(w);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t v = h ? x >> 16 : x & 0xFFFFu;  // 2-bit fields to 4-bit fields
+        v = (v | v << 8) & 0x00FF00FFu;
+        v = (v | v << 4) & 0x0F0F0F0Fu;
+        v = (v | v << 2) & 0x33333333u;
+        sel[2 * h] = v;
+        sel[2 * h + 1] = v >> 16;
+    }
+}
+
+__device__ __forceinline__ uint4 packed_lookup(uint32_t table, const uint32_t sel[4])
+{
+    // (the selector's upper half is ignored)
+    return make_uint4(__byte_perm(table, 0u, sel[0]), __byte_perm(table, 0u, sel[1]), __byte_perm(table, 0u, sel[2]),
+                      __byte_perm(table, 0u, sel[3]));
+}
 
 // TMA descriptors of the tensor form (kernel parameter, __grid_constant__)
 struct MmaMaps {

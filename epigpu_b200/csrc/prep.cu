@@ -167,7 +167,6 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     const double unit = 1.0 / scale;  // 2^-sy
 
     int8_t *dg = o.ydig + (size_t)t * 5 * Np;  // rows D, w, d2, d1, d0
-    double *qd = o.qd + (size_t)t * Np, *Yd = o.qd + ((size_t)ntraits + t) * Np;
     double s1[4] = {0.0, 0.0, 0.0, 0.0};  // sums of y^2 (as floats), ytilde^2, Y, d0^2
     double ymax = -INFINITY, nymin = -INFINITY;
     for (int k = tid; k < Np; k += nt) {
@@ -183,13 +182,15 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
         const long long a0 = ((Y + 128) & 255) - 128, Y1 = (Y - a0) / 256;
         const long long a1 = ((Y1 + 128) & 255) - 128, a2 = (Y1 - a1) / 256;
         const double yq = (double)Y * unit;
-        o.y[(size_t)t * Np + k] = yc;
+        if (o.y) o.y[(size_t)t * Np + k] = yc;
         dg[(size_t)Np + k] = (int8_t)v;
         dg[2 * (size_t)Np + k] = (int8_t)a2;
         dg[3 * (size_t)Np + k] = (int8_t)a1;
         dg[4 * (size_t)Np + k] = (int8_t)a0;
-        qd[k] = yq * yq;
-        Yd[k] = (double)Y;
+        if (o.qd) {
+            o.qd[(size_t)t * Np + k] = yq * yq;
+            o.qd[((size_t)ntraits + t) * Np + k] = (double)Y;
+        }
         if (v) {
             s1[0] += (double)yc * (double)yc;
             s1[1] += yq * yq;
@@ -209,7 +210,8 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     for (int k = tid; k < Np; k += nt) {  // (each thread reads what it wrote)
         double D = 0.0;
         if (dg[(size_t)Np + k]) {
-            const double x = s * (Yd[k] * unit);
+            const int Y = dg[4 * (size_t)Np + k] + 256 * dg[3 * (size_t)Np + k] + 65536 * dg[2 * (size_t)Np + k];
+            const double x = s * ((double)Y * unit);
             D = fmin(127.0, fmax(-127.0, rint(x + (double)dm)));
             const double r = x - (D - (double)dm);
             e[0] += r * r;

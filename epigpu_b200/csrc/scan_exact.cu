@@ -16,6 +16,34 @@ namespace epi {
 
 constexpr int EXACT_NT = 256;
 
+// RAW (epi_scan_block_noalloc): the genotypes come from the reference's packed words, ytilde from
+// the digits, the missing sums by the SNP's place in the block (qm, sm, nm of the i side, then of
+// the j side), and the hits go out as 24-byte rows.
+
+// the sum of ytilde^2 over the individuals missing at both SNPs, as missing_both_q, from the packed words
+__device__ __forceinline__ double missing_both_packed(const ScanArgs &a, const uint32_t *ri, const uint32_t *rj)
+{
+    const int8_t *dg = a.ydig;
+    double part = 0.0;
+    for (int w = threadIdx.x & 31; 16 * w < a.nid; w += 32) {
+        const uint32_t x = packed_word(ri, w, a.npack, a.remain) & packed_word(rj, w, a.npack, a.remain);
+        uint32_t m = x & (x >> 1) & 0x55555555u;  // both bits of both codes
+        while (m) {
+            const int k = 16 * w + 15 - ((31 - __clz(m)) >> 1);
+            m &= ~(0x80000000u >> __clz(m));
+            if (k < a.nid && dg[a.Np + k]) {
+                const int Y = dg[4 * a.Np + k] + 256 * dg[3 * a.Np + k] + 65536 * dg[2 * a.Np + k];
+                const double yq = (double)Y * a.yscale[0];
+                part += yq * yq;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+    return part;
+}
+
+template <bool RAW>
 __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -42,8 +70,16 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
         const float mI = screen_lo(ord2f(__shfl_sync(0xffffffffu, lI, 0)));
         if (c.fu <= (report ? fminf(t1c, mF) : mF) && (!a.test_int || c.f2u <= (report ? fminf(t2c, mI) : mI))) continue;
 
-        const uint4 *hi = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp1 * a.Np);
-        const uint4 *hj = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp2 * a.Np);
+        const uint4 *hi = nullptr, *hj = nullptr;
+        const uint32_t *ri = nullptr, *rj = nullptr;
+        if (RAW) {
+            const size_t npack1 = a.npack + (a.remain > 0);
+            ri = reinterpret_cast<const uint32_t *>(a.gpack) + c.snp1 * npack1;
+            rj = reinterpret_cast<const uint32_t *>(a.gpack) + c.snp2 * npack1;
+        } else {
+            hi = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp1 * a.Np);
+            hj = reinterpret_cast<const uint4 *>(a.hcodes + (size_t)c.snp2 * a.Np);
+        }
         const uint4 *dg = reinterpret_cast<const uint4 *>(a.ydig + ((size_t)t * 5 + 1) * a.Np);
         int acc[9][4];
 #pragma unroll
@@ -51,7 +87,19 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[k][r] = 0;
         for (int k = lane; k < nc; k += 32) {
-            const uint4 vi = hi[k], vj = hj[k];
+            uint4 vi, vj;
+            if (RAW) {
+                const auto one_hot = [&](const uint32_t *row) {
+                    uint32_t sel[4];
+                    packed_selectors(packed_word(row, k, a.npack, a.remain), sel);
+                    return packed_lookup(PACKED_TABLE(1u, 2u, 4u, 0u), sel);
+                };
+                vi = one_hot(ri);
+                vj = one_hot(rj);
+            } else {
+                vi = hi[k];
+                vj = hj[k];
+            }
             const uint4 d[4] = {dg[k], dg[nc + k], dg[2 * nc + k], dg[3 * nc + k]};
             const uint32_t wi[4] = {vi.x, vi.y, vi.z, vi.w}, wj[4] = {vj.x, vj.y, vj.z, vj.w};
 #pragma unroll
@@ -84,7 +132,11 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
             N += n[k];
         }
         // the sum of squares: see scan_mma.cu
-        const size_t mi = (size_t)t * a.nsnp + c.snp1, mj = (size_t)t * a.nsnp + c.snp2;
+        size_t mi = (size_t)t * a.nsnp + c.snp1, mj = (size_t)t * a.nsnp + c.snp2;
+        if (RAW) {
+            mi = c.snp1 - a.blocks[0].start1;
+            mj = RAW_SNPS + c.snp2 - a.blocks[0].start2;
+        }
         const double sc = a.yscale[t];
         const int nmm = N + (int)(a.nm[mi] - a.nvalid[t] + a.nm[mj]);
         double qmm = 0.0;
@@ -92,10 +144,12 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
             const double ymm = (st - a.ytot[t] + a.sm[mi] + a.sm[mj]) * sc;
             qmm = ymm * ymm;
         } else if (nmm >= 2) {
-            qmm = missing_both_q(a, t, c.snp1, c.snp2);
+            qmm = RAW ? missing_both_packed(a, ri, rj) : missing_both_q(a, t, c.snp1, c.snp2);
         }
         const PairStat s = pair_stat_exact(n, si, sc, a.qtot[t] - a.qm[mi] - a.qm[mj] + qmm, a.test_int != 0);
-        emit_hit(a, lane == 0 && report && is_hit(a, s), c.snp1, c.snp2, s, t, c.block);
+        const bool hit = lane == 0 && report && is_hit(a, s);
+        if (RAW) emit_row(a, hit, c.snp1, c.snp2, s);
+        else emit_hit(a, hit, c.snp1, c.snp2, s, t, c.block);
         if (lane == 0) {
             auto raise = [](unsigned int *max, unsigned int *low, double F) {
                 if (!(F == F)) return;
@@ -111,7 +165,8 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
 
 cudaError_t exact_enqueue(const ScanArgs &a, int sm_count, cudaStream_t stream)
 {
-    k_exact<<<2 * sm_count, EXACT_NT, 0, stream>>>(a);
+    if (a.gpack) k_exact<true><<<2 * sm_count, EXACT_NT, 0, stream>>>(a);
+    else k_exact<false><<<2 * sm_count, EXACT_NT, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

@@ -99,6 +99,9 @@ constexpr uint32_t XB_BYTES = 6 * TJ * KS;     // the streamed-B variant: one CT
 // raw stage: the j-tile's one-hot rows and the trait's digit rows, 1024-aligned sections
 constexpr int RAW_J = 0, RAW_D = (TJ * KS + 1023) / 1024 * 1024;
 constexpr int RAW_STAGE = 4 * 1024;
+// raw stage of RAW: the packed words of 40 + 21 SNPs (32 bytes each), then the digit rows D and w
+constexpr int PACKED_ROWS = TI + TJ, PACKED_D = PACKED_ROWS * 32, PACKED_STAGE = PACKED_D + 2 * KS;
+static_assert(PACKED_D % 16 == 0, "digit rows are read in words of 16 bytes");
 // producer work items per stage: (j-SNP, 16-individual chunk); 128 producer threads take the
 // first 128 and the threads below XTRA one more (the j-SNPs 16..20, same chunk)
 constexpr int XTRA = TJ * 8 - 128;
@@ -141,10 +144,17 @@ static_assert(6 * 3 * (ROUNDS - 1) + RCOLS <= NH && bcol(11, TJ - 1) < N && bcol
 // SCR (the screened scan, 1 or 2 phenotype digits; 0: all digits): B holds the column types of w
 // and of the screen's digits only, 3 (1 + SCR) per j-SNP and TJH j-SNPs in each CTA's half: a
 // tile is 42 j-SNPs wide with one digit, 28 with two (screen_epilogue below).
-template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false, int SCR_ = 0>
+//
+// RAW (epi_scan_block_noalloc: no memory for expanded rows): warps 13 and 14 copy the reference's
+// packed words of the CTA's 40 i-SNPs and 21 j-SNPs into the raw ring (cp.async, 4 bytes: the
+// caller's rows have no larger alignment) and three producer groups of 4 warps on alternate stages
+// (4-7, 16-19, 20-23) build A and B from them; CTA 0's full barrier counts the 8 producer warps of
+// a stage. 24 warps, launched with 80 registers each: epilogue 104, producers 72, the others 40
+// (59,392 of 61,440).
+template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false, int SCR_ = 0, bool RAW_ = false>
 struct Rings {
     static constexpr int STAGES = S, RSTAGES = RSx, EPW = EPW_, PW = PW_, SCR = SCR_;
-    static constexpr bool XF = XF_;
+    static constexpr bool XF = XF_, RAW = RAW_;
     static constexpr int TY = SCR ? 3 * (1 + SCR) : TYH;  // column types of a j-SNP in a CTA's half
     static constexpr int TJH = (TYH * TJ) / TY;           // j-SNPs in a half: 21 (all digits, one), 14 (two)
     static constexpr int TJT = SCR ? 2 * TJH : TJ;        // j-SNPs per tile
@@ -152,17 +162,21 @@ struct Rings {
     static constexpr uint32_t RAW_BYTES = (TJH + RAW_ROWS) * KS;
     static_assert(TY * TJH == TYH * TJ, "every variant fills 126 of a half's 128 rows");
     static_assert(!XF || (EPW == 2 && PW == 1) || (EPW == 4 && PW == 1 && SCR), "streamed-B layouts");
-    static constexpr int NWARPS = (EPW == 2 && PW == 1) ? 15 : 20;
+    static constexpr int NWARPS = RAW ? 24 : (EPW == 2 && PW == 1) ? 15 : 20;
     static constexpr int NTHREADS = NWARPS * 32;
-    static constexpr int PROD_REGS = PW == 2 ? 88 : 56;
+    static constexpr int PROD_REGS = RAW ? 72 : PW == 2 ? 88 : 56, EPI_REGS = RAW ? 104 : 128;
+    static constexpr int LAUNCH_REGS = RAW ? 80 : 96;
     // register budgets by warpgroup (setmaxnreg); with four epilogue warpgroups all keep the launch's 96
-    static constexpr bool REBALANCE = NWARPS == 20 && EPW < 4;
-    static_assert((EPW == 2 || EPW == 3 || XF) && (PW == 1 || PW == 2) && !(EPW == 3 && PW == 2), "warp roles");
-    static_assert(!REBALANCE || EPW * 128 * 128 + PW * 128 * PROD_REGS + 128 * 40 <= NTHREADS * 96, "register split");
+    static constexpr bool REBALANCE = NWARPS >= 20 && EPW < 4;
+    static_assert(RAW ? EPW == 2 && PW == 3 && SCR == 1 && !XF
+                      : (EPW == 2 || EPW == 3 || XF) && (PW == 1 || PW == 2) && !(EPW == 3 && PW == 2),
+                  "warp roles");
+    static_assert(!REBALANCE || EPW * 128 * EPI_REGS + PW * 128 * PROD_REGS + 128 * 40 <= NTHREADS * LAUNCH_REGS,
+                  "register split");
     struct Smem {
         uint8_t a[STAGES][A_STAGE];
         uint8_t b[STAGES][B_STAGE];
-        uint8_t raw[RSTAGES][XF ? 16 : RAW_STAGE];  // (unused with streamed B)
+        uint8_t raw[RSTAGES][XF ? 16 : RAW ? PACKED_STAGE : RAW_STAGE];  // (unused with streamed B)
         // full: CTA 0 -- its A stage landed (its TMA), CTA 1's forward of its own, and both B
         // halves built (4 local + 4 remote producer warps): 10 arrivals; CTA 1 -- its A stage
         // landed (1). empty: the MMAs reading the slot are done (both CTAs, one commit)
@@ -504,8 +518,8 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
         const bool ivalid = lane < 30 && di < un.bd.size1;
         const float4 ts = a.tscr[2 * t + C::SCR - 1];
         const float d0 = ts.x, E = ts.y, qtot = ts.z, s2y = ts.w;
-        const float *qmf = a.qmf + (size_t)t * a.nsnp;
-        const float qmi = ivalid ? s2y * qmf[gi] : 0.0f;
+        const float *qmf_j = a.qmf_j + (size_t)t * a.nsnp;
+        const float qmi = ivalid ? s2y * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
         const bool report = a.report_trait < 0 || a.report_trait == t;
         unsigned int lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
         unsigned int lI = ti ? reinterpret_cast<volatile unsigned int *>(a.lowf2)[t] : 0u;
@@ -536,7 +550,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                 valid[h] = ivalid && dj + C::TJH * h < un.bd.size2 && gi > gj + C::TJH * h;
                 // (the last round takes in the j-SNPs of the one before where three do not divide)
                 if (C::TJH % 3 != 0) valid[h] = valid[h] && round_j<C>(r) + ga >= 3 * r;
-                qmj[h] = valid[h] ? s2y * qmf[gj + C::TJH * h] : 0.0f;
+                qmj[h] = valid[h] ? s2y * qmf_j[gj + C::TJH * h] : 0.0f;
             }
             uint32_t v[2][3 * C::TY];
             load_round<C>(acc, r, v);
@@ -662,6 +676,148 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
     }
 }
 
+// RAW: the loader warps. A stage is 61 rows of 8 words; a lane copies word c of every eighth row
+// (A rows first, then B rows), and 16 lanes a chunk of the digit rows. Rows of SNPs that are not
+// there and words past the last one are left as they are: those pairs are masked in the epilogue,
+// and individuals past the last one have zero digits and flags on the B side.
+template <class C>
+__device__ __forceinline__ void raw_loader(const ScanArgs &a, typename C::Smem &sm, uint32_t rank, int pair, int npairs)
+{
+    volatile int *abort = &sm.abort;
+    const int t = threadIdx.x - 13 * 32, c = t & 7, rg = t >> 3;  // 64 lanes
+    const int nks = a.Np / KS, npack1 = a.npack + (a.remain > 0);
+    const long long stride8 = 8LL * npack1;
+    uint32_t rs = 0, rph = 0;
+    bool ok = true;
+    for (Walker<C> un(a, pair, npairs); !un.done && ok; un.next()) {
+        const int iA = un.i0 + TI * (int)rank, jB = un.j0 + C::TJH * (int)rank;
+        const int nA = min(TI, un.bd.size1 - iA), nB = min(C::TJH, un.bd.size2 - jB);  // rows that are there
+        const int32_t *pA = a.gpack + (long long)(un.bd.start1 + iA + rg) * npack1 + c;
+        const int32_t *pB = a.gpack + (long long)(un.bd.start2 + jB + rg) * npack1 + c;
+        for (int ks = 0; ks < nks; ++ks) {
+            if (!tc::mbar_wait(&sm.raw_empty[rs], rph ^ 1u, abort, a.wait_ns)) {
+                fail(a, sm, 14);
+                ok = false;
+                break;
+            }
+            uint8_t *const raw = sm.raw[rs];
+            if (8 * ks + c < npack1) {
+                const int32_t *src = pA;
+#pragma unroll
+                for (int x = 0; x < TI / 8; ++x, src += stride8)
+                    if (rg + 8 * x < nA) tc::cp_async4(raw + (rg + 8 * x) * 32 + 4 * c, src);
+                src = pB;
+#pragma unroll
+                for (int x = 0; x < (C::TJH + 7) / 8; ++x, src += stride8)
+                    if (rg + 8 * x < nB) tc::cp_async4(raw + (TI + rg + 8 * x) * 32 + 4 * c, src);
+            }
+            pA += 8;
+            pB += 8;
+            if (t < 16)  // row t / 8 (D, w), chunk c
+                tc::cp_async16(raw + PACKED_D + 16 * t, a.ydig + (size_t)(t >> 3) * a.Np + ks * KS + 16 * c);
+            tc::cp_async_arrive(&sm.raw_full[rs]);
+            advance<C::RSTAGES>(rs, rph);
+        }
+    }
+    tc::cp_async_wait_all();
+}
+
+// RAW: one warp of a producer group: per thread one chunk c of 16 individuals (a packed word) of
+// a few adjacent SNPs, whose rows in the operand tile follow each other. The first two warps build
+// A, 8 threads by 5 SNPs and three genotype rows (15 stores of 16 bytes), the other two B, 7 by 3
+// SNPs and six column types (18 stores). A word's 16 codes become byte-permute selectors, and every
+// row is one table look-up per four individuals. With the rows' addresses as eight precomputed
+// swizzled starts plus constants a stage is about 180 instructions; three groups give each three
+// stage times for its latency.
+template <class C>
+__device__ __forceinline__ void raw_producers(const ScanArgs &a, typename C::Smem &sm, uint32_t rank, int pair,
+                                              int npairs)
+{
+    constexpr int STAGES = C::STAGES, RSTAGES = C::RSTAGES, PW = C::PW;
+    constexpr int SA = 5, SB = 3;  // SNPs per thread
+    static_assert(8 * SA == TI && 7 * SB == C::TJH && 10 % SA == 0, "producer rows");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int *abort = &sm.abort;
+    const int pg = warp < 8 ? 0 : (warp >> 2) - 3;  // warps 4-7, 16-19, 20-23
+    const int t = threadIdx.x & 63, c = t & 7, rg = t >> 3;
+    const bool sideA = (threadIdx.x & 64) == 0;
+    const int nks = a.Np / KS;
+    const long long total = a.seg_units > pair ? ((a.seg_units - 1 - pair) / npairs + 1) * nks : 0;  // stages
+    int ks = pg % nks;  // of stage q
+    uint32_t stage = pg % STAGES, phase = pg / STAGES & 1, rs = pg % RSTAGES, rph = pg / RSTAGES & 1;
+    // tile rows nb, nb + 1, ..: A rows 32 (s / 10) + 3 (s % 10) + g of i-SNP s, B rows 6 s + 2 g + i; row
+    // n's chunk c is at n 128 + ((c ^ (n & 7)) << 4)
+    const int nb = sideA ? 32 * (SA * rg / 10) + 3 * (SA * rg % 10) : C::TY * SB * rg;
+    const int word0 = sideA ? 32 * SA * rg + 4 * c : 32 * (TI + SB * rg) + 4 * c;  // its first word in a raw stage
+    uint32_t at[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) at[k] = nb * 128 + ((c ^ ((nb + k) & 7)) << 4);
+    for (long long q = pg; q < total; q += PW) {
+        if (!tc::mbar_wait(&sm.raw_full[rs], rph, abort, a.wait_ns) ||
+            !tc::mbar_wait(&sm.empty[stage], phase ^ 1u, abort, a.wait_ns)) {
+            fail(a, sm, 13);
+            return;
+        }
+        const uint8_t *const raw = sm.raw[rs];
+        const bool tail = 8 * ks + c == a.npack && a.remain > 0;
+        auto word = [&](int x) {
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(raw + word0 + 32 * x);
+            return tail ? (w << (32 - 2 * a.remain)) | (0xFFFFFFFFu >> (2 * a.remain)) : w;
+        };
+        if (sideA) {
+            uint8_t *const base = sm.a[stage];
+#pragma unroll
+            for (int x = 0; x < SA; ++x) {
+                uint32_t sel[4];
+                packed_selectors(word(x), sel);
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    constexpr uint32_t tables[3] = {PACKED_TABLE(1u, 0u, 0u, 0u), PACKED_TABLE(0u, 1u, 0u, 0u),
+                                                    PACKED_TABLE(0u, 0u, 1u, 0u)};
+                    const int i = 3 * x + g;
+                    *reinterpret_cast<uint4 *>(base + at[i & 7] + 128 * i) = packed_lookup(tables[g], sel);
+                }
+            }
+        } else if (rg < 7) {
+            uint8_t *const base = sm.b[stage];
+            const uint4 d[2] = {*reinterpret_cast<const uint4 *>(raw + PACKED_D + KS + 16 * c),  // w, D
+                                *reinterpret_cast<const uint4 *>(raw + PACKED_D + 16 * c)};
+#pragma unroll
+            for (int x = 0; x < SB; ++x) {
+                uint32_t sel[4];
+                packed_selectors(word(x), sel);
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    constexpr uint32_t tables[3] = {PACKED_TABLE(0xFFu, 0u, 0u, 0u), PACKED_TABLE(0u, 0xFFu, 0u, 0u),
+                                                    PACKED_TABLE(0u, 0u, 0xFFu, 0u)};
+                    const uint4 M = packed_lookup(tables[g], sel);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int i = C::TY * x + 2 * g + k;
+                        *reinterpret_cast<uint4 *>(base + at[i & 7] + 128 * i) =
+                            make_uint4(M.x & d[k].x, M.y & d[k].y, M.z & d[k].z, M.w & d[k].w);
+                    }
+                }
+            }
+        }
+        // (the raw slot is released after the stores, which consume every value loaded from it)
+        tc::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+            tc::mbar_arrive(&sm.raw_empty[rs]);
+            if (rank == 0) tc::mbar_arrive(&sm.full[stage]);
+            else tc::mbar_arrive_remote(&sm.full[stage], 0);
+        }
+        ks += PW;
+        while (ks >= nks) ks -= nks;
+#pragma unroll
+        for (int x = 0; x < PW; ++x) {
+            advance<STAGES>(stage, phase);
+            advance<RSTAGES>(rs, rph);
+        }
+    }
+}
+
 template <class C>
 __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const __grid_constant__ MmaMaps maps)
 {
@@ -702,11 +858,11 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     unsigned int *const mxf2 = smax_local ? smax + a.ntraits : a.maxf2;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            tc::mbar_init(&sm.full[s], rank == 0 ? (C::XF ? 1 : 10) : 1);
+            tc::mbar_init(&sm.full[s], rank == 0 ? (C::XF ? 1 : C::RAW ? 8 : 10) : 1);
             tc::mbar_init(&sm.empty[s], 1);
         }
         for (int r = 0; r < RSTAGES; ++r) {
-            tc::mbar_init(&sm.raw_full[r], 1);
+            tc::mbar_init(&sm.raw_full[r], C::RAW ? 64 : 1);
             tc::mbar_init(&sm.raw_empty[r], 4);
         }
         for (int b = 0; b < 2; ++b) {
@@ -728,13 +884,15 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     // epilogue warps: 0-3, 8-11 (and 16-19 with three per lane quarter, 4-7 too with four); producer warps: 4-7
     // (and 16-19 with two producer groups)
     const bool epi_warp = warp < 4 || (warp >= 8 && warp < 12) || (EPW >= 3 && warp >= 16) || (EPW == 4 && warp < 8);
-    const bool prod_warp = !C::XF && ((warp >= 4 && warp < 8) || (PW == 2 && warp >= 16));
+    const bool prod_warp = !C::XF && ((warp >= 4 && warp < 8) || (PW >= 2 && warp >= 16));
     if constexpr (C::REBALANCE) {
-        if (epi_warp) tc::setmaxnreg_inc<128>();
+        if (epi_warp) tc::setmaxnreg_inc<C::EPI_REGS>();
         else if (prod_warp) tc::setmaxnreg_dec<C::PROD_REGS>();
         else tc::setmaxnreg_dec<40>();
     }
-    if (prod_warp) {
+    if (C::RAW && prod_warp) {
+        if constexpr (C::RAW) raw_producers<C>(a, sm, rank, pair, npairs);
+    } else if (prod_warp) {
         // ---------------- B producers: thread -> (j-SNP, 16-individual chunk) ----------------
         // items (jj, c) with jj < 16 for every thread, and (16 + t/8, c) for t < XTRA; with two
         // groups, group pg builds the stages whose sequence number is pg modulo 2 (and follows
@@ -810,7 +968,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             }
         }
     } else if (C::SCR && epi_warp) {
-        screen_epilogue<C>(a, sm, tmem, rank, pair, npairs);
+        if constexpr (C::SCR != 0) screen_epilogue<C>(a, sm, tmem, rank, pair, npairs);
     } else if (epi_warp) {
         // ---------------- epilogue: the j rounds split over the warps of each lane quarter ----------------
         // warps 0-3 (group 0), 8-11 (group 1), 16-19 (group 2): rounds [rb(g), rb(g + 1))
@@ -1016,7 +1174,9 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             accph[buf] ^= 1u;
             buf ^= 1;
         }
-    } else if (warp == 13) {
+    } else if (C::RAW && (warp == 13 || warp == 14)) {
+        if constexpr (C::RAW) raw_loader<C>(a, sm, rank, pair, npairs);
+    } else if (warp == 13 && !C::RAW) {
         // ---------------- A loader: this CTA's indicator rows, one slot per operand stage ----
         if (lane == 0) {
             uint32_t as = 0, aph = 0, issued_a = 0;
@@ -1063,7 +1223,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 if (!tc::mbar_wait(&sm.full[slot], par, &no_abort, a.wait_ns)) fail(a, sm, 8);
             }
         }
-    } else if (warp == 14 && !C::XF) {
+    } else if (warp == 14 && !C::XF && !C::RAW) {
         // ---------------- raw loader: j one-hot rows and trait digit rows ----------------
         // gated only by the B producers' consumption, so it runs up to RSTAGES stages ahead
         // of them (the j rows come from DRAM once per pair tile)
@@ -1097,7 +1257,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
                 if (!tc::mbar_wait(&sm.raw_full[slot], par, &no_abort, a.wait_ns)) fail(a, sm, 11);
             }
         }
-    } else if (warp == 12 && lane == 0 && rank == 1 && !C::XF) {
+    } else if (warp == 12 && lane == 0 && rank == 1 && !C::XF && !C::RAW) {
         // ---------------- A forwarder (CTA 1, warp 12) ----------------
         // each of this CTA's A stages, once landed, counts as one arrival on CTA 0's full
         uint32_t as = 0, aph = 0;
@@ -1374,6 +1534,16 @@ static cudaError_t with_variant(int v, int screen, F f)
     case 2: return with_rings<2>(v, f);
     }
     return cudaErrorInvalidValue;
+}
+
+using RawRings = mma::Rings<6, 8, 2, 3, false, 1, true>;
+
+// The same for the kernel of epi_scan_block_noalloc.
+cudaError_t mma_raw_prepare(int grid_request, int *grid) { return prepare<RawRings>(-1, 1, grid_request, grid); }
+cudaError_t mma_raw_enqueue(const ScanArgs &a, int grid, cudaStream_t stream)
+{
+    static const MmaMaps none = {};
+    return enqueue<RawRings>(a, none, grid, stream);
 }
 
 // The launch shape of a scan with variant v, resolved before any stream capture: the kernel's

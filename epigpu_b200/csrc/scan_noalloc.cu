@@ -1,9 +1,14 @@
-// scan_noalloc.cu -- the allocation-free entry point (epi_scan_block_noalloc) and the
-// kernel it runs: a popcount-form pair scan that reads the reference's packed genotype
-// words directly (src/readplink.c:1066-1102) and writes 24-byte result rows, with all of its
-// working memory in one fixed device array.
+// scan_noalloc.cu -- the allocation-free entry point (epi_scan_block_noalloc): a scan that reads
+// the reference's packed genotype words directly (src/readplink.c:1066-1102) and writes 24-byte
+// result rows, with all of its working memory in one fixed device array.
 //
-// The kernel is the reference's per-individual method (src/EpiOpenCL.c:110-228: unpack two
+// Two ways, chosen on the device. The tensor form's one-digit screen (scan_mma.cu: its RAW
+// variant builds both operands from the packed words; k_exact settles what it passes on) in parts
+// of 2,048 x 2,048 SNPs; and, where the screen would pass on too much (low thresholds, many
+// individuals) or its candidate list runs over, the plain kernel below. At 1,203 individuals x
+// 2,502 SNPs the plain kernel takes 4.7 ms, ten FP32 operations per pair and individual.
+//
+// The plain kernel is the reference's per-individual method (src/EpiOpenCL.c:110-228: unpack two
 // SNPs, count the 3x3 genotype cells, add the phenotype into its cell) on the CUDA cores.
 // Persistent, one 512-thread CTA per SM, pulling 64 x 32 SNP-pair tiles from a queue. Per
 // tile it walks the individuals in stages of 64:
@@ -16,6 +21,9 @@
 //     individual) and Q += U_V*F_Q (sum of y^2 over valid individuals, q = y^2 - mean y^2).
 // Each thread owns 4 whole pairs (the warp's four i-SNPs x the lane's j-SNP).
 // Epilogue: FP64 SSB/SSI/F/F2 per pair, warp-aggregated atomic row append, maximum F.
+#include <cmath>
+#include <cstddef>
+
 #include "epi_internal.cuh"
 #include "epigpu.h"
 
@@ -116,6 +124,7 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = a.Wp / KW;
+    if (RAW && a.counters[CNT_OVERFLOW] == 0ull) return;  // the screen has done it
     // maxima of F and F2 per trait: per CTA in shared memory (flushed to global memory once,
     // at the end) up to SMAX_TRAITS traits, else the global maxima directly
     const bool smax_local = a.ntraits <= SMAX_TRAITS;
@@ -272,25 +281,58 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
 // Some callers cannot allocate GPU memory: code that must not call cudaMalloc while it runs
 // (a latency-critical service or a real-time loop after start-up), or a host framework
 // that hands out device memory only from its own pool. They pass device buffers for every
-// input and output, and the scan's working memory -- hit/tile counters, the block
-// descriptor, the per-trait maxima and the centred phenotype arrays -- lives in the fixed
-// array below, sized for at most EPI_NOALLOC_MAX_NID individuals (about 520 KiB, held by
-// every GPU that loads the library until the process exits).
+// input and output, and the scan's working memory -- counters, the block descriptor, the
+// maxima, and what either way keeps of the phenotype -- lives in the fixed array below, sized
+// for at most EPI_NOALLOC_MAX_NID individuals (about 520 KiB, held by every GPU that loads the
+// library until the process exits).
 // ---------------------------------------------------------------------------------------
 namespace epi {
+cudaError_t launch_traits(const float *yraw, const uint8_t *valid, int mode, int nid, int Np, int ntraits,
+                          const TraitArrays &o, TraitInfo *info, cudaStream_t stream);
+cudaError_t exact_enqueue(const ScanArgs &a, int sm_count, cudaStream_t stream);
+cudaError_t mma_raw_prepare(int grid_request, int *grid);
+cudaError_t mma_raw_enqueue(const ScanArgs &a, int grid, cudaStream_t stream);
+int mma_tile_i();
+int mma_tile_j(int screen);
+int mma_screen_max_nid();
+
 namespace noalloc {
 
-constexpr int NP_MAX = 65536;  // individuals, padded to a multiple of 128
+constexpr int NP_MAX = 65536;        // individuals, padded to a multiple of 128
+constexpr int NP_SCREEN_MAX = 32768; // of the screen (mma_screen_max_nid is a little below)
 
-struct Scratch {
-    unsigned long long counters[4];  // hits found, tile queue, error flag, error site
-    unsigned int maxf[2];            // order-encoded max F and max F2
-    double qc;                       // mean of the centred phenotype's square
+// What both ways keep; the counters' overflow flag selects the plain kernel.
+struct Head {
+    unsigned long long counters[NCOUNTERS];
+    unsigned int maxf[2], lowf[2];  // order-encoded max F and max F2; the screen's lower bounds of them
+    double qc;                      // mean of the centred phenotype's square (plain kernel)
     BlockDesc block;
-    float y[NP_MAX];                 // centred phenotype (0 where missing)
-    float q[NP_MAX];                 // y^2 - qc (0 where missing)
+};
+
+struct Scratch {  // plain kernel
+    Head h;
+    alignas(16) float y[NP_MAX];     // centred phenotype (0 where missing)
+    alignas(16) float q[NP_MAX];     // y^2 - qc (0 where missing)
     uint32_t wmask[NP_MAX / 32];     // phenotype-valid bits
 };
+
+struct ScreenScratch {  // screen: layouts as in epi_internal.cuh, one trait, one part of the block
+    Head h;
+    TraitInfo info;
+    double ysq, qtot, yscale[3];
+    alignas(16) float4 tscr[2];
+    uint32_t wmask[NP_SCREEN_MAX / 32];
+    alignas(16) int8_t ydig[5 * NP_SCREEN_MAX];
+    // per SNP of the part, i side then j side
+    double qm[2 * RAW_SNPS], sm[2 * RAW_SNPS], nm[2 * RAW_SNPS];
+    float qmf[2 * RAW_SNPS];
+    Cand cand[10000];
+};
+static_assert(sizeof(ScreenScratch) <= sizeof(Scratch), "both ways share the array");
+// read in words of 16 bytes (k_scan_popc: y, q; the screen: tscr, ydig)
+static_assert(offsetof(Scratch, y) % 16 == 0 && offsetof(Scratch, q) % 16 == 0 && offsetof(ScreenScratch, tscr) % 16 == 0 &&
+                  offsetof(ScreenScratch, ydig) % 16 == 0,
+              "alignment");
 
 // The scratch: one copy per device, shared by every call on that device. In host code this
 // name only stands for the array; the device address comes from cudaGetSymbolAddress.
@@ -334,15 +376,17 @@ __device__ __forceinline__ double block_max(double v, double *sv)
 // centred by the valid mean and scaled by the power of two that brings its largest magnitude
 // into [0.5, 1) (exact, so F and F2 are unchanged, and a trait in units of 1e20 or 1e-20
 // neither overflows nor underflows the single-precision squares).
+// Only where the overflow flag asks for the plain kernel.
 __global__ void __launch_bounds__(1024) k_prep(Scratch *s, const float *__restrict__ phen, int nid, int Np, int Wp,
                                                int safe, BlockDesc bd)
 {
     __shared__ double sv[32];
     __shared__ long long sn[32];
     const int tid = threadIdx.x;
-    if (tid < 4) s->counters[tid] = 0ull;
-    if (tid < 2) s->maxf[tid] = 0x007fffffu;  // order-encoded -inf
-    if (tid == 0) s->block = bd;
+    if (s->h.counters[CNT_OVERFLOW] == 0ull) return;
+    if (tid < 4) s->h.counters[tid] = 0ull;
+    if (tid < 2) s->h.maxf[tid] = ENC_NEG_INF;
+    if (tid == 0) s->h.block = bd;
     double sum = 0.0;
     long long n = 0;
     for (int k = tid; k < nid; k += blockDim.x) {
@@ -372,7 +416,7 @@ __global__ void __launch_bounds__(1024) k_prep(Scratch *s, const float *__restri
     }
     block_sum(s2, dummy, sv, sn);
     const double c = n ? s2 / (double)n : 0.0;
-    if (tid == 0) s->qc = c;
+    if (tid == 0) s->h.qc = c;
     for (int k = tid; k < Np; k += blockDim.x) {
         const float y = k < nid ? phen[k] : -9.0f;
         const bool ok = k < nid && (safe || y != -9.0f);
@@ -389,7 +433,7 @@ __global__ void __launch_bounds__(1024) k_prep(Scratch *s, const float *__restri
     }
 }
 
-__global__ void k_finish(const Scratch *s, int64_t *nhits, float *maxf, int test_int)
+__global__ void k_finish(const Head *s, int64_t *nhits, float *maxf, int test_int)
 {
     if (threadIdx.x != 0) return;
     *nhits = (int64_t)s->counters[0];
@@ -397,6 +441,98 @@ __global__ void k_finish(const Scratch *s, int64_t *nhits, float *maxf, int test
         maxf[0] = ord2f(s->maxf[0]);
         maxf[1] = test_int ? ord2f(s->maxf[1]) : 0.0f;
     }
+}
+
+// Start of a call: counters and maxima reset, and the choice of the way -- the screen while it is
+// expected to pass on at most one pair in 250 (the rule of epi_scan, epi_capi.cu: screen_digits,
+// here for one trait and one digit; R = E / sigma, known on the device only). `on`: the screen
+// handles these sizes.
+__global__ void k_begin(ScreenScratch *s, int on, int want_int, float t1, float t2, double pairs, double top8, double top4)
+{
+    const int tid = threadIdx.x;
+    if (tid < NCOUNTERS) s->h.counters[tid] = 0ull;
+    if (tid < 2) s->h.maxf[tid] = s->h.lowf[tid] = ENC_NEG_INF;
+    __syncthreads();
+    if (tid != 0) return;
+    bool screen = on != 0;
+    if (screen) {
+        const double r = s->info.r1, nv = s->info.nv;
+        auto tail = [](double root, bool four) {
+            const double h = root > 0.0 ? 0.5 * root * root : 0.0;
+            return exp(-h) * (four ? 1.0 + h : 1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0)));
+        };
+        auto part = [&](double thr, double df, double top, bool four) {
+            if (!(thr > 0.0)) return 1.0;
+            const double d2 = nv > 10.0 ? nv - 9.0 : 1.0;
+            return tail(fmin(fmax(0.0, top - r), sqrt(df * thr * nv / (d2 + df * thr))) - r, four);
+        };
+        double share = part(t1, 8.0, top8, false);
+        if (want_int) share += part(t2, 4.0, top4, true);
+        screen = isfinite(r) && (share <= 1.0 / 250.0 || share * pairs <= 1024.0);
+    }
+    if (!screen) s->h.counters[CNT_OVERFLOW] = 1ull;
+}
+
+// Start of a part of the block: its descriptor, an empty candidate list, and per SNP of either
+// side, one warp each, the sums over the individuals missing at it (as k_qmiss, prep.cu) from the
+// packed words and the digits.
+__global__ void k_part(ScreenScratch *s, BlockDesc bd, const int32_t *__restrict__ gpack, int nid, int npack, int remain,
+                       int Np)
+{
+    if (s->h.counters[CNT_OVERFLOW]) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s->h.block = bd;
+        s->h.counters[CNT_CAND] = 0ull;
+    }
+    const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (q >= bd.size1 + bd.size2) return;
+    const int snp = q < bd.size1 ? bd.start1 + q : bd.start2 + q - bd.size1;
+    const uint32_t *row = reinterpret_cast<const uint32_t *>(gpack) + (size_t)snp * (npack + (remain > 0));
+    const int8_t *dg = s->ydig;
+    const double unit = s->yscale[0];
+    double x = 0.0, r = 0.0;
+    int cnt = 0;
+    for (int w = lane; 16 * w < nid; w += 32) {
+        const uint32_t v = packed_word(row, w, npack, remain);
+        uint32_t m = v & (v >> 1) & 0x55555555u;
+        while (m) {
+            const int k = 16 * w + 15 - ((31 - __clz(m)) >> 1);
+            m &= ~(0x80000000u >> __clz(m));
+            if (k < nid && dg[Np + k]) {
+                const int Y = dg[4 * Np + k] + 256 * dg[3 * Np + k] + 65536 * dg[2 * Np + k];
+                const double yq = (double)Y * unit;
+                x += yq * yq;
+                r += (double)Y;
+                ++cnt;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        r += __shfl_xor_sync(0xffffffffu, r, o);
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        const int o = q < bd.size1 ? q : RAW_SNPS + q - bd.size1;
+        s->qm[o] = x;
+        s->sm[o] = r;
+        s->nm[o] = (double)cnt;
+        s->qmf[o] = (float)x;
+    }
+}
+
+// Root of the largest of n draws of chi-squared with 8 or 4 degrees of freedom, about.
+static double top_root(double n, bool four)
+{
+    double lo = 0.0, hi = 1500.0;
+    const double p = n > 2.0 ? 1.0 / n : 0.5;
+    for (int k = 0; k < 60; ++k) {
+        const double x = 0.5 * (lo + hi), h = 0.5 * x;
+        const double t = exp(-h) * (four ? 1.0 + h : 1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0)));
+        (t > p ? lo : hi) = x;
+    }
+    return sqrt(lo);
 }
 
 constexpr int MAX_DEVICES = 64;
@@ -423,6 +559,7 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= noalloc::MAX_DEVICES) return EPI_E_NODEVICE;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t smem = sizeof(popc_raw::Smem) + 8;  // + per-CTA maxima of one trait
+    int screen_grid = 0;  // the screen's kernel: its attribute and launch shape (a look-up after the first call)
 
     // set-up, once per device with that device current: the device check, the SM count and
     // the kernel's shared-memory attribute
@@ -437,6 +574,7 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
             return EPI_E_CUDA;
         noalloc::g_sms[dev] = sms;
     }
+    if (mma_raw_prepare(noalloc::g_sms[dev], &screen_grid) != cudaSuccess) return EPI_E_CUDA;
     // The scratch array's device address. In host code g_scratch only stands for the array;
     // the address comes from the runtime, for the current device. It is looked up on every
     // call (a host-side table lookup once the module is loaded), so that a device reset
@@ -444,6 +582,7 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     void *ptr = nullptr;
     if (cudaGetSymbolAddress(&ptr, noalloc::g_scratch) != cudaSuccess || ptr == nullptr) return EPI_E_CUDA;
     noalloc::Scratch *scr = (noalloc::Scratch *)ptr;
+    noalloc::ScreenScratch *ss = (noalloc::ScreenScratch *)ptr;
 
     const int Wp = ((nid + 31) / 32 + 3) / 4 * 4;
     const int Np = 32 * Wp;
@@ -469,9 +608,9 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     a.y = scr->y;
     a.q = scr->q;
     a.wmask = scr->wmask;
-    a.qc = &scr->qc;
+    a.qc = &scr->h.qc;
     a.ntraits = 1;
-    a.blocks = &scr->block;
+    a.blocks = &scr->h.block;
     a.nblocks = 1;
     a.ntiles = ntiles;
     a.test_int = opts->test == 'i';
@@ -481,21 +620,82 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     a.t2 = opts->t2;
     a.rows = reinterpret_cast<HitRow *>(d_hits);
     a.cap = cap;
-    a.counters = scr->counters;
-    a.maxf = &scr->maxf[0];
-    a.maxf2 = &scr->maxf[1];
+    a.counters = scr->h.counters;
+    a.maxf = &scr->h.maxf[0];
+    a.maxf2 = &scr->h.maxf[1];
 
+    // the screen, part by part, while the overflow flag is clear
+    const bool screen = ntiles > 0 && Np <= mma_screen_max_nid();
+    cudaError_t e = cudaSuccess;
+    if (screen) {
+        const TraitArrays out = {nullptr, ss->wmask, ss->ydig, nullptr, &ss->ysq, &ss->qtot, ss->yscale, ss->tscr};
+        e = launch_traits(d_phen, nullptr, opts->safe ? VALID_ALL : VALID_NOT9, nid, Np, 1, out, &ss->info, st);
+    }
+    const double pairs = (double)block->size1 * block->size2;
+    noalloc::k_begin<<<1, 32, 0, st>>>(ss, screen, a.test_int, a.t1, a.t2, pairs, noalloc::top_root(pairs, false),
+                                       noalloc::top_root(pairs, true));
+    if (screen) {
+        ScanArgs p = a;
+        p.wmask = ss->wmask;
+        p.ydig = ss->ydig;
+        p.tscr = ss->tscr;
+        p.yscale = ss->yscale;
+        p.ytot = ss->yscale + 1;
+        p.nvalid = ss->yscale + 2;
+        p.qtot = &ss->qtot;
+        p.qm = ss->qm;
+        p.sm = ss->sm;
+        p.nm = ss->nm;
+        p.lowf = &ss->h.lowf[0];
+        p.lowf2 = &ss->h.lowf[1];
+        p.cand = ss->cand;
+        p.cand_cap = sizeof(ss->cand) / sizeof(ss->cand[0]);
+        p.wait_ns = 2000000000ull;
+        p.xsi = 1;
+        p.xsj = 1 << 30;
+        p.seg1 = {1, 0, 0};
+        const int TI = mma_tile_i(), TJ = mma_tile_j(1);
+        for (int i = 0; i < block->size1; i += RAW_SNPS)
+            for (int j = 0; j < block->size2; j += RAW_SNPS) {
+                BlockDesc d;
+                d.start1 = block->start1 + i;
+                d.size1 = block->size1 - i < RAW_SNPS ? block->size1 - i : RAW_SNPS;
+                d.start2 = block->start2 + j;
+                d.size2 = block->size2 - j < RAW_SNPS ? block->size2 - j : RAW_SNPS;
+                d.tiles_i = (d.size1 + TI - 1) / TI;
+                d.tiles_j = (d.size2 + TJ - 1) / TJ;
+                d.tile_base = 0;
+                p.seg_units = 0;  // tiles that hold a pair (scan_mma.cu: Walker)
+                for (int ti = 0; ti < d.tiles_i; ++ti) {
+                    const long long end = (long long)d.start1 + ((ti + 1) * TI < d.size1 ? (ti + 1) * TI : d.size1);
+                    const long long x = end - 1 - d.start2, n = x <= 0 ? 0 : (x + TJ - 1) / TJ;
+                    p.seg_units += n < d.tiles_j ? n : d.tiles_j;
+                }
+                if (p.seg_units == 0) continue;  // no pair with snp1 > snp2
+                // the per-SNP sums, indexed by SNP
+                p.qmf = (const float *)((uintptr_t)ss->qmf - sizeof(float) * (uintptr_t)d.start1);
+                p.qmf_j = (const float *)((uintptr_t)(ss->qmf + RAW_SNPS) - sizeof(float) * (uintptr_t)d.start2);
+                const unsigned snps = (unsigned)(d.size1 + d.size2);
+                noalloc::k_part<<<(snps + 7) / 8, 256, 0, st>>>(ss, d, d_gpack, nid, a.npack, a.remain, Np);
+                const long long want = 2 * p.seg_units;
+                if (e == cudaSuccess) e = mma_raw_enqueue(p, (int)(want < screen_grid ? want : screen_grid), st);
+                if (e == cudaSuccess) e = exact_enqueue(p, noalloc::g_sms[dev], st);
+            }
+    }
+    // the plain kernel, where the flag is set
     noalloc::k_prep<<<1, 1024, 0, st>>>(scr, d_phen, nid, Np, Wp, opts->safe, bd);
     if (ntiles > 0) {
         const int grid = (int)(ntiles < noalloc::g_sms[dev] ? ntiles : noalloc::g_sms[dev]);
         popc_raw::k_scan_popc<true><<<grid, popc_raw::NT, smem, st>>>(a);
     }
-    noalloc::k_finish<<<1, 32, 0, st>>>(scr, d_nhits, d_maxf, a.test_int);
-    if (cudaGetLastError() != cudaSuccess) return EPI_E_CUDA;
-    unsigned long long found = 0ull;
-    if (cudaMemcpyAsync(&found, &scr->counters[0], sizeof(found), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    noalloc::k_finish<<<1, 32, 0, st>>>(&scr->h, d_nhits, d_maxf, a.test_int);
+    if (cudaGetLastError() != cudaSuccess || e != cudaSuccess) return EPI_E_CUDA;
+    unsigned long long state[3] = {0ull, 0ull, 0ull};  // hits, tile queue, error flag
+    if (cudaMemcpyAsync(state, scr->h.counters, sizeof(state), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return EPI_E_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return EPI_E_CUDA;
+    if (state[2] != 0) return EPI_E_TIMEOUT;
+    const unsigned long long found = state[0];
     // as epi_scan: more hits than `cap` is reported (the first `cap` rows are written, and
     // *d_nhits holds the total)
     return (int64_t)found > cap ? EPI_E_OVERFLOW : EPI_OK;

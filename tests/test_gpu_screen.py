@@ -133,3 +133,44 @@ def test_automatic_form_of_few_individuals(gpu_ctx, nid, test):
     assert np.all(np.abs(auto["F"] - plain["F"]) <= 2e-5 * kappa * np.maximum(plain["F"], 1.0))
     assert np.all(np.abs(auto["F2"] - plain["F2"]) <= 2e-5 * kappa * np.maximum(plain["F2"], 1.0))
     assert np.allclose(ex["max_f"], px["max_f"], rtol=2e-5 * kappa)
+
+
+@pytest.mark.parametrize("nid,nsnp,block", [(17, 90, (0, 90, 0, 90)), (128, 130, (0, 130, 0, 130)),
+                                            (600, 2200, (0, 2200, 0, 2200)), (1203, 2150, (51, 2070, 3, 2147)),
+                                            (2000, 300, (200, 100, 7, 150)), (9001, 201, (0, 201, 0, 201)),
+                                            (32700, 50, (0, 50, 0, 50))], ids=str)
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_block_scan_without_allocation(gpu_ctx, nid, nsnp, block, test):
+    """epi_scan_block_noalloc builds the operands from the packed words (a full or a partial last
+    one) and goes through a block in parts of 2,048 SNPs: the rows and maxima of epi_scan, bit for
+    bit where both go by the digits, within the parity bar where the plain kernel runs (32,700)."""
+    import ctypes
+    torch = pytest.importorskip("torch")
+    codes = synth.genotype_codes(nid, nsnp, seed=nid)
+    codes[3], codes[7], codes[11] = 0, 3, 2
+    y = synth.planted_phenotype(codes, [(1, 20), (33, 5)], seed=nid, var_frac=min(0.3, 60.0 / nid), miss=0.02)
+    packed = synth.pack(codes)
+    t1, t2 = synth.f_threshold(8, max(nid - 9, 2), 1e-5), synth.f_threshold(4, max(nid - 9, 2), 1e-5)
+    opts = capi.default_opts(test=test, t1=t1, t2=t2, form=capi.FORM_TENSOR)
+    gpu_ctx.load_packed(packed, nid)
+    gpu_ctx.set_phenotype(y)
+    want, n, ex = gpu_ctx.scan([block], opts)
+    want = want[np.lexsort((want["snp2"], want["snp1"]))]
+    gp, ph = torch.from_numpy(packed).cuda(), torch.from_numpy(y).cuda()
+    rows = torch.zeros((1 << 16, 6), dtype=torch.int32, device="cuda")
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    maxf = torch.zeros(2, dtype=torch.float32, device="cuda")
+    b = capi.Block(*block)
+    for _ in range(2):
+        st = capi.load().epi_scan_block_noalloc(gp.data_ptr(), nid, nsnp, ph.data_ptr(), ctypes.byref(b),
+                                                ctypes.byref(opts), rows.data_ptr(), rows.shape[0],
+                                                count.data_ptr(), maxf.data_ptr(), None)
+        assert st == capi.EPI_OK and int(count) == n
+        got = rows[:n].cpu().numpy().copy().view(capi.HIT_DTYPE).reshape(-1)
+        got = got[np.lexsort((got["snp2"], got["snp1"]))]
+        top = np.array([ex["max_f"][0], ex["max_f2"][0]])
+        if nid <= 2000:  # (above, too many pairs pass the screen at these thresholds: the plain kernel)
+            assert np.array_equal(got, want) and np.array_equal(maxf.cpu().numpy(), top)
+        else:
+            assert all(np.array_equal(got[f], want[f]) for f in ("snp1", "snp2", "df1", "df2"))
+            assert np.allclose(got["F"], want["F"], rtol=2e-5) and np.allclose(maxf.cpu().numpy(), top, rtol=2e-5)
