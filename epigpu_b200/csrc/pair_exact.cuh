@@ -103,6 +103,20 @@ __device__ __forceinline__ double missing_both_q(const ScanArgs &a, int t, int s
     return part;
 }
 
+template <class T>
+__device__ __forceinline__ T pick3(T x0, T x1, T x2, int idx)
+{
+    return idx == 0 ? x0 : (idx == 1 ? x1 : x2);
+}
+
+// approximate reciprocal of the screen (one MUFU operation, relative error ~2^-23; 1/0 = +inf)
+__device__ __forceinline__ float rcp_fast(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // x lowered by the screen's margin (relative 1e-3); -inf and NaN stay as they are
 __device__ __forceinline__ float screen_lo(float x) { return x - 1e-3f * fabsf(x); }
 

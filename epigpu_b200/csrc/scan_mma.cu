@@ -287,20 +287,6 @@ __device__ __forceinline__ uint32_t sel3(const uint32_t v[3], int idx)
     return idx == 0 ? v[0] : (idx == 1 ? v[1] : v[2]);
 }
 
-template <class T>
-__device__ __forceinline__ T pick3(T x0, T x1, T x2, int idx)
-{
-    return idx == 0 ? x0 : (idx == 1 ? x1 : x2);
-}
-
-// approximate reciprocal of the screen (one MUFU operation, relative error ~2^-23; 1/0 = +inf)
-__device__ __forceinline__ float rcp_fast(float x)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
 // The same statistics in FP32, as a screen: relative error ~1e-6 for the centred trait and
 // the exact integer cells this gets (no cancellation beyond SSW = Q - ... at large N).
 // A pair whose screened F and F2 are clearly below every threshold and below the running

@@ -27,12 +27,14 @@
 // likewise the counts, and Q = Qtot - QM_i - QM_j + QMM. Deriving the most frequent
 // genotypes keeps the FP32 sums to the smaller cells. Each thread owns 8 whole pairs (the
 // warp's 8 i-SNPs x the lane's j-SNP), so the reduction over individuals stays in registers.
-// Epilogue: FP64 SSB/SSI/F/F2 per pair (src/EpiOpenCL.c:231-247, :452-486), warp-aggregated
-// atomic hit append, per-trait maxima (warp-shuffle reductions).
+// Epilogue: an FP32 screen (upper bounds of F and F2) settles all pairs but those that may be a hit
+// or raise a maximum; for these FP64 SSB/SSI/F/F2 (src/EpiOpenCL.c:231-247, :452-486),
+// warp-aggregated atomic hit append, per-trait maxima (warp-shuffle reductions).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include "epi_internal.cuh"
+#include "pair_exact.cuh"
 #include "tc_ptx.cuh"
 
 namespace epi {
@@ -133,6 +135,74 @@ __device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairIn p)
         if (a.dump_df2) a.dump_df2[o] = s.d2;
     }
     return s;
+}
+
+// What the screen keeps of this lane's j-SNP for a tile: the marginals of its genotypes A, B and
+// most frequent one (count, sum of y) and the sum of y^2 over its missing calls.
+struct JSide {
+    float N[3], C[3], q;
+};
+
+// Upper bounds of one pair's F and F2 in FP32, from the same sums that eval_pair works with; rows
+// and columns in the order A, B, most frequent (F and F2 do not depend on it). SSB and SSI carry an
+// absolute error below 1e-5 of SSY here -- rounding of the marginals, of the cell means and of the
+// sums -- which is added; NaN where SSW is then below 1e-3 of SSY, too little to be told from it.
+// n2, s2: individuals missing at i by the j genotype in that order.
+__device__ __forceinline__ void upper_f32(const PairIn &p, const JSide &j, const float iN[2], const float iC[2], float iq,
+                                          float ysq, const float n3[3], const float s3[3], bool want_int, float &F,
+                                          float &F2)
+{
+    float n[9], S[9];
+    n[0] = (float)(p.C[0] & 0xffffu);
+    n[1] = (float)(p.C[0] >> 16);
+    n[3] = (float)(p.C[1] & 0xffffu);
+    n[4] = (float)(p.C[1] >> 16);
+    S[0] = p.S[0];
+    S[1] = p.S[1];
+    S[3] = p.S[2];
+    S[4] = p.S[3];
+    n[2] = iN[0] - n[0] - n[1] - (float)(p.C[2] & 0xffffu);
+    n[5] = iN[1] - n[3] - n[4] - (float)(p.C[2] >> 16);
+    S[2] = iC[0] - S[0] - S[1] - p.SJ[0];
+    S[5] = iC[1] - S[3] - S[4] - p.SJ[1];
+    float N = 0.0f, St = 0.0f, nfac = 0.0f, P = 0.0f;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+        n[6 + b] = j.N[b] - n[b] - n[3 + b] - n3[b];
+        S[6 + b] = j.C[b] - S[b] - S[3 + b] - s3[b];
+    }
+    float mc[9];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        S[c] = n[c] > 0.0f ? S[c] : 0.0f;  // (a derived sum of an empty cell holds rounding only)
+        N += n[c];
+        St += S[c];
+        nfac += n[c] > 0.0f ? 1.0f : 0.0f;
+        mc[c] = S[c] * rcp_fast(n[c] + 1e-30f);
+        P = fmaf(S[c], mc[c], P);
+    }
+    const float m = St * rcp_fast(N + 1e-30f), M = St * m;
+    const float Y = ysq - iq - j.q + p.sp.w - M, slack = 1e-5f * (Y + M);
+    const float SSB = P - M + slack, W = Y - SSB;
+    const float d1 = nfac - 1.0f, d2 = N - nfac;
+    const bool ok = W > 1e-3f * Y;
+    const float nan = __int_as_float(0x7fc00000);
+    F = ok ? SSB * d2 * rcp_fast(d1 * W) : nan;
+    F2 = 0.0f;
+    if (want_int) {
+        float row[3], col[3], SSI = slack;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            row[i] = (S[3 * i] + S[3 * i + 1] + S[3 * i + 2]) * rcp_fast(n[3 * i] + n[3 * i + 1] + n[3 * i + 2] + 1e-30f);
+            col[i] = (S[i] + S[3 + i] + S[6 + i]) * rcp_fast(n[i] + n[3 + i] + n[6 + i] + 1e-30f);
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            const float t = mc[c] - row[c / 3] - col[c % 3] + m;
+            SSI = fmaf(n[c] * t, t, SSI);
+        }
+        F2 = ok ? SSI * d2 * rcp_fast(4.0f * W) : nan;
+    }
 }
 
 __device__ __forceinline__ bool bit(uint32_t w, int t) { return (w >> t) & 1u; }
@@ -336,39 +406,73 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
 
         // epilogue
         const bool report = a.report_trait < 0 || a.report_trait == t;
+        const bool dumping = t == a.report_trait && (a.dump_counts || a.dump_F || a.dump_F2 || a.dump_df1 || a.dump_df2);
+        const float t1c = screen_lo(a.t1), t2c = screen_lo(a.t2);
+        const float ysq = (float)a.ysq[t];
+        JSide js;
+        {
+            const int gj = min(j0 + jl, bd.size2 - 1);
+            const size_t mj = (size_t)t * a.nsnp + bd.start2 + gj;
+            const int A = mjj == 0 ? 1 : 0, B = mjj == 2 ? 1 : 2;
+            js.N[0] = (float)a.pmN[3 * mj + A];
+            js.N[1] = (float)a.pmN[3 * mj + B];
+            js.N[2] = (float)a.pmN[3 * mj + mjj];
+            js.C[0] = (float)a.pmC[3 * mj + A];
+            js.C[1] = (float)a.pmC[3 * mj + B];
+            js.C[2] = (float)a.pmC[3 * mj + mjj];
+            js.q = (float)a.pmQ[mj];
+        }
         // unrolled: S and C are indexed by constants only, so they stay in registers
 #pragma unroll
         for (int ii = 0; ii < PI; ++ii) {
             const int gi = i0 + ib + ii, gj = j0 + jl;
             const bool valid = gi < bd.size1 && gj < bd.size2 && (bd.start1 + gi > bd.start2 + gj);
+            PairIn p;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p.S[c] = ii % 2 ? S[ii / 2][c].y : S[ii / 2][c].x;
+            const float2 sj = sm.spj[ii][tid];
+            p.SJ[0] = sj.x;
+            p.SJ[1] = sj.y;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) p.C[c] = C[ii][c];
+            p.sp = sm.sps[ii][tid];
+            p.spn = sm.spn[ii][tid];
+            p.maj = sm.maj[ib + ii];
+            p.majj = mjj;
+            p.trait = t;
+            p.si = bd.start1 + gi;
+            p.sj = bd.start2 + gj;
+            p.gi = gi;
+            p.gj = gj;
+            p.size2 = bd.size2;
+            bool exact = valid;
+            if (!dumping) {
+                const size_t mi = (size_t)t * a.nsnp + bd.start1 + min(gi, bd.size1 - 1);
+                const int A = p.maj == 0 ? 1 : 0, B = p.maj == 2 ? 1 : 2;
+                const float iN[2] = {(float)a.pmN[3 * mi + A], (float)a.pmN[3 * mi + B]};
+                const float iC[2] = {(float)a.pmC[3 * mi + A], (float)a.pmC[3 * mi + B]};
+                const float g0 = (float)(p.spn.x & 0xffffu), g1 = (float)(p.spn.x >> 16), g2 = (float)p.spn.y;
+                const float n3[3] = {mjj == 0 ? g1 : g0, mjj == 2 ? g1 : g2, pick3(g0, g1, g2, mjj)};
+                const float s3[3] = {mjj == 0 ? p.sp.y : p.sp.x, mjj == 2 ? p.sp.y : p.sp.z,
+                                     pick3(p.sp.x, p.sp.y, p.sp.z, mjj)};
+                float uF, uF2;
+                upper_f32(p, js, iN, iC, (float)a.pmQ[mi], ysq, n3, s3, a.test_int != 0, uF, uF2);
+                // the CTA's maxima so far are exact values and bound the final ones from below
+                const unsigned int m1 = reinterpret_cast<volatile unsigned int *>(mxf)[t];
+                const unsigned int m2 = a.test_int ? reinterpret_cast<volatile unsigned int *>(mxf2)[t] : 0u;
+                const float l1 = m1 ? screen_lo(ord2f(m1)) : -INFINITY, l2 = m2 ? screen_lo(ord2f(m2)) : -INFINITY;
+                exact = valid && (!(uF <= (report ? fminf(t1c, l1) : l1)) ||
+                                  (a.test_int && !(uF2 <= (report ? fminf(t2c, l2) : l2))));
+            }
+            if (!__any_sync(0xffffffffu, exact)) continue;
             PairStat s;
             s.nfac = s.d1 = s.d2 = 0;
             s.F = s.F2 = 0.0;
-            if (valid) {
-                PairIn p;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) p.S[c] = ii % 2 ? S[ii / 2][c].y : S[ii / 2][c].x;
-                const float2 sj = sm.spj[ii][tid];
-                p.SJ[0] = sj.x;
-                p.SJ[1] = sj.y;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) p.C[c] = C[ii][c];
-                p.sp = sm.sps[ii][tid];
-                p.spn = sm.spn[ii][tid];
-                p.maj = sm.maj[ib + ii];
-                p.majj = sm.majj[jl];
-                p.trait = t;
-                p.si = bd.start1 + gi;
-                p.sj = bd.start2 + gj;
-                p.gi = gi;
-                p.gj = gj;
-                p.size2 = bd.size2;
-                s = eval_pair(a, p);
-            }
-            const bool hit = valid && report && is_hit(a, s);
+            if (exact) s = eval_pair(a, p);
+            const bool hit = exact && report && is_hit(a, s);
             emit_hit(a, hit, bd.start1 + gi, bd.start2 + gj, s, t, blk);
-            fold_max(&mxf[t], valid, s.F);
-            if (a.test_int) fold_max(&mxf2[t], valid, s.F2);
+            fold_max(&mxf[t], exact, s.F);
+            if (a.test_int) fold_max(&mxf2[t], exact, s.F2);
         }
     }
     __syncthreads();
