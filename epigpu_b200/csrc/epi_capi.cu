@@ -57,12 +57,38 @@ cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int n
 bool mma_needs_x(int v, int screen);
 cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int screen,
                           int8_t *x, cudaStream_t stream);
-// Start of a scan: counters to zero, the per-trait maxima of F and F2 and the screen's lower
-// bounds of them to the order-encoded -inf.
+// Counters to zero, the per-trait maxima of F and F2 and the screen's lower bounds of them to the
+// order-encoded -inf: before the first scan of a context, and after its number of traits changed.
 __global__ void k_scan_init(unsigned long long *counters, unsigned int *maxf, int n)
 {
     if (threadIdx.x < NCOUNTERS) counters[threadIdx.x] = 0ull;
     for (int i = threadIdx.x; i < n; i += blockDim.x) maxf[i] = ENC_NEG_INF;
+}
+
+// End of a scan, one block: the counters, the maxima and the first FINISH_HITS hits written
+// straight into pinned host memory, then the counters and maxima reset for the next scan. Against
+// a reset kernel before the scan, two copies after it and a third, with a second
+// synchronisation, for the hits, a small scan's call is 15 us shorter (N = 500 x 2,000 SNPs).
+constexpr int FINISH_HITS = 1024;
+__global__ void __launch_bounds__(256) k_finish(unsigned long long *counters, unsigned int *maxf, int ntraits,
+                                                const DevHit *__restrict__ hits, long long cap,
+                                                unsigned long long *out_counters, DevHit *out_hits)
+{
+    static_assert(sizeof(DevHit) == 2 * sizeof(uint4), "copied in two words of 16 bytes");
+    const unsigned long long found = counters[0];
+    const int n = (int)min(min(found, (unsigned long long)cap), (unsigned long long)FINISH_HITS);
+    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x)
+        reinterpret_cast<uint4 *>(out_hits)[i] = reinterpret_cast<const uint4 *>(hits)[i];
+    unsigned int *const out_max = reinterpret_cast<unsigned int *>(out_counters + NCOUNTERS);
+    for (int i = threadIdx.x; i < 4 * ntraits; i += blockDim.x) {
+        if (i < 2 * ntraits) out_max[i] = maxf[i];
+        maxf[i] = ENC_NEG_INF;
+    }
+    __syncthreads();  // counters[0] read by every thread
+    if (threadIdx.x < NCOUNTERS) {
+        out_counters[threadIdx.x] = counters[threadIdx.x];
+        counters[threadIdx.x] = 0ull;
+    }
 }
 }  // namespace epi
 
@@ -136,6 +162,11 @@ struct epi_ctx {
     BlockDesc *h_blocks = nullptr;
     int h_blocks_cap = 0;
     unsigned char *h_arena = nullptr;
+    DevHit *h_hits = nullptr;  // its last part: the first hits of a scan, written by k_finish
+    // what the device holds: counters and maxima as k_finish leaves them for this many traits (0: to
+    // be initialised), and the block schedule
+    int clean_traits = 0;
+    std::vector<BlockDesc> dev_blocks;
     unsigned long long *h_state = nullptr;  // the counters, then 2 x ntraits encoded maxima
     size_t h_state_cap = 0;
     // the device part of the last scan, captured as a CUDA graph, and what it was captured for
@@ -191,7 +222,8 @@ static cudaError_t ensure_own(T **p, size_t *cap_bytes, size_t bytes, bool *own)
 
 // Pinned host memory of `count` elements: the arena's part for it, or an allocation of its own
 // where that is too small.
-constexpr size_t ARENA_STATE = 0, ARENA_INFO = 16384, ARENA_BLOCKS = 32768, ARENA_BYTES = 65536;
+constexpr size_t ARENA_STATE = 0, ARENA_INFO = 16384, ARENA_BLOCKS = 32768, ARENA_HITS = 65536,
+                 ARENA_BYTES = ARENA_HITS + epi::FINISH_HITS * sizeof(DevHit);
 template <class T, class N>
 static cudaError_t ensure_pinned(epi_ctx *ctx, T **p, N *cap, size_t count, size_t at, size_t end)
 {
@@ -273,6 +305,7 @@ epi_status epi_open(int32_t device, epi_ctx **out)
     ctx->sm_count = sms;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&ctx->h_arena, ARENA_BYTES, cudaHostAllocDefault);
+    if (e == cudaSuccess) ctx->h_hits = (DevHit *)(ctx->h_arena + ARENA_HITS);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
@@ -635,14 +668,16 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     }
     r.ntiles = base;
     size_t bcap = (size_t)ctx->blocks_cap * sizeof(BlockDesc);
+    if (bcap < (size_t)std::max(nblocks, 1) * sizeof(BlockDesc)) ctx->dev_blocks.clear();
     CK(ensure(&ctx->d_blocks, &bcap, (size_t)std::max(nblocks, 1) * sizeof(BlockDesc)));
     ctx->blocks_cap = (int)(bcap / sizeof(BlockDesc));
-    CK(ensure_pinned(ctx, &ctx->h_blocks, &ctx->h_blocks_cap, (size_t)nblocks, ARENA_BLOCKS, ARENA_BYTES));
+    CK(ensure_pinned(ctx, &ctx->h_blocks, &ctx->h_blocks_cap, (size_t)nblocks, ARENA_BLOCKS, ARENA_HITS));
     CK(ensure_pinned(ctx, &ctx->h_state, &ctx->h_state_cap, epi::NCOUNTERS + (size_t)ctx->ntraits, ARENA_STATE,
                      ARENA_INFO));
     if (ctx->maxf_cap < 4 * ctx->ntraits) {  // maxima, then the screen's lower bounds of them
         if (ctx->d_maxf) cudaFree(ctx->d_maxf);
         ctx->d_maxf = nullptr;
+        ctx->clean_traits = 0;
         CK(cudaMalloc((void **)&ctx->d_maxf, 4 * (size_t)ctx->ntraits * sizeof(unsigned int)));
         ctx->maxf_cap = 4 * ctx->ntraits;
     }
@@ -778,20 +813,16 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
 }
 
 // The device part of a scan, on the context's stream and nothing but stream operations (so it
-// can be captured): counters and maxima reset, the block schedule uploaded from pinned memory,
-// the selected form's persistent kernel between the timing events, and the counters and maxima
-// read back into pinned memory.
-cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, int nblocks, bool capturing)
+// can be captured): the selected form's kernels between the timing events, and k_finish, which
+// hands counters, maxima and the first hits to the host and resets them. What it expects on the
+// device (clean counters and maxima, the block schedule) launch_run has put there.
+cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, bool capturing)
 {
     cudaStream_t s = ctx->stream;
     // under stream capture the timing events are recorded as external records, which become
     // event nodes of the graph (so they time every replay); a direct launch records them plainly
     const unsigned int ev_flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-    epi::k_scan_init<<<1, 256, 0, s>>>(ctx->d_counters, ctx->d_maxf, 4 * ctx->ntraits);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && nblocks)
-        e = cudaMemcpyAsync(ctx->d_blocks, ctx->h_blocks, nblocks * sizeof(BlockDesc), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev0, s, ev_flags);
+    cudaError_t e = cudaEventRecordWithFlags(ctx->ev0, s, ev_flags);
     if (e == cudaSuccess && r.ntiles > 0) {
         if (r.form != EPI_FORM_TENSOR) e = epi::popc_enqueue(r.variant, r.args, ctx->pmaps, grid, s);
         else if (!r.screen) e = epi::mma_enqueue(r.variant, 0, r.args, ctx->maps, grid, s);
@@ -810,12 +841,11 @@ cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, int nblocks, 
         }
     }
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(ctx->ev1, s, ev_flags);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ctx->h_state, ctx->d_counters, epi::NCOUNTERS * sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(ctx->h_state + epi::NCOUNTERS, ctx->d_maxf, 2 * (size_t)ctx->ntraits * sizeof(unsigned int),
-                            cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) {
+        epi::k_finish<<<1, 256, 0, s>>>(ctx->d_counters, ctx->d_maxf, ctx->ntraits, r.args.hits, r.args.cap, ctx->h_state,
+                                        ctx->h_hits);
+        e = cudaGetLastError();
+    }
     return e;
 }
 
@@ -844,12 +874,25 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
             grid = (int)std::min<int64_t>(units, ctx->sm_count);
         }
     }
-    if (nblocks) memcpy(ctx->h_blocks, r.desc.data(), nblocks * sizeof(BlockDesc));
-    // the state reset and the scan kernel, or the screen and the exact kernel of every segment
+    if ((int)ctx->dev_blocks.size() < nblocks ||
+        memcmp(ctx->dev_blocks.data(), r.desc.data(), nblocks * sizeof(BlockDesc)) != 0) {
+        ctx->dev_blocks.clear();
+        memcpy(ctx->h_blocks, r.desc.data(), nblocks * sizeof(BlockDesc));
+        CK(cudaMemcpyAsync(ctx->d_blocks, ctx->h_blocks, nblocks * sizeof(BlockDesc), cudaMemcpyHostToDevice,
+                           ctx->stream));
+        ctx->dev_blocks = r.desc;
+    }
+    if (ctx->clean_traits != ctx->ntraits) {
+        epi::k_scan_init<<<1, 256, 0, ctx->stream>>>(ctx->d_counters, ctx->d_maxf, 4 * ctx->ntraits);
+        CK(cudaGetLastError());
+    }
+    ctx->clean_traits = 0;  // until the launch below has succeeded
+    // the scan kernel, or the screen and the exact kernel of every segment, and k_finish
     ctx->last_launches = 1 + (r.ntiles > 0 ? (r.screen ? 2 * r.segments : 1) : 0);
     ctx->last_form = r.form;
     if (!use_graph) {
-        CK(enqueue_scan(ctx, r, grid, nblocks, false));
+        CK(enqueue_scan(ctx, r, grid, false));
+        ctx->clean_traits = ctx->ntraits;
         return EPI_OK;
     }
     std::vector<unsigned char> key;
@@ -871,7 +914,7 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
         ctx->gexec = nullptr;
         ctx->gkey.clear();
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        const cudaError_t e = enqueue_scan(ctx, r, grid, nblocks, true);
+        const cudaError_t e = enqueue_scan(ctx, r, grid, true);
         cudaGraph_t g = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &g);  // ends the capture in any case
         if (e != cudaSuccess || e2 != cudaSuccess) {
@@ -885,6 +928,7 @@ epi_status launch_run(epi_ctx *ctx, ScanRun &r, int nblocks, bool use_graph)
         ctx->gkey = std::move(key);
     }
     CK(cudaGraphLaunch(ctx->gexec, ctx->stream));
+    ctx->clean_traits = ctx->ntraits;
     return EPI_OK;
 }
 
@@ -1076,9 +1120,13 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     ctx->last_pairs = pairs * ctx->ntraits;
 
     const unsigned int *mx = reinterpret_cast<const unsigned int *>(ctx->h_state + epi::NCOUNTERS);
-    std::vector<DevHit> dh((size_t)found);
-    if (found) {
-        CK(cudaMemcpyAsync(dh.data(), ctx->d_hits, (size_t)found * sizeof(DevHit), cudaMemcpyDeviceToHost,
+    // k_finish has brought the first hits; more come by a copy
+    std::vector<DevHit> copied;
+    const DevHit *dh = ctx->h_hits;
+    if (found > epi::FINISH_HITS) {
+        copied.resize((size_t)found);
+        dh = copied.data();
+        CK(cudaMemcpyAsync(copied.data(), ctx->d_hits, (size_t)found * sizeof(DevHit), cudaMemcpyDeviceToHost,
                            ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
     }
