@@ -360,8 +360,9 @@ __device__ __forceinline__ void advance(uint32_t &slot, uint32_t &phase)
 // indicators less the constant) and SSI that of a symmetric map of norm <= 1 (the cells' mean
 // less the row and column means plus the grand mean), so in units of D
 //     sqrt(SSB) <= sqrt(SSB_D) + E,     sqrt(SSI) <= sqrt(SSI_D) + E,
-// and likewise from below with - E. The sum of squares is exact up to the individuals missing
-// at both SNPs: Qtot - QM_i - QM_j <= Q <= Qtot - max(QM_i, QM_j). A pair whose upper bounds of
+// and likewise from below with - E (and the same of P, the squared norm of the projection onto the
+// cells' indicators with the constant: SSB = P - M). The sum of squares is exact up to the
+// individuals missing at both SNPs: Qtot - QM_i - QM_j <= Q <= Qtot - max(QM_i, QM_j). A pair whose upper bounds of
 // F and F2 stay below the thresholds and below the largest lower bounds met so far is neither
 // a hit nor a maximum; every other pair (about 1e-4 of them at the usual thresholds) goes to
 // the candidate list, which k_exact evaluates from the 24-bit digits. The bounds of FP32
@@ -394,13 +395,6 @@ __device__ __forceinline__ float2 int_float2(uint32_t x, uint32_t y)
     return add2(make_float2(__int_as_float((int)(x + 0x4B400000u)), __int_as_float((int)(y + 0x4B400000u))), m);
 }
 
-// The pair sums that the common path needs, per genotype row of the i-SNP and added up over
-// the triplet of lanes that holds the three rows: sum of S^2 / n, the count (plus 65,536 times
-// the number of occupied cells: both are exact together, below 2^24) and the sum.
-struct RowSums {
-    float2 P, NF, S;
-};
-
 // A lane's accumulator row of a round, the j-SNPs 3 r .. 3 r + 2 of each half (the last three
 // where fewer are left): v[h][TY c + (1 + SCR) b + s], the count (s = 0) and the digit sums of
 // genotype b of j-SNP c
@@ -431,10 +425,14 @@ __device__ __forceinline__ void cell2(const uint32_t v[2][3 * C::TY], int k, flo
     else S = fma2(md0, n, S);  // exactly 0 in an empty cell
 }
 
-// 2 X - R - C - M of the lane's pair in half h: SSI_D = P + this (all nine cells, gathered
-// from the triplet's rows; the rows' order does not matter)
+// All that the screen can tell of the lane's pair in half h, from its nine cells, gathered from the
+// triplet's rows (the rows' order does not matter): P, M, the count, the occupied cells, and
+// I0 = 2 X - R - C - M, so that SSI_D = P + I0
+struct Table {
+    float P, M, N, nf, I0;
+};
 template <class C>
-__device__ __forceinline__ float interaction(const uint32_t v[3 * C::TY], float d0, int ga, int s1, int s2)
+__device__ __forceinline__ Table gather_table(const uint32_t v[3 * C::TY], float d0, int ga, int s1, int s2)
 {
     const int o1 = (ga + 2) % 3, o2 = (ga + 1) % 3;  // the columns this lane offers the others
     float n[9], S[9];
@@ -452,13 +450,19 @@ __device__ __forceinline__ float interaction(const uint32_t v[3 * C::TY], float 
             else S[cell] = s == 1 ? 256.0f * f : S[cell] + f;
         }
     }
-    float cb[3], N = 0.f, St = 0.f, RC = 0.f, X = 0.f;
+    Table t = {0.f, 0.f, 0.f, 0.f, 0.f};
+    float cb[3], St = 0.f, RC = 0.f, X = 0.f;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        t.P = fmaf(S[c], S[c] * rcp_fast(n[c] + 1e-30f), t.P);
+        t.nf += n[c] > 0.0f ? 1.0f : 0.0f;
+    }
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
         const float nb = n[b] + n[3 + b] + n[6 + b], Sb = S[b] + S[3 + b] + S[6 + b];
         cb[b] = Sb * rcp_fast(nb + 1e-30f);
         RC = fmaf(Sb, cb[b], RC);
-        N += nb;
+        t.N += nb;
         St += Sb;
     }
 #pragma unroll
@@ -468,16 +472,20 @@ __device__ __forceinline__ float interaction(const uint32_t v[3 * C::TY], float 
         RC = fmaf(Sa, ra, RC);
         X = fmaf(ra, fmaf(n[3 * k + 2], cb[2], fmaf(n[3 * k + 1], cb[1], n[3 * k] * cb[0])), X);
     }
-    return fmaf(2.0f, X, -RC) - St * St * rcp_fast(N + 1e-30f);
+    t.M = St * St * rcp_fast(t.N + 1e-30f);
+    t.I0 = fmaf(2.0f, X, -RC) - t.M;
+    return t;
 }
 
 // One warp of the epilogue: its j rounds of every unit. A round is three j-SNPs of each B half
 // (columns 18 r of either half), so a lane forms the pairs (i, j0 + 3 r + ga) and
-// (i, j0 + 21 + 3 r + ga), the two halves side by side in packed FP32 (f32x2) operations. SSI
-// is at most SSB (the map above has norm <= 1 on the cells' means), so one sum over the cells
-// settles both tests for all but a few pairs in a thousand: each lane forms the sums of its own
-// genotype row for the three j-SNPs and the triplet adds them up, three values a pair instead of
-// twelve; all nine cells meet in one lane only where a pair passes (the columns are read again).
+// (i, j0 + 21 + 3 r + ga), the two halves side by side in packed FP32 (f32x2) operations. What all
+// pairs need is little. With P the sum of S^2 / n over the cells, SSW = Q - P and SSB = P - M <= P, SSI
+// is at most SSB (the map above has norm <= 1 on the cells' means) and d2 at most the trait's valid
+// individuals, so P and the number of occupied cells settle both tests for all but a few pairs
+// in a thousand: each lane forms them for its own genotype row and the three j-SNPs, and the triplet
+// adds them up, three values for the two pairs instead of 36. All nine cells meet in one lane only
+// where a pair passes (the columns are read again).
 template <class C>
 __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::Smem &sm, uint32_t tmem, uint32_t rank,
                                                 int pair, int npairs)
@@ -514,8 +522,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
             return report ? fminf(tc, l) : l;
         };
         float tF = threshold(lF, t1c), tI = ti ? 4.0f * threshold(lI, t2c) : INFINITY;
-        // SSY >= Q - (sqrt(M) + E)^2 >= Q - 2 M - 2 E^2
-        const float qi = qtot - qmi - 2.0f * E * E;
+        const float qi = qtot - qmi, nv = (float)a.nvalid[t];
         if (!tc::mbar_wait(&sm.acc_full[buf], (accph >> buf) & 1u, abort, a.wait_ns)) {
             fail(a, sm, 3);
             break;
@@ -541,22 +548,17 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
             uint32_t v[2][3 * C::TY];
             load_round<C>(acc, r, v);
             const float2 tiny = make_float2(1e-30f, 1e-30f), md0 = make_float2(-d0, -d0);
-            const float2 k64 = make_float2(65536.0f, 65536.0f);
-            RowSums w[3];
+            float2 P2[3], nf2[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                float2 nf = make_float2(0.f, 0.f), n = nf;
-                w[c].P = w[c].S = nf;
+                P2[c] = nf2[c] = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int b = 0; b < 3; ++b) {
                     float2 nb, Sb;
                     cell2<C>(v, C::TY * c + (1 + C::SCR) * b, md0, nb, Sb);
-                    w[c].P = fma2(Sb, mul2(Sb, rcp2(add2(nb, tiny))), w[c].P);
-                    w[c].S = add2(w[c].S, Sb);
-                    n = add2(n, nb);
-                    nf = add2(nf, make_float2(__saturatef(nb.x), __saturatef(nb.y)));
+                    P2[c] = fma2(Sb, mul2(Sb, rcp2(add2(nb, tiny))), P2[c]);
+                    nf2[c] = add2(nf2[c], make_float2(__saturatef(nb.x), __saturatef(nb.y)));
                 }
-                w[c].NF = fma2(nf, k64, n);
             }
             // the pair (i, j-SNP c = ga) is this lane's: each lane adds what the triplet's other
             // two offer it, the lane of row ga + 1 its column (ga + 1) + 2 = ga (mod 3)
@@ -565,53 +567,49 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                 const float for1 = is1 ? x0 : is2 ? x1 : x2, for2 = is1 ? x2 : is2 ? x0 : x1;
                 return own + __shfl_sync(0xffffffffu, for1, s1) + __shfl_sync(0xffffffffu, for2, s2);
             };
+            const float P[2] = {gather(P2[0].x, P2[1].x, P2[2].x), gather(P2[0].y, P2[1].y, P2[2].y)};
+            // occupied cells of both halves in one value, 16 nf1 + nf0 (nf <= 9)
+            const float nf01 = gather(fmaf(16.0f, nf2[0].y, nf2[0].x), fmaf(16.0f, nf2[1].y, nf2[1].x),
+                                      fmaf(16.0f, nf2[2].y, nf2[2].x));
+            // nf1 = (nf01 - 4.5) / 16 to the nearest integer, since 0 <= nf0 <= 9
+            const float nf1 = fmaf(nf01 - 4.5f, 0.0625f, 12582912.0f) - 12582912.0f;
+            const float nf[2] = {fmaf(-16.0f, nf1, nf01), nf1};
             bool cand[2];
-            float P[2], M[2], d1[2], d2[2], uB[2], W[2];
             bool any = false;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                auto x = [&](const float2 &y) { return h ? y.y : y.x; };
-                P[h] = gather(x(w[0].P), x(w[1].P), x(w[2].P));
-                const float St = gather(x(w[0].S), x(w[1].S), x(w[2].S));
-                const float NF = gather(x(w[0].NF), x(w[1].NF), x(w[2].NF));
-                // NF = 65536 nfac + N with N < 32768: nfac by rounding to the nearest integer
-                const float nf = fmaf(NF, 1.0f / 65536.0f, 12582912.0f) - 12582912.0f;
-                const float N = fmaf(-65536.0f, nf, NF);
-                M[h] = St * St * rcp_fast(N + 1e-30f);
-                d1[h] = nf - 1.0f;
-                d2[h] = N - nf;
-                // upper bound of SSB, lower bounds of SSY and SSW
-                const float sB = sqrt_fast(fmaxf(fmaf(P[h], 1.0f + SLK_B, -M[h]), 0.0f)) + E;
-                const float Y = fmaf(-2.0f, M[h], qi - qmj[h]);
-                uB[h] = sB * sB;
-                W[h] = Y - uB[h];
-                const float lhs = uB[h] * d2[h];
-                // one occupied cell: F is 0/0, never a hit or a maximum (F2 is 0); no individual:
-                // neither is defined. W too small a part of Y to be told from rounding: unknown
-                cand[h] = valid[h] && ((d1[h] > 0.0f && !(lhs <= tF * d1[h] * W[h])) ||
-                                       (d1[h] >= 0.0f && (!(W[h] > 1e-3f * Y) || !(lhs <= tI * W[h]))));
-                cand[h] = cand[h] && (ti || d1[h] > 0.0f);
-                W[h] = W[h] > 1e-3f * Y ? W[h] : __int_as_float(0x7fc00000);
+                const float sB = sqrt_fast(P[h] * (1.0f + SLK_B)) + E, u = sB * sB;  // >= P >= SSB >= SSI
+                const float Q = qi - qmj[h], W = Q - u, lhs = u * nv, d1 = nf[h] - 1.0f;
+                // one occupied cell: F is 0/0, never a hit or a maximum (F2 is 0); none: neither is
+                // defined. W too small a part of Q to be told from rounding: unknown
+                cand[h] = valid[h] && d1 >= (ti ? 0.0f : 1.0f) &&
+                          (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs <= tF * d1 * W)) || !(lhs <= tI * W));
                 any = any || cand[h];
             }
             if (__any_sync(0xffffffffu, any)) {
-                // raise the lower bounds of the maxima by this round's pairs first, then list the
-                // pairs that still matter
-                if (ti) load_round<C>(acc, r, v);
+                // tighter bounds from all nine cells; they raise the lower bounds of the maxima first,
+                // then the pairs that still matter are listed
+                load_round<C>(acc, r, v);
                 float fu[2], f2u[2];
                 unsigned int bF = 0u, bI = 0u;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const float I0 = ti ? interaction<C>(v[h], d0, ga, s1, s2) : 0.0f;
-                    const float sI = sqrt_fast(fmaxf(fmaf(P[h], 1.0f + SLK_I, I0), 0.0f)) + E;
-                    fu[h] = d1[h] > 0.0f ? uB[h] * d2[h] / (d1[h] * W[h]) : -INFINITY;
-                    f2u[h] = ti ? sI * sI * d2[h] / (4.0f * W[h]) : -INFINITY;
-                    const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(P[h], 1.0f - SLK_B, -M[h]), 0.0f)) - E, 0.0f);
-                    const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(P[h], 1.0f - SLK_I, I0), 0.0f)) - E, 0.0f);
-                    const float Wu = (qtot - fmaxf(qmi, qmj[h])) - lB * lB;  // SSW <= Q - SSB
-                    if (cand[h] && W[h] == W[h] && Wu > 0.0f) {
-                        if (d1[h] > 0.0f) bF = max(bF, f2ord(screen_lo(lB * lB * d2[h] / (d1[h] * Wu))));
-                        if (ti) bI = max(bI, f2ord(screen_lo(lo * lo * d2[h] / (4.0f * Wu))));
+                    const Table x = gather_table<C>(v[h], d0, ga, s1, s2);
+                    const float d1 = x.nf - 1.0f, d2 = x.N - x.nf, Q = qi - qmj[h];
+                    const float sP = sqrt_fast(x.P * (1.0f + SLK_B)) + E;
+                    const float sB = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_B, -x.M), 0.0f)) + E;
+                    const float sI = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_I, x.I0), 0.0f)) + E;
+                    const float W0 = Q - sP * sP, W = W0 > 1e-3f * Q ? W0 : __int_as_float(0x7fc00000);
+                    fu[h] = d1 > 0.0f ? sB * sB * d2 / (d1 * W) : -INFINITY;
+                    f2u[h] = ti ? sI * sI * d2 / (4.0f * W) : -INFINITY;
+                    // from below: SSB, SSI and, for SSW <= Q - P from above, P
+                    const float lP = fmaxf(sqrt_fast(x.P * (1.0f - SLK_B)) - E, 0.0f);
+                    const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_B, -x.M), 0.0f)) - E, 0.0f);
+                    const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_I, x.I0), 0.0f)) - E, 0.0f);
+                    const float Wu = (qtot - fmaxf(qmi, qmj[h])) - lP * lP;
+                    if (cand[h] && W == W && Wu > 0.0f) {
+                        if (d1 > 0.0f) bF = max(bF, f2ord(screen_lo(lB * lB * d2 / (d1 * Wu))));
+                        if (ti) bI = max(bI, f2ord(screen_lo(lo * lo * d2 / (4.0f * Wu))));
                     }
                 }
                 bF = __reduce_max_sync(0xffffffffu, bF);
