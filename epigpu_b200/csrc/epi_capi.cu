@@ -42,6 +42,7 @@ bool mma_available();
 int mma_tile_i();
 int mma_tile_j(int screen);
 int mma_x_rows(int screen);
+int mma_x_sets(int screen, int ntraits);
 int mma_min_nid();
 int mma_max_nid();
 int mma_screen_max_nid();
@@ -534,7 +535,7 @@ int pick_form(const epi_ctx *ctx, const epi_scan_opts *o)
 // 32 GiB and half the device's free memory (beyond, that variant is not a candidate).
 static size_t x_bytes(const epi_ctx *ctx, int screen)
 {
-    return (size_t)epi::mma_x_rows(screen) * ctx->nsnp * ctx->Np * ctx->ntraits;
+    return (size_t)epi::mma_x_rows(screen) * ctx->nsnp * ctx->Np * epi::mma_x_sets(screen, ctx->ntraits);
 }
 static bool x_usable(const epi_ctx *ctx, int screen)
 {
@@ -601,7 +602,21 @@ static double screen_share(const epi_ctx *ctx, const epi_scan_opts *o, double pa
     return share / ctx->ntraits;
 }
 
-// The digits of the screen for a scan of `pairs` pairs, or 0 for all digits without a screen. A
+// Whether the one-digit screen takes the traits in groups of five that share their counts (screen
+// 3): all have the same valid individuals, their groups take fewer tiles (a tile is 14 j-SNPs by
+// five traits against 42 by one: not for 1 to 3 or 6 traits), the expanded rows fit, and no other
+// kernel variant is asked for.
+static bool group_traits(const epi_ctx *ctx, const epi_scan_opts *o)
+{
+    const int T = ctx->ntraits, G = epi::GROUP_TRAITS;
+    if (o->tile_config != 0 && o->tile_config != 6) return false;
+    if (T <= 3 * ((T + G - 1) / G)) return false;
+    for (int t = 0; t < T; ++t)
+        if (ctx->h_info[t].same_mask == 0.0) return false;
+    return x_usable(ctx, 3);
+}
+
+// The digits of the screen for a scan of `pairs` pairs (3: one digit, grouped traits), or 0 for all digits without a screen. A
 // candidate costs about as much as 110 pairs of the one-digit screen (11 ns against 0.1 ns at
 // N = 10,000, both in proportion to N), a pair with two digits 1.5 and with all digits 2 of them:
 // so one digit up to a share of 1 in 250 (0.72 of the time with all digits there), two up to 1 in
@@ -614,7 +629,7 @@ static int screen_digits(const epi_ctx *ctx, const epi_scan_opts *o, double pair
     if (!(pairs >= 1.0) || ctx->Np > epi::mma_screen_max_nid()) return 0;
     const double tests = pairs * ctx->ntraits;
     const double one = screen_share(ctx, o, pairs, 1);
-    if (one <= 1.0 / 250.0 || one * tests <= 1024.0) return 1;
+    if (one <= 1.0 / 250.0 || one * tests <= 1024.0) return group_traits(ctx, o) ? 3 : 1;
     const double two = screen_share(ctx, o, pairs, 2);
     return two <= 1.0 / 400.0 || two * tests <= 1024.0 ? 2 : 0;
 }
@@ -701,7 +716,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
                 r.units += x <= 0 ? 0 : std::min<int64_t>(d.tiles_j, (x + TJ - 1) / TJ);
             }
         r.trait_units = r.units;
-        r.units *= ctx->ntraits;
+        r.units *= epi::mma_x_sets(screen, ctx->ntraits);
         if (r.units == 0) r.ntiles = 0;  // no pair at all
     }
     size_t cand = 0;  // bytes of the candidate list
@@ -831,8 +846,9 @@ cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, bool capturin
             for (int k = 0; k < r.segments && e == cudaSuccess; ++k) {
                 a.segment = k;
                 int64_t u0 = 0, u1 = 0;
-                a.seg0 = r.at(r.units / r.segments * k, ctx->ntraits, &u0);
-                a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), ctx->ntraits, &u1);
+                const int sets = epi::mma_x_sets(r.screen, ctx->ntraits);
+                a.seg0 = r.at(r.units / r.segments * k, sets, &u0);
+                a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), sets, &u1);
                 a.seg_units = u1 - u0;
                 if (a.seg_units == 0) continue;
                 e = epi::mma_enqueue(r.variant, r.screen, a, ctx->maps, grid, s);
@@ -983,6 +999,11 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     if (nv == 1) {
         *v = 0;
         *how = "only candidate";
+        return EPI_OK;
+    }
+    if (screen == 3) {  // grouped traits have one kernel
+        *v = 5;
+        *how = "8-bit screen, traits in groups";
         return EPI_OK;
     }
     // sample: an off-diagonal s x s block (every pair valid) when the genome holds one, with

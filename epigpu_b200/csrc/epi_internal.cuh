@@ -81,11 +81,15 @@ struct TraitArrays {
     float4 *tscr;
 };
 
-// Per trait, for the choice of the screen: the number of valid individuals and E / sigma of the
-// screen with one digit and with two (+inf where the trait has no variance).
+// Per trait, for the choice of the screen: the number of valid individuals, E / sigma of the
+// screen with one digit and with two (+inf where the trait has no variance), and whether its
+// valid individuals are those of the first trait.
 struct TraitInfo {
-    double nv, r1, r2;
+    double nv, r1, r2, same_mask;
 };
+
+// The screen with several traits a tile (scan_mma.cu): traits in a group.
+constexpr int GROUP_TRAITS = 5;
 
 // A place in the tensor form's order of units: the begin of a row group.
 struct SegPos {
@@ -100,7 +104,7 @@ struct Cand {
 };
 
 // epi_scan_block_noalloc goes through its block in parts of at most this many SNPs a side
-constexpr int RAW_SNPS = 2048;
+constexpr int RAW_SNPS = 3072;
 
 // 64-bit counters of a scan: hits found, tile queue (plain form), error flag and site, then
 // whether the candidate list overflowed, and from CNT_CAND on the candidates of each segment

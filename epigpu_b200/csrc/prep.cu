@@ -139,6 +139,9 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     const float *y = yraw + (size_t)t * nid;
     const uint8_t *vb = mode == VALID_BYTES ? valid + (size_t)t * nid : nullptr;
     auto ok = [&](int k) { return k < nid && (mode == VALID_ALL || (vb ? vb[k] != 0 : y[k] != -9.0f)); };
+    // trait 0's
+    auto ok0 = [&](int k) { return k < nid && (mode == VALID_ALL || (vb ? valid[k] != 0 : yraw[k] != -9.0f)); };
+    bool differs = false;
 
     double s0[2] = {0.0, 0.0};
     for (int k = tid; k < Np; k += nt) {  // (Np and the block are multiples of a warp)
@@ -149,7 +152,9 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
             s0[0] += (double)y[k];
             s0[1] += 1.0;
         }
+        differs = differs || v != ok0(k);
     }
+    differs = __syncthreads_or(differs);
     block_sum(s0, sv);
     const double nv = s0[1], mu = nv > 0.0 ? s0[0] / nv : 0.0;
 
@@ -230,6 +235,7 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     o.tscr[2 * t] = make_float4(dm, (float)(sqrt(e[0]) * (1.0 + 1e-6)), (float)q8, (float)(s * s));
     o.tscr[2 * t + 1] = make_float4(0.0f, (float)(sqrt(e16) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
     info[t].nv = nv;
+    info[t].same_mask = differs ? 0.0 : 1.0;
     info[t].r1 = q8 > 0.0 ? sqrt(e[0] * nv / q8) : INFINITY;
     info[t].r2 = q16 > 0.0 ? sqrt(e16 * nv / q16) : INFINITY;
 }
@@ -277,12 +283,13 @@ __global__ void k_qmiss(const uint32_t *__restrict__ missbits, int nsnp, int Wp,
 // The streamed-B variant's expanded B rows: row (u nsnp + s) R + r of the u-th set of R = 3 G rows
 // per SNP holds [g_s(k) == b] * digit(k) for every individual k, r = G b + i and digit the i-th of
 // the set's G digit rows -- the rows the tensor form's producers otherwise build in shared
-// memory. Full digits: two sets of G = 2 rows per trait, (w, d2) for CTA 0's half and (d1, d0) for
+// memory. GROUP: one set per group of five traits with the same mask, w and their D's (zero past
+// the last trait). Full digits: two sets of G = 2 rows per trait, (w, d2) for CTA 0's half and (d1, d0) for
 // CTA 1's; the screen: one set per trait, (w, D) or (w, d2, d1). ydig's rows per trait are D, w,
 // d2, d1, d0. One thread per 16 individuals of (set, s).
-template <int G, bool FULL>
+template <int G, bool FULL, bool GROUP = false>
 __global__ void k_expand(const uint8_t *__restrict__ hcodes, const int8_t *__restrict__ ydig, int nsnp, int Np,
-                         int sets, int8_t *__restrict__ x)
+                         int sets, int ntraits, int8_t *__restrict__ x)
 {
     const int nc = Np / 16;
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -295,8 +302,10 @@ __global__ void k_expand(const uint8_t *__restrict__ hcodes, const int8_t *__res
     uint4 d[G];
 #pragma unroll
     for (int i = 0; i < G; ++i) {
-        const int row = FULL ? 1 + 2 * (u & 1) + i : G == 2 ? 1 - i : 1 + i;
-        d[i] = reinterpret_cast<const uint4 *>(ydig + ((size_t)trait * 5 + row) * Np)[c];
+        const int row = FULL ? 1 + 2 * (u & 1) + i : GROUP ? (i == 0 ? 1 : 0) : G == 2 ? 1 - i : 1 + i;
+        const int tr = GROUP ? (G - 1) * u + (i == 0 ? 0 : i - 1) : trait;
+        d[i] = tr < ntraits ? reinterpret_cast<const uint4 *>(ydig + ((size_t)tr * 5 + row) * Np)[c]
+                            : make_uint4(0u, 0u, 0u, 0u);
     }
     uint4 *out = reinterpret_cast<uint4 *>(x + ((size_t)u * nsnp + s) * 3 * G * (size_t)Np) + c;
 #pragma unroll
@@ -441,13 +450,14 @@ cudaError_t launch_qmiss(const uint32_t *missbits, int nsnp, int Wp, const uint3
 cudaError_t launch_expand(const uint8_t *hcodes, const int8_t *ydig, int nsnp, int Np, int ntraits, int screen,
                           int8_t *x, cudaStream_t stream)
 {
-    const int sets = screen ? ntraits : 2 * ntraits;
+    const int sets = screen == 0 ? 2 * ntraits : screen == 3 ? (ntraits + GROUP_TRAITS - 1) / GROUP_TRAITS : ntraits;
     const long long total = (long long)sets * nsnp * (Np / 16);
     const int nt = 256;
     const unsigned nb = (unsigned)((total + nt - 1) / nt);
-    if (screen == 0) k_expand<2, true><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
-    else if (screen == 1) k_expand<2, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
-    else k_expand<3, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, x);
+    if (screen == 0) k_expand<2, true><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, ntraits, x);
+    else if (screen == 1) k_expand<2, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, ntraits, x);
+    else if (screen == 2) k_expand<3, false><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, ntraits, x);
+    else k_expand<GROUP_TRAITS + 1, false, true><<<nb, nt, 0, stream>>>(hcodes, ydig, nsnp, Np, sets, ntraits, x);
     return cudaGetLastError();
 }
 

@@ -151,13 +151,19 @@ static_assert(6 * 3 * (ROUNDS - 1) + RCOLS <= NH && bcol(11, TJ - 1) < N && bcol
 // (4-7, 16-19, 20-23) build A and B from them; CTA 0's full barrier counts the 8 producer warps of
 // a stage. 24 warps, launched with 80 registers each: epilogue 104, producers 72, the others 40
 // (59,392 of 61,440).
-template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false, int SCR_ = 0, bool RAW_ = false>
+//
+// GT > 1 (streamed B, one digit): traits with the same valid individuals in groups of GT. Their counts
+// are the same, so a j-SNP has 3 (1 + GT) column types for GT traits, w and their D's: 18 for five,
+// and a tile of 14 j-SNPs makes 70 tests per i-SNP instead of 42 (group_epilogue below).
+template <int S, int RSx, int EPW_ = 2, int PW_ = 1, bool XF_ = false, int SCR_ = 0, bool RAW_ = false, int GT_ = 1>
 struct Rings {
-    static constexpr int STAGES = S, RSTAGES = RSx, EPW = EPW_, PW = PW_, SCR = SCR_;
+    static constexpr int STAGES = S, RSTAGES = RSx, EPW = EPW_, PW = PW_, SCR = SCR_, GT = GT_;
     static constexpr bool XF = XF_, RAW = RAW_;
-    static constexpr int TY = SCR ? 3 * (1 + SCR) : TYH;  // column types of a j-SNP in a CTA's half
-    static constexpr int TJH = (TYH * TJ) / TY;           // j-SNPs in a half: 21 (all digits, one), 14 (two)
+    static_assert(GT == 1 || (XF && SCR == 1 && EPW == 2 && PW == 1), "grouped traits: streamed B, one digit");
+    static constexpr int TY = SCR ? 3 * (1 + SCR * GT) : TYH;  // column types of a j-SNP in a CTA's half
+    static constexpr int TJH = (TYH * TJ) / TY;  // j-SNPs in a half: 21 (all digits, one), 14 (two), 7 (groups)
     static constexpr int TJT = SCR ? 2 * TJH : TJ;        // j-SNPs per tile
+    using OneTrait = Rings<S, RSx, EPW_, PW_, XF_, SCR_, RAW_, 1>;
     static constexpr int RAW_ROWS = SCR == 0 ? ND : 1 + SCR;  // digit rows of a raw stage
     static constexpr uint32_t RAW_BYTES = (TJH + RAW_ROWS) * KS;
     static_assert(TY * TJH == TYH * TJ, "every variant fills 126 of a half's 128 rows");
@@ -384,6 +390,8 @@ __device__ __forceinline__ float sqrt_fast(float x)
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+
+__device__ __forceinline__ float int_float(uint32_t x) { return __int_as_float((int)(x + 0x4B400000u)) - 12582912.0f; }
 
 // Integers below 2^22 in magnitude as floats (exact): an integer addition into the mantissa of
 // 1.5 x 2^23 and a float subtraction. The conversion instruction runs on the pipe of the
@@ -646,6 +654,189 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                 if (ti) {
                     lI = max(lI, reinterpret_cast<volatile unsigned int *>(a.lowf2)[t]);
                     tI = 4.0f * threshold(lI, t2c);
+                }
+            }
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+            if (rank == 0) tc::mbar_arrive(&sm.acc_empty[buf]);
+            else tc::mbar_arrive_remote(&sm.acc_empty[buf], 0);
+        }
+        accph ^= 1u << buf;
+        buf ^= 1;
+    }
+}
+
+// The epilogue of grouped traits: as screen_epilogue, for GT traits at once. A round is three j-SNPs
+// of one half (all its columns: 3 TY); the counts, their reciprocals and the occupied cells are
+// formed once, then per trait P of the lane's own genotype row and the triplet's sum: about 90
+// operations per test against 150. A trait whose bounds pass goes through the nine cells one by one
+// (gather_table on its columns).
+template <class C>
+__device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Smem &sm, uint32_t tmem, uint32_t rank,
+                                               int pair, int npairs)
+{
+    constexpr int EPW = C::EPW, GT = C::GT, TY = C::TY, NC = 3 * TY;
+    constexpr int RND = (C::TJH + 2) / 3;  // rounds of a half
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int *abort = &sm.abort;
+    const int e = warp & 3, part = warp < 4 ? 0 : 1;
+    const int ii = 10 * e + lane / 3, ga = lane % 3, tbase = (lane / 3) * 3;
+    const int s1 = tbase + (ga + 1) % 3, s2 = tbase + (ga + 2) % 3;
+    const bool is1 = ga == 1, is2 = ga == 2;
+    const uint32_t tl = tmem + ((uint32_t)(32 * e) << 16);
+    const bool ti = a.test_int != 0;
+    const float t1c = screen_lo(a.t1), t2c = screen_lo(a.t2);
+    uint32_t accph = 0u;
+    int buf = 0;
+    auto gather = [&](float x0, float x1, float x2) {
+        const float own = is1 ? x1 : is2 ? x2 : x0;
+        const float for1 = is1 ? x0 : is2 ? x1 : x2, for2 = is1 ? x2 : is2 ? x0 : x1;
+        return own + __shfl_sync(0xffffffffu, for1, s1) + __shfl_sync(0xffffffffu, for2, s2);
+    };
+    for (Walker<C> un(a, pair, npairs); !un.done; un.next()) {
+        const int t0 = un.trait * GT, nt = min(GT, a.ntraits - t0);  // the group's traits
+        const int di = un.i0 + TI * (int)rank + ii;
+        const int gi = un.bd.start1 + di;
+        const bool ivalid = lane < 30 && di < un.bd.size1;
+        const float nv = (float)a.nvalid[t0];  // the same for the group
+        // thresholds per trait: the report threshold or the lower bound of the maximum
+        float tF[GT], tI[GT], qi[GT];
+        bool unknown = false;
+#pragma unroll
+        for (int g = 0; g < GT; ++g) {
+            const int t = t0 + min(g, nt - 1);
+            const float4 ts = a.tscr[2 * t];
+            const bool report = a.report_trait < 0 || a.report_trait == t;
+            const unsigned int lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
+            const unsigned int lI = ti ? reinterpret_cast<volatile unsigned int *>(a.lowf2)[t] : 0u;
+            const float bF = screen_lo(ord2f(lF)), bI = screen_lo(ord2f(lI));
+            tF[g] = report ? fminf(t1c, bF) : bF;
+            tI[g] = !ti ? INFINITY : 4.0f * (report ? fminf(t2c, bI) : bI);
+            qi[g] = ivalid ? ts.z - ts.w * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
+            unknown = unknown || lF == ENC_NEG_INF || (ti && lI == ENC_NEG_INF);
+        }
+        if (!tc::mbar_wait(&sm.acc_full[buf], (accph >> buf) & 1u, abort, a.wait_ns)) {
+            fail(a, sm, 3);
+            break;
+        }
+        tc::tc_fence_after();
+        const uint32_t acc = tl + acc_col(buf);
+        // (unknown maxima: the rounds run twice, as in screen_epilogue)
+        for (int pass = unknown ? 0 : 1; pass < 2; ++pass) {
+#pragma unroll 1
+            for (int q = part; q < 2 * RND; q += EPW) {
+                const int h = q / RND, r = q % RND;
+                const int jr = round_j<C>(r) + ga;  // the lane's j-SNP of the half
+                const int dj = un.j0 + C::TJH * h + jr, gj = un.bd.start2 + dj;
+                const bool valid = ivalid && jr >= 3 * r && dj < un.bd.size2 && gi > gj;
+                const uint32_t col = acc + h * NH + TY * round_j<C>(r);
+                uint32_t v[NC];
+                static_assert(NC == 54, "columns of a round: 32 + 16 + 4 + 2");
+                tc::tmem_ld32(col, v);
+                tc::tmem_ld16(col + 32, v + 32);
+                tc::tmem_ld4(col + 48, v[48], v[49], v[50], v[51]);
+                tc::tmem_ld2(col + 52, v + 52);
+                tc::tmem_wait_ld();
+                float n[3][3], rn[3][3], nf[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    nf[c] = 0.0f;
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        n[c][b] = int_float(v[TY * c + (1 + GT) * b]);
+                        rn[c][b] = rcp_fast(n[c][b] + 1e-30f);
+                        nf[c] += __saturatef(n[c][b]);
+                    }
+                }
+                const float d1 = gather(nf[0], nf[1], nf[2]) - 1.0f;
+                uint32_t cand = 0u;
+#pragma unroll
+                for (int g = 0; g < GT; ++g) {
+                    const int t = t0 + min(g, nt - 1);
+                    const float4 ts = a.tscr[2 * t];
+                    float P[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        P[c] = 0.0f;
+#pragma unroll
+                        for (int b = 0; b < 3; ++b) {
+                            const float S = fmaf(-ts.x, n[c][b], int_float(v[TY * c + (1 + GT) * b + 1 + g]));
+                            P[c] = fmaf(S, S * rn[c][b], P[c]);
+                        }
+                    }
+                    const float qmj = valid ? ts.w * a.qmf_j[(size_t)t * a.nsnp + gj] : 0.0f;
+                    const float sB = sqrt_fast(gather(P[0], P[1], P[2]) * (1.0f + SLK_B)) + ts.y, u = sB * sB;
+                    const float Q = qi[g] - qmj, W = Q - u, lhs = u * nv;
+                    const bool c = valid && g < nt && d1 >= (ti ? 0.0f : 1.0f) &&
+                                   (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs <= tF[g] * d1 * W)) || !(lhs <= tI[g] * W));
+                    if (c) cand |= 1u << g;
+                }
+                uint32_t some = __reduce_or_sync(0xffffffffu, cand);
+                while (some) {  // traits with a pair that passes, one after the other (rare)
+                    const int g = __ffs(some) - 1, t = t0 + g;
+                    some &= some - 1u;
+                    const float4 ts = a.tscr[2 * t];
+                    const float E = ts.y;
+                    // the trait's columns as a one-digit round: counts and D sums (read again, since the
+                    // trait is not known at compile time)
+                    uint32_t w[18];
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) {
+                        const uint32_t cc = col + TY * (k / 3) + (1 + GT) * (k % 3);
+                        tc::tmem_ld1(cc, w[2 * k]);
+                        tc::tmem_ld1(cc + 1 + g, w[2 * k + 1]);
+                    }
+                    tc::tmem_wait_ld();
+                    const Table x = gather_table<typename C::OneTrait>(w, ts.x, ga, s1, s2);
+                    const bool mine = cand >> g & 1u;
+                    const bool report = a.report_trait < 0 || a.report_trait == t;
+                    const float qm = ivalid ? ts.w * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
+                    const float qmj = valid ? ts.w * a.qmf_j[(size_t)t * a.nsnp + gj] : 0.0f;
+                    const float e1 = x.nf - 1.0f, d2 = x.N - x.nf, Q = ts.z - qm - qmj;
+                    const float sP = sqrt_fast(x.P * (1.0f + SLK_B)) + E;
+                    const float sB = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_B, -x.M), 0.0f)) + E;
+                    const float sI = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_I, x.I0), 0.0f)) + E;
+                    const float W0 = Q - sP * sP, W = W0 > 1e-3f * Q ? W0 : __int_as_float(0x7fc00000);
+                    const float fu = e1 > 0.0f ? sB * sB * d2 / (e1 * W) : -INFINITY;
+                    const float f2u = ti ? sI * sI * d2 / (4.0f * W) : -INFINITY;
+                    const float lP = fmaxf(sqrt_fast(x.P * (1.0f - SLK_B)) - E, 0.0f);
+                    const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_B, -x.M), 0.0f)) - E, 0.0f);
+                    const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_I, x.I0), 0.0f)) - E, 0.0f);
+                    const float Wu = (ts.z - fmaxf(qm, qmj)) - lP * lP;
+                    unsigned int bF = 0u, bI = 0u;
+                    if (mine && W == W && Wu > 0.0f) {
+                        if (e1 > 0.0f) bF = f2ord(screen_lo(lB * lB * d2 / (e1 * Wu)));
+                        if (ti) bI = f2ord(screen_lo(lo * lo * d2 / (4.0f * Wu)));
+                    }
+                    bF = __reduce_max_sync(0xffffffffu, bF);
+                    bI = __reduce_max_sync(0xffffffffu, bI);
+                    // what is known now of this trait's maxima, this round's pairs included
+                    unsigned int oF = 0u, oI = 0u;
+                    if (lane == 0) {
+                        oF = atomicMax(&a.lowf[t], bF);
+                        if (ti) oI = atomicMax(&a.lowf2[t], bI);
+                    }
+                    bF = max(bF, __shfl_sync(0xffffffffu, oF, 0));
+                    bI = max(bI, __shfl_sync(0xffffffffu, oI, 0));
+                    const float kF = screen_lo(ord2f(bF)), kI = screen_lo(ord2f(bI));
+                    const float hF = report ? fminf(t1c, kF) : kF, hI = report ? fminf(t2c, kI) : kI;
+#pragma unroll
+                    for (int k = 0; k < GT; ++k)
+                        if (k == g) {
+                            tF[k] = hF;
+                            if (ti) tI[k] = 4.0f * hI;
+                        }
+                    const bool c = mine && pass == 1 && (!(fu <= hF) || (ti && !(f2u <= hI)));
+                    const unsigned int mask = __ballot_sync(0xffffffffu, c);
+                    if (!mask) continue;
+                    const int leader = __ffs(mask) - 1;
+                    unsigned long long base = 0ull;
+                    if (lane == leader)
+                        base = atomicAdd(&a.counters[CNT_CAND + a.segment], (unsigned long long)__popc(mask));
+                    base = __shfl_sync(0xffffffffu, base, leader) + __popc(mask & ((1u << lane) - 1u));
+                    if (c && (long long)base < a.cand_cap) a.cand[base] = Cand{gi, gj, t, un.block, fu, f2u};
                 }
             }
         }
@@ -952,7 +1143,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             }
         }
     } else if (C::SCR && epi_warp) {
-        if constexpr (C::SCR != 0) screen_epilogue<C>(a, sm, tmem, rank, pair, npairs);
+        if constexpr (C::GT > 1) group_epilogue<C>(a, sm, tmem, rank, pair, npairs);
+        else if constexpr (C::SCR != 0) screen_epilogue<C>(a, sm, tmem, rank, pair, npairs);
     } else if (epi_warp) {
         // ---------------- epilogue: the j rounds split over the warps of each lane quarter ----------------
         // warps 0-3 (group 0), 8-11 (group 1), 16-19 (group 2): rounds [rb(g), rb(g + 1))
@@ -1320,6 +1512,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
 }  // namespace mma
 
 using Screen2Digits = mma::Rings<6, 6, 2, 1, false, 2>;
+using GroupRings = mma::Rings<7, 1, 2, 1, true, 1, false, GROUP_TRAITS>;
+struct GroupOf { using type = GroupRings; };
 
 // Tensor maps of the tensor form's TMA loads: the genotype-indicator rows h3 [3 nsnp][Np]
 // with 30-row boxes (A), the one-hot genotype bytes [nsnp][Np] with 16-row boxes (j side) and
@@ -1365,16 +1559,22 @@ cudaError_t mma_encode_traits(MmaMaps *maps, const int8_t *ydig, int ntraits, in
 // The streamed-B variant's expanded rows [ntraits][2][nsnp][6][Np], in boxes of one CTA half
 // of a j tile (21 SNPs x 6 types = 126 rows)
 // expanded rows per SNP and trait
-int mma_x_rows(int screen) { return screen ? 3 * (1 + screen) : mma::NTYPE; }
+int mma_x_rows(int screen) { return screen == 3 ? 3 * (1 + GROUP_TRAITS) : screen ? 3 * (1 + screen) : mma::NTYPE; }
+// sets of them: per trait, or per group of traits
+int mma_x_sets(int screen, int ntraits) { return screen == 3 ? (ntraits + GROUP_TRAITS - 1) / GROUP_TRAITS : ntraits; }
 
 cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits, int screen)
 {
-    return encode_2d(&maps->hx, x, (uint64_t)Np, (uint64_t)mma_x_rows(screen) * nsnp * ntraits, mma::TYH * mma::TJ);
+    return encode_2d(&maps->hx, x, (uint64_t)Np, (uint64_t)mma_x_rows(screen) * nsnp * mma_x_sets(screen, ntraits),
+                     mma::TYH * mma::TJ);
 }
 
 bool mma_available() { return true; }
 int mma_tile_i() { return mma::TIP; }  // the host tiles blocks by CTA-pair tiles
-int mma_tile_j(int screen) { return screen == 0 ? mma::TJ : screen == 1 ? 2 * mma::TJ : Screen2Digits::TJT; }
+int mma_tile_j(int screen)
+{
+    return screen == 0 ? mma::TJ : screen == 1 ? 2 * mma::TJ : screen == 2 ? Screen2Digits::TJT : GroupRings::TJT;
+}
 // The automatic choice takes this form from here on. Kernel time against the plain form, 8 df and
 // 4 df, B200: N = 64 x 2,000 SNPs 64 us and 320, N = 150 x 240 22 and 88, N = 231 x 2,003 69 and
 // 443, N = 126 x 30,000 6.3 ms and 61. With few individuals many pairs fit nearly perfectly and
@@ -1516,6 +1716,7 @@ static cudaError_t with_variant(int v, int screen, F f)
     case 0: return with_rings<0>(v, f);
     case 1: return with_rings<1>(v, f);
     case 2: return with_rings<2>(v, f);
+    case 3: return f(GroupOf());  // one variant only
     }
     return cudaErrorInvalidValue;
 }

@@ -4,7 +4,8 @@
 //
 // Two ways, chosen on the device. The tensor form's one-digit screen (scan_mma.cu: its RAW
 // variant builds both operands from the packed words; k_exact settles what it passes on) in parts
-// of 2,048 x 2,048 SNPs; and, where the screen would pass on too much (low thresholds, many
+// of 3,072 x 3,072 SNPs (the fixed array holds what either side needs per SNP, and a list of 8,000
+// candidates); and, where the screen would pass on too much (low thresholds, many
 // individuals) or its candidate list runs over, the plain kernel below. At 1,203 individuals x
 // 2,502 SNPs the plain kernel takes 4.7 ms, ten FP32 operations per pair and individual.
 //
@@ -326,7 +327,7 @@ struct ScreenScratch {  // screen: layouts as in epi_internal.cuh, one trait, on
     // per SNP of the part, i side then j side
     double qm[2 * RAW_SNPS], sm[2 * RAW_SNPS], nm[2 * RAW_SNPS];
     float qmf[2 * RAW_SNPS];
-    Cand cand[10000];
+    Cand cand[8000];
 };
 static_assert(sizeof(ScreenScratch) <= sizeof(Scratch), "both ways share the array");
 // read in words of 16 bytes (k_scan_popc: y, q; the screen: tscr, ydig)

@@ -274,7 +274,7 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t &a, uint32_t &
                  : "memory");
 }
 
-// 32 lanes x 16, 8, 2 or 1 consecutive columns
+// 32 lanes x 16, 32, 8, 2 or 1 consecutive columns
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *v)
 {
     asm volatile(
@@ -289,6 +289,19 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *v)
 __device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t *v)
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *v)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v)

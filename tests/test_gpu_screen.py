@@ -84,6 +84,19 @@ def test_variants_and_maxima(gpu_ctx, tile):
         assert _check(gpu_ctx, blocks, 3, "i", 1e6, 1e6, tile) == 0
 
 
+@pytest.mark.parametrize("ntraits", [4, 5, 8, 13])
+@pytest.mark.parametrize("sizes", [[15, 2], [81, 85, 1]], ids=str)
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_traits_with_one_mask_go_in_groups(gpu_ctx, ntraits, sizes, test):
+    """Traits with the same valid individuals, five to a group (a full group and a partial one)."""
+    nid = 700
+    blocks = _load(gpu_ctx, nid, sizes, ntraits, seed=ntraits, masks=False)
+    t1, t2 = synth.f_threshold(8, nid - 9, 1e-5), synth.f_threshold(4, nid - 9, 1e-5)
+    _check(gpu_ctx, blocks, ntraits, test, t1, t2, screened=True)
+    gpu_ctx.scan(blocks, capi.default_opts(test=test, t1=t1, t2=t2, form=capi.FORM_TENSOR), ntraits=ntraits)
+    assert "groups" in gpu_ctx.scan_config()
+
+
 @pytest.mark.parametrize("nid,screened", [(6017, True), (12200, None), (32641, False)])
 def test_many_individuals(gpu_ctx, nid, screened):
     blocks = _load(gpu_ctx, nid, [300, 41], 1, seed=nid, miss=0.02)
@@ -136,13 +149,13 @@ def test_automatic_form_of_few_individuals(gpu_ctx, nid, test):
 
 
 @pytest.mark.parametrize("nid,nsnp,block", [(17, 90, (0, 90, 0, 90)), (128, 130, (0, 130, 0, 130)),
-                                            (600, 2200, (0, 2200, 0, 2200)), (1203, 2150, (51, 2070, 3, 2147)),
+                                            (600, 3100, (0, 3100, 0, 3100)), (1203, 3200, (51, 3090, 3, 3197)),
                                             (2000, 300, (200, 100, 7, 150)), (9001, 201, (0, 201, 0, 201)),
                                             (32700, 50, (0, 50, 0, 50))], ids=str)
 @pytest.mark.parametrize("test", ["f", "i"])
 def test_block_scan_without_allocation(gpu_ctx, nid, nsnp, block, test):
     """epi_scan_block_noalloc builds the operands from the packed words (a full or a partial last
-    one) and goes through a block in parts of 2,048 SNPs: the rows and maxima of epi_scan, bit for
+    one) and goes through a block in parts of 3,072 SNPs: the rows and maxima of epi_scan, bit for
     bit where both go by the digits, within the parity bar where the plain kernel runs (32,700)."""
     import ctypes
     torch = pytest.importorskip("torch")
