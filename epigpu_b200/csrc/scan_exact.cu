@@ -86,27 +86,42 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
         for (int k = 0; k < 9; ++k)
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[k][r] = 0;
-        for (int k = lane; k < nc; k += 32) {
-            uint4 vi, vj;
+        // the chunks of the next step are fetched while this one's are worked on: a step waits about as
+        // long for its loads as it computes, and few candidates leave few warps to hide that
+        uint4 vi, vj, d[4];
+        uint32_t pi = 0u, pj = 0u;
+        auto fetch = [&](int k) {
+            if (k >= nc) return;
             if (RAW) {
-                const auto one_hot = [&](const uint32_t *row) {
-                    uint32_t sel[4];
-                    packed_selectors(packed_word(row, k, a.npack, a.remain), sel);
-                    return packed_lookup(PACKED_TABLE(1u, 2u, 4u, 0u), sel);
-                };
-                vi = one_hot(ri);
-                vj = one_hot(rj);
+                pi = packed_raw(ri, k, a.npack + (a.remain > 0));
+                pj = packed_raw(rj, k, a.npack + (a.remain > 0));
             } else {
                 vi = hi[k];
                 vj = hj[k];
             }
-            const uint4 d[4] = {dg[k], dg[nc + k], dg[2 * nc + k], dg[3 * nc + k]};
-            const uint32_t wi[4] = {vi.x, vi.y, vi.z, vi.w}, wj[4] = {vj.x, vj.y, vj.z, vj.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) d[r] = dg[r * nc + k];
+        };
+        fetch(lane);
+        for (int k = lane; k < nc; k += 32) {
+            uint4 ci = vi, cj = vj;
+            const uint4 e[4] = {d[0], d[1], d[2], d[3]};
+            if (RAW) {
+                const auto one_hot = [&](uint32_t w) {
+                    uint32_t sel[4];
+                    packed_selectors(packed_aligned(w, k, a.npack, a.remain), sel);
+                    return packed_lookup(PACKED_TABLE(1u, 2u, 4u, 0u), sel);
+                };
+                ci = one_hot(pi);
+                cj = one_hot(pj);
+            }
+            fetch(k + 32);
+            const uint32_t wi[4] = {ci.x, ci.y, ci.z, ci.w}, wj[4] = {cj.x, cj.y, cj.z, cj.w};
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 int dx[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) dx[r] = (int)(x == 0 ? d[r].x : x == 1 ? d[r].y : x == 2 ? d[r].z : d[r].w);
+                for (int r = 0; r < 4; ++r) dx[r] = (int)(x == 0 ? e[r].x : x == 1 ? e[r].y : x == 2 ? e[r].z : e[r].w);
 #pragma unroll
                 for (int g = 0; g < 3; ++g) {
                     const uint32_t mi = (wi[x] >> g) & 0x01010101u;
