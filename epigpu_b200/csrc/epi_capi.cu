@@ -532,7 +532,7 @@ int pick_form(const epi_ctx *ctx, const epi_scan_opts *o)
 
 // Builds the kernel arguments and tile schedule for `blocks` and uploads the schedule.
 // Bytes of the streamed-B variant's expanded rows, and whether they may be allocated: at most
-// 32 GiB and half the device's free memory (beyond, that variant is not a candidate).
+// 64 GiB and half the device's free memory (beyond, that variant is not a candidate).
 static size_t x_bytes(const epi_ctx *ctx, int screen)
 {
     return (size_t)epi::mma_x_rows(screen) * ctx->nsnp * ctx->Np * epi::mma_x_sets(screen, ctx->ntraits);
@@ -543,7 +543,7 @@ static bool x_usable(const epi_ctx *ctx, int screen)
     if (need <= ctx->x_cap) return true;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
-    return need <= (32ull << 30) && need <= fr / 2 + ctx->x_cap;
+    return need <= (64ull << 30) && need <= fr / 2 + ctx->x_cap;
 }
 
 // The streamed-B variant as an autotuner candidate: only up to 6,144 padded individuals. Its
@@ -1051,7 +1051,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
                                     : snprintf(buf + len, sizeof(buf) - len, "%s n/a", c ? " /" : "");
     *v = best;
     *how = buf;
-    // the streamed-B candidate's expanded rows (up to 32 GiB) are released when it lost
+    // the streamed-B candidate's expanded rows (up to 64 GiB) are released when it lost
     if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best, screen) && ctx->d_x && ctx->own_x) {
         CK(cudaStreamSynchronize(ctx->stream));
         cudaFree(ctx->d_x);
