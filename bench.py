@@ -513,22 +513,30 @@ def main():
         pairs_launch = pairs_step
         if used_form == "tensor":
             int8 = int8_peak_tops()
-            # algorithmic int8 ops per pair: 3 genotype rows x 12 column types (3 genotypes x
-            # {count, 3 y digits}) per individual; the 256 x 256 pair tile of 80 x 21 pairs
-            # carries 39.0 (8 padding rows per CTA, 4 zero columns)
-            ops_pair = 2.0 * 36.0 * nid
+            # int8 MACs per pair, individual and trait of the kernel that ran: 3 genotype rows x
+            # the column types of 3 genotypes -- the screen carries the count and one digit of
+            # the phenotype (two with 16 bits; the count and five traits' digits for five traits
+            # in groups), the kernel without it the count and three digits. A 256 x 256 pair
+            # tile issues 8% more (8 padding rows per CTA, 4 zero columns).
+            types = (6.0 / 5.0 if "in groups" in kernel_config else 2.0 if "8-bit screen" in kernel_config
+                     else 3.0 if "16-bit screen" in kernel_config else 4.0)
+            macs_pair = 9.0 * types
+            ops_pair = 2.0 * macs_pair * nid
             achieved = pairs_launch * ops_pair / kern_s / 1e12
-            # DRAM bytes per launch: the ncu capture of the same kernel on the cfg3m workload
-            # (N=10,000, M=20,000, operands larger than L2) read and wrote 16.89 GB for
-            # 199,990,000 pairs over Np = 10,112 padded individuals; the j rows are streamed
-            # once per i tile, so the bytes scale with pairs x Np
+            # DRAM bytes per launch: the ncu capture of the screen with streamed B and its exact
+            # kernel on the cfg3m workload (N=10,000, M=20,000, operands larger than L2) read and
+            # wrote 32.92 GB for 199,990,000 pairs over Np = 10,112 padded individuals; a
+            # super-tile's rows are read once, so the bytes scale with pairs x Np. Other kernels:
+            # not captured.
             np_pad = (nid + 127) // 128 * 128
-            traffic = 16.89e9 / (199990000.0 * 10112.0) * pairs_launch * np_pad
+            traffic = (32.92e9 / (199990000.0 * 10112.0) * pairs_launch * np_pad
+                       if "streamed from HBM" in kernel_config and "8-bit screen" in kernel_config and ntraits == 1
+                       else None)
             # peak: twice the dense bf16 rate of MEASURED_PEAKS.json (dense int8 runs at twice
             # bf16; the file holds no int8 figure); beside it, a cuBLAS int8 GEMM timed in this run
             bf16x2 = 2.0 * peaks["bf16_tflops"]
             roof = {"bound": "tensor", "achieved": achieved, "peak": bf16x2, "unit": "TOP/s",
-                    "frac": achieved / bf16x2,
+                    "frac": achieved / bf16x2, "int8_macs_per_pair_individual": macs_pair,
                     "peak_source": "2 x dense bf16 of MEASURED_PEAKS.json (%s, %.1f TFLOP/s burst)"
                                    % (peak_kind, peaks["bf16_tflops"]),
                     "cublas_int8_same_run": int8, "frac_of_cublas_int8_same_run": achieved / int8,
