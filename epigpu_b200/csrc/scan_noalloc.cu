@@ -58,13 +58,10 @@ __device__ __forceinline__ void count9(uint32_t c[5], const uint4 &p, const uint
     c[4] += __popc(p.z & r.z);
 }
 
-// Genotype bit-planes of 32 individuals (word w) of one SNP: from the library's plane array,
-// or, in the allocation-free variant, decoded straight from the reference's packed row
-// (src/readplink.c:1066-1102: MSB-first words, right-aligned tail word).
-template <bool RAW>
+// Genotype bit-planes of 32 individuals (word w) of one SNP, decoded from the reference's packed
+// row (src/readplink.c:1066-1102: MSB-first words, right-aligned tail word).
 __device__ __forceinline__ uint4 load_planes(const ScanArgs &a, int snp, int w)
 {
-    if (!RAW) return a.planes[(size_t)snp * a.Wp + w];
     const int npack1 = a.remain ? a.npack + 1 : a.npack;
     const uint32_t *row = reinterpret_cast<const uint32_t *>(a.gpack) + (size_t)snp * npack1;
     uint32_t p0 = 0, p1 = 0, p2 = 0;
@@ -116,16 +113,14 @@ __device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairAcc acc,
     return s;
 }
 
-// RAW = false: the library path (epi_scan). RAW = true: the allocation-free variant,
-// reading the reference's packed words and writing 24-byte rows (epi_scan_block_noalloc).
-template <bool RAW>
+// Runs when the screen did not or its list ran over (the array's overflow flag).
 __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = a.Wp / KW;
-    if (RAW && a.counters[CNT_OVERFLOW] == 0ull) return;  // the screen has done it
+    if (a.counters[CNT_OVERFLOW] == 0ull) return;  // the screen has done it
     // maxima of F and F2 per trait: per CTA in shared memory (flushed to global memory once,
     // at the end) up to SMAX_TRAITS traits, else the global maxima directly
     const bool smax_local = a.ntraits <= SMAX_TRAITS;
@@ -171,7 +166,7 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
                     const int i = tid >> 3, part = tid & 7;
                     const int gi = i0 + i;
                     uint4 P = make_uint4(0, 0, 0, 0);
-                    if (gi < bd.size1) P = load_planes<RAW>(a, bd.start1 + gi, w0 + (part >> 2));
+                    if (gi < bd.size1) P = load_planes(a, bd.start1 + gi, w0 + (part >> 2));
                     const float4 ya = *reinterpret_cast<const float4 *>(yt + k0 + 8 * part);
                     const float4 yb = *reinterpret_cast<const float4 *>(yt + k0 + 8 * part + 4);
                     const float yv[8] = {ya.x, ya.y, ya.z, ya.w, yb.x, yb.y, yb.z, yb.w};
@@ -189,13 +184,13 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
                 if (tid < KW * TI) {
                     const int w = tid / TI, i = tid % TI, gi = i0 + i;
                     uint4 P = make_uint4(0, 0, 0, 0);
-                    if (gi < bd.size1) P = load_planes<RAW>(a, bd.start1 + gi, w0 + w);
+                    if (gi < bd.size1) P = load_planes(a, bd.start1 + gi, w0 + w);
                     const uint32_t W = wt[w0 + w];
                     sm.pi[w][i] = make_uint4(P.x & W, P.y & W, P.z & W, 0u);
                 } else if (tid < KW * TI + KW * TJ) {
                     const int idx = tid - KW * TI, w = idx / TJ, j = idx % TJ, gj = j0 + j;
                     uint4 P = make_uint4(0, 0, 0, 0);
-                    if (gj < bd.size2) P = load_planes<RAW>(a, bd.start2 + gj, w0 + w);
+                    if (gj < bd.size2) P = load_planes(a, bd.start2 + gj, w0 + w);
                     sm.pj[w][j] = P;
                 } else if (tid < KW * TI + KW * TJ + KP) {
                     const int kp = tid - KW * TI - KW * TJ;
@@ -259,8 +254,7 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
                     s = eval_pair(a, acc, qc, t, gi, gj, bd.size2);
                 }
                 const bool hit = valid && report && is_hit(a, s);
-                if (RAW) emit_row(a, hit, bd.start1 + gi, bd.start2 + gj, s);
-                else emit_hit(a, hit, bd.start1 + gi, bd.start2 + gj, s, t, b);
+                emit_row(a, hit, bd.start1 + gi, bd.start2 + gj, s);
                 fold_max(&mxf[t], valid, s.F);
                 if (a.test_int) fold_max(&mxf2[t], valid, s.F2);
             }
@@ -570,7 +564,7 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
             return EPI_E_NODEVICE;
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
             return EPI_E_CUDA;
-        if (cudaFuncSetAttribute(popc_raw::k_scan_popc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        if (cudaFuncSetAttribute(popc_raw::k_scan_popc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
             return EPI_E_CUDA;
         noalloc::g_sms[dev] = sms;
@@ -687,7 +681,7 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     noalloc::k_prep<<<1, 1024, 0, st>>>(scr, d_phen, nid, Np, Wp, opts->safe, bd);
     if (ntiles > 0) {
         const int grid = (int)(ntiles < noalloc::g_sms[dev] ? ntiles : noalloc::g_sms[dev]);
-        popc_raw::k_scan_popc<true><<<grid, popc_raw::NT, smem, st>>>(a);
+        popc_raw::k_scan_popc<<<grid, popc_raw::NT, smem, st>>>(a);
     }
     noalloc::k_finish<<<1, 32, 0, st>>>(&scr->h, d_nhits, d_maxf, a.test_int);
     if (cudaGetLastError() != cudaSuccess || e != cudaSuccess) return EPI_E_CUDA;
