@@ -8,25 +8,33 @@
 // j-SNPs (planes of g==0, g==1, g==2, g!=3 per 32 individuals)
 // arrive by TMA, 64 individuals per stage, in a three-stage ring. Each SNP's two genotypes
 // other than its most frequent one are its dense genotypes A and B. Per stage:
-//   * expansion (all threads, double-buffered): for each i-SNP, U_A = [g_i==A]*y and
-//     U_B = [g_i==B]*y floats in shared memory, two i-SNPs side by side, with the
-//     phenotype-masked plane words of A, B and of the missing calls;
+//   * expansion (all threads, double-buffered): the phenotype-masked plane words of A, B and of the
+//     missing calls of each i-SNP, and 13 tables of 32 partial sums: entry e of table g is the sum of
+//     y over the individuals 5g + b whose bit b is set in e (the last table has four);
 //   * cell counts of the dense 2x2 cells and of the individuals missing at j: AND + __popc of
 //     32-bit plane words, 16-bit packed counters;
-//   * cell sums S_{Ai,Aj}, S_{Ai,Bj}, S_{Bi,Aj}, S_{Bi,Bj}: each lane holds its own j-SNP's
-//     plane words and adds the warp's broadcast U values into the cells its genotype bits
-//     select (4 FP32 adds per pair and individual, predicated by the bits; the bit of the
-//     lane's j-SNP is the same for two i-SNPs, so each predicated instruction is a packed
-//     f32x2 add serving two pairs, rounded like two scalar adds);
+//   * cell sums S_{Ai,Aj}, S_{Ai,Bj}, S_{Bi,Aj}, S_{Bi,Bj}: the same ANDed words, five individuals at
+//     a time, select an entry of each table. A lane holds entry `lane` of the 13 tables in
+//     registers, so a look-up is one shift and one warp shuffle (which reads the low five bits of its
+//     index) and one add; three chains of adds per cell;
 //   * individuals missing at the j-SNP (per lane, sparse): their sums by the i genotype;
 //   * individuals missing at the i-SNP (warp-uniform, sparse): their sums and counts by the
 //     j genotype, and the sum of y^2 of individuals missing at both SNPs.
+// Four FP32 adds per pair and individual, predicated by the bits, took 93 cycles of an SM per 32
+// individuals and 32 pairs (32 of them the packed adds, 16 the shared-memory broadcasts of the
+// i-SNP's values, much of the rest read-modify-writes of the sparse sums in shared memory). The
+// look-ups take 60 (26 shuffles, LSU at 55%, issue at 50%: bound by their latency chains), and the
+// sparse sums stand in registers, which four pairs per thread leave room for: 69 cycles at 1%
+// missing calls, 10.0 -> 7.4 ms at N = 4,000 x 4,001 SNPs. More warps with two pairs each (768 or
+// 1,024 threads), look-ups in shared memory instead of shuffles and for the individuals missing at j
+// measured 7.8 to 9.4 ms. Their partial sums of five add fewer roundings than one add per
+// individual.
 // The most frequent genotypes' row and column and the sum of squares come from per-(trait,
 // SNP) FP64 marginals in the epilogue: S_{a,Mj} = R_a(i) - S_{a,Aj} - S_{a,Bj} - S_{a,3}
 // (R_a(i) = sum of y over g_i = a), then S_{Mi,b} = C_b(j) - S_{Ai,b} - S_{Bi,b} - S_{3,b},
 // likewise the counts, and Q = Qtot - QM_i - QM_j + QMM. Deriving the most frequent
-// genotypes keeps the FP32 sums to the smaller cells. Each thread owns 8 whole pairs (the
-// warp's 8 i-SNPs x the lane's j-SNP), so the reduction over individuals stays in registers.
+// genotypes keeps the FP32 sums to the smaller cells. Each thread owns 4 whole pairs (the
+// warp's 4 i-SNPs x the lane's j-SNP), so the reduction over individuals stays in registers.
 // Epilogue: an FP32 screen (upper bounds of F and F2) settles all pairs but those that may be a hit
 // or raise a maximum; for these FP64 SSB/SSI/F/F2 (src/EpiOpenCL.c:231-247, :452-486),
 // warp-aggregated atomic hit append, per-trait maxima (warp-shuffle reductions).
@@ -52,19 +60,18 @@ struct Shape {
     static constexpr int KW = 2;              // 32-individual words per stage
     static constexpr int KI = 32 * KW;        // individuals per stage
     static constexpr int RS = 3;              // TMA ring depth
+    static constexpr int G = (KI + 4) / 5;    // tables of partial sums, five individuals each
     static constexpr uint32_t STAGE_BYTES = (TI + TJ) * KW * 16;  // transaction bytes per stage
-    static_assert(TI * KW <= NT - KI / 4 && TI <= 256 && TJ <= 256 && TI + TJ <= NT, "expansion roles");
+    static_assert(KW == 2 && 32 * G <= NT && TI * KW <= NT - KI / 4 && TI <= 256 && TJ <= 256 && TI + TJ <= NT,
+                  "expansion roles");
     static_assert(PI % 2 == 0, "i-SNPs in pairs (packed FP32 adds)");
 
     struct Smem {
         uint4 raw_i[RS][TI][KW];  // TMA: plane words of the i-tile (row = SNP)
         uint4 raw_j[RS][TJ][KW];  // TMA: plane words of the j-tile
-        float4 u[2][KI][TI / 2];  // (U_A, U_A', U_B, U_B') of i-SNPs 2p, 2p + 1 at individual k
+        float tab[2][G][32];      // sums of y over the subsets of five individuals
         uint4 pm[2][KW][TI];      // (P_A & W, P_B & W, missing & W, W) of each i-SNP
         float y[2][KI];           // the stage's trait values (0 where invalid)
-        float4 sps[PI][NT];       // per pair: sums over individuals missing at i by g_j: S_30..S_32, QMM
-        uint2 spn[PI][NT];        // and counts: n_30 | n_31 << 16, n_32
-        float2 spj[PI][NT];       // per pair: sums over individuals missing at j by g_i: S_{Ai,3}, S_{Bi,3}
         uint64_t full[RS];
         uint8_t maj[TI];          // most frequent genotype of each i-SNP
         uint8_t majj[TJ];         // and of each j-SNP
@@ -269,12 +276,6 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
         if (tid < TI) sm.maj[tid] = i0 + tid < bd.size1 ? a.maj[bd.start1 + i0 + tid] : (uint8_t)0;
         else if (tid < TI + TJ)
             sm.majj[tid - TI] = j0 + tid - TI < bd.size2 ? a.maj[bd.start2 + j0 + tid - TI] : (uint8_t)0;
-#pragma unroll
-        for (int ii = 0; ii < PI; ++ii) {
-            sm.sps[ii][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
-            sm.spn[ii][tid] = make_uint2(0u, 0u);
-            sm.spj[ii][tid] = make_float2(0.f, 0.f);
-        }
         auto issue = [&](int st) {  // thread 0: the TMA loads of stage st
             const int r = st % RS;
             tc::mbar_arrive_expect_tx(&sm.full[r], Sh::STAGE_BYTES);
@@ -285,25 +286,16 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
             for (int st = 0; st < min(RS, nst); ++st) issue(st);
         __syncthreads();  // maj
 
-        // expansion of stage st into buffer b: work item -> (pair of i-SNPs, 4 individuals),
-        // consecutive threads on consecutive i-SNP pairs (contiguous stores, the same trait
-        // words in a warp)
+        // expansion of stage st into buffer b
         auto expand = [&](int st, int b) {
             const int r = st % RS;
-            for (int it = tid; it < 8 * TI; it += NT) {
-                const int p = it % (TI / 2), part = it / (TI / 2), w = part >> 3, k4 = 4 * (part & 7);
-                const uint4 P0 = sm.raw_i[r][2 * p][w], P1 = sm.raw_i[r][2 * p + 1][w];
-                const int m0 = sm.maj[2 * p], m1 = sm.maj[2 * p + 1];
-                const uint32_t PA0 = m0 == 0 ? P0.y : P0.x, PB0 = m0 == 2 ? P0.y : P0.z;
-                const uint32_t PA1 = m1 == 0 ? P1.y : P1.x, PB1 = m1 == 2 ? P1.y : P1.z;
-                const float4 y4 = __ldg(reinterpret_cast<const float4 *>(yt + KI * st + 32 * w + k4));
-                const float yv[4] = {y4.x, y4.y, y4.z, y4.w};
+            if (tid < 32 * Sh::G) {
+                const int g = tid >> 5;
+                float v = 0.f;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int k = k4 + e;
-                    sm.u[b][32 * w + k][p] = make_float4(bit(PA0, k) ? yv[e] : 0.f, bit(PA1, k) ? yv[e] : 0.f,
-                                                         bit(PB0, k) ? yv[e] : 0.f, bit(PB1, k) ? yv[e] : 0.f);
-                }
+                for (int e = 0; e < 5; ++e)
+                    if (5 * g + e < KI && bit(lane, e)) v += __ldg(yt + KI * st + 5 * g + e);
+                sm.tab[b][g][lane] = v;
             }
             if (tid < TI * KW) {
                 const int i = tid % TI, w = tid / TI;
@@ -324,12 +316,18 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
 
         float2 S[PI / 2][4];  // the cell sums of i-SNPs ib + 2p (x) and ib + 2p + 1 (y)
         uint32_t C[PI][3];
+        float4 sps[PI];       // per pair: sums over individuals missing at i by g_j: S_30..S_32, QMM
+        uint2 spn[PI];        // and counts: n_30 | n_31 << 16, n_32
+        float2 spj[PI];       // per pair: sums over individuals missing at j by g_i: S_{Ai,3}, S_{Bi,3}
 #pragma unroll
         for (int ii = 0; ii < PI; ++ii) {
             if (ii % 2 == 0)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) S[ii / 2][c] = make_float2(0.f, 0.f);
             C[ii][0] = C[ii][1] = C[ii][2] = 0u;
+            sps[ii] = make_float4(0.f, 0.f, 0.f, 0.f);
+            spn[ii] = make_uint2(0u, 0u);
+            spj[ii] = make_float2(0.f, 0.f);
         }
         const int mjj = sm.majj[jl];  // this lane's j-SNP: its dense genotypes' planes
 
@@ -339,67 +337,97 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
                 wait_stage(st + 1);
                 expand(st + 1, b ^ 1);
             }
+            float T[Sh::G];  // this lane's entries of the tables
+#pragma unroll
+            for (int g = 0; g < Sh::G; ++g) T[g] = sm.tab[b][g][lane];
+            const uint4 pj[2] = {sm.raw_j[r][jl][0], sm.raw_j[r][jl][1]};
+            const uint32_t Xj[2][2] = {{mjj == 0 ? pj[0].y : pj[0].x, mjj == 0 ? pj[1].y : pj[1].x},   // A
+                                       {mjj == 2 ? pj[0].y : pj[0].z, mjj == 2 ? pj[1].y : pj[1].z}};  // B
+            const uint32_t Mj[2] = {~pj[0].w, ~pj[1].w};
+#pragma unroll
+            for (int q = 0; q < PI / 2; ++q) {
+                const uint4 pm[2][2] = {{sm.pm[b][0][ib + 2 * q], sm.pm[b][1][ib + 2 * q]},
+                                        {sm.pm[b][0][ib + 2 * q + 1], sm.pm[b][1][ib + 2 * q + 1]}};
+                // the dense cells: counts, and sums by look-up (all lanes of the warp are here)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t x[2][2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                        for (int w = 0; w < 2; ++w) x[e][w] = (c < 2 ? pm[e][w].x : pm[e][w].y) & Xj[c & 1][w];
+                        C[2 * q + e][c >> 1] += (uint32_t)(__popc(x[e][0]) + __popc(x[e][1])) << (16 * (c & 1));
+                    }
+                    float2 s[3];
+#pragma unroll
+                    for (int g = 0; g < Sh::G; ++g) {
+                        const int k = 5 * g;
+                        float2 v;
+                        v.x = __shfl_sync(0xffffffffu, T[g], (int)(k < 32 ? __funnelshift_r(x[0][0], x[0][1], k) : x[0][1] >> (k - 32)));
+                        v.y = __shfl_sync(0xffffffffu, T[g], (int)(k < 32 ? __funnelshift_r(x[1][0], x[1][1], k) : x[1][1] >> (k - 32)));
+                        if (g < 3) s[g] = v;
+                        else { s[g % 3].x += v.x; s[g % 3].y += v.y; }
+                    }
+                    s[0].x += s[1].x; s[0].y += s[1].y; s[0].x += s[2].x; s[0].y += s[2].y;
+                    S[q][c].x += s[0].x; S[q][c].y += s[0].y;
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int ii = 2 * q + e;
+                    // the sparse individuals missing at i
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        uint32_t m = pm[e][w].z;  // the same in every lane of the warp
+                        if (!m) continue;
+                        spn[ii].x += (uint32_t)__popc(m & pj[w].x) + ((uint32_t)__popc(m & pj[w].y) << 16);
+                        spn[ii].y += (uint32_t)__popc(m & pj[w].z);
 #pragma unroll 1
-            for (int w = 0; w < KW; ++w) {
-                const uint4 pj = sm.raw_j[r][jl][w];
-                const uint32_t PAj = mjj == 0 ? pj.y : pj.x, PBj = mjj == 2 ? pj.y : pj.z, Mj = ~pj.w;
-                // counts and the sparse individuals missing at i
-#pragma unroll
-                for (int ii = 0; ii < PI; ++ii) {
-                    const uint4 pm = sm.pm[b][w][ib + ii];
-                    C[ii][0] += __popc(pm.x & PAj) + (__popc(pm.x & PBj) << 16);
-                    C[ii][1] += __popc(pm.y & PAj) + (__popc(pm.y & PBj) << 16);
-                    C[ii][2] += __popc(pm.x & Mj) + (__popc(pm.y & Mj) << 16);
-                    uint32_t m = pm.z;  // the same in every lane of the warp
-                    while (m) {
-                        const int k = __ffs(m) - 1;
-                        m &= m - 1u;
-                        const float yv = sm.y[b][32 * w + k];
-                        const bool g0 = bit(pj.x, k), g1 = bit(pj.y, k), g2 = bit(pj.z, k);
-                        float4 acc = sm.sps[ii][tid];
-                        uint2 nn = sm.spn[ii][tid];
-                        acc.x += g0 ? yv : 0.f;
-                        acc.y += g1 ? yv : 0.f;
-                        acc.z += g2 ? yv : 0.f;
-                        acc.w += (g0 || g1 || g2) ? 0.f : yv * yv;
-                        nn.x += (g0 ? 1u : 0u) + (g1 ? 0x10000u : 0u);
-                        nn.y += g2 ? 1u : 0u;
-                        sm.sps[ii][tid] = acc;
-                        sm.spn[ii][tid] = nn;
-                    }
-                }
-                // individuals missing at this lane's j-SNP (and phenotype-valid): their sums by
-                // the i genotype (per lane; rare)
-                uint32_t mj = Mj & sm.pm[b][w][ib].w;
-                while (mj) {
-                    const int k = __ffs(mj) - 1;
-                    mj &= mj - 1u;
-                    const float yv = sm.y[b][32 * w + k];
-#pragma unroll
-                    for (int ii = 0; ii < PI; ++ii) {
-                        const uint2 pab = *reinterpret_cast<const uint2 *>(&sm.pm[b][w][ib + ii]);
-                        float2 acc = sm.spj[ii][tid];
-                        acc.x += bit(pab.x, k) ? yv : 0.f;
-                        acc.y += bit(pab.y, k) ? yv : 0.f;
-                        sm.spj[ii][tid] = acc;
-                    }
-                }
-                // sums: this lane's j genotype bit of individual k selects the cells the U
-                // values go to; one packed FP32 add serves two i-SNPs (the same j bit)
-#pragma unroll
-                for (int k = 0; k < 32; ++k) {
-                    const bool fA = bit(PAj, k), fB = bit(PBj, k);
-#pragma unroll
-                    for (int q = 0; q < PI / 2; ++q) {
-                        const float4 uu = sm.u[b][32 * w + k][ib / 2 + q];
-                        const float2 ua = make_float2(uu.x, uu.y), ub = make_float2(uu.z, uu.w);
-                        if (fA) S[q][0] = __fadd2_rn(S[q][0], ua);
-                        if (fB) S[q][1] = __fadd2_rn(S[q][1], ua);
-                        if (fA) S[q][2] = __fadd2_rn(S[q][2], ub);
-                        if (fB) S[q][3] = __fadd2_rn(S[q][3], ub);
+                        while (m) {
+                            const int k = __ffs(m) - 1;
+                            m &= m - 1u;
+                            const float yv = sm.y[b][32 * w + k];
+                            if (bit(pj[w].x, k)) sps[ii].x += yv;
+                            if (bit(pj[w].y, k)) sps[ii].y += yv;
+                            if (bit(pj[w].z, k)) sps[ii].z += yv;
+                            if (bit(Mj[w], k)) sps[ii].w = fmaf(yv, yv, sps[ii].w);
+                        }
                     }
                 }
             }
+            // individuals missing at this lane's j-SNP (and phenotype-valid): their sums by
+            // the i genotype (per lane; rare)
+            uint32_t mj = Mj[0] & sm.pm[b][0][ib].w, mj1 = Mj[1] & sm.pm[b][1][ib].w;
+            int w = 0;
+            if (!mj) {
+                mj = mj1;
+                mj1 = 0u;
+                w = 1;
+            }
+#pragma unroll 1
+            while (mj) {
+                const int k = __ffs(mj) - 1;
+                mj &= mj - 1u;
+                const float yv = sm.y[b][32 * w + k];
+                const uint4 *const row = &sm.pm[b][w][ib];
+                if (!mj) {
+                    mj = mj1;
+                    mj1 = 0u;
+                    w = 1;
+                }
+#pragma unroll
+                for (int ii = 0; ii < PI; ++ii) {
+                    const uint2 pab = *reinterpret_cast<const uint2 *>(row + ii);
+                    if (bit(pab.x, k)) {
+                        spj[ii].x += yv;
+                        C[ii][2] += 1u;
+                    }
+                    if (bit(pab.y, k)) {
+                        spj[ii].y += yv;
+                        C[ii][2] += 0x10000u;
+                    }
+                }
+            }
+            __syncwarp();
             __syncthreads();  // stage st consumed (its ring slot and U buffer), st + 1 expanded
             if (tid == 0 && st + RS < nst) issue(st + RS);
         }
@@ -430,13 +458,12 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
             PairIn p;
 #pragma unroll
             for (int c = 0; c < 4; ++c) p.S[c] = ii % 2 ? S[ii / 2][c].y : S[ii / 2][c].x;
-            const float2 sj = sm.spj[ii][tid];
-            p.SJ[0] = sj.x;
-            p.SJ[1] = sj.y;
+            p.SJ[0] = spj[ii].x;
+            p.SJ[1] = spj[ii].y;
 #pragma unroll
             for (int c = 0; c < 3; ++c) p.C[c] = C[ii][c];
-            p.sp = sm.sps[ii][tid];
-            p.spn = sm.spn[ii][tid];
+            p.sp = sps[ii];
+            p.spn = spn[ii];
             p.maj = sm.maj[ib + ii];
             p.majj = mjj;
             p.trait = t;
@@ -484,12 +511,12 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
 }  // namespace popc
 
 // The tile shapes the autotuner chooses among:
-//   0  64 x 64 tile, 8 pairs per thread (8 x 2 warps): fewest shared-memory loads per add
-//   1  64 x 32 tile, 4 pairs per thread (16 x 1 warps): fewest registers, most warps per i-SNP
-//   2  32 x 128 tile, 8 pairs per thread (4 x 4 warps): the i-side expansion shared by more lanes
-using Shape0 = popc::Shape<8, 2, 8>;
+//   0  32 x 64 tile (8 x 2 warps)
+//   1  64 x 32 tile (16 x 1 warps): the j side's words shared by more warps
+//   2  16 x 128 tile (4 x 4 warps): the i side's
+using Shape0 = popc::Shape<8, 2, 4>;
 using Shape1 = popc::Shape<16, 1, 4>;
-using Shape2 = popc::Shape<4, 4, 8>;
+using Shape2 = popc::Shape<4, 4, 4>;
 constexpr int POPC_SHAPES = 3;
 
 int popc_shapes() { return POPC_SHAPES; }
@@ -497,9 +524,9 @@ int popc_shapes() { return POPC_SHAPES; }
 // Tile size (i x j SNPs) and a description of shape v.
 void popc_shape(int v, int *ti, int *tj, const char **desc)
 {
-    static const char *names[POPC_SHAPES] = {"64x64 tile, 8 pairs/thread, 8x2 warps",
+    static const char *names[POPC_SHAPES] = {"32x64 tile, 4 pairs/thread, 8x2 warps",
                                              "64x32 tile, 4 pairs/thread, 16x1 warps",
-                                             "32x128 tile, 8 pairs/thread, 4x4 warps"};
+                                             "16x128 tile, 4 pairs/thread, 4x4 warps"};
     const int tis[POPC_SHAPES] = {Shape0::TI, Shape1::TI, Shape2::TI};
     const int tjs[POPC_SHAPES] = {Shape0::TJ, Shape1::TJ, Shape2::TJ};
     *ti = tis[v];
