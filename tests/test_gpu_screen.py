@@ -148,6 +148,27 @@ def test_automatic_form_of_few_individuals(gpu_ctx, nid, test):
     assert np.allclose(ex["max_f"], px["max_f"], rtol=2e-5 * kappa)
 
 
+@pytest.mark.parametrize("nid", [31, 59, 64, 66, 128, 191, 257])
+@pytest.mark.parametrize("miss", [0.0, 0.01, 0.4])
+@pytest.mark.parametrize("tile", [1, 2, 3])
+def test_plain_form_sums_by_look_up(gpu_ctx, nid, miss, tile):
+    """The plain form's cell sums (tables over five individuals, 13 a stage of 64) at the edges of the
+    tables, words and stages, without, with few and with many missing calls: the counts and degrees
+    of freedom of the tensor form's dump, F and F2 within 1e-5 of SSY in SSB, SSI and SSW."""
+    for block in _load(gpu_ctx, nid, [135, 70], 1, seed=nid, miss=miss):
+        want = gpu_ctx.scan_dump(block, capi.default_opts(test="i", form=capi.FORM_TENSOR))
+        got = gpu_ctx.scan_dump(block, capi.default_opts(test="i", form=capi.FORM_POPC, tile_config=tile))
+        s1, m1, s2, m2 = block
+        tri = (np.arange(m1)[:, None] + s1) > (np.arange(m2)[None, :] + s2)
+        for f in ("counts", "df1", "df2"):
+            assert np.array_equal(got[f][tri], want[f][tri])
+        ok = tri & (want["df1"] > 0) & (want["df2"] > 2)
+        d1, d2 = want["df1"][ok].astype(float), want["df2"][ok].astype(float)
+        kappa = 1.0 + want["F"][ok] * d1 / d2  # SSY / SSW
+        assert np.all(np.abs(got["F"][ok] - want["F"][ok]) <= 1e-5 * kappa ** 2 * d2 / d1 + 1e-6 * want["F"][ok])
+        assert np.all(np.abs(got["F2"][ok] - want["F2"][ok]) <= 1e-5 * kappa ** 2 * d2 / 4 + 1e-6 * want["F2"][ok])
+
+
 @pytest.mark.parametrize("nid,nsnp,block", [(17, 90, (0, 90, 0, 90)), (128, 130, (0, 130, 0, 130)),
                                             (600, 3100, (0, 3100, 0, 3100)), (1203, 3200, (51, 3090, 3, 3197)),
                                             (2000, 300, (200, 100, 7, 150)), (9001, 201, (0, 201, 0, 201)),
