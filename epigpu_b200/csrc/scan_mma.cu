@@ -25,6 +25,11 @@
 // grows, so the screen bounds them from above) and forms SSB / SSI / F / F2 in FP64 for every
 // pair that could be a hit or a new maximum.
 //
+// That is the kernel with all digits. The screen (SCR) carries only the count and one or two
+// 8-bit phenotype digits, bounds F and F2 (screen_epilogue) and lists the pairs it cannot
+// settle for k_exact (scan_exact.cu): 42 or 28 j-SNPs per tile instead of 21, or 14 j-SNPs by
+// five traits that share their counts (group_epilogue). RAW is the screen on the packed words.
+//
 // The GEMM runs on a CTA pair (a cluster of two CTAs on two SMs, tcgen05 cta_group::2): one
 // MMA of M = 256 rows (each CTA's 40 i-SNPs, 3 genotype rows each, in its own shared memory)
 // by N = 256 columns (the 252 columns of 21 j-SNPs plus 4 zero columns; each CTA holds and

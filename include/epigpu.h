@@ -79,8 +79,8 @@ typedef struct epi_scan_opts {
                             * launch; 1: every operation is launched directly */
     int32_t tile_config;   /* 0: the kernel variant (plain form: tile shape, 3 candidates;
                             * tensor form: ring depths, epilogue warps, producer groups and
-                            * streamed B, 6 candidates, streamed B only up to 6,144 padded
-                            * individuals) is chosen by the autotuner, which times every
+                            * streamed B, 6 candidates, streamed B only where its expanded
+                            * rows fit in memory) is chosen by the autotuner, which times every
                             * candidate on a sample block once per device, form, individual
                             * count and trait count; k >= 1: candidate k (epi_scan_config
                             * names it) */
@@ -178,8 +178,9 @@ epi_status epi_get_stream(const epi_ctx *ctx, void **stream);
  * For callers that cannot allocate GPU memory while they run: a service or real-time loop
  * that forbids cudaMalloc after start-up, or a host framework that hands out device memory
  * only from its own pool. Every input and output is a device buffer the caller owns; the
- * call makes no cudaMalloc, cudaFree or other allocating call. The plain popcount form
- * runs on the calling thread's current device, on `stream` (a cudaStream_t; NULL = the
+ * call makes no cudaMalloc, cudaFree or other allocating call. The tensor-core screen, or
+ * the plain popcount form where the screen would pass on too many pairs, runs on the
+ * calling thread's current device, on `stream` (a cudaStream_t; NULL = the
  * default stream), and the call returns once the scan has finished.
  *
  *   d_gpack  device, nsnp x (nid/16 + (nid%16 > 0)) int32: the reference's packed words
