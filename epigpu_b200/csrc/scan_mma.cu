@@ -438,6 +438,14 @@ __device__ __forceinline__ void cell2(const uint32_t v[2][3 * C::TY], int k, flo
     else S = fma2(md0, n, S);  // exactly 0 in an empty cell
 }
 
+// A lower bound of a trait's maximum, which other warps raise meanwhile: lane 0's reading for the whole
+// warp. Whether the rounds run twice (seed) hangs on it, and the rounds hold full-warp operations, so
+// lanes with different readings of it could end up in different passes.
+__device__ __forceinline__ unsigned int bound_now(const unsigned int *low)
+{
+    return __shfl_sync(0xffffffffu, *reinterpret_cast<const volatile unsigned int *>(low), 0);
+}
+
 // All that the screen can tell of the lane's pair in half h, from its nine cells, gathered from the
 // triplet's rows (the rows' order does not matter): P, M, the count, the occupied cells, and
 // I0 = 2 X - R - C - M, so that SSI_D = P + I0
@@ -528,8 +536,8 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
         const float *qmf_j = a.qmf_j + (size_t)t * a.nsnp;
         const float qmi = ivalid ? s2y * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
         const bool report = a.report_trait < 0 || a.report_trait == t;
-        unsigned int lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
-        unsigned int lI = ti ? reinterpret_cast<volatile unsigned int *>(a.lowf2)[t] : 0u;
+        unsigned int lF = bound_now(a.lowf + t);
+        unsigned int lI = ti ? bound_now(a.lowf2 + t) : 0u;
         auto threshold = [&](unsigned int low, float tc) {
             const float l = screen_lo(ord2f(low));
             return report ? fminf(tc, l) : l;
@@ -654,10 +662,10 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
             if (seed && r + 1 == r_end) {
                 seed = false;
                 r = r_begin - 1;
-                lF = max(lF, reinterpret_cast<volatile unsigned int *>(a.lowf)[t]);
+                lF = max(lF, bound_now(a.lowf + t));
                 tF = threshold(lF, t1c);
                 if (ti) {
-                    lI = max(lI, reinterpret_cast<volatile unsigned int *>(a.lowf2)[t]);
+                    lI = max(lI, bound_now(a.lowf2 + t));
                     tI = 4.0f * threshold(lI, t2c);
                 }
             }
@@ -714,8 +722,8 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
             const int t = t0 + min(g, nt - 1);
             const float4 ts = a.tscr[2 * t];
             const bool report = a.report_trait < 0 || a.report_trait == t;
-            const unsigned int lF = reinterpret_cast<volatile unsigned int *>(a.lowf)[t];
-            const unsigned int lI = ti ? reinterpret_cast<volatile unsigned int *>(a.lowf2)[t] : 0u;
+            const unsigned int lF = bound_now(a.lowf + t);
+            const unsigned int lI = ti ? bound_now(a.lowf2 + t) : 0u;
             const float bF = screen_lo(ord2f(lF)), bI = screen_lo(ord2f(lI));
             tF[g] = report ? fminf(t1c, bF) : bF;
             tI[g] = !ti ? INFINITY : 4.0f * (report ? fminf(t2c, bI) : bI);
