@@ -117,6 +117,14 @@ __device__ __forceinline__ float rcp_fast(float x)
     return r;
 }
 
+// approximate square root (relative error ~2^-23)
+__device__ __forceinline__ float sqrt_fast(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // x lowered by the screen's margin (relative 1e-3); -inf and NaN stay as they are
 __device__ __forceinline__ float screen_lo(float x) { return x - 1e-3f * fabsf(x); }
 

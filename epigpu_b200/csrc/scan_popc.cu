@@ -151,10 +151,18 @@ struct JSide {
 };
 
 // Upper bounds of one pair's F and F2 in FP32, from the same sums that eval_pair works with; rows
-// and columns in the order A, B, most frequent (F and F2 do not depend on it). SSB and SSI carry an
-// absolute error below 1e-5 of SSY here -- rounding of the marginals, of the cell means and of the
-// sums -- which is added; NaN where SSW is then below 1e-3 of SSY, too little to be told from it.
-// n2, s2: individuals missing at i by the j genotype in that order.
+// and columns in the order A, B, most frequent (F and F2 do not depend on it). n3, s3: individuals
+// missing at i by the j genotype in that order. What FP32 costs against eval_pair's FP64, with u = 2^-24:
+//   * the sum of squares Q is a difference of numbers up to the trait's whole one, ysq, however little
+//     of it the pair keeps (outliers that it misses): four values rounded to FP32 and three operations,
+//     below 6 u ysq = 3.6e-7 ysq;
+//   * the five derived cell sums are differences of marginals: each is good to 4 u (the most frequent
+//     cell 8 u) of the magnitudes it was formed from, together below E = 16 u B, B the sum of all of
+//     them. sqrt(P), sqrt(SSB) and sqrt(SSI), P the sum of S^2 / n, are norms of the cell sums or of
+//     maps of them of norm <= 1 (scan_mma.cu: the screen), so each is within E of its own;
+//   * forming P, M and SSI: below 1e-5 of Q.
+// NaN where SSW is then below 1e-3 of Q, too little to be told from the subtraction's rounding.
+constexpr float SLK_Q = 4e-7f, SLK_S = 1e-6f, SLK_P = 1e-5f;
 __device__ __forceinline__ void upper_f32(const PairIn &p, const JSide &j, const float iN[2], const float iC[2], float iq,
                                           float ysq, const float n3[3], const float s3[3], bool want_int, float &F,
                                           float &F2)
@@ -189,12 +197,17 @@ __device__ __forceinline__ void upper_f32(const PairIn &p, const JSide &j, const
         P = fmaf(S[c], mc[c], P);
     }
     const float m = St * rcp_fast(N + 1e-30f), M = St * m;
-    const float Y = ysq - iq - j.q + p.sp.w - M, slack = 1e-5f * (Y + M);
-    const float SSB = P - M + slack, W = Y - SSB;
+    const float Q = fmaf(-SLK_Q, ysq, ysq - iq - j.q + p.sp.w), slack = SLK_P * Q;
+    const float B = fabsf(iC[0]) + fabsf(iC[1]) + fabsf(j.C[0]) + fabsf(j.C[1]) + fabsf(j.C[2]) + fabsf(S[0]) +
+                    fabsf(S[1]) + fabsf(S[3]) + fabsf(S[4]) + fabsf(p.SJ[0]) + fabsf(p.SJ[1]) + fabsf(s3[0]) +
+                    fabsf(s3[1]) + fabsf(s3[2]);
+    const float E = SLK_S * B;
+    const float sP = sqrt_fast(P + slack) + E, sB = sqrt_fast(fmaxf(P - M + slack, 0.0f)) + E;
+    const float W = Q - sP * sP;  // (Q <= 0: NaN or negative)
     const float d1 = nfac - 1.0f, d2 = N - nfac;
-    const bool ok = W > 1e-3f * Y;
+    const bool ok = W > 1e-3f * Q;
     const float nan = __int_as_float(0x7fc00000);
-    F = ok ? SSB * d2 * rcp_fast(d1 * W) : nan;
+    F = ok ? sB * sB * d2 * rcp_fast(d1 * W) : nan;
     F2 = 0.0f;
     if (want_int) {
         float row[3], col[3], SSI = slack;
@@ -208,7 +221,8 @@ __device__ __forceinline__ void upper_f32(const PairIn &p, const JSide &j, const
             const float t = mc[c] - row[c / 3] - col[c % 3] + m;
             SSI = fmaf(n[c] * t, t, SSI);
         }
-        F2 = ok ? SSI * d2 * rcp_fast(4.0f * W) : nan;
+        const float sI = sqrt_fast(SSI) + E;
+        F2 = ok ? sI * sI * d2 * rcp_fast(4.0f * W) : nan;
     }
 }
 

@@ -39,3 +39,50 @@ def test_unknown_maxima_of_many_traits(gpu_ctx, masks):
         for t in range(0, ntraits, 9):
             F, F2, *_ = _dumped(gpu_ctx, block, "i", capi.FORM_TENSOR, trait=t)
             assert (ex["max_f"][t], ex["max_f2"][t]) == _maxima(F, F2, "i"), t
+
+
+def _check_thresholds(ctx, block, test, form, among, seed, n=24, config=None):
+    """Thresholds a relative 1e-4 below F of pairs drawn from `among` (a mask of the dumped pairs): each scan
+    must return that pair and all others above, and the dump's maxima."""
+    F, F2, df1, i, j = _dumped(ctx, block, test, form)
+    top = np.flatnonzero(among & (F > 0))
+    top = top[np.argsort(F[top])[-400:]]
+    for k in np.random.default_rng(seed).choice(top, n, replace=False):
+        t1 = np.float32(F[k] * np.float32(1.0 - 1e-4))
+        hits, total, ex = ctx.scan([block], capi.default_opts(test=test, form=form, t1=t1, t2=1e30))
+        if config is not None:
+            assert config in ctx.scan_config()
+        want = (F > t1) & ((df1 > 5) if test == "i" else True)
+        got = set(zip(hits["snp1"], hits["snp2"], hits["F"]))
+        assert total == want.sum() and got == set(zip(i[want], j[want], F[want]))
+        assert (ex["max_f"][0], ex["max_f2"][0]) == _maxima(F, F2, test)
+
+
+@pytest.mark.parametrize("test", ["f", "i"])
+@pytest.mark.parametrize("nid,sd", [(1000, 3e3), (1000, 1e4), (4000, 3e4)])
+def test_plain_form_with_outliers_that_pairs_miss(gpu_ctx, nid, sd, test):
+    """Two opposite outliers hold nearly all of the trait's sum of squares; a pair that misses one at
+    either SNP keeps a millionth of it and less. No hit and no maximum may be lost."""
+    nsnp = 240
+    codes = synth.genotype_codes(nid, nsnp, seed=nid, miss=0.0)
+    codes[:nsnp // 2, 0], codes[nsnp // 2:, 1] = 3, 3
+    y = np.random.default_rng(nid + 1).standard_normal(nid)
+    y[0], y[1] = sd, -sd
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_phenotype(y.astype(np.float32))
+    block = (0, nsnp, 0, nsnp)
+    *_, i, j = _dumped(gpu_ctx, block, test, capi.FORM_POPC)
+    _check_thresholds(gpu_ctx, block, test, capi.FORM_POPC, (i >= nsnp // 2) & (j < nsnp // 2), 5)
+
+
+@pytest.mark.parametrize("miss", [0.4, 0.97])
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_plain_form_with_many_missing_calls(gpu_ctx, miss, test):
+    nid, nsnp = 1500, 200
+    codes = synth.genotype_codes(nid, nsnp, seed=17, miss=0.0)
+    codes[nsnp // 2:][np.random.default_rng(18).random((nsnp - nsnp // 2, nid)) < miss] = 3
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_phenotype(np.random.default_rng(19).standard_normal(nid).astype(np.float32))
+    block = (0, nsnp, 0, nsnp)
+    *_, i, j = _dumped(gpu_ctx, block, test, capi.FORM_POPC)
+    _check_thresholds(gpu_ctx, block, test, capi.FORM_POPC, (i >= nsnp // 2) & (j < nsnp // 2), 6)
