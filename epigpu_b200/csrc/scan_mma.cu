@@ -378,12 +378,14 @@ __device__ __forceinline__ void advance(uint32_t &slot, uint32_t &phase)
 // a hit nor a maximum; every other pair (about 1e-4 of them at the usual thresholds) goes to
 // the candidate list, which k_exact evaluates from the 24-bit digits. The bounds of FP32
 // rounding: P, R, C, M and X below are sums of squares of the centred trait's cell sums, each
-// at most P in magnitude and good to ~1e-6 of it, hence the slack SLK_B and SLK_I; the
-// thresholds are lowered by a relative 1e-3, which covers the rest.
+// at most P in magnitude and good to ~1e-6 of it, hence the slack SLK_B and SLK_I. Q is a difference
+// of floats up to Qtot, however little of it the pair keeps: six roundings, below 6 x 2^-24 Qtot, hence
+// SLK_Q (E is no cover for it: it is 0 for a trait of two values). The thresholds are lowered by a
+// relative 1e-3, which covers the rest.
 //
 // Six column types (nine) instead of twelve per j-SNP: a pair MMA serves 80 x 42 (28) pairs
 // instead of 80 x 21.
-constexpr float SLK_B = 4e-6f, SLK_I = 1.2e-5f;
+constexpr float SLK_B = 4e-6f, SLK_I = 1.2e-5f, SLK_Q = 4e-7f;
 
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -537,7 +539,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
             return report ? fminf(tc, l) : l;
         };
         float tF = threshold(lF, t1c), tI = ti ? 4.0f * threshold(lI, t2c) : INFINITY;
-        const float qi = qtot - qmi, nv = (float)a.nvalid[t];
+        const float qi = fmaf(-SLK_Q, qtot, qtot - qmi), nv = (float)a.nvalid[t];
         if (!tc::mbar_wait(&sm.acc_full[buf], (accph >> buf) & 1u, abort, a.wait_ns)) {
             fail(a, sm, 3);
             break;
@@ -621,7 +623,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                     const float lP = fmaxf(sqrt_fast(x.P * (1.0f - SLK_B)) - E, 0.0f);
                     const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_B, -x.M), 0.0f)) - E, 0.0f);
                     const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_I, x.I0), 0.0f)) - E, 0.0f);
-                    const float Wu = (qtot - fmaxf(qmi, qmj[h])) - lP * lP;
+                    const float Wu = fmaf(SLK_Q, qtot, qtot - fmaxf(qmi, qmj[h])) - lP * lP;
                     if (cand[h] && W == W && Wu > 0.0f) {
                         if (d1 > 0.0f) bF = max(bF, f2ord(screen_lo(lB * lB * d2 / (d1 * Wu))));
                         if (ti) bI = max(bI, f2ord(screen_lo(lo * lo * d2 / (4.0f * Wu))));
@@ -721,7 +723,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
             const float bF = screen_lo(ord2f(lF)), bI = screen_lo(ord2f(lI));
             tF[g] = report ? fminf(t1c, bF) : bF;
             tI[g] = !ti ? INFINITY : 4.0f * (report ? fminf(t2c, bI) : bI);
-            qi[g] = ivalid ? ts.z - ts.w * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
+            qi[g] = ivalid ? fmaf(-SLK_Q, ts.z, ts.z - ts.w * a.qmf[(size_t)t * a.nsnp + gi]) : 0.0f;
             unknown = unknown || lF == ENC_NEG_INF || (ti && lI == ENC_NEG_INF);
         }
         if (!tc::mbar_wait(&sm.acc_full[buf], (accph >> buf) & 1u, abort, a.wait_ns)) {
@@ -801,7 +803,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
                     const bool report = a.report_trait < 0 || a.report_trait == t;
                     const float qm = ivalid ? ts.w * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
                     const float qmj = valid ? ts.w * a.qmf_j[(size_t)t * a.nsnp + gj] : 0.0f;
-                    const float e1 = x.nf - 1.0f, d2 = x.N - x.nf, Q = ts.z - qm - qmj;
+                    const float e1 = x.nf - 1.0f, d2 = x.N - x.nf, Q = fmaf(-SLK_Q, ts.z, ts.z - qm) - qmj;
                     const float sP = sqrt_fast(x.P * (1.0f + SLK_B)) + E;
                     const float sB = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_B, -x.M), 0.0f)) + E;
                     const float sI = sqrt_fast(fmaxf(fmaf(x.P, 1.0f + SLK_I, x.I0), 0.0f)) + E;
@@ -811,7 +813,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
                     const float lP = fmaxf(sqrt_fast(x.P * (1.0f - SLK_B)) - E, 0.0f);
                     const float lB = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_B, -x.M), 0.0f)) - E, 0.0f);
                     const float lo = fmaxf(sqrt_fast(fmaxf(fmaf(x.P, 1.0f - SLK_I, x.I0), 0.0f)) - E, 0.0f);
-                    const float Wu = (ts.z - fmaxf(qm, qmj)) - lP * lP;
+                    const float Wu = fmaf(SLK_Q, ts.z, ts.z - fmaxf(qm, qmj)) - lP * lP;
                     unsigned int bF = 0u, bI = 0u;
                     if (mine && W == W && Wu > 0.0f) {
                         if (e1 > 0.0f) bF = f2ord(screen_lo(lB * lB * d2 / (e1 * Wu)));

@@ -86,3 +86,36 @@ def test_plain_form_with_many_missing_calls(gpu_ctx, miss, test):
     block = (0, nsnp, 0, nsnp)
     *_, i, j = _dumped(gpu_ctx, block, test, capi.FORM_POPC)
     _check_thresholds(gpu_ctx, block, test, capi.FORM_POPC, (i >= nsnp // 2) & (j < nsnp // 2), 6)
+
+
+@pytest.mark.parametrize("nid,ntraits,config", [(30700, 1, "8-bit screen"), (30700, 4, "groups"), (15000, 1, "16-bit screen")])
+def test_screen_with_snps_of_a_dozen_calls(gpu_ctx, nid, ntraits, config):
+    """SNPs known in a dozen individuals against SNPs known in all, where the screen's phenotype is exact
+    (two values) or nearly (16 bits): a pair's sum of squares is a difference of floats thousands of
+    times its size, and E widens the bounds by next to nothing. (The counts of the two values, 15,271 of
+    30,700 and 6 of 12, leave Q 2.4e-4 too large.)"""
+    sparse, full, calls = 150, 210, 12
+    codes = synth.genotype_codes(nid, sparse + full, seed=nid, miss=0.0)
+    rng = np.random.default_rng(nid + 1)
+    y = rng.standard_normal(nid)
+    high = y >= np.sort(y)[-15271] if nid == 30700 else y >= 0
+    if nid == 30700:
+        y = np.where(high, 1.0, -1.0)
+    for s in range(sparse):
+        keep = np.concatenate([rng.choice(np.flatnonzero(high == h), calls // 2, replace=False) for h in (True, False)])
+        gone = np.ones(nid, dtype=bool)
+        gone[keep] = False
+        codes[s, gone] = 3
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_traits(np.repeat(y[:, None], ntraits, 1).astype(np.float32))
+    block = (0, sparse + full, 0, sparse + full)
+    F, F2, df1, i, j = _dumped(gpu_ctx, block, "f", capi.FORM_TENSOR)
+    values = np.unique(F[(j < sparse) & (i >= sparse) & np.isfinite(F) & (F > 3) & (F < 1e5)])
+    assert len(values) >= 5
+    for v in values[-24:]:
+        t1 = np.float32(v * np.float32(1.0 - 1e-4))
+        hits, total, ex = gpu_ctx.scan([block], capi.default_opts(t1=t1, form=capi.FORM_TENSOR), ntraits=ntraits)
+        assert config in gpu_ctx.scan_config()
+        want = F > t1
+        assert total == want.sum() and set(zip(hits["snp1"], hits["snp2"])) == set(zip(i[want], j[want]))
+        assert ex["max_f"][0] == _maxima(F, F2, "f")[0]
