@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(EXACT_NT, 2) k_exact(ScanArgs a)
         }
         const float mF = screen_lo(ord2f(__shfl_sync(0xffffffffu, lF, 0)));
         const float mI = screen_lo(ord2f(__shfl_sync(0xffffffffu, lI, 0)));
-        if (c.fu <= (report ? fminf(t1c, mF) : mF) && (!a.test_int || c.f2u <= (report ? fminf(t2c, mI) : mI))) continue;
+        if (c.fu < (report ? fminf(t1c, mF) : mF) && (!a.test_int || c.f2u < (report ? fminf(t2c, mI) : mI))) continue;
 
         const uint4 *hi = nullptr, *hj = nullptr;
         const uint32_t *ri = nullptr, *rj = nullptr;

@@ -381,7 +381,8 @@ __device__ __forceinline__ void advance(uint32_t &slot, uint32_t &phase)
 // at most P in magnitude and good to ~1e-6 of it, hence the slack SLK_B and SLK_I. Q is a difference
 // of floats up to Qtot, however little of it the pair keeps: six roundings, below 6 x 2^-24 Qtot, hence
 // SLK_Q (E is no cover for it: it is 0 for a trait of two values). The thresholds are lowered by a
-// relative 1e-3, which covers the rest.
+// relative 1e-3, which covers the rest. A pair is settled only below a bound, never at it: where every
+// F is 0 the pair that raised the lower bound to 0 has to reach k_exact, or no pair would make the maximum.
 //
 // Six column types (nine) instead of twelve per j-SNP: a pair MMA serves 80 x 42 (28) pairs
 // instead of 80 x 21.
@@ -600,7 +601,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                 // one occupied cell: F is 0/0, never a hit or a maximum (F2 is 0); none: neither is
                 // defined. W too small a part of Q to be told from rounding: unknown
                 cand[h] = valid[h] && d1 >= (ti ? 0.0f : 1.0f) &&
-                          (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs <= tF * d1 * W)) || !(lhs <= tI * W));
+                          (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs < tF * d1 * W)) || !(lhs < tI * W));
                 any = any || cand[h];
             }
             if (__any_sync(0xffffffffu, any)) {
@@ -643,7 +644,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const bool c = cand[h] && !seed && (!(fu[h] <= tF) || !(4.0f * f2u[h] <= tI));
+                    const bool c = cand[h] && !seed && (!(fu[h] < tF) || !(4.0f * f2u[h] < tI));
                     const unsigned int mask = __ballot_sync(0xffffffffu, c);
                     if (!mask) continue;
                     const int leader = __ffs(mask) - 1;
@@ -779,7 +780,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
                     const float sB = sqrt_fast(gather(P[0], P[1], P[2]) * (1.0f + SLK_B)) + ts.y, u = sB * sB;
                     const float Q = qi[g] - qmj, W = Q - u, lhs = u * nv;
                     const bool c = valid && g < nt && d1 >= (ti ? 0.0f : 1.0f) &&
-                                   (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs <= tF[g] * d1 * W)) || !(lhs <= tI[g] * W));
+                                   (!(W > 1e-3f * Q) || (d1 > 0.0f && !(lhs < tF[g] * d1 * W)) || !(lhs < tI[g] * W));
                     if (c) cand |= 1u << g;
                 }
                 uint32_t some = __reduce_or_sync(0xffffffffu, cand);
@@ -837,7 +838,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
                             tF[k] = hF;
                             if (ti) tI[k] = 4.0f * hI;
                         }
-                    const bool c = mine && pass == 1 && (!(fu <= hF) || (ti && !(f2u <= hI)));
+                    const bool c = mine && pass == 1 && (!(fu < hF) || (ti && !(f2u < hI)));
                     const unsigned int mask = __ballot_sync(0xffffffffu, c);
                     if (!mask) continue;
                     const int leader = __ffs(mask) - 1;

@@ -119,3 +119,43 @@ def test_screen_with_snps_of_a_dozen_calls(gpu_ctx, nid, ntraits, config):
         want = F > t1
         assert total == want.sum() and set(zip(hits["snp1"], hits["snp2"])) == set(zip(i[want], j[want]))
         assert ex["max_f"][0] == _maxima(F, F2, "f")[0]
+
+
+def _noalloc(packed, nid, y, block, **opts):
+    """epi_scan_block_noalloc on copies of the inputs: status, rows, maxima of F and F2."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+    gp, ph = torch.from_numpy(packed).cuda(), torch.from_numpy(np.ascontiguousarray(y, dtype=np.float32)).cuda()
+    rows = torch.zeros((1 << 20, 6), dtype=torch.int32, device="cuda")
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    maxf = torch.zeros(2, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    o, b = capi.default_opts(**opts), capi.Block(*block)
+    st = capi.load().epi_scan_block_noalloc(gp.data_ptr(), nid, packed.shape[0], ph.data_ptr(), ctypes.byref(b),
+                                            ctypes.byref(o), rows.data_ptr(), rows.shape[0], count.data_ptr(),
+                                            maxf.data_ptr(), None)
+    got = rows[:int(count)].cpu().numpy().copy().view(capi.HIT_DTYPE).reshape(-1)
+    return st, got[np.lexsort((got["snp2"], got["snp1"]))], maxf.cpu().numpy()
+
+
+@pytest.mark.parametrize("test", ["f", "i"])
+@pytest.mark.parametrize("ntraits", [1, 4])
+@pytest.mark.parametrize("nid", [256, 1024])
+def test_pairs_that_explain_nothing(gpu_ctx, nid, ntraits, test):
+    """Two halves with the same genotypes and opposite values of +-1: every cell's sum is 0, the screen's
+    phenotype is exact and every F is 0. The largest is 0, not the -inf of no pair."""
+    nsnp = 100
+    codes = np.tile(synth.genotype_codes(nid // 2, nsnp, seed=nid, miss=0.01), 2)
+    half = np.where(np.random.default_rng(1).random((nid // 2, ntraits)) < 0.5, 1.0, -1.0)
+    y = np.concatenate([half, -half]).astype(np.float32)
+    packed, block = synth.pack(codes), (0, nsnp, 0, nsnp)
+    gpu_ctx.load_packed(packed, nid)
+    gpu_ctx.set_traits(y)
+    for t1 in (0.0, 5.0):
+        _, total, ex = gpu_ctx.scan([block], capi.default_opts(test=test, t1=t1, t2=t1, form=capi.FORM_TENSOR),
+                                    ntraits=ntraits)
+        F, F2, *_ = _dumped(gpu_ctx, block, test, capi.FORM_TENSOR)
+        assert total == 0 and _maxima(F, F2, test) == (0.0, 0.0)
+        assert np.all(ex["max_f"] == 0.0) and np.all(ex["max_f2"] == 0.0)
+    st, rows, top = _noalloc(packed, nid, y[:, 0], block, test=test, t1=5.0, t2=5.0)
+    assert st == capi.EPI_OK and len(rows) == 0 and np.array_equal(top, [0.0, 0.0])
