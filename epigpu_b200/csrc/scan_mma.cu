@@ -1184,7 +1184,7 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
             tc::tc_fence_after();
             const uint32_t acc = tl + acc_col(buf);
             const bool report = a.report_trait < 0 || a.report_trait == t;
-            const bool dumping = t == a.report_trait && (a.dump_counts || a.dump_F);
+            const bool dumping = t == a.report_trait && (a.dump_counts || a.dump_F || a.dump_F2 || a.dump_df1 || a.dump_df2);
             const float t1c = screen_lo(a.t1), t2c = screen_lo(a.t2), scf = (float)sc;
             unsigned int fmx = 0u, f2mx = 0u;  // this thread's largest F, F2 of the tile (encoded)
             // screen against the CTA's maxima so far (exact values, a lower bound of the final

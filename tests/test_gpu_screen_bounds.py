@@ -159,3 +159,24 @@ def test_pairs_that_explain_nothing(gpu_ctx, nid, ntraits, test):
         assert np.all(ex["max_f"] == 0.0) and np.all(ex["max_f2"] == 0.0)
     st, rows, top = _noalloc(packed, nid, y[:, 0], block, test=test, t1=5.0, t2=5.0)
     assert st == capi.EPI_OK and len(rows) == 0 and np.array_equal(top, [0.0, 0.0])
+
+
+@pytest.mark.parametrize("form", [capi.FORM_POPC, capi.FORM_TENSOR], ids=["plain", "tensor"])
+def test_dump_of_one_output(gpu_ctx, form):
+    """Every output of epi_scan_dump by itself, the others null."""
+    import ctypes
+    nid, nsnp = 300, 60
+    codes = synth.genotype_codes(nid, nsnp, seed=8)
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_phenotype(synth.phenotype(nid, seed=9))
+    block = (0, nsnp, 0, nsnp)
+    o, b = capi.default_opts(test="i", form=form), capi.Block(*block)
+    whole = gpu_ctx.scan_dump(block, o)
+    for k, name in enumerate(("counts", "F", "F2", "df1", "df2")):
+        out = np.full_like(whole[name], -77)
+        args = [None] * 5
+        args[k] = out.ctypes.data_as(ctypes.c_void_p)
+        assert gpu_ctx.lib.epi_scan_dump(gpu_ctx.h, ctypes.byref(b), ctypes.byref(o), 0, *args) == capi.EPI_OK
+        i, j = np.tril_indices(nsnp, -1)
+        np.testing.assert_array_equal(out[i, j], whole[name][i, j], err_msg=name)
+        assert np.all(out[j, i] == -77)  # pairs that are not tested are left alone
