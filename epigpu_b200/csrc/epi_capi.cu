@@ -750,6 +750,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     }
     if (cand) CK(ensure_own(&ctx->d_cand, &ctx->cand_cap, cand, &ctx->own_cand));
     if (needs_x && ctx->x_valid != screen) {
+        ctx->x_valid = -1;  // until the rows are there: the old ones may be gone when the allocation fails
         CK(ensure_own(&ctx->d_x, &ctx->x_cap, x_bytes(ctx, screen), &ctx->own_x));
         CK(epi::launch_expand(ctx->d_hcodes, ctx->d_ydig, ctx->nsnp, ctx->Np, ctx->ntraits, screen, ctx->d_x,
                               ctx->stream));

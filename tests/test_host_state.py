@@ -1,0 +1,104 @@
+"""The library's host side (epi_capi.cu) over a CUDA runtime and kernels that do nothing
+(fake/fake_cuda.cpp): what a context holds after an allocation has failed, and which kernels a
+scan is given. No GPU: the fake checks that every launch's memory is allocated."""
+import ctypes
+import pathlib
+import subprocess
+
+import numpy as np
+import pytest
+
+from epigpu_b200 import build, capi, synth
+
+HERE = pathlib.Path(__file__).resolve().parent
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fake")
+    nvcc, inc = build._nvcc(), ["-I", str(build.INCLUDE), "-I", str(build.CSRC)]
+    capi_o, fake_o, so = (str(d / n) for n in ("capi.o", "fake.o", "libfake.so"))
+    flags = [f for f in build.NVCC_FLAGS if f != "-lineinfo"]
+    subprocess.run([nvcc, *flags, *inc, "-c", str(build.CSRC / "epi_capi.cu"), "-o", capi_o], check=True)
+    subprocess.run([nvcc, *flags, *inc, "-c", str(HERE / "fake" / "fake_cuda.cpp"), "-o", fake_o], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", capi_o, fake_o, "-o", so, "-lpthread"], check=True)
+    syms = subprocess.run(["nm", "-D", "--undefined-only", so], capture_output=True, text=True).stdout
+    assert "cuda" not in syms, syms  # nothing left to a real runtime
+    # (the allocation-free call is in another file of the library)
+    sigs = dict(capi._SIGS)
+    del sigs["epi_scan_block_noalloc"]
+    lib = ctypes.CDLL(so)
+    for name, (res, args) in sigs.items():
+        getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    lib.fake_error.restype = ctypes.c_char_p
+    lib.fake_limit.argtypes = [ctypes.c_size_t]
+    lib.fake_used.restype = ctypes.c_size_t
+    lib.fake_rate.argtypes = [ctypes.c_double]
+    lib.fake_traits.argtypes = [ctypes.c_double] * 3
+    return lib
+
+
+class Ctx:
+    """A context over the fake runtime; every call is checked for launches on memory that is not there."""
+
+    def __init__(self, lib):
+        self.lib, self.h = lib, ctypes.c_void_p()
+        lib.fake_reset()
+        assert lib.epi_open(0, ctypes.byref(self.h)) == capi.EPI_OK
+        self.nid = self.nsnp = self.ntraits = 0
+
+    def _done(self, st):
+        assert self.lib.fake_error() == b"", self.lib.fake_error()
+        return st
+
+    def load(self, nid, nsnp):
+        g = np.zeros((nsnp, (nid + 15) // 16), dtype=np.int32)
+        self.nid, self.nsnp = nid, nsnp
+        return self._done(self.lib.epi_load_packed(self.h, g.ctypes.data, nid, nsnp, nid // 16, nid % 16))
+
+    def traits(self, ntraits=1):
+        y = np.zeros((ntraits, self.nid), dtype=np.float32)
+        self.ntraits = ntraits
+        return self._done(self.lib.epi_set_traits(self.h, y.ctypes.data, self.nid, ntraits, None))
+
+    def scan(self, blocks=None, **opts):
+        """Status, and the launches by kind: the kernel with all digits and with the screens 1 to 3, the
+        exact kernel, the plain kernel; and the graphs captured."""
+        o = capi.default_opts(**opts)
+        arr = capi.blocks_array(blocks or [(0, self.nsnp, 0, self.nsnp)])
+        n = (ctypes.c_int * 7)()
+        self.lib.fake_count(n)
+        nh = ctypes.c_int64()
+        st = self.lib.epi_scan(self.h, ctypes.cast(arr, ctypes.c_void_p), len(blocks or [0]), ctypes.byref(o), None, 0,
+                               ctypes.byref(nh), None, None, None, None)
+        self.lib.fake_count(n)
+        names = ("full", "one", "two", "groups", "exact", "plain", "captures")
+        return self._done(st), {k: v for k, v in zip(names, n) if v}
+
+    def close(self):
+        self.lib.epi_close(self.h)
+        assert self.lib.fake_error() == b"" and self.lib.fake_used() == 0  # all memory given back
+
+
+@pytest.fixture
+def ctx(library):
+    c = Ctx(library)
+    yield c
+    c.close()
+
+
+HIGH, LOW = dict(t1=8.0, t2=11.0), dict(t1=0.5, t2=0.5)  # screened, and not (one pair in 400 or more passes)
+STREAMED = dict(form=capi.FORM_TENSOR, tile_config=6)
+
+
+@pytest.mark.parametrize("first,second", [(HIGH, LOW), (LOW, HIGH)], ids=["one digit, all", "all, one digit"])
+def test_expanded_rows_after_a_failed_allocation(ctx, first, second):
+    """A scan that changes the kind of expanded rows frees the old ones; where the new ones then cannot
+    be allocated, the next scan of the first kind has to expand its rows again."""
+    assert ctx.load(4000, 100000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    for failing in range(4):
+        assert ctx.scan(**STREAMED, **first)[0] == capi.EPI_OK
+        ctx.lib.fake_fail_after(failing)
+        ctx.scan(**STREAMED, **second)
+        ctx.lib.fake_fail_after(-1)
+        assert ctx.scan(**STREAMED, **first)[0] == capi.EPI_OK
