@@ -255,6 +255,30 @@ static cudaError_t ensure(T **p, size_t *cap_bytes, size_t bytes)
     return e;
 }
 
+// The expanded rows that are not a part of the slab (up to 64 GiB), given back.
+static void release_x(epi_ctx *ctx)
+{
+    if (!ctx->d_x || !ctx->own_x) return;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->d_x);
+    ctx->d_x = nullptr;
+    ctx->own_x = false;
+    ctx->x_cap = 0;
+    ctx->x_valid = -1;
+}
+
+// f(), which allocates for new genotypes or traits; where memory runs out, once more without the
+// expanded rows, which the new data have made useless.
+template <class F>
+static cudaError_t without_x(epi_ctx *ctx, F f)
+{
+    cudaError_t e = f();
+    if (e != cudaErrorMemoryAllocation || !ctx->d_x || !ctx->own_x) return e;
+    cudaGetLastError();
+    release_x(ctx);
+    return f();
+}
+
 extern "C" {
 
 void epi_default_opts(epi_scan_opts *o)
@@ -370,21 +394,26 @@ epi_status epi_load_packed(epi_ctx *ctx, const int32_t *gpack, int32_t nid, int3
     const int npack1 = remain ? npack + 1 : npack;
     const int Wp = ((nid + 31) / 32 + 3) / 4 * 4;  // multiple of 4 words = 128 individuals
     const int Wc = 2 * Wp;
-    CK(ensure(&ctx->d_raw, &ctx->raw_cap, (size_t)nsnp * npack1 * sizeof(int32_t)));
-    CK(ensure(&ctx->d_planes, &ctx->planes_cap, (size_t)nsnp * Wp * sizeof(uint4)));
-    CK(ensure(&ctx->d_hcodes, &ctx->hcodes_cap, (size_t)nsnp * Wp * 32));
-    CK(ensure(&ctx->d_h3, &ctx->h3_cap, 3 * (size_t)nsnp * Wp * 32));
-    CK(ensure(&ctx->d_missbits, &ctx->missbits_cap, (size_t)nsnp * Wp * sizeof(uint32_t)));
-    CK(ensure(&ctx->d_maj, &ctx->maj_cap, (size_t)nsnp));
+    // no genotypes until the new ones are there: an allocation that fails below has freed the old ones
+    ctx->nid = ctx->nsnp = 0;
+    ctx->qm_valid = false;
+    ctx->pm_valid = false;
+    ctx->x_valid = -1;
+    ctx->scr_full = false;
+    CK(without_x(ctx, [&] {
+        cudaError_t e = ensure(&ctx->d_raw, &ctx->raw_cap, (size_t)nsnp * npack1 * sizeof(int32_t));
+        if (e == cudaSuccess) e = ensure(&ctx->d_planes, &ctx->planes_cap, (size_t)nsnp * Wp * sizeof(uint4));
+        if (e == cudaSuccess) e = ensure(&ctx->d_hcodes, &ctx->hcodes_cap, (size_t)nsnp * Wp * 32);
+        if (e == cudaSuccess) e = ensure(&ctx->d_h3, &ctx->h3_cap, 3 * (size_t)nsnp * Wp * 32);
+        if (e == cudaSuccess) e = ensure(&ctx->d_missbits, &ctx->missbits_cap, (size_t)nsnp * Wp * sizeof(uint32_t));
+        if (e == cudaSuccess) e = ensure(&ctx->d_maj, &ctx->maj_cap, (size_t)nsnp);
+        return e;
+    }));
     CK(cudaMemcpyAsync(ctx->d_raw, gpack, (size_t)nsnp * npack1 * sizeof(int32_t), cudaMemcpyHostToDevice,
                        ctx->stream));
     CK(epi::launch_unpack(ctx->d_raw, nsnp, nid, npack, remain, ctx->d_planes, Wp, nullptr, Wc, ctx->d_hcodes,
                           ctx->d_h3, ctx->d_missbits, ctx->stream));
     CK(epi::launch_major(ctx->d_planes, nsnp, Wp, ctx->d_maj, ctx->stream));
-    ctx->qm_valid = false;
-    ctx->pm_valid = false;
-    ctx->x_valid = -1;
-    ctx->scr_full = false;
     CK(epi::mma_encode_genotypes(&ctx->maps, ctx->d_hcodes, ctx->d_h3, nsnp, 32 * Wp));
     if (ctx->traits_nid != nid) ctx->ntraits = 0;  // traits no longer match
     ctx->nid = nid;
@@ -412,16 +441,19 @@ static epi_status set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t 
     ctx->ntraits = 0;  // until the new ones are there
     // buffers are kept across calls while they are large enough: a cudaFree would
     // synchronise the device on every trait upload
-    CK(ensure(&ctx->d_yraw, &ctx->yraw_cap, cells * sizeof(float)));
-    if (mode == epi::VALID_BYTES) CK(ensure(&ctx->d_yvalid, &ctx->yvalid_cap, cells));
-    CK(ensure(&ctx->d_y, &ctx->y_cap, T * Np * sizeof(float)));
-    CK(ensure(&ctx->d_wmask, &ctx->wmask_cap, T * Wp * sizeof(uint32_t)));
-    CK(ensure(&ctx->d_ysq, &ctx->ysq_cap, T * sizeof(double)));
-    CK(ensure(&ctx->d_ydig, &ctx->ydig_cap, 5 * T * Np));
-    CK(ensure(&ctx->d_qd, &ctx->qd_cap, 2 * T * Np * sizeof(double)));
-    CK(ensure(&ctx->d_qtot, &ctx->qtot_cap, T * sizeof(double)));
-    CK(ensure(&ctx->d_yscale, &ctx->yscale_cap, 3 * T * sizeof(double)));
-    CK(ensure(&ctx->d_tscr, &ctx->tscr_cap, 2 * T * sizeof(float4)));
+    CK(without_x(ctx, [&] {
+        cudaError_t e = ensure(&ctx->d_yraw, &ctx->yraw_cap, cells * sizeof(float));
+        if (e == cudaSuccess && mode == epi::VALID_BYTES) e = ensure(&ctx->d_yvalid, &ctx->yvalid_cap, cells);
+        if (e == cudaSuccess) e = ensure(&ctx->d_y, &ctx->y_cap, T * Np * sizeof(float));
+        if (e == cudaSuccess) e = ensure(&ctx->d_wmask, &ctx->wmask_cap, T * Wp * sizeof(uint32_t));
+        if (e == cudaSuccess) e = ensure(&ctx->d_ysq, &ctx->ysq_cap, T * sizeof(double));
+        if (e == cudaSuccess) e = ensure(&ctx->d_ydig, &ctx->ydig_cap, 5 * T * Np);
+        if (e == cudaSuccess) e = ensure(&ctx->d_qd, &ctx->qd_cap, 2 * T * Np * sizeof(double));
+        if (e == cudaSuccess) e = ensure(&ctx->d_qtot, &ctx->qtot_cap, T * sizeof(double));
+        if (e == cudaSuccess) e = ensure(&ctx->d_yscale, &ctx->yscale_cap, 3 * T * sizeof(double));
+        if (e == cudaSuccess) e = ensure(&ctx->d_tscr, &ctx->tscr_cap, 2 * T * sizeof(float4));
+        return e;
+    }));
     CK(ensure_pinned(ctx, &ctx->h_info, &ctx->h_info_cap, T, ARENA_INFO, ARENA_BLOCKS));
     CK(epi::mma_encode_traits(&ctx->maps, ctx->d_ydig, ntraits, Np));
     CK(cudaMemcpyAsync(ctx->d_yraw, y, cells * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
@@ -692,6 +724,7 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
     if (ctx->maxf_cap < 4 * ctx->ntraits) {  // maxima, then the screen's lower bounds of them
         if (ctx->d_maxf) cudaFree(ctx->d_maxf);
         ctx->d_maxf = nullptr;
+        ctx->maxf_cap = 0;
         ctx->clean_traits = 0;
         CK(cudaMalloc((void **)&ctx->d_maxf, 4 * (size_t)ctx->ntraits * sizeof(unsigned int)));
         ctx->maxf_cap = 4 * ctx->ntraits;
@@ -1053,14 +1086,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
     *v = best;
     *how = buf;
     // the streamed-B candidate's expanded rows (up to 64 GiB) are released when it lost
-    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best, screen) && ctx->d_x && ctx->own_x) {
-        CK(cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->d_x);
-        ctx->d_x = nullptr;
-        ctx->own_x = false;
-        ctx->x_cap = 0;
-        ctx->x_valid = -1;
-    }
+    if (form == EPI_FORM_TENSOR && !epi::mma_needs_x(best, screen)) release_x(ctx);
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune.push_back({ctx->device, form, ctx->Np, ctx->ntraits, best, screen, *how});
     return EPI_OK;

@@ -102,3 +102,49 @@ def test_expanded_rows_after_a_failed_allocation(ctx, first, second):
         ctx.scan(**STREAMED, **second)
         ctx.lib.fake_fail_after(-1)
         assert ctx.scan(**STREAMED, **first)[0] == capi.EPI_OK
+
+
+@pytest.mark.parametrize("form", [capi.FORM_TENSOR, capi.FORM_POPC], ids=["tensor", "plain"])
+def test_a_load_that_fails_leaves_no_genotypes(ctx, form):
+    """Whichever allocation of a larger upload fails, the next scan is refused; the context is whole again
+    after the next upload, its traits kept where the number of individuals is the same."""
+    for failing in range(8):
+        assert ctx.load(1000, 300) == capi.EPI_OK and ctx.traits(2) == capi.EPI_OK
+        assert ctx.scan(form=form, **HIGH)[0] == capi.EPI_OK
+        ctx.lib.fake_fail_after(failing)
+        st = ctx.load(1000, 400 * (failing + 1))
+        ctx.lib.fake_fail_after(-1)
+        if st != capi.EPI_OK:
+            assert st == capi.EPI_E_NOMEM
+            assert ctx.scan(form=form, **HIGH) == (capi.EPI_E_STATE, {})
+            assert ctx.load(1000, 300) == capi.EPI_OK
+        assert ctx.scan(form=form, **HIGH)[0] == capi.EPI_OK
+
+
+def test_traits_and_scans_that_fail_leave_nothing_half_done(ctx):
+    """Every allocation of a larger set of traits and of the scan after it fails once; the calls after
+    that, with these or with fewer traits, find memory for all that they launch."""
+    assert ctx.load(1000, 300) == capi.EPI_OK
+    for form in (capi.FORM_TENSOR, capi.FORM_POPC):
+        for failing in range(16):
+            assert ctx.traits(1) == capi.EPI_OK and ctx.scan(form=form, **HIGH)[0] == capi.EPI_OK
+            ctx.lib.fake_fail_after(failing)
+            ctx.nsnp = 300
+            if ctx.traits(40 * (failing + 1)) == capi.EPI_OK:
+                ctx.scan(form=form, **HIGH)
+            else:
+                assert ctx.scan(form=form, **HIGH)[0] == capi.EPI_E_STATE
+            ctx.lib.fake_fail_after(-1)
+            assert ctx.traits(3) == capi.EPI_OK and ctx.scan(form=form, **HIGH)[0] == capi.EPI_OK
+
+
+def test_expanded_rows_make_room_for_a_larger_fileset(ctx):
+    """The rows of the fileset before it (20 GB) are given back where the new one does not fit beside them."""
+    assert ctx.load(4000, 800000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    assert ctx.scan(**STREAMED, **HIGH)[0] == capi.EPI_OK
+    used = ctx.lib.fake_used()
+    assert used > 35e9
+    ctx.lib.fake_limit(used + (4 << 30))
+    assert ctx.load(4000, 1600000) == capi.EPI_OK
+    ctx.lib.fake_limit(180 << 30)
+    assert ctx.scan(**STREAMED, **HIGH)[0] == capi.EPI_OK
