@@ -575,7 +575,7 @@ static bool x_usable(const epi_ctx *ctx, int screen)
     if (need <= ctx->x_cap) return true;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
-    return need <= (64ull << 30) && need <= fr / 2 + ctx->x_cap;
+    return need <= (64ull << 30) && need <= fr / 2 + (ctx->own_x ? ctx->x_cap : 0);  // (the slab's part stays)
 }
 
 // The streamed-B variant as an autotuner candidate: only up to 6,144 padded individuals. Its
@@ -765,18 +765,27 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         cand = (size_t)cand_capacity(tests / r.segments) * sizeof(epi::Cand);
     }
     if (!ctx->d_slab) {
-        // the first scan's memory in one piece: hits (2^20), candidates, expanded B rows
+        // the first scan's memory in one piece: hits (2^20), candidates, expanded B rows; the hits alone
+        // where that is too much
         const size_t hits = sizeof(DevHit) << 20, cand_part = (cand + 255) & ~(size_t)255;
         const size_t x = needs_x && x_bytes(ctx, screen) <= (256u << 20) ? x_bytes(ctx, screen) : 0;
-        CK(cudaMalloc(&ctx->d_slab, hits + cand_part + x));
+        bool whole = true;
+        cudaError_t e = cudaMalloc(&ctx->d_slab, hits + cand_part + x);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            whole = false;
+            e = cudaMalloc(&ctx->d_slab, hits);
+        }
+        if (e != cudaSuccess) ctx->d_slab = nullptr;
+        CK(e);
         unsigned char *const p = (unsigned char *)ctx->d_slab;
         ctx->d_hits = (DevHit *)p;
         ctx->hit_cap = 1 << 20;
-        if (cand) {
+        if (cand && whole) {
             ctx->d_cand = (epi::Cand *)(p + hits);
             ctx->cand_cap = cand;
         }
-        if (x) {
+        if (x && whole) {
             ctx->d_x = (int8_t *)(p + hits + cand_part);
             ctx->x_cap = x;
         }
@@ -1195,10 +1204,18 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
         pairs += block_pairs(e);
     }
     int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs) : 0;
-    s = pick_variant(ctx, opts, form, screen, &variant, &how);
-    if (s != EPI_OK) return s;
     ScanRun r;
-    s = setup_run(ctx, blocks, nblocks, opts, r, variant, screen);
+    const auto prepare = [&]() {
+        const epi_status st = pick_variant(ctx, opts, form, screen, &variant, &how);
+        return st == EPI_OK ? setup_run(ctx, blocks, nblocks, opts, r, variant, screen) : st;
+    };
+    s = prepare();
+    if (s == EPI_E_NOMEM && screen) {
+        // no room for the candidates' list or the expanded rows: all digits need neither
+        screen = 0;
+        ctx->err.clear();
+        s = prepare();
+    }
     if (s != EPI_OK) return s;
     unsigned long long found = 0;
     for (int attempt = 0; attempt < 2; ++attempt) {
@@ -1218,8 +1235,7 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
             ctx->scr_full_t1 = opts->t1;
             ctx->scr_full_t2 = opts->t2;
             screen = 0;
-            s = pick_variant(ctx, opts, form, screen, &variant, &how);
-            if (s == EPI_OK) s = setup_run(ctx, blocks, nblocks, opts, r, variant, screen);
+            s = prepare();
             if (s != EPI_OK) return s;
             attempt = -1;
             continue;

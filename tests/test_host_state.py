@@ -148,3 +148,16 @@ def test_expanded_rows_make_room_for_a_larger_fileset(ctx):
     assert ctx.load(4000, 1600000) == capi.EPI_OK
     ctx.lib.fake_limit(180 << 30)
     assert ctx.scan(**STREAMED, **HIGH)[0] == capi.EPI_OK
+
+
+@pytest.mark.parametrize("free_mb", list(range(34, 100, 8)) + list(range(100, 700, 50)))
+def test_a_scan_that_the_screen_has_no_room_for(ctx, free_mb):
+    """The hits' buffer (32 MB) is all that a first scan cannot do without: where the candidates' list or
+    the expanded rows (100 and 184 MB here) do not fit, the kernel with all digits makes the scan."""
+    assert ctx.load(1000, 30000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    ctx.lib.fake_limit(ctx.lib.fake_used() + (free_mb << 20))
+    for _ in range(2):
+        st, n = ctx.scan(**HIGH)
+        assert st == capi.EPI_OK and (n.get("one", 0) > 0 or n.get("full", 0) > 0)
+    if free_mb >= 650:
+        assert n == {"one": 1, "exact": 1}
