@@ -96,6 +96,32 @@ __global__ void __launch_bounds__(256) k_finish(unsigned long long *counters, un
 using epi::BlockDesc;
 using epi::DevHit;
 
+// The last screened scan whose candidates ran over their list (genotypes in linkage around a strong
+// effect). No scan that asks for as much or more is screened again while the same genotypes and traits
+// are loaded.
+struct Overrun {
+    bool on = false, want_int = false;
+    int report = 0;
+    float t1 = 0.0f, t2 = 0.0f;
+    double tests = 0.0;
+
+    void record(const epi_scan_opts *o, double tests_)
+    {
+        on = true;
+        want_int = o->test == 'i';
+        report = o->report_trait;
+        t1 = o->t1;
+        t2 = o->t2;
+        tests = tests_;
+    }
+    // as many tests or more, for the same trait or all, at the same or lower thresholds of the tests made
+    bool covers(const epi_scan_opts *o, double tests_) const
+    {
+        return on && tests_ >= tests && (o->report_trait == report || o->report_trait < 0) && o->t1 <= t1 &&
+               (!want_int || (o->test == 'i' && o->t2 <= t2));
+    }
+};
+
 struct epi_ctx {
     int device = -1;
     int sm_count = 0;
@@ -130,16 +156,13 @@ struct epi_ctx {
     int x_valid = -1;  // -1: none, 0: of all digits, 1, 2: of the screen with that many digits
     // screened scan: constants per trait and per (trait, SNP), the candidate list; per trait
     // E / sigma of either screen and the number of valid individuals (pinned, written by k_traits;
-    // screen_digits); the thresholds of a scan
-    // whose candidates did not fit the list (no scan at these or lower ones is screened again
-    // until other genotypes or traits are loaded)
+    // screen_digits)
     float4 *d_tscr = nullptr;
     epi::Cand *d_cand = nullptr;
     size_t tscr_cap = 0, cand_cap = 0;
     epi::TraitInfo *h_info = nullptr;
     int h_info_cap = 0;
-    bool scr_full = false;
-    float scr_full_t1 = 0.0f, scr_full_t2 = 0.0f;
+    Overrun overrun;
     // plain form: marginals per (trait, SNP) and the sum of y^2 per trait
     double *d_pmC = nullptr, *d_pmQ = nullptr, *d_ysq = nullptr;
     int32_t *d_pmN = nullptr;
@@ -399,7 +422,7 @@ epi_status epi_load_packed(epi_ctx *ctx, const int32_t *gpack, int32_t nid, int3
     ctx->qm_valid = false;
     ctx->pm_valid = false;
     ctx->x_valid = -1;
-    ctx->scr_full = false;
+    ctx->overrun.on = false;
     CK(without_x(ctx, [&] {
         cudaError_t e = ensure(&ctx->d_raw, &ctx->raw_cap, (size_t)nsnp * npack1 * sizeof(int32_t));
         if (e == cudaSuccess) e = ensure(&ctx->d_planes, &ctx->planes_cap, (size_t)nsnp * Wp * sizeof(uint4));
@@ -468,7 +491,7 @@ static epi_status set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t 
     ctx->qm_valid = false;
     ctx->pm_valid = false;
     ctx->x_valid = -1;
-    ctx->scr_full = false;
+    ctx->overrun.on = false;
     return EPI_OK;
 }
 
@@ -634,6 +657,20 @@ static double screen_share(const epi_ctx *ctx, const epi_scan_opts *o, double pa
     return share / ctx->ntraits;
 }
 
+// Capacity of the candidate list of a segment: one percent of its pair tests (where the screen stops
+// paying), 2^16 to 2^22 entries (100 MB); a longer list ends the screened scan.
+constexpr double CAND_MAX = 4194304.0;
+static int64_t cand_capacity(double tests)
+{
+    return (int64_t)std::min(CAND_MAX, std::max(65536.0, tests / 100.0));
+}
+
+// Segments that keep the candidates expected of the largest list at half of it (a list of one percent
+// holds twice what the screen is chosen for, 1 in 250). A segment boundary costs 30 us; at 1 in 250 a
+// segment is 5e8 tests, 0.05 s at N = 10,000.
+constexpr int MAX_SEGMENTS = 1024;
+static double segments_for(double tests, double share) { return 2.0 * share * tests / CAND_MAX; }
+
 // Whether the one-digit screen takes the traits in groups of five that share their counts (screen
 // 3): all have the same valid individuals, their groups take fewer tiles (a tile is 14 j-SNPs by
 // five traits against 42 by one: not for 1 to 3 or 6 traits), the expanded rows fit, and no other
@@ -655,26 +692,28 @@ static bool group_traits(const epi_ctx *ctx, const epi_scan_opts *o)
 // 400, or where that is at most 1,024 candidates in all (fewer than the exact kernel's warps). For
 // a normal trait R is 0.0092 sqrt(N) with one digit: the rule turns to two at 10,000 to 14,000
 // individuals at p = 1e-6, and to all digits at thresholds that let one pair in 400 through.
-static int screen_digits(const epi_ctx *ctx, const epi_scan_opts *o, double pairs)
+// `share` is the share expected of the chosen screen; more than its lists would hold refuses it.
+static int screen_digits(const epi_ctx *ctx, const epi_scan_opts *o, double pairs, double *share)
 {
-    if (ctx->scr_full && o->t1 <= ctx->scr_full_t1 && o->t2 <= ctx->scr_full_t2) return 0;
-    if (!(pairs >= 1.0) || ctx->Np > epi::mma_screen_max_nid()) return 0;
+    *share = 0.0;
     const double tests = pairs * ctx->ntraits;
+    if (ctx->overrun.covers(o, tests)) return 0;
+    if (!(pairs >= 1.0) || ctx->Np > epi::mma_screen_max_nid()) return 0;
+    const double most = (double)MAX_SEGMENTS / segments_for(tests, 1.0);
     const double one = screen_share(ctx, o, pairs, 1);
-    if (one <= 1.0 / 250.0 || one * tests <= 1024.0) return group_traits(ctx, o) ? 3 : 1;
+    if ((one <= 1.0 / 250.0 || one * tests <= 1024.0) && one <= most) {
+        *share = one;
+        return group_traits(ctx, o) ? 3 : 1;
+    }
     const double two = screen_share(ctx, o, pairs, 2);
-    return two <= 1.0 / 400.0 || two * tests <= 1024.0 ? 2 : 0;
+    if ((two > 1.0 / 400.0 && two * tests > 1024.0) || two > most) return 0;
+    *share = two;
+    return 2;
 }
 
-// Capacity of the candidate list: one percent of the pair tests (where the screen stops paying),
-// 2^16 to 2^22 entries (100 MB); a longer list ends the screened scan.
-static int64_t cand_capacity(double tests)
-{
-    return (int64_t)std::min(4194304.0, std::max(65536.0, tests / 100.0));
-}
-
+// share: of the pair tests that the screen is expected to pass on
 epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const epi_scan_opts *o, ScanRun &r,
-                     int variant, int screen)
+                     int variant, int screen, double share = 0.0)
 {
     r.form = pick_form(ctx, o);
     r.variant = variant;
@@ -760,8 +799,10 @@ epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const e
         // short, the exact maxima of the first ones tighten the screen of the later ones and a
         // list that runs over costs a part of the scan only. A segment boundary idles the GPU for
         // about 30 us, so a segment lasts 5 ms or more (600 cycles a stage, two SMs a unit).
+        // More than eight only where their lists would run over.
         const double ms = (double)r.units / (ctx->sm_count / 2) * (ctx->Np / 128) * 600.0 / 1.9e6;
-        r.segments = (int)std::min((double)epi::MAX_SEGMENTS, std::max(1.0, ms / 5.0));
+        r.segments = (int)std::max(std::min(8.0, std::max(1.0, ms / 5.0)),
+                                   std::min((double)MAX_SEGMENTS, std::ceil(segments_for(tests, share))));
         cand = (size_t)cand_capacity(tests / r.segments) * sizeof(epi::Cand);
     }
     if (!ctx->d_slab) {
@@ -886,14 +927,15 @@ cudaError_t enqueue_scan(epi_ctx *ctx, const ScanRun &r, int grid, bool capturin
         else if (!r.screen) e = epi::mma_enqueue(r.variant, 0, r.args, ctx->maps, grid, s);
         else {
             epi::ScanArgs a = r.args;
+            a.segment = -1;
             for (int k = 0; k < r.segments && e == cudaSuccess; ++k) {
-                a.segment = k;
                 int64_t u0 = 0, u1 = 0;
                 const int sets = epi::mma_x_sets(r.screen, ctx->ntraits);
                 a.seg0 = r.at(r.units / r.segments * k, sets, &u0);
                 a.seg1 = r.at(k + 1 == r.segments ? r.units : r.units / r.segments * (k + 1), sets, &u1);
                 a.seg_units = u1 - u0;
                 if (a.seg_units == 0) continue;
+                a.segment = (a.segment + 1) % epi::CAND_RING;
                 e = epi::mma_enqueue(r.variant, r.screen, a, ctx->maps, grid, s);
                 if (e == cudaSuccess) e = epi::exact_enqueue(a, ctx->sm_count, s);
             }
@@ -1203,11 +1245,12 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
             return set_err(ctx, EPI_E_INVALID, "block %d out of range", b);
         pairs += block_pairs(e);
     }
-    int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs) : 0;
+    double share = 0.0;
+    int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs, &share) : 0;
     ScanRun r;
     const auto prepare = [&]() {
         const epi_status st = pick_variant(ctx, opts, form, screen, &variant, &how);
-        return st == EPI_OK ? setup_run(ctx, blocks, nblocks, opts, r, variant, screen) : st;
+        return st == EPI_OK ? setup_run(ctx, blocks, nblocks, opts, r, variant, screen, share) : st;
     };
     s = prepare();
     if (s == EPI_E_NOMEM && screen) {
@@ -1218,11 +1261,13 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     }
     if (s != EPI_OK) return s;
     unsigned long long found = 0;
+    bool again = false;
     for (int attempt = 0; attempt < 2; ++attempt) {
         r.args.hits = ctx->d_hits;
         r.args.cap = ctx->hit_cap;
-        // the rescan after a regrow is launched directly (a one-off shape)
-        s = launch_run(ctx, r, nblocks, !opts->no_graph && attempt == 0);
+        // the rescans, after a regrow or a list that ran over, are launched directly (one-off shapes)
+        s = launch_run(ctx, r, nblocks, !opts->no_graph && !again);
+        again = true;
         if (s != EPI_OK) return s;
         CK(cudaStreamSynchronize(ctx->stream));
         const unsigned long long *cnt = ctx->h_state;
@@ -1230,10 +1275,8 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
             return set_err(ctx, EPI_E_TIMEOUT, "a bounded device wait of the scan kernel gave up (site %llu)",
                            cnt[3]);
         if (screen && cnt[epi::CNT_OVERFLOW] != 0) {
-            // more candidates than the list holds: once more with all digits, directly
-            ctx->scr_full = true;
-            ctx->scr_full_t1 = opts->t1;
-            ctx->scr_full_t2 = opts->t2;
+            // more candidates than the list holds: once more with all digits
+            ctx->overrun.record(opts, (double)pairs * ctx->ntraits);
             screen = 0;
             s = prepare();
             if (s != EPI_OK) return s;

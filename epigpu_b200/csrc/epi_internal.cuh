@@ -107,8 +107,9 @@ struct Cand {
 constexpr int RAW_SNPS = 3072;
 
 // 64-bit counters of a scan: hits found, tile queue (plain form), error flag and site, then
-// whether the candidate list overflowed, and from CNT_CAND on the candidates of each segment
-constexpr int CNT_OVERFLOW = 4, CNT_CAND = 5, MAX_SEGMENTS = 8, NCOUNTERS = CNT_CAND + MAX_SEGMENTS + 3;
+// whether the candidate list overflowed, and from CNT_CAND on the candidates of a segment: the segments
+// take CAND_RING counters in turn, and each one's screen sets the next one's to zero
+constexpr int CNT_OVERFLOW = 4, CNT_CAND = 5, CAND_RING = 8, NCOUNTERS = CNT_CAND + CAND_RING + 3;
 
 struct ScanArgs {
     // genotypes
@@ -155,7 +156,7 @@ struct ScanArgs {
     const float *qmf, *qmf_j;  // indexed by SNP; qmf_j: of the j side (the same array but in epi_scan_block_noalloc)
     Cand *cand;
     int64_t cand_cap;
-    int32_t segment;
+    int32_t segment;  // its counter, 0 .. CAND_RING - 1
     unsigned int *lowf, *lowf2;
     // outputs
     DevHit *hits;

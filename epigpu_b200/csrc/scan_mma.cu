@@ -1020,6 +1020,8 @@ __global__ void __launch_bounds__(C::NTHREADS, 1) k_scan_mma(ScanArgs a, const _
     // an earlier segment's candidates did not fit: the host scans again without the screen (the
     // flag is written between the segments' kernels only, so every thread reads the same)
     if (C::SCR && a.counters[CNT_OVERFLOW]) return;
+    // the next segment's candidates: nothing else in this segment touches their counter
+    if (C::SCR && !C::RAW && blockIdx.x == 0 && threadIdx.x == 0) a.counters[CNT_CAND + (a.segment + 1) % CAND_RING] = 0ull;
 
     if (warp == 12) {
         tc::tmem_alloc_pair(&sm.tmem_base, TMEM_COLS);

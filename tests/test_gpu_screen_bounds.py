@@ -180,3 +180,30 @@ def test_dump_of_one_output(gpu_ctx, form):
         i, j = np.tril_indices(nsnp, -1)
         np.testing.assert_array_equal(out[i, j], whole[name][i, j], err_msg=name)
         assert np.all(out[j, i] == -77)  # pairs that are not tested are left alone
+
+
+def test_more_segments_than_counters(gpu_ctx):
+    """Two traits of 100,000 SNPs at 8,000 individuals and p = 4e-5: more than eight segments, so their
+    candidate counters come round again. The same hits and maxima as from 15 scans of eight segments at most."""
+    nid, nsnp, ntraits = 8000, 100000, 2
+    rng = np.random.default_rng(31)
+    gpu_ctx.load_packed(synth.packed_on_gpu(nid, nsnp, seed=32), nid)
+    gpu_ctx.set_traits(rng.standard_normal((nid, ntraits)).astype(np.float32), rng.random((nid, ntraits)) >= 0.02)
+    opts = capi.default_opts(test="i", t1=synth.f_threshold(8, nid - 9, 4e-5), t2=synth.f_threshold(4, nid - 9, 4e-5),
+                             report_trait=-1)
+
+    def scan(block):
+        hits, total, ex = gpu_ctx.scan([block], opts, ntraits=ntraits, want_traits=True)
+        assert "8-bit screen" in gpu_ctx.scan_config() and total == len(hits) > 0
+        return hits, ex["trait"], ex["max_f"], ex["max_f2"], gpu_ctx.last_timing()[2]
+
+    def ordered(hits, trait):
+        o = np.lexsort((hits["snp2"], hits["snp1"], trait))
+        return hits[o], trait[o]
+    hits, trait, mf, mf2, launches = scan((0, nsnp, 0, nsnp))
+    assert launches > 1 + 2 * 8
+    parts = [scan((i, 20000, j, 20000)) for i in range(0, nsnp, 20000) for j in range(0, i + 1, 20000)]
+    assert max(p[4] for p in parts) <= 1 + 2 * 8
+    for a, b in zip(ordered(hits, trait), ordered(np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts]))):
+        assert np.array_equal(a, b)
+    assert np.array_equal(np.max([p[2] for p in parts], 0), mf) and np.array_equal(np.max([p[3] for p in parts], 0), mf2)

@@ -161,3 +161,47 @@ def test_a_scan_that_the_screen_has_no_room_for(ctx, free_mb):
         assert st == capi.EPI_OK and (n.get("one", 0) > 0 or n.get("full", 0) > 0)
     if free_mb >= 650:
         assert n == {"one": 1, "exact": 1}
+
+
+def _share(t1, t2, test, nid, pairs, r):
+    """The share of a trait's pairs that the screen is expected to pass on (epi_capi.cu: screen_share)."""
+    from scipy import stats
+    total = 0.0
+    for df, thr in ((8, t1), (4, t2))[:2 if test == "i" else 1]:
+        top = np.sqrt(stats.chi2.isf(1.0 / pairs, df))
+        root = min(top - r, np.sqrt(df * thr * nid / (nid - 9 + df * thr))) - r
+        total += stats.chi2.sf(max(0.0, root) ** 2, df)
+    return total
+
+
+@pytest.mark.parametrize("ntraits,nsnp", [(1, 3000), (1, 40000), (8, 250000), (8, 400000)])
+@pytest.mark.parametrize("r", [0.3, 0.8, 1.0])
+def test_the_candidates_that_are_expected_fit_their_lists(ctx, ntraits, nsnp, r):
+    """The list of a segment stops at 2^22 entries however large the scan: with the share of candidates
+    that the dispatch itself expects, no screened scan is thrown away and made again."""
+    nid, t1, t2 = 8000, 5.7, 8.4
+    ctx.lib.fake_traits(r, 0.002, 0.0)
+    assert ctx.load(nid, nsnp) == capi.EPI_OK and ctx.traits(ntraits) == capi.EPI_OK
+    ctx.lib.fake_rate(_share(t1, t2, "i", nid, nsnp * (nsnp - 1) / 2, r))
+    st, n = ctx.scan(test="i", t1=t1, t2=t2, report_trait=-1, form=capi.FORM_TENSOR, tile_config=1)
+    assert st == capi.EPI_OK and len({"full", "one", "two"} & set(n)) == 1
+    assert n.get("one", 0) + n.get("two", 0) == n.get("exact", 0)
+
+
+def test_what_a_scan_that_ran_over_says_of_others(ctx):
+    """After a list ran over, a scan that asks for as much is made with all digits at once, without a
+    second graph; one that asks for less (higher thresholds of the tests it makes, fewer pairs, one trait
+    of many) is screened."""
+    assert ctx.load(1000, 3000) == capi.EPI_OK and ctx.traits(2) == capi.EPI_OK
+    f = dict(test="f", t1=8.0, t2=1.0, tile_config=1)
+    ctx.lib.fake_traits(0.5, 0.002, 0.0)
+    ctx.lib.fake_rate(0.05)
+    assert ctx.scan(**f) == (capi.EPI_OK, {"one": 1, "exact": 1, "full": 1, "captures": 1})
+    assert ctx.scan(**f) == (capi.EPI_OK, {"full": 1, "captures": 1})
+    assert ctx.scan(**f) == (capi.EPI_OK, {"full": 1})
+    ctx.lib.fake_rate(0.0)
+    for same in (dict(t2=99.0), dict(t1=7.0), dict(report_trait=-1), dict(test="i", t2=99.0)):  # (8 df: t2 is not used)
+        assert "one" not in ctx.scan(**dict(f, **same))[1], same
+    for less in (dict(t1=8.5), dict(report_trait=1)):
+        assert "full" not in ctx.scan(**dict(f, **less))[1], less
+    assert "full" not in ctx.scan([(0, 300, 0, 300)], **f)[1]
