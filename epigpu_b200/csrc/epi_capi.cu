@@ -97,16 +97,30 @@ using epi::BlockDesc;
 using epi::DevHit;
 
 // The last screened scan whose candidates ran over their list (genotypes in linkage around a strong
-// effect). No scan that asks for as much or more is screened again while the same genotypes and traits
-// are loaded.
+// effect; the share expected of unassociated ones does not foresee it). No scan that asks for as much
+// or more is screened again while the same genotypes and traits are loaded, nor, since the next trait of
+// a panel is likely to be such another, for the next 1, 2, 4 .. 64 changes of them: a loop over such
+// traits then spends under a twentieth of its time on screens that come to nothing, where each one's
+// screen cost up to half as much again as the scan with all digits.
 struct Overrun {
-    bool on = false, want_int = false;
-    int report = 0;
+    bool on = false, changed = false, want_int = false;
+    int report = 0, left = 0, next = 1;  // changes that it still holds for, and the next time
     float t1 = 0.0f, t2 = 0.0f;
     double tests = 0.0;
 
+    // before a scan
+    void begin()
+    {
+        if (changed && left-- == 0) on = false;
+        if (!on) left = 0;
+        changed = false;
+    }
     void record(const epi_scan_opts *o, double tests_)
     {
+        if (!on) {
+            left = next;
+            next = std::min(2 * next, 64);
+        }
         on = true;
         want_int = o->test == 'i';
         report = o->report_trait;
@@ -115,10 +129,16 @@ struct Overrun {
         tests = tests_;
     }
     // as many tests or more, for the same trait or all, at the same or lower thresholds of the tests made
-    bool covers(const epi_scan_opts *o, double tests_) const
+    bool as_hard(const epi_scan_opts *o, double tests_) const
     {
-        return on && tests_ >= tests && (o->report_trait == report || o->report_trait < 0) && o->t1 <= t1 &&
+        return tests_ >= tests && (o->report_trait == report || o->report_trait < 0) && o->t1 <= t1 &&
                (!want_int || (o->test == 'i' && o->t2 <= t2));
+    }
+    bool covers(const epi_scan_opts *o, double tests_) const { return on && as_hard(o, tests_); }
+    // after a screened scan whose list held
+    void held(const epi_scan_opts *o, double tests_)
+    {
+        if (as_hard(o, tests_)) next = 1;
     }
 };
 
@@ -422,7 +442,8 @@ epi_status epi_load_packed(epi_ctx *ctx, const int32_t *gpack, int32_t nid, int3
     ctx->qm_valid = false;
     ctx->pm_valid = false;
     ctx->x_valid = -1;
-    ctx->overrun.on = false;
+    if (ctx->traits_nid != nid) ctx->overrun = Overrun();
+    ctx->overrun.changed = true;
     CK(without_x(ctx, [&] {
         cudaError_t e = ensure(&ctx->d_raw, &ctx->raw_cap, (size_t)nsnp * npack1 * sizeof(int32_t));
         if (e == cudaSuccess) e = ensure(&ctx->d_planes, &ctx->planes_cap, (size_t)nsnp * Wp * sizeof(uint4));
@@ -491,7 +512,7 @@ static epi_status set_traits(epi_ctx *ctx, const float *y, int32_t nid, int32_t 
     ctx->qm_valid = false;
     ctx->pm_valid = false;
     ctx->x_valid = -1;
-    ctx->overrun.on = false;
+    ctx->overrun.changed = true;
     return EPI_OK;
 }
 
@@ -1246,6 +1267,7 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
         pairs += block_pairs(e);
     }
     double share = 0.0;
+    ctx->overrun.begin();
     int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs, &share) : 0;
     ScanRun r;
     const auto prepare = [&]() {
@@ -1283,6 +1305,7 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
             attempt = -1;
             continue;
         }
+        if (screen) ctx->overrun.held(opts, (double)pairs * ctx->ntraits);
         found = cnt[0];
         if ((int64_t)found <= ctx->hit_cap) break;
         // every hit is needed to put the first `cap` in output order: grow and rescan

@@ -205,3 +205,34 @@ def test_what_a_scan_that_ran_over_says_of_others(ctx):
     for less in (dict(t1=8.5), dict(report_trait=1)):
         assert "full" not in ctx.scan(**dict(f, **less))[1], less
     assert "full" not in ctx.scan([(0, 300, 0, 300)], **f)[1]
+
+
+@pytest.mark.parametrize("loads", [False, True], ids=["traits", "filesets"])
+def test_a_loop_over_traits_that_run_over(ctx, loads):
+    """Each step of a loop loads another trait (or fileset, too) for which the screen's list runs over: the
+    screen is tried after 1, 2, 4 .. 64 steps, not in each; it is back within as many steps once the list
+    holds, in every step from then on, and a cohort of another size starts afresh."""
+    f = dict(t1=8.0, tile_config=1)
+    assert ctx.load(1000, 3000) == capi.EPI_OK
+
+    def steps(n):
+        tried, captures = 0, 0
+        for _ in range(n):
+            assert not loads or ctx.load(1000, 3000) == capi.EPI_OK
+            assert ctx.traits() == capi.EPI_OK
+            for _ in range(2):  # (a second scan of the same data is never screened after the first ran over)
+                st, k = ctx.scan(**f)
+                assert st == capi.EPI_OK
+                tried += k.get("one", 0)
+                captures += k.get("captures", 0)
+        return tried, captures
+    ctx.lib.fake_rate(0.05)
+    tried, captures = steps(200)
+    assert 4 <= tried <= 10 and captures <= 2 * tried
+    ctx.lib.fake_rate(0.0)
+    steps(65)
+    assert steps(10)[0] == 20
+    ctx.lib.fake_rate(0.05)
+    assert steps(2)[0] == 1
+    assert ctx.load(900, 3000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    assert ctx.scan(**f)[1].get("one") == 1
