@@ -435,13 +435,14 @@ __device__ __forceinline__ void cell2(const uint32_t v[2][3 * C::TY], int k, flo
     else S = fma2(md0, n, S);  // exactly 0 in an empty cell
 }
 
-// A lower bound of a trait's maximum, which other warps raise meanwhile: lane 0's reading for the whole
-// warp. Whether the rounds run twice (seed) hangs on it, and the rounds hold full-warp operations, so
-// lanes with different readings of it could end up in different passes.
-__device__ __forceinline__ unsigned int bound_now(const unsigned int *low)
-{
-    return __shfl_sync(0xffffffffu, *reinterpret_cast<const volatile unsigned int *>(low), 0);
-}
+// What other warps change meanwhile, a lower bound of a trait's maximum or the number of candidates:
+// lane 0's reading for the whole warp. Whether a unit's rounds run, and whether they run twice (seed),
+// hangs on it, and the rounds hold full-warp operations, so lanes with different readings of it could
+// end up in different passes. (Loads first, then the shuffles: each load is a trip to L2.)
+template <class T>
+__device__ __forceinline__ T peek(const T *p) { return *reinterpret_cast<const volatile T *>(p); }
+template <class T>
+__device__ __forceinline__ T lane0(T x) { return __shfl_sync(0xffffffffu, x, 0); }
 
 // All that the screen can tell of the lane's pair in half h, from its nine cells, gathered from the
 // triplet's rows (the rows' order does not matter): P, M, the count, the occupied cells, and
@@ -533,8 +534,12 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
         const float *qmf_j = a.qmf_j + (size_t)t * a.nsnp;
         const float qmi = ivalid ? s2y * a.qmf[(size_t)t * a.nsnp + gi] : 0.0f;
         const bool report = a.report_trait < 0 || a.report_trait == t;
-        unsigned int lF = bound_now(a.lowf + t);
-        unsigned int lI = ti ? bound_now(a.lowf2 + t) : 0u;
+        unsigned int lF = peek(a.lowf + t), lI = ti ? peek(a.lowf2 + t) : 0u;
+        // a list that has run over: what is left is listed nowhere and need not be screened
+        const unsigned long long listed = lane0(peek(a.counters + CNT_CAND + a.segment));
+        const int r_first = (long long)listed > a.cand_cap ? r_end : r_begin;
+        lF = lane0(lF);
+        lI = lane0(lI);
         auto threshold = [&](unsigned int low, float tc) {
             const float l = screen_lo(ord2f(low));
             return report ? fminf(tc, l) : l;
@@ -552,7 +557,7 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
         // that pass would list a tenth of them.
         bool seed = lF == ENC_NEG_INF || (ti && lI == ENC_NEG_INF);
 #pragma unroll 1
-        for (int r = r_begin; r < r_end; ++r) {
+        for (int r = r_first; r < r_end; ++r) {
             const int dj = un.j0 + round_j<C>(r) + ga, gj = un.bd.start2 + dj;
             bool valid[2];
             float qmj[2];
@@ -659,10 +664,10 @@ __device__ __forceinline__ void screen_epilogue(const ScanArgs &a, typename C::S
             if (seed && r + 1 == r_end) {
                 seed = false;
                 r = r_begin - 1;
-                lF = max(lF, bound_now(a.lowf + t));
+                lF = max(lF, lane0(peek(a.lowf + t)));
                 tF = threshold(lF, t1c);
                 if (ti) {
-                    lI = max(lI, bound_now(a.lowf2 + t));
+                    lI = max(lI, lane0(peek(a.lowf2 + t)));
                     tI = 4.0f * threshold(lI, t2c);
                 }
             }
@@ -714,13 +719,20 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
         // thresholds per trait: the report threshold or the lower bound of the maximum
         float tF[GT], tI[GT], qi[GT];
         bool unknown = false;
+        unsigned int low[GT][2];
+#pragma unroll
+        for (int g = 0; g < GT; ++g) {
+            const int t = t0 + min(g, nt - 1);
+            low[g][0] = peek(a.lowf + t);
+            low[g][1] = ti ? peek(a.lowf2 + t) : 0u;
+        }
+        const bool full = (long long)lane0(peek(a.counters + CNT_CAND + a.segment)) > a.cand_cap;
 #pragma unroll
         for (int g = 0; g < GT; ++g) {
             const int t = t0 + min(g, nt - 1);
             const float4 ts = a.tscr[2 * t];
             const bool report = a.report_trait < 0 || a.report_trait == t;
-            const unsigned int lF = bound_now(a.lowf + t);
-            const unsigned int lI = ti ? bound_now(a.lowf2 + t) : 0u;
+            const unsigned int lF = lane0(low[g][0]), lI = lane0(low[g][1]);
             const float bF = screen_lo(ord2f(lF)), bI = screen_lo(ord2f(lI));
             tF[g] = report ? fminf(t1c, bF) : bF;
             tI[g] = !ti ? INFINITY : 4.0f * (report ? fminf(t2c, bI) : bI);
@@ -734,7 +746,7 @@ __device__ __forceinline__ void group_epilogue(const ScanArgs &a, typename C::Sm
         tc::tc_fence_after();
         const uint32_t acc = tl + acc_col(buf);
         // (unknown maxima: the rounds run twice, as in screen_epilogue)
-        for (int pass = unknown ? 0 : 1; pass < 2; ++pass) {
+        for (int pass = full ? 2 : unknown ? 0 : 1; pass < 2; ++pass) {
 #pragma unroll 1
             for (int q = part; q < 2 * RND; q += EPW) {
                 const int h = q / RND, r = q % RND;
