@@ -7,6 +7,7 @@
 // (epigpu_b200/host/scan_driver.c).
 #include "epigpu.h"
 #include "epi_internal.cuh"
+#include "screen_rule.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -540,15 +541,7 @@ void epi_permute_phenotype(float *phen, int32_t nid, uint32_t seed)
 
 }  // extern "C"
 
-// number of pairs (gx, gy) of a block with start1+gx > start2+gy: the sum over gx of
-// clamp(gx + d, 0, size2), d = start1 - start2
-static int64_t block_pairs(const epi_block &b)
-{
-    const int64_t d = (int64_t)b.start1 - b.start2, m1 = b.size1, m2 = b.size2;
-    const int64_t lo = std::min(m1, std::max<int64_t>(0, -d));      // gx + d <= 0 below lo
-    const int64_t hi = std::min(m1, std::max<int64_t>(lo, m2 - d));  // gx + d >= m2 from hi on
-    return (hi - lo) * d + (lo + hi - 1) * (hi - lo) / 2 + (m1 - hi) * m2;
-}
+static int64_t block_pairs(const epi_block &b) { return epi::pairs_below(b.start1, b.size1, b.start2, b.size2); }
 
 namespace {
 
@@ -632,48 +625,18 @@ static bool x_usable(const epi_ctx *ctx, int screen)
 // N = 10,000 under the power cap (605 ms at 1,567 MHz against 640 ms for two producer groups).
 static bool x_candidate(const epi_ctx *ctx, int screen) { return (screen || ctx->Np <= 6144) && x_usable(ctx, screen); }
 
-// Upper tails of the chi-squared distribution with 8 and 4 degrees of freedom.
-static double chi8(double x) { const double h = 0.5 * x; return std::exp(-h) * (1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0))); }
-static double chi4(double x) { const double h = 0.5 * x; return std::exp(-h) * (1.0 + h); }
-
-// x with tail(x) = p (bisection; both tails fall from 1)
-static double chi_quantile(double (*tail)(double), double p)
-{
-    double lo = 0.0, hi = 1500.0;
-    for (int k = 0; k < 60; ++k) {
-        const double mid = 0.5 * (lo + hi);
-        (tail(mid) > p ? lo : hi) = mid;
-    }
-    return lo;
-}
-
 // The share of a scan's pair tests that the screen with `digits` phenotype digits (1 or 2,
-// scan_mma.cu) is expected to pass on, for unassociated genotypes. SSB and SSI are then about
-// sigma^2 times chi-squared with 8 and 4 degrees of freedom; a pair is passed on when its root is
-// within R = E / sigma of the threshold's, or of the largest lower bound so far, itself R below
-// the largest of `pairs` draws.
+// scan_mma.cu) is expected to pass on (screen_rule.cuh).
 static double screen_share(const epi_ctx *ctx, const epi_scan_opts *o, double pairs, int digits)
 {
-    const bool want_int = o->test == 'i';
-    const double top8 = std::sqrt(chi_quantile(chi8, std::min(0.5, 1.0 / pairs)));
-    const double top4 = std::sqrt(chi_quantile(chi4, std::min(0.5, 1.0 / pairs)));
+    const double top8 = epi::chi_top(pairs, 8), top4 = epi::chi_top(pairs, 4);
     double share = 0.0;
     for (int t = 0; t < ctx->ntraits; ++t) {
         const double r = digits == 1 ? ctx->h_info[t].r1 : ctx->h_info[t].r2, nv = ctx->h_info[t].nv;
         if (!std::isfinite(r)) return INFINITY;
         const bool report = o->report_trait < 0 || o->report_trait == t;
-        auto part = [&](double thr, double df, double top, double (*tail)(double)) {
-            double root = std::max(0.0, top - r);
-            if (report) {
-                if (!(thr > 0.0)) return 1.0;
-                const double d2 = std::max(1.0, nv - 9.0);
-                root = std::min(root, std::sqrt(df * thr * nv / (d2 + df * thr)));
-            }
-            root = std::max(0.0, root - r);
-            return tail(root * root);
-        };
-        share += part(o->t1, 8.0, top8, chi8);
-        if (want_int) share += part(o->t2, 4.0, top4, chi4);
+        share += epi::screen_share_of(o->t1, report, 8, top8, r, nv);
+        if (o->test == 'i') share += epi::screen_share_of(o->t2, report, 4, top4, r, nv);
     }
     return share / ctx->ntraits;
 }

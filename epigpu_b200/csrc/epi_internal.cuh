@@ -68,6 +68,18 @@ struct HitRow {
     float F, F2;
 };
 
+// Number of pairs (gx, gy) of a block with start1 + gx > start2 + gy: the sum over gx of
+// clamp(gx + d, 0, size2), d = start1 - start2.
+inline int64_t pairs_below(int64_t start1, int64_t m1, int64_t start2, int64_t m2)
+{
+    const int64_t d = start1 - start2;
+    int64_t lo = -d > 0 ? -d : 0, hi = m2 - d;  // gx + d <= 0 below lo and >= m2 from hi on
+    if (lo > m1) lo = m1;
+    if (hi < lo) hi = lo;
+    if (hi > m1) hi = m1;
+    return (hi - lo) * d + (lo + hi - 1) * (hi - lo) / 2 + (m1 - hi) * m2;
+}
+
 // Which phenotype values count: those that are not -9, those whose `valid` byte is set, or all.
 enum { VALID_NOT9 = 0, VALID_BYTES = 1, VALID_ALL = 2 };
 
@@ -103,8 +115,9 @@ struct Cand {
     float fu, f2u;
 };
 
-// epi_scan_block_noalloc goes through its block in parts of at most this many SNPs a side
-constexpr int RAW_SNPS = 3072;
+// epi_scan_block_noalloc goes through its block in parts of at most this many SNPs a side, with a list
+// of at most this many candidates
+constexpr int RAW_SNPS = 3072, RAW_CAND = 8000;
 
 // 64-bit counters of a scan: hits found, tile queue (plain form), error flag and site, then
 // whether the candidate list overflowed, and from CNT_CAND on the candidates of a segment: the segments

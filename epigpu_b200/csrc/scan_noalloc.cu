@@ -2,11 +2,12 @@
 // the reference's packed genotype words directly (src/readplink.c:1066-1102) and writes 24-byte
 // result rows, with all of its working memory in one fixed device array.
 //
-// Two ways, chosen on the device. The tensor form's one-digit screen (scan_mma.cu: its RAW
+// Two ways. The tensor form's one-digit screen (scan_mma.cu: its RAW
 // variant builds both operands from the packed words; k_exact settles what it passes on) in parts
-// of 3,072 x 3,072 SNPs (the fixed array holds what either side needs per SNP, and a list of 8,000
-// candidates); and, where the screen would pass on too much (low thresholds, many
-// individuals) or its candidate list runs over, the plain kernel below. At 1,203 individuals x
+// of up to 3,072 x 3,072 SNPs (the fixed array holds what either side needs per SNP, and a list of 8,000
+// candidates), a second time with a small first part where a list ran over that was expected to be near
+// full; and, where the screen would pass on too much (low thresholds, many
+// individuals) or its list runs over all the same, the plain kernel below. At 1,203 individuals x
 // 2,502 SNPs the plain kernel takes 4.7 ms, ten FP32 operations per pair and individual.
 //
 // The plain kernel is the reference's per-individual method (src/EpiOpenCL.c:110-228: unpack two
@@ -22,11 +23,13 @@
 //     individual) and Q += U_V*F_Q (sum of y^2 over valid individuals, q = y^2 - mean y^2).
 // Each thread owns 4 whole pairs (the warp's four i-SNPs x the lane's j-SNP).
 // Epilogue: FP64 SSB/SSI/F/F2 per pair, warp-aggregated atomic row append, maximum F.
+#include <algorithm>
 #include <cmath>
 #include <cstddef>
 
 #include "epi_internal.cuh"
 #include "epigpu.h"
+#include "screen_rule.cuh"
 
 namespace epi {
 namespace popc_raw {
@@ -113,14 +116,12 @@ __device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairAcc acc,
     return s;
 }
 
-// Runs when the screen did not or its list ran over (the array's overflow flag).
 __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = a.Wp / KW;
-    if (a.counters[CNT_OVERFLOW] == 0ull) return;  // the screen has done it
     // maxima of F and F2 per trait: per CTA in shared memory (flushed to global memory once,
     // at the end) up to SMAX_TRAITS traits, else the global maxima directly
     const bool smax_local = a.ntraits <= SMAX_TRAITS;
@@ -296,7 +297,7 @@ namespace noalloc {
 constexpr int NP_MAX = 65536;        // individuals, padded to a multiple of 128
 constexpr int NP_SCREEN_MAX = 32768; // of the screen (mma_screen_max_nid is a little below)
 
-// What both ways keep; the counters' overflow flag selects the plain kernel.
+// What both ways keep; the counters' overflow flag ends the screen.
 struct Head {
     unsigned long long counters[NCOUNTERS];
     unsigned int maxf[2], lowf[2];  // order-encoded max F and max F2; the screen's lower bounds of them
@@ -321,7 +322,7 @@ struct ScreenScratch {  // screen: layouts as in epi_internal.cuh, one trait, on
     // per SNP of the part, i side then j side
     double qm[2 * RAW_SNPS], sm[2 * RAW_SNPS], nm[2 * RAW_SNPS];
     float qmf[2 * RAW_SNPS];
-    Cand cand[8000];
+    Cand cand[RAW_CAND];
 };
 static_assert(sizeof(ScreenScratch) <= sizeof(Scratch), "both ways share the array");
 // read in words of 16 bytes (k_scan_popc: y, q; the screen: tscr, ydig)
@@ -371,14 +372,12 @@ __device__ __forceinline__ double block_max(double v, double *sv)
 // centred by the valid mean and scaled by the power of two that brings its largest magnitude
 // into [0.5, 1) (exact, so F and F2 are unchanged, and a trait in units of 1e20 or 1e-20
 // neither overflows nor underflows the single-precision squares).
-// Only where the overflow flag asks for the plain kernel.
 __global__ void __launch_bounds__(1024) k_prep(Scratch *s, const float *__restrict__ phen, int nid, int Np, int Wp,
                                                int safe, BlockDesc bd)
 {
     __shared__ double sv[32];
     __shared__ long long sn[32];
     const int tid = threadIdx.x;
-    if (s->h.counters[CNT_OVERFLOW] == 0ull) return;
     if (tid < 4) s->h.counters[tid] = 0ull;
     if (tid < 2) s->h.maxf[tid] = ENC_NEG_INF;
     if (tid == 0) s->h.block = bd;
@@ -438,34 +437,40 @@ __global__ void k_finish(const Head *s, int64_t *nhits, float *maxf, int test_in
     }
 }
 
-// Start of a call: counters and maxima reset, and the choice of the way -- the screen while it is
-// expected to pass on at most one pair in 250 (the rule of epi_scan, epi_capi.cu: screen_digits,
-// here for one trait and one digit; R = E / sigma, known on the device only). `on`: the screen
-// handles these sizes.
-__global__ void k_begin(ScreenScratch *s, int on, int want_int, float t1, float t2, double pairs, double top8, double top4)
+// The candidates expected of the first part of a block, and of the largest of the others: their pairs and
+// the roots of the largest draws that the screen's lower bounds come from. In the first part these are
+// R below the draws (screen_rule.cuh); from the second on k_exact has put them at the first part's own
+// largest F.
+struct PartSizes {
+    double first, others, top8[2], top4[2];
+};
+__host__ __device__ inline double fullest_list(const PartSizes &p, int want_int, double t1, double t2, double r, double nv)
+{
+    double n[2];
+    for (int k = 0; k < 2; ++k) {
+        double share = screen_share_of(t1, true, 8, p.top8[k] + k * r, r, nv);
+        if (want_int) share += screen_share_of(t2, true, 4, p.top4[k] + k * r, r, nv);
+        n[k] = share * (k ? p.others : p.first);
+    }
+    return (n[0] > n[1] ? n[0] : n[1]) / RAW_CAND;
+}
+
+// Start of a pass over the parts: counters and maxima reset, and the overflow flag set, so that the
+// parts' kernels return at once, where the lists are expected to be fuller than `most` (R = E / sigma
+// is known on the device only). A candidate takes about as long as 110 pairs of the screen, the plain
+// kernel 20 to 40 times as long as the screen: no share that the lists hold is too large.
+__global__ void k_begin(ScreenScratch *s, int fresh, int want_int, float t1, float t2, PartSizes p, double most)
 {
     const int tid = threadIdx.x;
     if (tid < NCOUNTERS) s->h.counters[tid] = 0ull;
-    if (tid < 2) s->h.maxf[tid] = s->h.lowf[tid] = ENC_NEG_INF;
+    if (tid < 2) {
+        s->h.maxf[tid] = ENC_NEG_INF;
+        if (fresh) s->h.lowf[tid] = ENC_NEG_INF;  // (a pass that was given up has left bounds that hold)
+    }
     __syncthreads();
     if (tid != 0) return;
-    bool screen = on != 0;
-    if (screen) {
-        const double r = s->info.r1, nv = s->info.nv;
-        auto tail = [](double root, bool four) {
-            const double h = root > 0.0 ? 0.5 * root * root : 0.0;
-            return exp(-h) * (four ? 1.0 + h : 1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0)));
-        };
-        auto part = [&](double thr, double df, double top, bool four) {
-            if (!(thr > 0.0)) return 1.0;
-            const double d2 = nv > 10.0 ? nv - 9.0 : 1.0;
-            return tail(fmin(fmax(0.0, top - r), sqrt(df * thr * nv / (d2 + df * thr))) - r, four);
-        };
-        double share = part(t1, 8.0, top8, false);
-        if (want_int) share += part(t2, 4.0, top4, true);
-        screen = isfinite(r) && (share <= 1.0 / 250.0 || share * pairs <= 1024.0);
-    }
-    if (!screen) s->h.counters[CNT_OVERFLOW] = 1ull;
+    const double r = s->info.r1;
+    if (!(isfinite(r) && fullest_list(p, want_int, t1, t2, r, s->info.nv) <= most)) s->h.counters[CNT_OVERFLOW] = 1ull;
 }
 
 // Start of a part of the block: its descriptor, an empty candidate list, and per SNP of either
@@ -515,19 +520,6 @@ __global__ void k_part(ScreenScratch *s, BlockDesc bd, const int32_t *__restrict
         s->nm[o] = (double)cnt;
         s->qmf[o] = (float)x;
     }
-}
-
-// Root of the largest of n draws of chi-squared with 8 or 4 degrees of freedom, about.
-static double top_root(double n, bool four)
-{
-    double lo = 0.0, hi = 1500.0;
-    const double p = n > 2.0 ? 1.0 / n : 0.5;
-    for (int k = 0; k < 60; ++k) {
-        const double x = 0.5 * (lo + hi), h = 0.5 * x;
-        const double t = exp(-h) * (four ? 1.0 + h : 1.0 + h * (1.0 + h / 2.0 * (1.0 + h / 3.0)));
-        (t > p ? lo : hi) = x;
-    }
-    return sqrt(lo);
 }
 
 constexpr int MAX_DEVICES = 64;
@@ -619,17 +611,71 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
     a.maxf = &scr->h.maxf[0];
     a.maxf2 = &scr->h.maxf[1];
 
-    // the screen, part by part, while the overflow flag is clear
-    const bool screen = ntiles > 0 && Np <= mma_screen_max_nid();
+    // hits, maxima and the end of the scan; the counters come to the host
+    unsigned long long state[CNT_OVERFLOW + 1] = {0ull};  // hits, tile queue, error flag and site, overflow flag
     cudaError_t e = cudaSuccess;
+    const auto finish = [&]() -> epi_status {
+        noalloc::k_finish<<<1, 32, 0, st>>>(&scr->h, d_nhits, d_maxf, a.test_int);
+        if (cudaGetLastError() != cudaSuccess || e != cudaSuccess) return EPI_E_CUDA;
+        if (cudaMemcpyAsync(state, scr->h.counters, sizeof(state), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            return EPI_E_CUDA;
+        if (cudaStreamSynchronize(st) != cudaSuccess) return EPI_E_CUDA;
+        return state[2] != 0 ? EPI_E_TIMEOUT : EPI_OK;
+    };
+
+    // The screen, in one of two passes over parts of the block: the first `head` SNPs of either side, then
+    // 3,072 at a time.
+    //   first pass   head = 3,072: while the lists are expected to be at most three times full. The
+    //                expectation holds for unassociated SNPs; effects of 1% lift the bounds and leave a
+    //                fifth of it
+    //   second pass  after the first has run over: a head so small that its list should hold what its first
+    //                wave of tiles (2.5e5 pairs) lets through, for a normal trait that reaches 4.2 standard
+    //                deviations (R = 0.0097 sqrt(N)); the parts after it go by its largest F. Not where the
+    //                first pass's lists should have been a quarter full: what ran over then (linkage)
+    //                runs over again.
+    // 8,000 individuals x 3,000 SNPs, 8 df, p = 1e-6, no effects: the first pass runs over at 9,400 candidates,
+    // the second's parts have 4,700 and 600; without it the plain kernel took 38.7 ms.
+    bool done = false;
+    const bool screen = ntiles > 0 && Np <= mma_screen_max_nid();
+    int heads[2] = {RAW_SNPS, RAW_SNPS};
+    noalloc::PartSizes sizes[2];
+    const double most[2] = {3.0, 0.9}, usual = 0.0097 * std::sqrt((double)nid);
+    const auto fullest = [&](const noalloc::PartSizes &s, double r) {
+        return noalloc::fullest_list(s, a.test_int, a.t1, a.t2, r, nid);
+    };
+    const auto sizes_of = [&](int head, double wave) {
+        const auto pairs = [&](int i, int ni, int j, int nj) {
+            return (double)pairs_below(bd.start1 + i, std::max(0, std::min(ni, bd.size1 - i)), bd.start2 + j,
+                                       std::max(0, std::min(nj, bd.size2 - j)));
+        };
+        noalloc::PartSizes s;
+        s.first = pairs(0, head, 0, head);
+        s.others = std::max(std::max(pairs(head, RAW_SNPS, 0, head), pairs(0, head, head, RAW_SNPS)),
+                            pairs(head, RAW_SNPS, head, RAW_SNPS));
+        const double drawn[2] = {std::min(wave, s.first), s.first};
+        for (int k = 0; k < 2; ++k) {
+            s.top8[k] = chi_top(drawn[k], 8);
+            s.top4[k] = chi_top(drawn[k], 4);
+        }
+        return s;
+    };
     if (screen) {
         const TraitArrays out = {nullptr, ss->wmask, ss->ydig, nullptr, &ss->ysq, &ss->qtot, ss->yscale, ss->tscr};
         e = launch_traits(d_phen, nullptr, opts->safe ? VALID_ALL : VALID_NOT9, nid, Np, 1, out, &ss->info, st);
+        sizes[0] = sizes_of(RAW_SNPS, 1e300);
     }
-    const double pairs = (double)block->size1 * block->size2;
-    noalloc::k_begin<<<1, 32, 0, st>>>(ss, screen, a.test_int, a.t1, a.t2, pairs, noalloc::top_root(pairs, false),
-                                       noalloc::top_root(pairs, true));
-    if (screen) {
+    bool fresh = true;  // no bounds of an earlier pass yet
+    for (int pass = 0; screen && pass < 2 && !done; ++pass) {
+        if (pass == 1) {
+            if (fullest(sizes_of(RAW_SNPS, 2.5e5), usual) < 0.25) break;
+            do {
+                heads[1] = heads[1] * 3 / 4;
+                sizes[1] = sizes_of(heads[1], 2.5e5);
+            } while (fullest(sizes[1], usual) > 0.7 && heads[1] > 600);
+        }
+        if (fullest(sizes[pass], 0.0) > most[pass]) continue;  // too full for any trait
+        noalloc::k_begin<<<1, 32, 0, st>>>(ss, fresh, a.test_int, a.t1, a.t2, sizes[pass], most[pass]);
+        fresh = false;
         ScanArgs p = a;
         p.wmask = ss->wmask;
         p.ydig = ss->ydig;
@@ -644,19 +690,20 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
         p.lowf = &ss->h.lowf[0];
         p.lowf2 = &ss->h.lowf[1];
         p.cand = ss->cand;
-        p.cand_cap = sizeof(ss->cand) / sizeof(ss->cand[0]);
+        p.cand_cap = RAW_CAND;
         p.wait_ns = 2000000000ull;
         p.xsi = 1;
         p.xsj = 1 << 30;
         p.seg1 = {1, 0, 0};
         const int TI = mma_tile_i(), TJ = mma_tile_j(1);
-        for (int i = 0; i < block->size1; i += RAW_SNPS)
-            for (int j = 0; j < block->size2; j += RAW_SNPS) {
+        const int head = heads[pass];
+        for (int i = 0, ni = head; i < bd.size1; i += ni, ni = RAW_SNPS)
+            for (int j = 0, nj = head; j < bd.size2; j += nj, nj = RAW_SNPS) {
                 BlockDesc d;
-                d.start1 = block->start1 + i;
-                d.size1 = block->size1 - i < RAW_SNPS ? block->size1 - i : RAW_SNPS;
-                d.start2 = block->start2 + j;
-                d.size2 = block->size2 - j < RAW_SNPS ? block->size2 - j : RAW_SNPS;
+                d.start1 = bd.start1 + i;
+                d.size1 = std::min(ni, bd.size1 - i);
+                d.start2 = bd.start2 + j;
+                d.size2 = std::min(nj, bd.size2 - j);
                 d.tiles_i = (d.size1 + TI - 1) / TI;
                 d.tiles_j = (d.size2 + TJ - 1) / TJ;
                 d.tile_base = 0;
@@ -676,20 +723,20 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
                 if (e == cudaSuccess) e = mma_raw_enqueue(p, (int)(want < screen_grid ? want : screen_grid), st);
                 if (e == cudaSuccess) e = exact_enqueue(p, noalloc::g_sms[dev], st);
             }
+        const epi_status s = finish();
+        if (s != EPI_OK) return s;
+        done = state[CNT_OVERFLOW] == 0ull;
     }
-    // the plain kernel, where the flag is set
-    noalloc::k_prep<<<1, 1024, 0, st>>>(scr, d_phen, nid, Np, Wp, opts->safe, bd);
-    if (ntiles > 0) {
-        const int grid = (int)(ntiles < noalloc::g_sms[dev] ? ntiles : noalloc::g_sms[dev]);
-        popc_raw::k_scan_popc<<<grid, popc_raw::NT, smem, st>>>(a);
+    if (!done) {
+        // the plain kernel
+        noalloc::k_prep<<<1, 1024, 0, st>>>(scr, d_phen, nid, Np, Wp, opts->safe, bd);
+        if (ntiles > 0) {
+            const int grid = (int)(ntiles < noalloc::g_sms[dev] ? ntiles : noalloc::g_sms[dev]);
+            popc_raw::k_scan_popc<<<grid, popc_raw::NT, smem, st>>>(a);
+        }
+        const epi_status s = finish();
+        if (s != EPI_OK) return s;
     }
-    noalloc::k_finish<<<1, 32, 0, st>>>(&scr->h, d_nhits, d_maxf, a.test_int);
-    if (cudaGetLastError() != cudaSuccess || e != cudaSuccess) return EPI_E_CUDA;
-    unsigned long long state[3] = {0ull, 0ull, 0ull};  // hits, tile queue, error flag
-    if (cudaMemcpyAsync(state, scr->h.counters, sizeof(state), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        return EPI_E_CUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return EPI_E_CUDA;
-    if (state[2] != 0) return EPI_E_TIMEOUT;
     const unsigned long long found = state[0];
     // as epi_scan: more hits than `cap` is reported (the first `cap` rows are written, and
     // *d_nhits holds the total)

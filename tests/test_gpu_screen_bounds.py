@@ -207,3 +207,55 @@ def test_more_segments_than_counters(gpu_ctx):
     for a, b in zip(ordered(hits, trait), ordered(np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts]))):
         assert np.array_equal(a, b)
     assert np.array_equal(np.max([p[2] for p in parts], 0), mf) and np.array_equal(np.max([p[3] for p in parts], 0), mf2)
+
+
+@pytest.mark.parametrize("nid,nsnp,p,test", [(10000, 3300, 1e-6, "i"), (9500, 3000, 1e-6, "f"), (8000, 3000, 1e-6, "f")])
+def test_block_scan_in_parts_that_its_list_holds(gpu_ctx, nid, nsnp, p, test):
+    """epi_scan_block_noalloc where a part of 3,072 SNPs a side passes on more pairs than its list holds (no
+    effects, so the largest F is near): the second pass's small first part holds them, so the rows are the
+    exact kernel's, those of epi_scan bit for bit, and not the plain kernel's."""
+    codes = synth.genotype_codes(nid, nsnp, seed=nid, miss=0.01)
+    y = synth.phenotype(nid, seed=nid)
+    packed, block = synth.pack(codes), (0, nsnp, 0, nsnp)
+    opts = dict(test=test, t1=synth.f_threshold(8, nid - 9, p), t2=synth.f_threshold(4, nid - 9, p))
+    gpu_ctx.load_packed(packed, nid)
+    gpu_ctx.set_phenotype(y)
+    want, n, ex = gpu_ctx.scan([block], capi.default_opts(form=capi.FORM_TENSOR, **opts))
+    want = want[np.lexsort((want["snp2"], want["snp1"]))]
+    st, rows, top = _noalloc(packed, nid, y, block, **opts)
+    assert st == capi.EPI_OK and n > 0 and np.array_equal(rows, want)
+    assert np.array_equal(top, [ex["max_f"][0], ex["max_f2"][0]])
+
+
+@pytest.mark.parametrize("test", ["f", "i"])
+@pytest.mark.parametrize("where", ["first part", "last part"])
+def test_block_scan_whose_list_runs_over(gpu_ctx, where, test):
+    """SNPs in linkage around a strong effect fill the list of one part, the first or the last of four, which
+    have given rows, a count and maxima by then: all of it is made again by the plain kernel."""
+    nid, nsnp, linked = 600, 3500, 150
+    codes = synth.genotype_codes(nid, nsnp, seed=41, miss=0.01)
+    rng = np.random.default_rng(42)
+    at = 0 if where == "first part" else nsnp - linked
+    keep = rng.random((linked, nid)) < 0.85
+    codes[at:at + linked] = np.where(keep, codes[at], codes[at:at + linked])
+    pairs = [(5, 3), (900, 200), (3000, 1500)] if at else [(nsnp - 3, nsnp - 9), (2000, 1900), (3400, 800)]
+    y = synth.planted_phenotype(codes, pairs, seed=43, var_frac=0.08, miss=0.01)
+    y = np.where(y == -9.0, y, y + 0.8 * np.where(codes[at] == 3, 0, codes[at])).astype(np.float32)
+    packed, block = synth.pack(codes), (0, nsnp, 0, nsnp)
+    opts = dict(test=test, t1=synth.f_threshold(8, nid - 9, 1e-6), t2=synth.f_threshold(4, nid - 9, 1e-6))
+    gpu_ctx.load_packed(packed, nid)
+    gpu_ctx.set_phenotype(y)
+    want, n, ex = gpu_ctx.scan([block], capi.default_opts(form=capi.FORM_TENSOR, **opts))
+    want = want[np.lexsort((want["snp2"], want["snp1"]))]
+    assert n > 8000 + len(pairs)
+    for _ in range(2):
+        st, rows, top = _noalloc(packed, nid, y, block, **opts)
+        assert st == capi.EPI_OK
+        # (F of the plain kernel's FP32 sums: a pair at a threshold may fall on its other side)
+        both = {(a, b): f for a, b, f in zip(want["snp1"], want["snp2"], want["F"])}
+        got = {(a, b): f for a, b, f in zip(rows["snp1"], rows["snp2"], rows["F"])}
+        assert len(got) == len(rows) and abs(len(rows) - n) <= 3 and len(both.keys() ^ got.keys()) <= 3
+        common = sorted(both.keys() & got.keys())
+        np.testing.assert_allclose([got[k] for k in common], [both[k] for k in common], rtol=2e-5)
+        assert not np.array_equal([got[k] for k in common], [both[k] for k in common])  # the plain kernel's
+        np.testing.assert_allclose(top, [ex["max_f"][0], ex["max_f2"][0]], rtol=2e-5)
