@@ -591,12 +591,20 @@ epi_status check_opts(epi_ctx *ctx, const epi_scan_opts *o)
     return EPI_OK;
 }
 
+// The form of a scan without a screen. The automatic choice is the plain one below 256 individuals: it
+// keeps y in 32 bits, which the tensor form's digits do not.
 int pick_form(const epi_ctx *ctx, const epi_scan_opts *o)
 {
     if (o->form != EPI_FORM_AUTO) return o->form;
-    if (epi::mma_available() && ctx->nid >= epi::mma_min_nid() && ctx->Np <= epi::mma_max_nid())
-        return EPI_FORM_TENSOR;
-    return EPI_FORM_POPC;
+    return epi::mma_available() && ctx->nid >= 256 && ctx->Np <= epi::mma_max_nid() ? EPI_FORM_TENSOR : EPI_FORM_POPC;
+}
+
+// Whether the automatic choice of the plain form may be screened by the tensor form, whose candidates are
+// then evaluated from y (and no kernel variant of the plain form is asked for).
+bool screens_plain(const epi_ctx *ctx, const epi_scan_opts *o)
+{
+    return o->form == EPI_FORM_AUTO && pick_form(ctx, o) == EPI_FORM_POPC && o->tile_config == 0 && epi::mma_available() &&
+           ctx->nid >= epi::mma_min_nid();
 }
 
 // Builds the kernel arguments and tile schedule for `blocks` and uploads the schedule.
@@ -696,10 +704,10 @@ static int screen_digits(const epi_ctx *ctx, const epi_scan_opts *o, double pair
 }
 
 // share: of the pair tests that the screen is expected to pass on
-epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const epi_scan_opts *o, ScanRun &r,
+epi_status setup_run(epi_ctx *ctx, const epi_block *blocks, int nblocks, const epi_scan_opts *o, ScanRun &r, int form,
                      int variant, int screen, double share = 0.0)
 {
-    r.form = pick_form(ctx, o);
+    r.form = form;
     r.variant = variant;
     r.screen = screen;
     r.segments = 1;
@@ -1097,7 +1105,7 @@ epi_status pick_variant(epi_ctx *ctx, const epi_scan_opts *o, int form, int scre
             continue;
         }
         ScanRun r;
-        epi_status st = setup_run(ctx, &blk, 1, &o2, r, c, screen);
+        epi_status st = setup_run(ctx, &blk, 1, &o2, r, form, c, screen);
         if (st != EPI_OK) return st;
         r.args.hits = ctx->d_hits;
         r.args.cap = ctx->hit_cap;
@@ -1218,7 +1226,6 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     epi_status s = check_opts(ctx, opts);
     if (s != EPI_OK) return s;
     CK(cudaSetDevice(ctx->device));
-    const int form = pick_form(ctx, opts);
     int variant = 0;
     std::string how;
     int64_t pairs = 0;
@@ -1231,15 +1238,20 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
     }
     double share = 0.0;
     ctx->overrun.begin();
-    int screen = form == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs, &share) : 0;
+    const bool plain = screens_plain(ctx, opts);
+    int form = 0;
+    int screen = plain || pick_form(ctx, opts) == EPI_FORM_TENSOR ? screen_digits(ctx, opts, (double)pairs, &share) : 0;
     ScanRun r;
     const auto prepare = [&]() {
-        const epi_status st = pick_variant(ctx, opts, form, screen, &variant, &how);
-        return st == EPI_OK ? setup_run(ctx, blocks, nblocks, opts, r, variant, screen, share) : st;
+        form = plain && screen ? EPI_FORM_TENSOR : pick_form(ctx, opts);
+        epi_status st = pick_variant(ctx, opts, form, screen, &variant, &how);
+        if (st == EPI_OK) st = setup_run(ctx, blocks, nblocks, opts, r, form, variant, screen, share);
+        r.args.from_y = plain && screen;
+        return st;
     };
     s = prepare();
     if (s == EPI_E_NOMEM && screen) {
-        // no room for the candidates' list or the expanded rows: all digits need neither
+        // no room for the candidates' list or the expanded rows: without a screen there is need of neither
         screen = 0;
         ctx->err.clear();
         s = prepare();
@@ -1260,7 +1272,7 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
             return set_err(ctx, EPI_E_TIMEOUT, "a bounded device wait of the scan kernel gave up (site %llu)",
                            cnt[3]);
         if (screen && cnt[epi::CNT_OVERFLOW] != 0) {
-            // more candidates than the list holds: once more with all digits
+            // more candidates than the list holds: once more without a screen
             ctx->overrun.record(opts, (double)pairs * ctx->ntraits);
             screen = 0;
             s = prepare();
@@ -1336,7 +1348,7 @@ extern "C" epi_status epi_scan_dump(epi_ctx *ctx, const epi_block *block, const 
     s = pick_variant(ctx, &o, form, 0, &variant, &how);
     if (s != EPI_OK) return s;
     ScanRun r;
-    s = setup_run(ctx, block, 1, &o, r, variant, 0);
+    s = setup_run(ctx, block, 1, &o, r, form, variant, 0);
     if (s != EPI_OK) return s;
     const size_t np = (size_t)block->size1 * block->size2;
     int32_t *dc = nullptr, *dd1 = nullptr, *dd2 = nullptr;

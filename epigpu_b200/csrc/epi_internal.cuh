@@ -19,8 +19,8 @@
 //   tscr    float4 [T][2]         the screen with one digit and with two: (d0, E, s^2 Qtot, s^2);
 //                                 one digit: D approximates s (ytilde - c) with |D| <= 127,
 //                                 d0 = -s c is the D of the mean; two: D is the two upper digits
-//                                 of Y and d0 = 0; E = ||s ytilde - (D - d0)||_2 over the valid
-//                                 individuals
+//                                 of Y and d0 = 0; E = ||s ytilde - (D - d0)||_2 + s ||y - ytilde||_2
+//                                 over the valid individuals
 //   qmf     float [T][nsnp]       qm as floats
 //   qd      double [2][T][Np]     ytilde^2 (ytilde = Y 2^-sy, the quantised y), then Y itself;
 //                                 0 where invalid; per trait qtot = sum of ytilde^2, ytot = sum
@@ -170,6 +170,7 @@ struct ScanArgs {
     Cand *cand;
     int64_t cand_cap;
     int32_t segment;  // its counter, 0 .. CAND_RING - 1
+    int32_t from_y;   // the candidates are evaluated from y, not from the digits
     unsigned int *lowf, *lowf2;
     // outputs
     DevHit *hits;

@@ -72,7 +72,7 @@ __global__ void k_unpack(const int32_t *__restrict__ raw, int nsnp, int nid, int
     }
 }
 
-// Sum over the block of up to four values at once; every thread gets the sums. `sv` holds
+// Sum over the block of a few values at once; every thread gets the sums. `sv` holds
 // 32 x N doubles.
 template <int N>
 __device__ __forceinline__ void block_sum(double (&v)[N], double *sv)
@@ -127,14 +127,15 @@ __device__ __forceinline__ void block_max2(double &a, double &b, double *sv)
 //     and the valid flag; ytilde^2 = (Y 2^-sy)^2 (exact in FP64: |Y| < 2^23) and Y; their sums;
 //   * the screen's 8-bit phenotype D = round(s (ytilde - c)), c the middle of the values and s
 //     the scale that spreads them over -127..127, d0 = -s c (the D of the mean), and the norm
-//     E of what the rounding leaves; the same for the two upper digits of Y (scan_mma.cu).
+//     E of what the rounding leaves, that of ytilde against y included; the same for the two upper
+//     digits of Y (scan_mma.cu).
 // Four passes over the column; at 10,000 individuals about 15 us, where the same loops on one
 // host core and the upload of their eight arrays took 200 to 300 us.
 __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw, const uint8_t *__restrict__ valid,
                                                  int mode, int nid, int Np, int ntraits, TraitArrays o,
                                                  TraitInfo *__restrict__ info)
 {
-    __shared__ double sv[32 * 4];
+    __shared__ double sv[32 * 5];
     const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
     const float *y = yraw + (size_t)t * nid;
     const uint8_t *vb = mode == VALID_BYTES ? valid + (size_t)t * nid : nullptr;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     const double unit = 1.0 / scale;  // 2^-sy
 
     int8_t *dg = o.ydig + (size_t)t * 5 * Np;  // rows D, w, d2, d1, d0
-    double s1[4] = {0.0, 0.0, 0.0, 0.0};  // sums of y^2 (as floats), ytilde^2, Y, d0^2
+    double s1[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // sums of y^2 (as floats), ytilde^2, Y, d0^2, (y - ytilde)^2
     double ymax = -INFINITY, nymin = -INFINITY;
     for (int k = tid; k < Np; k += nt) {
         float yc = 0.0f;
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
             s1[1] += yq * yq;
             s1[2] += (double)Y;
             s1[3] += (double)(a0 * a0);
+            s1[4] += ((double)yc - yq) * ((double)yc - yq);
             ymax = yq > ymax ? yq : ymax;
             nymin = -yq > nymin ? -yq : nymin;
         }
@@ -232,8 +234,9 @@ __global__ void __launch_bounds__(1024) k_traits(const float *__restrict__ yraw,
     o.yscale[t] = unit;
     o.yscale[ntraits + t] = s1[2];
     o.yscale[2 * (size_t)ntraits + t] = nv;
-    o.tscr[2 * t] = make_float4(dm, (float)(sqrt(e[0]) * (1.0 + 1e-6)), (float)q8, (float)(s * s));
-    o.tscr[2 * t + 1] = make_float4(0.0f, (float)(sqrt(e16) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
+    const double ey = sqrt(s1[4]);
+    o.tscr[2 * t] = make_float4(dm, (float)((sqrt(e[0]) + s * ey) * (1.0 + 1e-6)), (float)q8, (float)(s * s));
+    o.tscr[2 * t + 1] = make_float4(0.0f, (float)((sqrt(e16) + s16 * ey) * (1.0 + 1e-6)), (float)q16, (float)(s16 * s16));
     info[t].nv = nv;
     info[t].same_mask = differs ? 0.0 : 1.0;
     info[t].r1 = q8 > 0.0 ? sqrt(e[0] * nv / q8) : INFINITY;

@@ -1599,7 +1599,7 @@ int mma_tile_j(int screen)
 {
     return screen == 0 ? mma::TJ : screen == 1 ? 2 * mma::TJ : screen == 2 ? Screen2Digits::TJT : GroupRings::TJT;
 }
-// The automatic choice takes this form from here on. Kernel time against the plain form, 8 df and
+// The automatic choice screens with this form from here on. Kernel time against the plain form, 8 df and
 // 4 df, B200: N = 64 x 2,000 SNPs 64 us and 320, N = 150 x 240 22 and 88, N = 231 x 2,003 69 and
 // 443, N = 126 x 30,000 6.3 ms and 61. With few individuals many pairs fit nearly perfectly and
 // the screen settles none of them: at N = 20 both take 0.3 ms.

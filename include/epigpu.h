@@ -67,7 +67,9 @@ typedef struct epi_scan_opts {
     float t2;              /* -I threshold for F2 (4 df) */
     int32_t form;          /* EPI_FORM_AUTO / _POPC (plain popcount form, up to 65,535 individuals)
                             * / _TENSOR (tcgen05, up to 2^24 individuals); AUTO takes the tensor
-                            * form from 64 individuals on */
+                            * form from 256 individuals on, and from 64 on where its screen
+                            * settles all but a few pairs, which are then evaluated from the
+                            * phenotype in 32 bits as in the plain form */
     int32_t report_trait;  /* trait whose hits are returned; -1 = every trait */
     int32_t wait_limit_ms; /* tensor form: every device-side wait gives up after this many
                             * milliseconds and the scan returns EPI_E_TIMEOUT; 0 = 2000 */

@@ -259,3 +259,44 @@ def test_block_scan_whose_list_runs_over(gpu_ctx, where, test):
         np.testing.assert_allclose([got[k] for k in common], [both[k] for k in common], rtol=2e-5)
         assert not np.array_equal([got[k] for k in common], [both[k] for k in common])  # the plain kernel's
         np.testing.assert_allclose(top, [ex["max_f"][0], ex["max_f2"][0]], rtol=2e-5)
+
+
+@pytest.mark.parametrize("nid", [64, 101, 150, 255])
+@pytest.mark.parametrize("sd", [0.0, 1e3], ids=["normal", "outlier"])
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_few_individuals_keep_32_bits(gpu_ctx, nid, sd, test):
+    """The automatic form of 64 to 255 individuals evaluates from the phenotype in 32 bits, as the plain form
+    does: F and F2 of every pair against FP64, with an outlier that most pairs miss (24-bit fixed point is
+    good to 2^-24 of the outlier). y carries a relative 2^-24, which moves the roots of SSB, SSI and SSW by
+    2^-24 of the norm of y over the pair's individuals; F is rounded to 32 bits."""
+    nsnp, u = 31, 2.0 ** -24
+    codes = synth.genotype_codes(nid, nsnp, seed=nid, miss=0.02)
+    codes[4:, 0] = 3
+    y = np.random.default_rng(nid).standard_normal(nid).astype(np.float32)
+    if sd:
+        y[0] = sd
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_phenotype(y)
+    hits, total, ex = gpu_ctx.scan([(0, nsnp, 0, nsnp)], capi.default_opts(test=test, safe=1, t1=1e-3, t2=1e-3))
+    assert "screen" in gpu_ctx.scan_config() and total > nsnp * (nsnp - 1) // 2 - 60
+    yc = y.astype(np.float64) - y.astype(np.float64).mean()
+    for h in hits:
+        gi, gj = codes[h["snp1"]], codes[h["snp2"]]
+        ok = (gi != 3) & (gj != 3)
+        cell, v = 3 * gi[ok].astype(int) + gj[ok], yc[ok]
+        n, S = np.bincount(cell, minlength=9), np.bincount(cell, v, minlength=9)
+        m, mc = v.mean(), S / np.maximum(n, 1)
+        ssb, ssw, d1, d2 = (n * (mc - m) ** 2).sum(), ((v - mc[cell]) ** 2).sum(), (n > 0).sum() - 1, ok.sum() - (n > 0).sum()
+        assert (h["df1"], h["df2"]) == (d1, d2)
+        norm = np.sqrt((v ** 2).sum())
+
+        def near(got, ss, df):
+            want = ss / df / (ssw / d2)
+            tol = u * (1.0 + 2.2 * norm / np.sqrt(ss) + 2.2 * norm / np.sqrt(ssw))
+            assert abs(got - want) <= tol * want, (got, want, tol)
+        near(h["F"], ssb, d1)
+        if test == "i":
+            n3, S3 = n.reshape(3, 3), S.reshape(3, 3)
+            row, col = S3.sum(1) / np.maximum(n3.sum(1), 1), S3.sum(0) / np.maximum(n3.sum(0), 1)
+            near(h["F2"], (n3 * (mc.reshape(3, 3) - row[:, None] - col[None] + m) ** 2).sum(), 4)
+    assert ex["max_f"][0] == hits["F"].max()

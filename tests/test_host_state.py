@@ -236,3 +236,24 @@ def test_a_loop_over_traits_that_run_over(ctx, loads):
     assert steps(2)[0] == 1
     assert ctx.load(900, 3000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
     assert ctx.scan(**f)[1].get("one") == 1
+
+
+def test_few_individuals_keep_the_plain_form_behind_the_screen(ctx):
+    """The automatic form below 256 individuals is the plain one: where its pairs cannot be screened (low
+    thresholds, a list that runs over, no memory, a tile shape of its own) and for the dump. From 64 on the
+    tensor form screens it."""
+    assert ctx.load(200, 5000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    ctx.lib.fake_traits(0.1, 0.001, 1.0)
+    st, n = ctx.scan(**HIGH)
+    assert st == capi.EPI_OK and n.pop("one") > 0 and set(n) == {"exact", "captures"}
+    assert set(ctx.scan(**LOW)[1]) == {"plain", "captures"}
+    assert set(ctx.scan(tile_config=2, **HIGH)[1]) == {"plain", "captures"}
+    ctx.lib.fake_rate(0.05)
+    assert set(ctx.scan(**HIGH)[1]) == {"one", "exact", "plain", "captures"}
+    assert set(ctx.scan(**HIGH)[1]) == {"plain", "captures"}
+    ctx.lib.fake_rate(0.0)
+    assert "full" in ctx.scan(form=capi.FORM_TENSOR, **LOW)[1]
+    assert ctx.load(63, 5000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    assert set(ctx.scan(**HIGH)[1]) == {"plain", "captures"}
+    assert ctx.load(256, 5000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    assert "full" in ctx.scan(**LOW)[1]
