@@ -1250,8 +1250,9 @@ extern "C" epi_status epi_scan(epi_ctx *ctx, const epi_block *blocks, int32_t nb
         return st;
     };
     s = prepare();
-    if (s == EPI_E_NOMEM && screen) {
+    if ((s == EPI_E_NOMEM || s == EPI_E_UNSUPPORTED) && screen) {
         // no room for the candidates' list or the expanded rows: without a screen there is need of neither
+        // (the variant that is asked for may stream B under the screen only)
         screen = 0;
         ctx->err.clear();
         s = prepare();

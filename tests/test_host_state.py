@@ -257,3 +257,16 @@ def test_few_individuals_keep_the_plain_form_behind_the_screen(ctx):
     assert set(ctx.scan(**HIGH)[1]) == {"plain", "captures"}
     assert ctx.load(256, 5000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
     assert "full" in ctx.scan(**LOW)[1]
+
+
+def test_requested_variants_where_expanded_rows_do_not_fit(ctx):
+    """Variant 3 streams B under the screen and does not without: where the rows do not fit it is refused no
+    more than before there was a screen. Variant 6 streams B always, and is."""
+    assert ctx.load(4000, 800000) == capi.EPI_OK and ctx.traits() == capi.EPI_OK
+    ctx.lib.fake_limit(ctx.lib.fake_used() + (10 << 30))
+    for k in range(1, 7):
+        st, n = ctx.scan(form=capi.FORM_TENSOR, tile_config=k, **HIGH)
+        if k == 6:
+            assert (st, n) == (capi.EPI_E_UNSUPPORTED, {})
+        else:
+            assert st == capi.EPI_OK and ("full" if k == 3 else "one") in n and len({"full", "one"} & set(n)) == 1
