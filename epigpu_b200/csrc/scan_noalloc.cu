@@ -691,7 +691,8 @@ extern "C" epi_status epi_scan_block_noalloc(const int32_t *d_gpack, int32_t nid
         p.lowf2 = &ss->h.lowf[1];
         p.cand = ss->cand;
         p.cand_cap = RAW_CAND;
-        p.wait_ns = 2000000000ull;
+        p.wait_ns = opts->wait_limit_ms > 0 ? (unsigned long long)opts->wait_limit_ms * 1000000ull : 2000000000ull;
+        p.debug_stall = opts->debug == EPI_DEBUG_STALL;
         p.xsi = 1;
         p.xsj = 1 << 30;
         p.seg1 = {1, 0, 0};

@@ -188,7 +188,8 @@ epi_status epi_get_stream(const epi_ctx *ctx, void **stream);
  *   d_gpack  device, nsnp x (nid/16 + (nid%16 > 0)) int32: the reference's packed words
  *   d_phen   device, nid floats; -9 = missing unless opts->safe
  *   block    the pairs to scan (snp1 in block 1 > snp2 in block 2), as for epi_scan
- *   opts     test, safe, t1, t2 as for epi_scan (form and chunk are ignored)
+ *   opts     test, safe, t1, t2 as for epi_scan; wait_limit_ms and debug as for epi_scan where the
+ *            tensor-core screen runs (a limit below 0 is the default one); the others are ignored
  *   d_hits   device, cap rows: the hits, in no particular order (epi_scan gives the
  *            reference's order; sort by (snp1, snp2) to compare)
  *   d_nhits  device, one int64: the number of hits; when it exceeds cap the first cap

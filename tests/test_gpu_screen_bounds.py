@@ -300,3 +300,21 @@ def test_few_individuals_keep_32_bits(gpu_ctx, nid, sd, test):
             row, col = S3.sum(1) / np.maximum(n3.sum(1), 1), S3.sum(0) / np.maximum(n3.sum(0), 1)
             near(h["F2"], (n3 * (mc.reshape(3, 3) - row[:, None] - col[None] + m) ** 2).sum(), 4)
     assert ex["max_f"][0] == hits["F"].max()
+
+
+def test_block_scan_without_allocation_times_out(gpu_ctx):
+    """A wait of the screen that runs out after wait_limit_ms ends epi_scan_block_noalloc with a status; the
+    next call is whole."""
+    import time
+    nid, nsnp = 1203, 300
+    codes = synth.genotype_codes(nid, nsnp, seed=61)
+    packed, y, block = synth.pack(codes), synth.phenotype(nid, seed=62), (0, nsnp, 0, nsnp)
+    opts = dict(test="i", t1=synth.f_threshold(8, nid - 9, 1e-3), t2=synth.f_threshold(4, nid - 9, 1e-3))
+    st, want, top = _noalloc(packed, nid, y, block, **opts)
+    assert st == capi.EPI_OK and len(want) > 0
+    t = time.perf_counter()
+    st, *_ = _noalloc(packed, nid, y, block, wait_limit_ms=20, debug=capi.DEBUG_STALL, **opts)
+    assert st == capi.EPI_E_TIMEOUT and time.perf_counter() - t < 10.0
+    for limit in (0, 20, -1):
+        st, rows, again = _noalloc(packed, nid, y, block, wait_limit_ms=limit, **opts)
+        assert st == capi.EPI_OK and np.array_equal(rows, want) and np.array_equal(again, top)
