@@ -318,3 +318,35 @@ def test_block_scan_without_allocation_times_out(gpu_ctx):
     for limit in (0, 20, -1):
         st, rows, again = _noalloc(packed, nid, y, block, wait_limit_ms=limit, **opts)
         assert st == capi.EPI_OK and np.array_equal(rows, want) and np.array_equal(again, top)
+
+
+@pytest.mark.parametrize("nid,nsnp,ntraits,form,config",
+                         [(96, 150, 1, capi.FORM_AUTO, "8-bit screen"), (96, 150, 1, capi.FORM_TENSOR, "8-bit screen"),
+                          (300, 167, 1, capi.FORM_AUTO, "8-bit screen"), (1153, 200, 1, capi.FORM_AUTO, "8-bit screen"),
+                          (700, 130, 5, capi.FORM_AUTO, "groups"), (15000, 140, 1, capi.FORM_AUTO, "16-bit screen")])
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_screened_scans_against_the_oracle(gpu_ctx, nid, nsnp, ntraits, form, config, test):
+    """The screen and the exact kernel against the FP64 oracle: the hits in its order, F within the parity bar
+    and the largest F, for every trait that is asked for in turn."""
+    import oracles
+    import parity
+    codes = synth.genotype_codes(nid, nsnp, seed=nid, miss=0.01)
+    block = (0, nsnp, 0, nsnp)
+    cols = np.stack([synth.planted_phenotype(codes, [(1, 20), (33, 5)], seed=nid + t, var_frac=min(0.3, 60.0 / nid), miss=0.0)
+                     for t in range(ntraits)], 1)
+    gpu_ctx.load_packed(synth.pack(codes), nid)
+    gpu_ctx.set_traits(cols, np.ones(cols.shape, dtype=np.uint8))
+    p = 1e-4 if nid < 15000 else 1e-3
+    t1, t2 = synth.f_threshold(8, nid - 9, p), synth.f_threshold(4, nid - 9, p)
+    for t in range(ntraits):
+        want, _, per = oracles.oracle_scan_block(codes, cols[:, t], block, test=test, t1=t1, t2=t2, per_pair=True)
+        near = parity.near_threshold(per, block, t1, t2, test, 1e-4)
+        opts = capi.default_opts(test=test, t1=t1, t2=t2, form=form, report_trait=t)
+        hits, total, ex = gpu_ctx.scan([block], opts, ntraits=ntraits)
+        assert config in gpu_ctx.scan_config() and total == len(hits) > 0
+        ok, msg = parity.compare_hit_lists(hits, want, near)
+        assert ok, msg
+        assert parity.f_errors(hits, per, block, 1e-5).max() <= 1.0
+        F = np.where(per["df1"] > 0, per["F"], -np.inf)[np.tril_indices(nsnp, -1)]
+        k = np.nanmax(F) * 8.0 / (nid - 9)  # about the largest SSB / SSW
+        assert abs(ex["max_f"][t] - np.nanmax(F)) <= 1e-5 * (1.0 + k) * np.nanmax(F)
