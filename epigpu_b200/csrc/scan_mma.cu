@@ -1540,9 +1540,10 @@ using GroupRings = mma::Rings<7, 1, 2, 1, true, 1, false, GROUP_TRAITS>;
 struct GroupOf { using type = GroupRings; };
 
 // Tensor maps of the tensor form's TMA loads: the genotype-indicator rows h3 [3 nsnp][Np]
-// with 30-row boxes (A), the one-hot genotype bytes [nsnp][Np] with 16-row boxes (j side) and
-// the trait digit rows [7T][Np] with 7-row boxes; all 128 bytes wide, 128-byte swizzled,
-// out-of-range rows read as zero.
+// with 30-row boxes (A), the one-hot genotype bytes [nsnp][Np] with boxes of a half's j-SNPs (21; 14 for
+// the screen with two digits) and the trait digit rows [5T][Np] with boxes of 4 (all digits), 2 and 3 rows
+// (the screen with one digit and with two); all 128 bytes wide, 128-byte swizzled, out-of-range rows read
+// as zero.
 static cudaError_t encode_2d(CUtensorMap *m, const void *base, uint64_t inner, uint64_t rows, uint32_t box_rows)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
@@ -1580,11 +1581,10 @@ cudaError_t mma_encode_traits(MmaMaps *maps, const int8_t *ydig, int ntraits, in
     return e;
 }
 
-// The streamed-B variant's expanded rows [ntraits][2][nsnp][6][Np], in boxes of one CTA half
-// of a j tile (21 SNPs x 6 types = 126 rows)
-// expanded rows per SNP and trait
+// The streamed-B variant's expanded rows ([ntraits][2][nsnp][6][Np] with all digits, prep.cu: k_expand) go
+// in boxes of one CTA half of a j tile (126 rows). Rows per SNP and set of them:
 int mma_x_rows(int screen) { return screen == 3 ? 3 * (1 + GROUP_TRAITS) : screen ? 3 * (1 + screen) : mma::NTYPE; }
-// sets of them: per trait, or per group of traits
+// and sets: one per trait, or per group of traits
 int mma_x_sets(int screen, int ntraits) { return screen == 3 ? (ntraits + GROUP_TRAITS - 1) / GROUP_TRAITS : ntraits; }
 
 cudaError_t mma_encode_x(MmaMaps *maps, const int8_t *x, int nsnp, int Np, int ntraits, int screen)
@@ -1607,7 +1607,6 @@ int mma_min_nid() { return 64; }
 int mma_max_nid() { return 1 << 24; }  // digit sums stay within int32
 // the screen's sums (127 per individual) stay below 2^22, its counts below 2^15
 int mma_screen_max_nid() { return (1 << 15) - mma::KS; }
-int mma_stage_individuals() { return mma::KS; }
 
 // The variants the autotuner chooses among -- operand slots and raw stages (each ~200-230 KB
 // of shared memory) and epilogue warps per TMEM lane quarter:

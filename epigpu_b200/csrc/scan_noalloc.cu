@@ -87,11 +87,10 @@ struct PairAcc {
     float Q;
 };
 
-// FP64 statistics of one pair from its packed counts, FP32 cell sums and y^2 sum; also
-// writes the optional per-pair dump. Kept out of line: the kernel's accumulators stay in
-// registers and only this call's arguments go through the stack.
-__device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairAcc acc, double qc, int t, int gi, int gj,
-                                           int size2)
+// FP64 statistics of one pair from its packed counts, FP32 cell sums and y^2 sum. Kept out of
+// line: the kernel's accumulators stay in registers and only this call's arguments go through
+// the stack.
+__device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairAcc acc, double qc)
 {
     int n[9];
     double Sd[9];
@@ -102,18 +101,7 @@ __device__ __noinline__ PairStat eval_pair(const ScanArgs &a, const PairAcc acc,
         Sd[c] = (double)acc.S[c];
         N += n[c];
     }
-    const PairStat s = pair_stat(n, Sd, (double)acc.Q + qc * (double)N, a.test_int != 0);
-    if (t == a.report_trait) {
-        const size_t o = (size_t)gi * size2 + gj;
-        if (a.dump_counts)
-#pragma unroll
-            for (int c = 0; c < 9; ++c) a.dump_counts[9 * o + c] = n[c];
-        if (a.dump_F) a.dump_F[o] = (float)s.F;
-        if (a.dump_F2) a.dump_F2[o] = (float)s.F2;
-        if (a.dump_df1) a.dump_df1[o] = s.d1;
-        if (a.dump_df2) a.dump_df2[o] = s.d2;
-    }
-    return s;
+    return pair_stat(n, Sd, (double)acc.Q + qc * (double)N, a.test_int != 0);
 }
 
 __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
@@ -252,7 +240,7 @@ __global__ void __launch_bounds__(NT, 1) k_scan_popc(ScanArgs a)
 #pragma unroll
                     for (int c = 0; c < 9; ++c) acc.S[c] = S[ii][c];
                     acc.Q = Q[ii];
-                    s = eval_pair(a, acc, qc, t, gi, gj, bd.size2);
+                    s = eval_pair(a, acc, qc);
                 }
                 const bool hit = valid && report && is_hit(a, s);
                 emit_row(a, hit, bd.start1 + gi, bd.start2 + gj, s);
@@ -368,7 +356,7 @@ __device__ __forceinline__ double block_max(double v, double *sv)
 }
 
 // One block: resets the counters and maxima (every call starts from zero), writes the block
-// descriptor, then the centred phenotype as the library's epi_set_traits does on the host:
+// descriptor, then the centred phenotype as k_traits (prep.cu) makes it for epi_set_traits:
 // centred by the valid mean and scaled by the power of two that brings its largest magnitude
 // into [0.5, 1) (exact, so F and F2 are unchanged, and a trait in units of 1e20 or 1e-20
 // neither overflows nor underflows the single-precision squares).

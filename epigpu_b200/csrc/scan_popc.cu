@@ -64,7 +64,7 @@ struct Shape {
     static constexpr uint32_t STAGE_BYTES = (TI + TJ) * KW * 16;  // transaction bytes per stage
     static_assert(KW == 2 && 32 * G <= NT && TI * KW <= NT - KI / 4 && TI <= 256 && TJ <= 256 && TI + TJ <= NT,
                   "expansion roles");
-    static_assert(PI % 2 == 0, "i-SNPs in pairs (packed FP32 adds)");
+    static_assert(PI % 2 == 0, "i-SNPs in pairs");
 
     struct Smem {
         uint4 raw_i[RS][TI][KW];  // TMA: plane words of the i-tile (row = SNP)
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(Sh::NT, 1) k_scan_popc(ScanArgs a, const __gri
                 }
             }
             __syncwarp();
-            __syncthreads();  // stage st consumed (its ring slot and U buffer), st + 1 expanded
+            __syncthreads();  // stage st consumed (its ring slot and expansion buffer), st + 1 expanded
             if (tid == 0 && st + RS < nst) issue(st + RS);
         }
 

@@ -81,11 +81,17 @@ typedef struct epi_scan_opts {
                             * launch; 1: every operation is launched directly */
     int32_t tile_config;   /* 0: the kernel variant (plain form: tile shape, 3 candidates;
                             * tensor form: ring depths, epilogue warps, producer groups and
-                            * streamed B, 6 candidates, streamed B only where its expanded
-                            * rows fit in memory) is chosen by the autotuner, which times every
-                            * candidate on a sample block once per device, form, individual
-                            * count and trait count; k >= 1: candidate k (epi_scan_config
-                            * names it) */
+                            * streamed B, 6 candidates) is chosen by the autotuner, which times
+                            * every candidate on a sample block once per device, form,
+                            * individual count and trait count; k >= 1: candidate k
+                            * (epi_scan_config names it). Streamed B keeps expanded genotype
+                            * rows on the GPU, 6 to 18 bytes per SNP, individual and trait or
+                            * group of traits (6 GB at 10,000 x 100,000): only where they take
+                            * 64 GiB and half of the free memory at most and, without the
+                            * screen, up to 6,144 individuals (padded to 128) unless asked for.
+                            * They are freed with the context, when the autotuner prefers
+                            * another candidate, and when a load needs their memory; candidates
+                            * 1, 2, 4 and 5 keep none */
     int32_t reserved[5];   /* set to 0 */
 } epi_scan_opts;
 
