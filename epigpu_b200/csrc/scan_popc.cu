@@ -23,7 +23,7 @@
 // Four FP32 adds per pair and individual, predicated by the bits, took 93 cycles of an SM per 32
 // individuals and 32 pairs (32 of them the packed adds, 16 the shared-memory broadcasts of the
 // i-SNP's values, much of the rest read-modify-writes of the sparse sums in shared memory). The
-// look-ups take 60 (26 shuffles, LSU at 55%, issue at 50%: bound by their latency chains), and the
+// look-ups take 60 (26 shuffles, LSU at 63%, issue at 65%: bound by their latency chains), and the
 // sparse sums stand in registers, which four pairs per thread leave room for: 69 cycles at 1%
 // missing calls, 10.0 -> 7.4 ms at N = 4,000 x 4,001 SNPs. More warps with two pairs each (768 or
 // 1,024 threads), look-ups in shared memory instead of shuffles and for the individuals missing at j
