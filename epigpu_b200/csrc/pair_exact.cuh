@@ -26,7 +26,8 @@ __device__ __forceinline__ double div_fast(double num, double den)
 // The reference's 8 df / 4 df statistics (src/EpiOpenCL.c:231-247, :452-486) in FP64 from
 // the exact integer cell counts n and digit sums si (S = si * sc), and Q = sum of y^2 over
 // the pair's valid individuals. Same quantities as pair_stat, arranged to avoid division
-// chains: reciprocals by rcp_d.
+// chains: reciprocals by rcp_d. A pair whose individuals all have one value of y has nothing to explain:
+// F and F2 are 0/0 (NaN, never a hit or a maximum), although SSB may hold a rounding of the cell means.
 __device__ __forceinline__ PairStat pair_stat_exact(const int n[9], const double si[9], double sc, double Q,
                                                     bool want_int)
 {
@@ -52,12 +53,17 @@ __device__ __forceinline__ PairStat pair_stat_exact(const int n[9], const double
             SSB = fma((double)n[c] * d, d, SSB);
         }
     }
-    const double SSW = ssw_floored(Q - St * m, SSB, SSW_FLOOR_EXACT);
+    const double SSY = Q - St * m;
+    const double SSW = ssw_floored(SSY, SSB, SSW_FLOOR_EXACT);
     r.nfac = nfac;
     r.d1 = nfac - 1;
     r.d2 = N - nfac;
     r.F = div_fast(SSB * (double)r.d2, SSW * (double)r.d1);
     r.F2 = 0.0;
+    if (!(SSY > 0.0)) {
+        r.F = r.F2 = __longlong_as_double(0x7ff8000000000000ll);
+        return r;
+    }
     if (want_int) {
         double row[3], col[3];
 #pragma unroll

@@ -350,3 +350,32 @@ def test_screened_scans_against_the_oracle(gpu_ctx, nid, nsnp, ntraits, form, co
         F = np.where(per["df1"] > 0, per["F"], -np.inf)[np.tril_indices(nsnp, -1)]
         k = np.nanmax(F) * 8.0 / (nid - 9)  # about the largest SSB / SSW
         assert abs(ex["max_f"][t] - np.nanmax(F)) <= 1e-5 * (1.0 + k) * np.nanmax(F)
+
+
+@pytest.mark.parametrize("nid", [150, 400, 3000])
+@pytest.mark.parametrize("test", ["f", "i"])
+def test_pairs_of_individuals_with_one_value(gpu_ctx, nid, test):
+    """SNPs known in a few individuals who all have the same value of a trait of two or three: nothing is
+    there to explain, F is 0/0 and not the infinity of a rounding over nothing. No hit, no maximum, in the
+    automatic form, the tensor form and the allocation-free call."""
+    nsnp, sparse = 90, 30
+    codes = synth.genotype_codes(nid, nsnp, seed=nid, miss=0.0)
+    rng = np.random.default_rng(nid + 1)
+    y = rng.integers(0, 3 if nid == 400 else 2, nid).astype(np.float32)
+    for s in range(sparse):
+        gone = np.ones(nid, dtype=bool)
+        gone[rng.choice(np.flatnonzero(y == s % 2), 5 + s % 7, replace=False)] = False
+        codes[s, gone] = 3
+    packed, block = synth.pack(codes), (0, nsnp, 0, nsnp)
+    t1, t2 = synth.f_threshold(8, nid - 9, 1e-3), synth.f_threshold(4, nid - 9, 1e-3)
+    gpu_ctx.load_packed(packed, nid)
+    gpu_ctx.set_phenotype(y)
+    F, F2, df1, i, j = _dumped(gpu_ctx, block, test, capi.FORM_TENSOR)
+    flat = j < sparse
+    top = np.nanmax(F[~flat])
+    for form in (capi.FORM_AUTO, capi.FORM_TENSOR):
+        hits, _, ex = gpu_ctx.scan([block], capi.default_opts(test=test, safe=1, t1=t1, t2=t2, form=form))
+        assert np.all(hits["snp2"] >= sparse) and abs(ex["max_f"][0] - top) <= 2e-5 * top
+    st, rows, most = _noalloc(packed, nid, y, block, test=test, safe=1, t1=t1, t2=t2)
+    assert st == capi.EPI_OK and np.all(rows["snp2"] >= sparse) and abs(most[0] - top) <= 2e-5 * top
+    assert not np.any(F[flat] > 0.01) and not (test == "i" and np.any(F2[flat] > 0.01))
